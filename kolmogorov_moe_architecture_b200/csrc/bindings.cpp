@@ -38,7 +38,7 @@ void gemm(const Tensor& A, const Tensor& B, const OptT& B2, Tensor C, const OptT
           int64_t c_gs, const OptT& tile_group, const OptT& num_m_tiles, const OptT& k_begin, const OptT& k_len,
           double alpha, double beta, const OptT& row_scale, const OptT& row_ptr, const OptT& alpha_dev,
           const OptT& beta_dev, bool sym_upper, double diag_add, int64_t k_split, const OptT& D2, double beta2,
-          Tensor status) {
+          int64_t b_rows, int64_t b_klen, Tensor status) {
   c10::cuda::CUDAGuard guard(A.device());
   need_bf16(A, "A");
   need_bf16(B, "B");
@@ -67,6 +67,8 @@ void gemm(const Tensor& A, const Tensor& B, const OptT& B2, Tensor C, const OptT
   d.sym_upper = sym_upper ? 1 : 0;
   d.diag_add = (float)diag_add;
   d.k_split = (int)k_split;
+  d.b_rows = (int)b_rows;
+  d.b_klen = (int)b_klen;
   const int64_t n_groups = mode == KMOE_GEMM_BATCHED ? groups : 1;
   if (alpha_dev.has_value() && alpha_dev->defined()) {
     need_f32(*alpha_dev, "alpha_dev");
@@ -243,23 +245,25 @@ std::tuple<Tensor, Tensor> swiglu_bwd(const Tensor& g, const Tensor& u, const Te
   const long long rows = g.numel() / cols;
   Tensor g2 = g.dim() == 1 ? g.unsqueeze(0) : g, u2 = u.dim() == 1 ? u.unsqueeze(0) : u;
   Tensor dg = at::empty(g.sizes(), g.options()), du = at::empty(g.sizes(), g.options());
-  check(kmoe_swiglu_bwd(g2.data_ptr(), u2.data_ptr(), dh.data_ptr(), dg.data_ptr(), du.data_ptr(), rows, cols,
+  check(kmoe_swiglu_bwd(g2.data_ptr(), u2.data_ptr(), dh.data_ptr(), dg.data_ptr(), du.data_ptr(), rows, cols, cols,
                         row_stride(g2), row_stride(u2), cols, (const int*)ptr_or_null(live_rows), cur_stream()),
         "swiglu_bwd");
   return {dg, du};
 }
 
-// dG and dU side by side in one (rows, 2 * cols) buffer: the [dG | dU] operand of a split-reduction GEMM
+// dG and dU side by side in one (rows, 2 * P) buffer, P = cols rounded up to 64 (zeros between cols and P): the
+// [dG | dU] operand of a split-reduction GEMM
 Tensor swiglu_bwd_cat(const Tensor& g, const Tensor& u, const Tensor& dh, const OptT& live_rows) {
   c10::cuda::CUDAGuard guard(g.device());
   need_bf16(g, "gate"); need_bf16(u, "up"); need_bf16(dh, "dh");
   TORCH_CHECK(dh.is_contiguous() && g.dim() == 2);
   const int cols = g.size(-1);
   const long long rows = g.numel() / cols;
-  Tensor out = at::empty({rows, 2 * (long long)cols}, g.options());
+  const int P = (cols + 63) / 64 * 64;
+  Tensor out = at::empty({rows, 2 * (long long)P}, g.options());
   char* base = reinterpret_cast<char*>(out.data_ptr());
-  check(kmoe_swiglu_bwd(g.data_ptr(), u.data_ptr(), dh.data_ptr(), base, base + 2LL * cols, rows, cols, row_stride(g),
-                        row_stride(u), 2LL * cols, (const int*)ptr_or_null(live_rows), cur_stream()),
+  check(kmoe_swiglu_bwd(g.data_ptr(), u.data_ptr(), dh.data_ptr(), base, base + 2LL * P, rows, cols, P, row_stride(g),
+                        row_stride(u), 2LL * P, (const int*)ptr_or_null(live_rows), cur_stream()),
         "swiglu_bwd_cat");
   return out;
 }

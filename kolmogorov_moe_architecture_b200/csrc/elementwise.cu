@@ -426,15 +426,20 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ g, const __n
 
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ u,
                                   const __nv_bfloat16* __restrict__ dh, __nv_bfloat16* __restrict__ dg,
-                                  __nv_bfloat16* __restrict__ du, long long rows, int cols, long long ldg,
-                                  long long ldu, long long ldo, const int* __restrict__ live_rows) {
-  const int vpr = cols / 8;
+                                  __nv_bfloat16* __restrict__ du, long long rows, int cols, int pcols,
+                                  long long ldg, long long ldu, long long ldo, const int* __restrict__ live_rows) {
+  const int vpr = pcols / 8;            // columns [cols, pcols) of both outputs are zeros
   if (live_rows != nullptr) rows = min(rows, (long long)*live_rows);
   const long long total = rows * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / vpr;
     const int c = (int)(i % vpr) * 8;
+    if (c >= cols) {
+      *reinterpret_cast<uint4*>(dg + r * ldo + c) = make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(du + r * ldo + c) = make_uint4(0, 0, 0, 0);
+      continue;
+    }
     float gv[8], uv[8], dv[8], og[8], ou[8];
     unpack8(*reinterpret_cast<const uint4*>(g + r * ldg + c), gv);
     unpack8(*reinterpret_cast<const uint4*>(u + r * ldu + c), uv);
@@ -720,12 +725,12 @@ extern "C" int kmoe_swiglu_fwd(const void* g, const void* u, void* h, long long 
 }
 
 extern "C" int kmoe_swiglu_bwd(const void* g, const void* u, const void* dh, void* dg, void* du, long long rows,
-                               int cols, long long ldg, long long ldu, long long ldo, const int* live_rows,
-                               cudaStream_t st) {
-  if (cols % 8 || ldg % 8 || ldu % 8 || ldo % 8) return -1;
-  swiglu_bwd_kernel<<<grid_for(rows * (cols / 8), 256), 256, 0, st>>>(
+                               int cols, int pcols, long long ldg, long long ldu, long long ldo,
+                               const int* live_rows, cudaStream_t st) {
+  if (pcols < cols || pcols % 8 || cols % 8 || ldg % 8 || ldu % 8 || ldo % 8) return -1;
+  swiglu_bwd_kernel<<<grid_for(rows * (pcols / 8), 256), 256, 0, st>>>(
       (const __nv_bfloat16*)g, (const __nv_bfloat16*)u, (const __nv_bfloat16*)dh, (__nv_bfloat16*)dg,
-      (__nv_bfloat16*)du, rows, cols, ldg, ldu, ldo, live_rows);
+      (__nv_bfloat16*)du, rows, cols, pcols, ldg, ldu, ldo, live_rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -55,6 +55,7 @@ struct GemmArgs {
   int sym_upper;              // C is symmetric (A == B): compute only tiles that touch the upper triangle
   float diag_add;             // added to C[i][i] after alpha (bf16 store path)
   int k_split;                // > 0: reduction elements [k_split, K) of B come from the second tensor map
+  int a_boxed, b_boxed;       // MN-major operand whose row count is no multiple of 64: one 64-row box per load
   const long long* row_ptr;   // optional: address of each output row (may be peer memory); 0 = row not stored
   int* status;
 };
@@ -187,6 +188,32 @@ __device__ __forceinline__ void epilogue_store_chunk(const GemmArgs& a, const ui
   }
 }
 
+// MN-major tile of ROWS operand rows (memory [K][rows]) into shared memory as ROWS / 64 blocks of 64 k-rows x 128
+// bytes.  A row count that is a multiple of 64 is described to TMA as (64, K, rows / 64) and the tile is one load;
+// any other count (expert width 2464, vocabulary 50257) as (rows, K), where a load brings one block and the unit
+// zero-fills what lies past the last row.  The second form costs ROWS / 64 issue slots of the producer thread
+// instead of one, which a reduction block of >= 500 ns hides.
+template <int ROWS>
+__device__ __forceinline__ void load_mn_tile(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int k, int row, int g,
+                                             int boxed) {
+  if (!boxed) {
+    tma_load_4d(dst, tm, bar, 0, k, row / 64, g);
+  } else {
+#pragma unroll
+    for (int j = 0; j < ROWS / 64; ++j) tma_load_4d(dst + j * BK * 128, tm, bar, row + j * 64, k, 0, g);
+  }
+}
+template <int ROWS>
+__device__ __forceinline__ void load_mn_tile_pair(uint8_t* dst, const CUtensorMap* tm, uint32_t bar, int k, int row,
+                                                  int g, int boxed) {
+  if (!boxed) {
+    tma_load_4d_pair(dst, tm, bar, 0, k, row / 64, g);
+  } else {
+#pragma unroll
+    for (int j = 0; j < ROWS / 64; ++j) tma_load_4d_pair(dst + j * BK * 128, tm, bar, row + j * 64, k, 0, g);
+  }
+}
+
 template <int BN, int A_MAJOR, int B_MAJOR>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -256,7 +283,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (A_MAJOR == KMOE_MAJOR_K)
             tma_load_4d(sa, &tmA, &full_bar[s], k, t.m_tile * BM, 0, t.g_a);
           else
-            tma_load_4d(sa, &tmA, &full_bar[s], 0, k, t.m_tile * (BM / 64), t.g_a);
+            load_mn_tile<BM>(sa, &tmA, &full_bar[s], k, t.m_tile * BM, t.g_a, args.a_boxed);
           if (!swiglu) {
             const bool second = args.k_split > 0 && k >= args.k_split;
             const CUtensorMap* tb = second ? &tmB2 : &tmB;
@@ -264,15 +291,15 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             if (B_MAJOR == KMOE_MAJOR_K)
               tma_load_4d(sb, tb, &full_bar[s], kb2, t.n_tile * BN, 0, t.g_b);
             else
-              tma_load_4d(sb, tb, &full_bar[s], 0, kb2, t.n_tile * (BN / 64), t.g_b);
+              load_mn_tile<BN>(sb, tb, &full_bar[s], kb2, t.n_tile * BN, t.g_b, args.b_boxed);
           } else {
             constexpr int HB = BN / 2;
             if (B_MAJOR == KMOE_MAJOR_K) {
               tma_load_4d(sb, &tmB, &full_bar[s], k, t.n_tile * HB, 0, t.g_b);
               tma_load_4d(sb + B_STAGE_BYTES / 2, &tmB2, &full_bar[s], k, t.n_tile * HB, 0, t.g_b);
             } else {
-              tma_load_4d(sb, &tmB, &full_bar[s], 0, k, t.n_tile * (HB / 64), t.g_b);
-              tma_load_4d(sb + B_STAGE_BYTES / 2, &tmB2, &full_bar[s], 0, k, t.n_tile * (HB / 64), t.g_b);
+              load_mn_tile<HB>(sb, &tmB, &full_bar[s], k, t.n_tile * HB, t.g_b, args.b_boxed);
+              load_mn_tile<HB>(sb + B_STAGE_BYTES / 2, &tmB2, &full_bar[s], k, t.n_tile * HB, t.g_b, args.b_boxed);
             }
           }
           if (++s == stages) { s = 0; ph ^= 1; }
@@ -548,7 +575,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           if (A_MAJOR == KMOE_MAJOR_K)
             tma_load_4d_pair(sa, &tmA, fb, k, arow, 0, t.g_a);
           else
-            tma_load_4d_pair(sa, &tmA, fb, 0, k, arow / 64, t.g_a);
+            load_mn_tile_pair<BM>(sa, &tmA, fb, k, arow, t.g_a, args.a_boxed);
           // B: this CTA's half of the tile's columns; with the SwiGLU epilogue the halves are the gate
           // weight (leader) and the up weight (peer), so accumulator columns [0, BN/2) hold the gate
           const bool second = !swiglu && args.k_split > 0 && k >= args.k_split;
@@ -558,7 +585,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           if (B_MAJOR == KMOE_MAJOR_K)
             tma_load_4d_pair(sb, tb, fb, kb2, brow, 0, t.g_b);
           else
-            tma_load_4d_pair(sb, tb, fb, 0, kb2, brow / 64, t.g_b);
+            load_mn_tile_pair<HALF_N>(sb, tb, fb, kb2, brow, t.g_b, args.b_boxed);
           if (++s == stages) { s = 0; ph ^= 1; }
         }
       }
@@ -849,6 +876,7 @@ static std::mutex g_tmap_mutex;
 // Operand tensor map (bf16, 128B swizzle), always rank 4 so one TMA instruction form serves all cases.
 //   K-major : dims {K, rows, 1, G}       box {64, tile_rows, 1, 1}
 //   MN-major: dims {64, K, rows/64, G}   box {64, 64, tile_rows/64, 1}   (memory is [K][rows], rows contiguous)
+//             dims {rows, K, 1, G}       box {64, 64, 1, 1}              when rows % 64 != 0 (see load_mn_tile)
 static int make_operand_tmap(CUtensorMap* out, const void* base, int major, long long rows, long long K,
                              long long ld, long long gstride, int groups, int tile_rows) {
   TmapKey key{base, major, rows, K, ld, gstride, groups, tile_rows};
@@ -870,10 +898,15 @@ static int make_operand_tmap(CUtensorMap* out, const void* base, int major, long
     strides[0] = (cuuint64_t)ld * 2; strides[1] = (cuuint64_t)rows * ld * 2; strides[2] = (cuuint64_t)gs * 2;
     box[0] = BK; box[1] = (cuuint32_t)tile_rows; box[2] = 1; box[3] = 1;
   } else {
-    if (rows % 64 != 0) return -11;
+    if (rows % 64 != 0) {
+      dims[0] = (cuuint64_t)rows; dims[1] = (cuuint64_t)K; dims[2] = 1; dims[3] = (cuuint64_t)G;
+      strides[0] = (cuuint64_t)ld * 2; strides[1] = (cuuint64_t)K * ld * 2; strides[2] = (cuuint64_t)gs * 2;
+      box[0] = 64; box[1] = BK; box[2] = 1; box[3] = 1;
+    } else {
     dims[0] = 64; dims[1] = (cuuint64_t)K; dims[2] = (cuuint64_t)(rows / 64); dims[3] = (cuuint64_t)G;
     strides[0] = (cuuint64_t)ld * 2; strides[1] = 128; strides[2] = (cuuint64_t)gs * 2;
     box[0] = 64; box[1] = BK; box[2] = (cuuint32_t)(tile_rows / 64); box[3] = 1;
+    }
   }
   const int rc = encode_bf16_4d(out, base, dims, strides, box);
   if (rc) return rc;
@@ -950,9 +983,10 @@ extern "C" void kmoe_gemm_clear_tensormap_cache(void) {
 
 extern "C" int kmoe_gemm(const KmoeGemmDesc* d, cudaStream_t stream) {
   using namespace kmoe;
-  // 16-byte rows for TMA: the reduction length only matters for an operand whose rows run along it
-  if (d->N % 8 != 0) return -1;
-  if ((d->a_major == KMOE_MAJOR_K || d->b_major == KMOE_MAJOR_K) && d->K % 8 != 0) return -1;
+  // 16-byte output vectors; the pitches of the operands are checked where their tensor maps are made (the lengths
+  // themselves are free: TMA zero-fills past the end of a row and past the last row)
+  if (d->N % 8 != 0 || d->ldc % (d->out_f32 ? 4 : 8) != 0) return -1;
+  if (d->b_rows < 0 || d->b_rows > d->N || d->b_klen < 0 || d->b_klen > (d->k_split ? d->k_split : d->K)) return -7;
   if (d->K <= 0 || d->M <= 0 || d->N <= 0) return -2;
   if (d->c_row_ptr != nullptr && (d->out_f32 || d->epilogue != KMOE_EPI_STORE)) return -3;
   if (d->k_split != 0 && (d->k_split % BK || d->k_split <= 0 || d->k_split >= d->K || d->B2 == nullptr ||
@@ -1011,18 +1045,22 @@ extern "C" int kmoe_gemm(const KmoeGemmDesc* d, cudaStream_t stream) {
   }
   const int a_groups = (d->mode == KMOE_GEMM_BATCHED && d->a_gstride != 0) ? d->groups : 1;
   const int b_groups = d->b_gstride != 0 ? d->groups : 1;
+  const int n_rows = d->b_rows > 0 ? d->b_rows : d->N;
+  a.a_boxed = d->a_major == KMOE_MAJOR_MN && d->M % 64 != 0;
+  a.b_boxed = d->b_major == KMOE_MAJOR_MN && n_rows % 64 != 0;
   CUtensorMap tA, tB, tB2;
   int rc = make_operand_tmap(&tA, d->A, d->a_major, d->M, k_extent_a, d->lda, d->a_gstride, a_groups, BM);
   if (rc) return rc;
   if (d->k_split > 0) k_extent_b = d->k_split;
-  rc = make_operand_tmap(&tB, d->B, d->b_major, d->N, k_extent_b, d->ldb, d->b_gstride, b_groups, b_box_rows);
+  if (d->b_klen > 0) k_extent_b = d->b_klen;
+  rc = make_operand_tmap(&tB, d->B, d->b_major, n_rows, k_extent_b, d->ldb, d->b_gstride, b_groups, b_box_rows);
   if (rc) return rc;
   if (d->k_split > 0) {
-    rc = make_operand_tmap(&tB2, d->B2, d->b_major, d->N, d->K - d->k_split, d->ldb, d->b_gstride, b_groups,
-                           b_box_rows);
+    rc = make_operand_tmap(&tB2, d->B2, d->b_major, n_rows, d->b_klen > 0 ? d->b_klen : d->K - d->k_split, d->ldb,
+                           d->b_gstride, b_groups, b_box_rows);
     if (rc) return rc;
   } else if (swiglu) {
-    rc = make_operand_tmap(&tB2, d->B2, d->b_major, d->N, k_extent_b, d->ldb, d->b_gstride, b_groups, b_box_rows);
+    rc = make_operand_tmap(&tB2, d->B2, d->b_major, n_rows, k_extent_b, d->ldb, d->b_gstride, b_groups, b_box_rows);
     if (rc) return rc;
   } else {
     tB2 = tB;

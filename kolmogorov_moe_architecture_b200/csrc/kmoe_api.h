@@ -58,6 +58,10 @@ typedef struct KmoeGemmDesc {
   // B and [k_split, K) from B2 (same layout, ldb and group stride; k_split a multiple of 64), while A is one
   // [M, K] operand.  C = A[:, :k_split] B^T + A[:, k_split:] B2^T in one pass, e.g. dX = [dG | dU] [W1 ; W2].
   int k_split;
+  // optional (0 = N / the whole length): rows of B that exist when N was rounded up to a whole output vector, and
+  // reduction elements of B (of each of B and B2 with k_split) that exist when the reduction was rounded up; what
+  // lies beyond reads as zero.  A must be finite there.
+  int b_rows, b_klen;
   int* status;             // device int; non-zero after the launch = a bounded wait expired
   int num_sms;             // 0 = query
 } KmoeGemmDesc;
@@ -150,7 +154,7 @@ int kmoe_rope(const void* x, const float* cs, const float* sn, void* out, int B,
 int kmoe_swiglu_fwd(const void* g, const void* u, void* h, long long rows, int cols, long long ldg, long long ldu,
                     const int* live_rows, cudaStream_t st);
 int kmoe_swiglu_bwd(const void* g, const void* u, const void* dh, void* dg, void* du, long long rows, int cols,
-                    long long ldg, long long ldu, long long ldo, const int* live_rows, cudaStream_t st);
+                    int pcols, long long ldg, long long ldu, long long ldo, const int* live_rows, cudaStream_t st);
 
 // --------------------------------------------------------------------------- Mamba
 // groups: number of parameter sets stacked along the first dimension of w / bias (A, D, dt_bias for the scan);

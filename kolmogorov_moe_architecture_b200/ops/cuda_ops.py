@@ -85,7 +85,7 @@ def gemm(A, B, C, *, M, N, Kd, mode=DENSE, epi=EPI_STORE, groups=1, a_major=MAJ_
          lda, ldb, ldc, ldd=0, a_gs=0, b_gs=0, c_gs=0, B2=None, D=None, G=None, U=None,
          tile_group=None, num_m_tiles=None, k_begin=None, k_len=None, alpha=1.0, beta=0.0, row_scale=None,
          row_ptr=None, alpha_dev=None, beta_dev=None, sym_upper=False, diag_add=0.0, k_split=0, D2=None,
-         beta2=0.0):
+         beta2=0.0, b_rows=0, b_klen=0):
     """``row_ptr`` (int64, one address per output row, 0 = skip) redirects each output row, e.g. into a
     peer GPU's buffer; ``C`` then only supplies the dtype.  ``alpha_dev`` / ``beta_dev`` (fp32, one entry
     per group of a batched GEMM) multiply alpha / beta with values that live on the device.  ``sym_upper``:
@@ -93,11 +93,13 @@ def gemm(A, B, C, *, M, N, Kd, mode=DENSE, epi=EPI_STORE, groups=1, a_major=MAJ_
     instead of computed.  ``diag_add`` is added to the main diagonal of the (bf16) result after ``alpha``.
     ``k_split`` > 0 (with ``B2``): the reduction is split, elements [0, k_split) multiply ``B`` and the rest
     ``B2``: ``C = A[:, :k_split] B^T + A[:, k_split:] B2^T`` in one pass.  ``D2`` / ``beta2``: a second addend
-    laid out like ``D`` (bf16 output): ``C = alpha A B + beta D + beta2 D2``; ``beta_dev`` scales both."""
+    laid out like ``D`` (bf16 output): ``C = alpha A B + beta D + beta2 D2``; ``beta_dev`` scales both.
+    ``b_rows`` / ``b_klen``: rows of ``B`` / reduction elements of ``B`` (and of ``B2``) that exist when ``N`` / the
+    reduction was rounded up; the rest reads as zero."""
     K.gemm(A, B, B2, C, D, G, U, mode, epi, M, N, Kd, groups, a_major, b_major, lda, ldb, ldc, ldd,
            a_gs, b_gs, c_gs, tile_group, num_m_tiles, k_begin, k_len, alpha, beta, row_scale, row_ptr,
            alpha_dev, beta_dev, sym_upper, float(diag_add), int(k_split), D2, float(beta2),
-           status_tensor(A.device))
+           b_rows, b_klen, status_tensor(A.device))
     _count()
     return C
 
@@ -596,11 +598,12 @@ class _GroupedSwiGLU(torch.autograd.Function):
         dH = torch.empty(max_rows, f, dtype=dout.dtype, device=dout.device)
         gemm(dYp, w3, dH, mode=GROUPED_M, M=max_rows, N=f, Kd=d, groups=E, lda=d, ldb=d, ldc=f, b_gs=f * d,
              tile_group=tile_group, num_m_tiles=nmt)
-        dGU = K.swiglu_bwd_cat(G, U, dH, meta[1:2])          # [dG | dU], one (rows, 2f) operand
-        dG, dU = dGU[:, :f], dGU[:, f:]
+        dGU = K.swiglu_bwd_cat(G, U, dH, meta[1:2])          # [dG | dU], one operand; P = f in whole 64-blocks
+        P = dGU.shape[1] // 2
+        dG, dU = dGU[:, :f], dGU[:, P:P + f]
         dXp = torch.empty(max_rows, d, dtype=dout.dtype, device=dout.device)
         # dXp = dG W1^T + dU W2^T in one grouped GEMM: the reduction runs over [dG | dU] and [W1 | W2]
-        gemm(dGU, w1, dXp, B2=w2, mode=GROUPED_M, M=max_rows, N=d, Kd=2 * f, k_split=f, groups=E, lda=2 * f,
+        gemm(dGU, w1, dXp, B2=w2, mode=GROUPED_M, M=max_rows, N=d, Kd=2 * P, k_split=P, b_klen=f, groups=E, lda=2 * P,
              ldb=f, ldc=d, b_gs=d * f, tile_group=tile_group, num_m_tiles=nmt)
         dx = K.moe_combine(dXp, pos, None, T, k)
         # weight gradients: per expert, reduction over that expert's (padded) row range
@@ -611,8 +614,8 @@ class _GroupedSwiGLU(torch.autograd.Function):
         sinks = [grad_sink(w) for w in (w1, w2, w3)]
         dw1, dw2, dw3 = [s[0] if s is not None else torch.empty_like(w) for s, w in zip(sinks, (w1, w2, w3))]
         common = dict(mode=BATCHED, groups=E, a_major=MAJ_MN, b_major=MAJ_MN, Kd=max_rows, k_begin=kb, k_len=kl)
-        gemm(Xp, dG, dw1, M=d, N=f, lda=d, ldb=2 * f, ldc=f, c_gs=d * f, **common)
-        gemm(Xp, dU, dw2, M=d, N=f, lda=d, ldb=2 * f, ldc=f, c_gs=d * f, **common)
+        gemm(Xp, dG, dw1, M=d, N=f, lda=d, ldb=2 * P, ldc=f, c_gs=d * f, **common)
+        gemm(Xp, dU, dw2, M=d, N=f, lda=d, ldb=2 * P, ldc=f, c_gs=d * f, **common)
         gemm(H, dYp, dw3, M=f, N=d, lda=f, ldb=d, ldc=d, c_gs=f * d, **common)
         _count(5)
         for s_ in sinks:
@@ -622,10 +625,18 @@ class _GroupedSwiGLU(torch.autograd.Function):
         return dx, dw1, dw2, dw3, None, dwts, None
 
 
+def _expert_widths_ok(d: int, f: int) -> bool:
+    """Widths the grouped GEMMs cover: whole 16-byte rows (what TMA can address) of at least one 64-element block.
+    An expert width that is no multiple of 64 (2464 in the 3B preset) costs a few more load instructions per block,
+    see ``load_mn_tile``."""
+    return d % 8 == 0 and f % 8 == 0 and d >= 64 and f >= 64
+
+
 def grouped_swiglu(x, w1, w2, w3, idx, weights, keep=None, moe_dtype="bf16"):
     T, d = x.shape
     f = w1.shape[2]
-    ok = _bf16(x) and _bf16(w1) and d % 64 == 0 and f % 64 == 0
+    ok = (_bf16(x) and _bf16(w1) and _bf16(w2) and _bf16(w3) and _expert_widths_ok(d, f)
+          and (moe_dtype != "mxfp8" or (d % 64 == 0 and f % 64 == 0)))
     if not ok:
         _fallback("grouped_swiglu", f"dtype {x.dtype}/{w1.dtype} d={d} f={f}")
         return eager.grouped_swiglu(x, w1, w2, w3, idx, weights, keep)
@@ -686,17 +697,18 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
         gemm(dY, w3, dH, mode=BATCHED, groups=E, M=BC, N=f, Kd=d, lda=d, ldb=d, ldc=f,
              a_gs=BC * d, b_gs=f * d, c_gs=BC * f)
         dGU = K.swiglu_bwd_cat(G, U, dH, None)
-        dG, dU = dGU[:, :f], dGU[:, f:]
+        P = dGU.shape[1] // 2                                # f in whole 64-element blocks
+        dG, dU = dGU[:, :f], dGU[:, P:P + f]
         dXg = torch.empty(E * BC, d, dtype=dout.dtype, device=dout.device)
-        gemm(dGU, w1, dXg, B2=w2, mode=BATCHED, groups=E, M=BC, N=d, Kd=2 * f, k_split=f, lda=2 * f, ldb=f, ldc=d,
-             a_gs=BC * 2 * f, b_gs=d * f, c_gs=BC * d)
+        gemm(dGU, w1, dXg, B2=w2, mode=BATCHED, groups=E, M=BC, N=d, Kd=2 * P, k_split=P, b_klen=f, lda=2 * P, ldb=f,
+             ldc=d, a_gs=BC * 2 * P, b_gs=d * f, c_gs=BC * d)
         dx = K.moe_combine(dXg, pos, None, T, E)
         H = K.swiglu_fwd(G, U, None)
         sinks = [grad_sink(w) for w in (w1, w2, w3)]
         dw1, dw2, dw3 = [s_[0] if s_ is not None else torch.empty_like(w) for s_, w in zip(sinks, (w1, w2, w3))]
         common = dict(mode=BATCHED, groups=E, a_major=MAJ_MN, b_major=MAJ_MN, Kd=BC)
-        gemm(Xg, dG, dw1, M=d, N=f, lda=d, ldb=2 * f, ldc=f, a_gs=BC * d, b_gs=BC * 2 * f, c_gs=d * f, **common)
-        gemm(Xg, dU, dw2, M=d, N=f, lda=d, ldb=2 * f, ldc=f, a_gs=BC * d, b_gs=BC * 2 * f, c_gs=d * f, **common)
+        gemm(Xg, dG, dw1, M=d, N=f, lda=d, ldb=2 * P, ldc=f, a_gs=BC * d, b_gs=BC * 2 * P, c_gs=d * f, **common)
+        gemm(Xg, dU, dw2, M=d, N=f, lda=d, ldb=2 * P, ldc=f, a_gs=BC * d, b_gs=BC * 2 * P, c_gs=d * f, **common)
         gemm(H, dY, dw3, M=f, N=d, lda=f, ldb=d, ldc=d, a_gs=BC * f, b_gs=BC * d, c_gs=f * d, **common)
         _count(5)
         for s_ in sinks:
@@ -710,7 +722,7 @@ def expert_choice_swiglu(x, w1, w2, w3, wts, tok):
     """x (B, S, d); wts, tok (B, E, C) from ``expert_choice_route``; returns (B, S, d)."""
     B, S, d = x.shape
     f = w1.shape[2]
-    ok = _bf16(x) and _bf16(w1) and d % 64 == 0 and f % 64 == 0 and tok.numel() > 0
+    ok = _bf16(x) and _bf16(w1) and _bf16(w2) and _bf16(w3) and _expert_widths_ok(d, f) and tok.numel() > 0
     if not ok:
         _fallback("expert_choice_swiglu", f"dtype {x.dtype}/{w1.dtype} d={d} f={f}")
         return eager.expert_choice_swiglu(x, w1, w2, w3, wts, tok)
@@ -1003,22 +1015,22 @@ class _MTPLoss(torch.autograd.Function):
             Wc = W.contiguous()
             dW = torch.empty_like(Wc) if need_grad else None
             loss_sum = torch.zeros((), dtype=torch.float32, device=hidden.device)
+            pitch = -(-V // 64) * 64        # whole 16-byte rows for TMA whatever the vocabulary (50257)
             for r0 in range(0, R, chunk_rows):
                 r1 = min(R, r0 + chunk_rows)
+                n = r1 - r0
                 hc = h2[r0:r1]
-                logits = mm_nt(hc, Wc)
-                rows = K.ce_fwd_bwd(logits, lab[r0:r1].contiguous(), gscale, ignore_index, need_grad)
+                buf = torch.empty(n, pitch, dtype=h2.dtype, device=h2.device)
+                # N in whole output vectors: the columns past V are products with rows of W that read as zero
+                gemm(hc, Wc, buf, M=n, N=-(-V // 8) * 8, Kd=d, lda=d, ldb=d, ldc=pitch, b_rows=V)
+                rows = K.ce_fwd_bwd(buf[:, :V], lab[r0:r1].contiguous(), gscale, ignore_index, need_grad)
                 _count()
                 loss_sum = loss_sum + rows.sum()
                 if need_grad:
-                    if dH_started:
-                        mm_nn(logits, Wc, out=dH[r0:r1], D=dH[r0:r1], beta=1.0)
-                    else:
-                        mm_nn(logits, Wc, out=dH[r0:r1])
-                    if r0 > 0:
-                        mm_tn(logits, hc, out=dW, D=dW, beta=1.0)
-                    else:
-                        mm_tn(logits, hc, out=dW)
+                    acc = dict(D=dH[r0:r1], beta=1.0) if dH_started else {}
+                    gemm(buf, Wc, dH[r0:r1], M=n, N=d, Kd=V, b_major=MAJ_MN, lda=pitch, ldb=d, ldc=d, **acc)
+                    acc = dict(D=dW, beta=1.0) if r0 > 0 else {}
+                    gemm(buf, hc, dW, M=V, N=d, Kd=n, a_major=MAJ_MN, b_major=MAJ_MN, lda=pitch, ldb=d, ldc=d, **acc)
             dH_started = dH_started or need_grad
             per.append(loss_sum / n_valid)
             dWs.append(dW)
@@ -1067,7 +1079,8 @@ def mtp_cross_entropy(hidden, head_weights: Sequence[torch.Tensor], labels, weig
                       chunk_rows: int = 8192):
     d = hidden.shape[-1]
     V = head_weights[0].shape[0]
-    ok = _bf16(hidden) and all(_bf16(w) for w in head_weights) and d % 64 == 0 and V % 64 == 0
+    # any vocabulary of at least one block: the logits buffer is padded to whole 64-element rows
+    ok = _bf16(hidden) and all(_bf16(w) for w in head_weights) and d % 64 == 0 and V >= 64
     if not ok:
         _fallback("mtp_cross_entropy", f"dtype {hidden.dtype} d={d} V={V}")
         return eager.mtp_cross_entropy(hidden, head_weights, labels, weights, ignore_index)

@@ -1,0 +1,129 @@
+"""Sizes that are no whole number of 64-element blocks on the GEMM paths: operand rows read in single boxes, padded
+split reductions, odd vocabularies."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(out, ref):
+    return ((out.double() - ref.double()).norm() / ref.double().norm().clamp(min=1e-30)).item()
+
+
+def _rand(*shape, scale=1.0):
+    return (torch.randn(*shape, device="cuda") * scale).to(torch.bfloat16)
+
+
+# One rounding of the result to bf16 is 2^-9 at most and about 1.7e-3 in the 2-norm; the sums are in 32 bits.
+ONE_ROUNDING = 4e-3
+
+
+@pytest.mark.parametrize("M,N,K", [(72, 72, 64), (136, 200, 72), (264, 328, 8), (2464, 1000, 192), (1000, 2464, 640)])
+def test_mn_major_rows_in_boxes(M, N, K):
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    a, b = _rand(K, M), _rand(K, N)
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    c.mm_tn(a, b, out=out)                                     # both operands MN-major
+    c.check_status()
+    assert _rel(out, a.double().t() @ b.double()) < ONE_ROUNDING
+    x = _rand(M, K)
+    assert _rel(c.mm_nn(x, b), x.double() @ b.double()) < ONE_ROUNDING
+    c.check_status()
+
+
+@pytest.mark.parametrize("rows,V,d", [(128, 65, 64), (300, 50257 % 1000 + 1000, 192), (136, 127, 128)])
+def test_odd_row_count_and_odd_reduction(rows, V, d):
+    """The three products of an output head whose vocabulary is odd; guard bands around every operand hold NaN."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    pitch = -(-V // 64) * 64
+    guard = torch.full((V + 64, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    W = guard[:V]
+    W.copy_(_rand(V, d))
+    h = _rand(rows, d)
+    buf = torch.full((rows, pitch), float("nan"), dtype=torch.bfloat16, device="cuda")
+    c.gemm(h, W, buf, M=rows, N=-(-V // 8) * 8, Kd=d, lda=d, ldb=d, ldc=pitch, b_rows=V)
+    assert _rel(buf[:, :V], h.double() @ W.double().t()) < ONE_ROUNDING
+    dh = torch.empty(rows, d, dtype=torch.bfloat16, device="cuda")
+    c.gemm(buf, W, dh, M=rows, N=d, Kd=V, b_major=c.MAJ_MN, lda=pitch, ldb=d, ldc=d)
+    assert _rel(dh, buf[:, :V].double() @ W.double()) < ONE_ROUNDING
+    dW = torch.full((V + 8, d), 7.0, dtype=torch.bfloat16, device="cuda")
+    c.gemm(buf, h, dW, M=V, N=d, Kd=rows, a_major=c.MAJ_MN, b_major=c.MAJ_MN, lda=pitch, ldb=d, ldc=d)
+    c.check_status()
+    assert _rel(dW[:V], buf[:, :V].double().t() @ h.double()) < ONE_ROUNDING
+    assert (dW[V:] == 7.0).all()
+
+
+# Rounded to bf16 on the way: gate, up, hidden, the rows and dH, dG, dU - seven roundings of about 1.7e-3 that add in
+# quadrature to 4.5e-3 at most; twice that.
+EXPERT_TOL = 9e-3
+
+
+def _expert_case(E, d, f):
+    return [_rand(E, d, f, scale=d ** -0.5), _rand(E, d, f, scale=d ** -0.5), _rand(E, f, d, scale=f ** -0.5)]
+
+
+@pytest.mark.parametrize("T,d,f,E,k", [(1, 64, 72, 3, 2), (200, 192, 88, 4, 2), (333, 72, 2464, 5, 1), (515, 1792, 136, 64, 2)])
+def test_expert_widths(T, d, f, E, k):
+    from kolmogorov_moe_architecture_b200 import ops
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops, eager
+    torch.manual_seed(T)
+    ws = _expert_case(E, d, f)
+    x = _rand(T, d)
+    wts, idx = eager.topk_softmax_route(torch.randn(T, E, device="cuda"), k)
+    wts = wts.to(torch.bfloat16)
+    go = _rand(T, d)
+    leaves = [t.clone().requires_grad_() for t in (x, *ws, wts)]
+    out = ops.grouped_swiglu(*leaves[:4], idx, leaves[4])
+    got = (out, *torch.autograd.grad(out, leaves, go))
+    cuda_ops.check_status()
+    ref_leaves = [t.double().requires_grad_() for t in (x, *ws, wts)]
+    ref = eager.grouped_swiglu(*ref_leaves[:4], idx, ref_leaves[4])
+    want = (ref, *torch.autograd.grad(ref, ref_leaves, go.double()))
+    for g, w in zip(got, want):
+        if w.norm() > 0:
+            assert _rel(g, w) < EXPERT_TOL
+
+
+@pytest.mark.parametrize("B,S,d,f,E", [(1, 65, 64, 72, 3), (2, 130, 136, 200, 4)])
+def test_expert_choice_widths(B, S, d, f, E):
+    from kolmogorov_moe_architecture_b200 import ops
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops, eager
+    torch.manual_seed(S)
+    ws = _expert_case(E, d, f)
+    x = _rand(B, S, d)
+    wts, tok = eager.expert_choice_route(torch.randn(B, S, E, device="cuda"), -(-S // E))
+    go = _rand(B, S, d)
+    leaves = [t.clone().requires_grad_() for t in (x, *ws, wts)]
+    out = ops.expert_choice_swiglu(*leaves, tok)
+    got = (out, *torch.autograd.grad(out, leaves, go))
+    cuda_ops.check_status()
+    ref_leaves = [t.double().requires_grad_() for t in (x, *ws, wts)]
+    ref = eager.expert_choice_swiglu(*ref_leaves, tok)
+    want = (ref, *torch.autograd.grad(ref, ref_leaves, go.double()))
+    for g, w in zip(got, want):
+        assert _rel(g, w) < EXPERT_TOL
+
+
+@pytest.mark.parametrize("B,S,d,V,chunk", [(1, 9, 64, 65, 8192), (2, 70, 128, 1001, 64), (2, 33, 64, 131, 8192)])
+def test_loss_vocabulary(B, S, d, V, chunk):
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops, eager
+    torch.manual_seed(V)
+    h = _rand(B, S, d)
+    Ws = [_rand(V, d, scale=0.1) for _ in range(3)]
+    labels = torch.randint(0, V, (B, S), device="cuda")
+    labels[:, ::7] = -100
+    wts = (0.5, 0.3, 0.2)
+    leaves = [t.clone().requires_grad_() for t in (h, *Ws)]
+    total, _ = cuda_ops.mtp_cross_entropy(leaves[0], leaves[1:], labels, wts, chunk_rows=chunk)
+    got = torch.autograd.grad(total, leaves)
+    cuda_ops.check_status()
+    ref_leaves = [t.double().requires_grad_() for t in (h, *Ws)]
+    ref = 0.0
+    for i, W in enumerate(ref_leaves[1:]):
+        lg = ref_leaves[0][:, : S - i - 1] @ W.t()
+        ref = ref + wts[i] * torch.nn.functional.cross_entropy(lg.reshape(-1, V), labels[:, i + 1:].reshape(-1), ignore_index=-100)
+    want = torch.autograd.grad(ref, ref_leaves)
+    # logits and their gradients are rounded to bf16, and dH / dW to bf16 once per head / row chunk
+    assert abs(total.item() - ref.item()) < 2e-3 * abs(ref.item())
+    for g, w in zip(got, want):
+        assert _rel(g, w) < EXPERT_TOL
