@@ -160,31 +160,211 @@ __device__ __forceinline__ void load8(const float* src, float* v) {
   v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-// Writes one 32-column chunk of one row: out = alpha*scale*acc + beta*D
-template <typename T>
-__device__ __forceinline__ void epilogue_store_chunk(const GemmArgs& a, const uint32_t (&acc)[32], bool have_acc,
-                                                     long long row_off_c, long long row_off_d, int col, float scale,
-                                                     float beta, long long row_addr, int row = -1) {
-  // row_addr != 0: the row's own base address (possibly on a peer GPU) replaces C + row offset
-  T* C = row_addr ? reinterpret_cast<T*>(row_addr) - row_off_c : reinterpret_cast<T*>(a.C);
-  const T* D = reinterpret_cast<const T*>(a.D);
+// Writes one 32-column chunk of one fp32 row: out = scale * acc + beta * D
+__device__ __forceinline__ void epilogue_store_chunk_f32(const GemmArgs& a, const uint32_t (&acc)[32], bool have_acc,
+                                                         long long row_off_c, long long row_off_d, int col, float scale,
+                                                         float beta) {
+  float* C = reinterpret_cast<float*>(a.C);
+  const float* D = reinterpret_cast<const float*>(a.D);
 #pragma unroll
   for (int j = 0; j < 32; j += 8) {
     if (col + j >= a.N) break;
     float v[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = have_acc ? __uint_as_float(acc[j + i]) * scale : 0.f;
-    if (a.diag_add != 0.f && row >= col + j && row < col + j + 8) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] += (col + j + i == row) ? a.diag_add : 0.f;
-    }
     if (D != nullptr) {
       float d[8];
       load8(D + row_off_d + col + j, d);
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] += beta * d[i];
     }
-    store8<T>(C + row_off_c + col + j, v);
+    store8<float>(C + row_off_c + col + j, v);
+  }
+}
+
+// ------------------------------------------------------------------ bf16 epilogue
+// An epilogue warp owns 32 accumulator rows (lane = row).  Each 64-column slab is read from tensor memory, finished
+// in registers, rounded into one of the warp's two 4 KB staging buffers (32 rows x 128 bytes in the 128-byte swizzle,
+// so that both the row-per-lane writes and TMA's reads are free of bank conflicts) and sent off by a TMA store, which
+// also clips at M and N.  The warp does not wait for the store: it returns to a buffer two slabs later, and the
+// accumulator goes back to the MMA warp as soon as the last slab is in registers.
+// A tile whose reduction is shorter than its epilogue is bound by this code (weight gradients of experts with few
+// tokens, orthogonalisation).  The staged form it replaces - shared memory, then one 128-byte line per 8 lanes - took
+// 6.1 us per 256 x 256 tile.
+constexpr int OUT_BUF_BYTES = 32 * 128;
+constexpr int OUT_STAGE_BYTES = 4 * 2 * OUT_BUF_BYTES;     // four epilogue warps, two buffers each
+
+struct OutStage {
+  uint8_t* base;
+  int buf;
+};
+__device__ __forceinline__ uint8_t* out_acquire(OutStage& o, int lane) {
+  if (lane == 0) tma_store_wait_read_but_one();
+  __syncwarp();
+  uint8_t* p = o.base + o.buf * OUT_BUF_BYTES;
+  o.buf ^= 1;
+  return p;
+}
+__device__ __forceinline__ void out_put_row(uint8_t* sb, int lane, const uint32_t (&p)[32]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    *reinterpret_cast<uint4*>(sb + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+        make_uint4(p[4 * j], p[4 * j + 1], p[4 * j + 2], p[4 * j + 3]);
+}
+__device__ __forceinline__ void out_send(const CUtensorMap* tm, const uint8_t* sb, int lane, int x, int y, int g) {
+  fence_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    tma_store_4d(tm, sb, x, y, 0, g);
+    tma_store_commit();
+  }
+}
+
+// C = scale * acc (+ diag) (+ beta D + beta2 D2), all in fp32 before the one rounding.  `mirror`: the tile lies above
+// the diagonal of a symmetric product and also writes its transpose (tmT: boxes of 32 columns x 64 rows).
+// wait() returns once the accumulator is complete (false: gave up), release() hands it back.
+template <int BN, class Wait, class Release>
+__device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtensorMap* tmC, const CUtensorMap* tmT,
+                                                OutStage& out, uint32_t t_row, bool have_acc, int row0, int n0, int g,
+                                                float scale, float beta, float beta2, bool mirror, int lane,
+                                                Wait wait, Release release) {
+  const int slabs = row0 < a.M ? min(BN / 64, ceil_div(a.N - n0, 64)) : 0;
+  const __nv_bfloat16* Dp = reinterpret_cast<const __nv_bfloat16*>(a.D);
+  const __nv_bfloat16* D2p = reinterpret_cast<const __nv_bfloat16*>(a.D2);
+  const bool diag = a.diag_add != 0.f && n0 < row0 + 32 && n0 + BN > row0;
+  const long long goff = (long long)g * a.c_gstride;
+  uint4 dpre[8];
+  auto load_addend = [&](const __nv_bfloat16* P, int col) {      // 8 lanes per row: full 128-byte lines
+#pragma unroll
+    for (int i8 = 0; i8 < 8; ++i8) {
+      const int grow = row0 + i8 * 4 + (lane >> 3);
+      const int gcol = col + (lane & 7) * 8;
+      dpre[i8] = (grow < a.M && gcol < a.N)
+                     ? __ldg(reinterpret_cast<const uint4*>(P + goff + (long long)grow * a.ldd + gcol))
+                     : make_uint4(0, 0, 0, 0);
+    }
+  };
+  if (Dp != nullptr && slabs > 0) load_addend(Dp, n0);           // under the wait for the accumulator
+  if (!wait()) return false;
+  if (slabs == 0) release();
+  // the loop stays rolled: unrolled, the epilogue outgrows the instruction cache
+#pragma unroll 1
+  for (int sl = 0; sl < slabs; ++sl) {
+    const int col = n0 + sl * 64;
+    uint32_t r[64];
+    if (have_acc) {
+      tmem_ld_32x32(t_row + sl * 64, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+      tmem_ld_32x32(t_row + sl * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+      tmem_ld_wait();
+    } else {
+#pragma unroll
+      for (int i = 0; i < 64; ++i) r[i] = 0u;
+    }
+    if (sl == slabs - 1) release();
+#pragma unroll
+    for (int i = 0; i < 64; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * scale);
+    if (diag) {
+#pragma unroll
+      for (int i = 0; i < 64; ++i)
+        if (col + i == row0 + lane) r[i] = __float_as_uint(__uint_as_float(r[i]) + a.diag_add);
+    }
+    uint8_t* sb = out_acquire(out, lane);
+    if (Dp != nullptr) {
+      // the addends pass through the staging buffer to reach the lane that owns their row
+#pragma unroll 1
+      for (int pass = 0; pass < (D2p != nullptr ? 2 : 1); ++pass) {
+        const float bcoef = pass == 0 ? beta : beta2;
+        if (pass == 1) load_addend(D2p, col);
+#pragma unroll
+        for (int i8 = 0; i8 < 8; ++i8) {
+          const int rr = i8 * 4 + (lane >> 3);
+          *reinterpret_cast<uint4*>(sb + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4)) = dpre[i8];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint4 q4 = *reinterpret_cast<const uint4*>(sb + lane * 128 + ((j ^ (lane & 7)) << 4));
+          const __nv_bfloat162* pq = reinterpret_cast<const __nv_bfloat162*>(&q4);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 f = __bfloat1622float2(pq[i]);
+            r[j * 8 + 2 * i] = __float_as_uint(__uint_as_float(r[j * 8 + 2 * i]) + bcoef * f.x);
+            r[j * 8 + 2 * i + 1] = __float_as_uint(__uint_as_float(r[j * 8 + 2 * i + 1]) + bcoef * f.y);
+          }
+        }
+        __syncwarp();
+      }
+      if (sl + 1 < slabs) load_addend(Dp, col + 64);
+    }
+    uint32_t p[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) p[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+    out_put_row(sb, lane, p);
+    out_send(tmC, sb, lane, col, row0, g);
+    if (mirror) {
+      // two lanes hold a 2 x 2 block: they swap its off-diagonal corner and each writes one word of the transpose
+      uint8_t* mb = out_acquire(out, lane);
+      const bool odd = lane & 1;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const uint32_t give = odd ? (p[i] & 0xffffu) : (p[i] >> 16);
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, give, 1);
+        const uint32_t word = odd ? (got | (p[i] & 0xffff0000u)) : ((p[i] & 0xffffu) | (got << 16));
+        *reinterpret_cast<uint32_t*>(mb + (2 * i + (odd ? 1 : 0)) * 64 + (lane >> 1) * 4) = word;
+      }
+      out_send(tmT, mb, lane, row0, col, g);
+    }
+  }
+  return true;
+}
+
+// H = silu(gate) * up * scale, with the pre-activations G and U stored as well when asked for.  The accumulator holds
+// HB gate columns followed by the HB up columns of the same outputs.
+template <int HB, class Release>
+__device__ __forceinline__ void store_tile_swiglu(const GemmArgs& a, const CUtensorMap* tmH, const CUtensorMap* tmG,
+                                                  const CUtensorMap* tmU, OutStage& out, uint32_t t_row, bool have_acc,
+                                                  int row0, int n0, int g, float scale, int lane, Release release) {
+  const int slabs = row0 < a.M ? min(HB / 64, ceil_div(a.N - n0, 64)) : 0;
+  if (slabs == 0) release();
+  // Three results per slab, one after the other: reading tensor memory again costs less than holding both slabs in
+  // registers (192 of them, which spilled).
+#pragma unroll 1
+  for (int sl = 0; sl < slabs; ++sl) {
+    const int col = n0 + sl * 64;
+    const int last = a.U_out != nullptr ? 2 : (a.G_out != nullptr ? 1 : 0);
+#pragma unroll 1
+    for (int what = 0; what <= last; ++what) {
+      if (what == 1 && a.G_out == nullptr) continue;
+      uint32_t p[32];
+      const uint32_t t_first = t_row + sl * 64 + (what == 2 ? HB : 0);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t x[32];
+        if (have_acc) {
+          tmem_ld_32x32(t_first + h * 32, x);
+          if (what == 0) {
+            uint32_t u[32];
+            tmem_ld_32x32(t_row + HB + sl * 64 + h * 32, u);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              x[i] = __float_as_uint(silu_f(__uint_as_float(x[i])) * __uint_as_float(u[i]) * scale);
+          } else {
+            tmem_ld_wait();
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) x[i] = 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          p[h * 16 + i] = pack_bf16(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1]));
+      }
+      if (sl == slabs - 1 && what == last) release();
+      uint8_t* sb = out_acquire(out, lane);
+      out_put_row(sb, lane, p);
+      out_send(what == 0 ? tmH : (what == 1 ? tmG : tmU), sb, lane, col, row0, g);
+    }
   }
 }
 
@@ -217,7 +397,9 @@ __device__ __forceinline__ void load_mn_tile_pair(uint8_t* dst, const CUtensorMa
 template <int BN, int A_MAJOR, int B_MAJOR>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmB2, const GemmArgs args, const int stages) {
+                 const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
+                 const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY, const GemmArgs args,
+                 const int stages) {
   constexpr int B_STAGE_BYTES = BN * BK * 2;
   constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
   constexpr uint32_t TMEM_COLS = 2 * BN;  // two accumulators
@@ -231,7 +413,6 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __shared__ uint64_t tmem_full[2];
   __shared__ uint64_t tmem_empty[2];
   __shared__ uint32_t tmem_base_slot;
-  __shared__ __align__(16) __nv_bfloat16 peer_stage[4][32][72];   // per epilogue warp: 32 rows x 64 columns (+pad)
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -354,37 +535,54 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     int it = 0;
     Tile t;
+    OutStage out{smem + stages * STAGE_BYTES + q * 2 * OUT_BUF_BYTES, 0};
     for (int idx = blockIdx.x; get_tile<BN>(args, idx, num_m, num_n, t); idx += gridDim.x) {
       const int acc = it & 1;
       const uint32_t acc_ph = (it >> 1) & 1;
       ++it;
-      if (!mbar_wait(&tmem_full[acc], acc_ph)) {
-        if (lane == 0) atomicExch(args.status, 4);
-        goto teardown;
-      }
-      tc_fence_after();
       const bool have_acc = t.k_blocks > 0;
-      const int row = t.m_tile * BM + q * 32 + lane;
+      const int row0 = t.m_tile * BM + q * 32;
+      const int row = row0 + lane;
       const bool row_ok = row < args.M;
-      const long long coff = (long long)t.g_c * args.c_gstride + (long long)row * args.ldc;
-      const long long doff = (long long)t.g_c * args.c_gstride + (long long)row * args.ldd;
       float scale = args.alpha;
       float beta = args.beta;
       if (args.alpha_dev != nullptr) scale *= args.alpha_dev[t.g_c];
       if (args.beta_dev != nullptr) beta *= args.beta_dev[t.g_c];
       if (args.row_scale != nullptr && row_ok) scale *= args.row_scale[row];
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
-      long long row_addr = 0;
-      bool store_ok = row_ok;
-      if (args.row_ptr != nullptr) {
-        row_addr = row_ok ? args.row_ptr[row] : 0;
-        store_ok = row_addr != 0;
+      auto wait = [&]() {
+        if (!mbar_wait(&tmem_full[acc], acc_ph)) {
+          if (lane == 0) atomicExch(args.status, 4);
+          return false;
+        }
+        tc_fence_after();
+        return true;
+      };
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+      };
+      if (!swiglu && !args.out_f32 && args.row_ptr == nullptr) {
+        if (!store_tile_bf16<BN>(args, &tmC, &tmX, out, t_row, have_acc, row0, t.n_tile * BN, t.g_c, scale, beta, 0.f,
+                                 false, lane, wait, release))
+          goto teardown;
+        continue;
       }
-      if (!swiglu && args.row_ptr != nullptr) {
+      if (!wait()) goto teardown;
+      if (swiglu) {
+        store_tile_swiglu<BN / 2>(args, &tmC, &tmX, &tmY, out, t_row, have_acc, row0, t.n_tile * (BN / 2), t.g_c, scale,
+                                  lane, release);
+        continue;
+      }
+      const long long coff = (long long)t.g_c * args.c_gstride + (long long)row * args.ldc;
+      const long long doff = (long long)t.g_c * args.c_gstride + (long long)row * args.ldd;
+      if (args.row_ptr != nullptr) {
         // Rows go to individual addresses, possibly on peer GPUs.  A lane holds one row, so a direct store
         // would emit 32 scattered 16-byte writes per instruction; the 64-column slab is staged in shared
         // memory instead and written back with 8 lanes per row: four full 128-byte lines per instruction.
-        __nv_bfloat16(*stg)[72] = peer_stage[q];
+        const long long row_addr = row_ok ? args.row_ptr[row] : 0;
+        __nv_bfloat16(*stg)[72] = reinterpret_cast<__nv_bfloat16(*)[72]>(out.base);      // 32 rows, within 8 KB
         const __nv_bfloat16* Dp = reinterpret_cast<const __nv_bfloat16*>(args.D);
 #pragma unroll 1
         for (int c = 0; c < BN; c += 64) {
@@ -423,7 +621,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
           __syncwarp();
         }
-      } else if (!swiglu) {
+      } else {
 #pragma unroll 1
         for (int c = 0; c < BN; c += 32) {
           uint32_t r[32];
@@ -432,52 +630,15 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tmem_ld_wait();
           }
           const int col = t.n_tile * BN + c;
-          if (store_ok && col < args.N) {
-            if (args.out_f32)
-              epilogue_store_chunk<float>(args, r, have_acc, coff, doff, col, scale, beta, row_addr);
-            else
-              epilogue_store_chunk<__nv_bfloat16>(args, r, have_acc, coff, doff, col, scale, beta, row_addr, row);
-          }
-        }
-      } else {
-        constexpr int HB = BN / 2;
-        __nv_bfloat16* H = reinterpret_cast<__nv_bfloat16*>(args.C);
-        __nv_bfloat16* G = reinterpret_cast<__nv_bfloat16*>(args.G_out);
-        __nv_bfloat16* U = reinterpret_cast<__nv_bfloat16*>(args.U_out);
-#pragma unroll 1
-        for (int c = 0; c < HB; c += 32) {
-          uint32_t g[32], u[32];
-          if (have_acc) {
-            tmem_ld_32x32(t_row + c, g);
-            tmem_ld_32x32(t_row + HB + c, u);
-            tmem_ld_wait();
-          }
-          const int col = t.n_tile * HB + c;
-          if (row_ok && col < args.N) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (col + j >= args.N) break;
-              float gv[8], uv[8], hv[8];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                gv[i] = have_acc ? __uint_as_float(g[j + i]) : 0.f;
-                uv[i] = have_acc ? __uint_as_float(u[j + i]) : 0.f;
-                hv[i] = silu_f(gv[i]) * uv[i] * scale;
-              }
-              store8<__nv_bfloat16>(H + coff + col + j, hv);
-              if (G != nullptr) store8<__nv_bfloat16>(G + coff + col + j, gv);
-              if (U != nullptr) store8<__nv_bfloat16>(U + coff + col + j, uv);
-            }
-          }
+          if (row_ok && col < args.N) epilogue_store_chunk_f32(args, r, have_acc, coff, doff, col, scale, beta);
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+      release();
     }
   }
 
 teardown:
+  if (warp >= 2 && lane == 0) tma_store_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -502,7 +663,9 @@ constexpr int PAIR_TM = 2 * BM;
 template <int BN, int A_MAJOR, int B_MAJOR>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                      const __grid_constant__ CUtensorMap tmB2, const GemmArgs args, const int stages) {
+                      const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
+                 const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY, const GemmArgs args,
+                 const int stages) {
   constexpr int HALF_N = BN / 2;
   constexpr int B_STAGE_BYTES = HALF_N * BK * 2;
   constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;   // per CTA
@@ -517,7 +680,6 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   __shared__ uint64_t tmem_full[2];
   __shared__ uint64_t tmem_empty[2];
   __shared__ uint32_t tmem_base_slot;
-  __shared__ __align__(16) __nv_bfloat16 out_stage[4][32][72];   // per epilogue warp: 32 rows x 64 columns (+pad)
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -639,210 +801,73 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const int q = warp & 3;
     int it = 0;
     Tile t;
-    __nv_bfloat16(*stg)[72] = out_stage[q];
+    OutStage out{smem + stages * STAGE_BYTES + q * 2 * OUT_BUF_BYTES, 0};
     for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t); idx += num_pairs) {
       const int acc = it & 1;
       const uint32_t acc_ph = (it >> 1) & 1;
       ++it;
-      const bool staged = !swiglu && !args.out_f32;   // this path awaits the accumulator itself
-      if (!staged) {
-        if (!mbar_wait(&tmem_full[acc], acc_ph)) {
-          if (lane == 0) atomicExch(args.status, 14);
-          goto teardown;
-        }
-        tc_fence_after();
-      }
       const bool have_acc = t.k_blocks > 0;
       const int row0 = t.m_tile * PAIR_TM + (int)rank * BM + q * 32;
       const int row = row0 + lane;
       const bool row_ok = row < args.M;
+      float scale = args.alpha;
+      float beta = args.beta, beta2 = args.beta2;
+      if (args.alpha_dev != nullptr) scale *= args.alpha_dev[t.g_c];
+      if (args.beta_dev != nullptr) {
+        beta *= args.beta_dev[t.g_c];
+        beta2 *= args.beta_dev[t.g_c];
+      }
+      if (args.row_scale != nullptr && row_ok) scale *= args.row_scale[row];
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
+      auto wait = [&]() {
+        if (!mbar_wait(&tmem_full[acc], acc_ph)) {
+          if (lane == 0) atomicExch(args.status, 14);
+          return false;
+        }
+        tc_fence_after();
+        return true;
+      };
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (leader) mbar_arrive(&tmem_empty[acc]);
+          else mbar_arrive_cluster(map_to_cta(&tmem_empty[acc], 0));
+        }
+      };
+      if (!swiglu && !args.out_f32) {
+        // symmetric product: a tile strictly above the diagonal also writes its transpose
+        const bool mirror = args.sym_upper && t.n_tile * BN >= (t.m_tile + 1) * PAIR_TM;
+        if (!store_tile_bf16<BN>(args, &tmC, &tmX, out, t_row, have_acc, row0, t.n_tile * BN, t.g_c, scale, beta, beta2,
+                                 mirror, lane, wait, release))
+          goto teardown;
+        continue;
+      }
+      if (!wait()) goto teardown;
+      if (swiglu) {
+        store_tile_swiglu<HALF_N>(args, &tmC, &tmX, &tmY, out, t_row, have_acc, row0, t.n_tile * HALF_N, t.g_c, scale,
+                                  lane, release);
+        continue;
+      }
       const long long goff = (long long)t.g_c * args.c_gstride;
       const long long coff = goff + (long long)row * args.ldc;
       const long long doff = goff + (long long)row * args.ldd;
-      float scale = args.alpha;
-      float beta = args.beta;
-      if (args.alpha_dev != nullptr) scale *= args.alpha_dev[t.g_c];
-      if (args.beta_dev != nullptr) beta *= args.beta_dev[t.g_c];
-      if (args.row_scale != nullptr && row_ok) scale *= args.row_scale[row];
-      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
-      if (!swiglu && !args.out_f32) {
-        // bf16 output: a lane holds one row, so each 64-column slab is staged in shared memory and written
-        // back with 8 lanes per row (four full 128-byte lines per store instruction).  The addend is read
-        // with the same pattern.
-        __nv_bfloat16* Cb = reinterpret_cast<__nv_bfloat16*>(args.C);
-        const __nv_bfloat16* Dp = reinterpret_cast<const __nv_bfloat16*>(args.D);
-        constexpr int SLABS = BN / 64;
-        if (!mbar_wait(&tmem_full[acc], acc_ph)) {
-          if (lane == 0) atomicExch(args.status, 14);
-          goto teardown;
-        }
-        tc_fence_after();
-        // symmetric product: a tile strictly above the diagonal also writes its transpose
-        const bool mirror = args.sym_upper && t.n_tile * BN >= (t.m_tile + 1) * PAIR_TM;
-        const bool diag = args.diag_add != 0.f && t.n_tile * BN < row0 + 32 && (t.n_tile + 1) * BN > row0;
-        // Addends of a symmetric product (and every second addend) are added before the slab is staged, each lane
-        // reading its own row, so that the mirrored tile is written from final values.
-        const __nv_bfloat16* D2p = reinterpret_cast<const __nv_bfloat16*>(args.D2);
-        const bool d_early = Dp != nullptr && (args.sym_upper || D2p != nullptr);
-        float beta2 = args.beta2;
-        if (args.beta_dev != nullptr) beta2 *= args.beta_dev[t.g_c];
-        // the slab loop stays rolled: unrolled, the epilogue outgrows the instruction cache and every tile
-        // of a short-reduction product stalls on instruction fetch
 #pragma unroll 1
-        for (int sl = 0; sl < SLABS; ++sl) {
-          const int c = sl * 64;
-          if (t.n_tile * BN + c >= args.N) break;
-          // the addend of this slab is requested first: its latency falls under the accumulator reads below
-          uint4 dpre[8];
-          auto load_addend = [&](const __nv_bfloat16* P) {      // 8 lanes per row: full 128-byte lines
-#pragma unroll
-            for (int i8 = 0; i8 < 8; ++i8) {
-              const int grow = row0 + i8 * 4 + (lane >> 3);
-              const int gcol = t.n_tile * BN + c + (lane & 7) * 8;
-              dpre[i8] = (grow < args.M && gcol < args.N)
-                             ? __ldg(reinterpret_cast<const uint4*>(P + goff + (long long)grow * args.ldd + gcol))
-                             : make_uint4(0, 0, 0, 0);
-            }
-          };
-          if (Dp != nullptr) load_addend(Dp);
-          uint32_t r[64];
-          if (have_acc) {
-            tmem_ld_32x32(t_row + c, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-            tmem_ld_32x32(t_row + c + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
-            tmem_ld_wait();
-          }
-#pragma unroll
-          for (int i = 0; i < 64; ++i) r[i] = have_acc ? __float_as_uint(__uint_as_float(r[i]) * scale) : 0u;
-          if (diag) {
-            const int col0 = t.n_tile * BN + c;
-#pragma unroll
-            for (int i = 0; i < 64; ++i)
-              if (col0 + i == row) r[i] = __float_as_uint(__uint_as_float(r[i]) + args.diag_add);
-          }
-          if (d_early) {
-            // the addends pass through the staging buffer to reach the lane that owns their row
-#pragma unroll 1
-            for (int pass = 0; pass < (D2p != nullptr ? 2 : 1); ++pass) {
-              const float bcoef = pass == 0 ? beta : beta2;
-              if (pass == 1) load_addend(D2p);
-#pragma unroll
-              for (int i8 = 0; i8 < 8; ++i8)
-                *reinterpret_cast<uint4*>(&stg[i8 * 4 + (lane >> 3)][(lane & 7) * 8]) = dpre[i8];
-              __syncwarp();
-#pragma unroll
-              for (int j8 = 0; j8 < 8; ++j8) {
-                const uint4 q4 = *reinterpret_cast<const uint4*>(&stg[lane][j8 * 8]);
-                const __nv_bfloat162* pq = reinterpret_cast<const __nv_bfloat162*>(&q4);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const float2 f = __bfloat1622float2(pq[i]);
-                  r[j8 * 8 + 2 * i] = __float_as_uint(__uint_as_float(r[j8 * 8 + 2 * i]) + bcoef * f.x);
-                  r[j8 * 8 + 2 * i + 1] = __float_as_uint(__uint_as_float(r[j8 * 8 + 2 * i + 1]) + bcoef * f.y);
-                }
-              }
-              __syncwarp();
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 64; j += 8) store8<__nv_bfloat16>(&stg[lane][j], reinterpret_cast<const float*>(&r[j]));
-          __syncwarp();
-#pragma unroll
-          for (int i8 = 0; i8 < 8; ++i8) {
-            const int rr = i8 * 4 + (lane >> 3);
-            const int cc = (lane & 7) * 8;
-            const int grow = row0 + rr;
-            const int gcol = t.n_tile * BN + c + cc;
-            if (grow < args.M && gcol < args.N) {
-              uint4 o = *reinterpret_cast<const uint4*>(&stg[rr][cc]);
-              if (Dp != nullptr && !d_early) {
-                float v[8];
-                const __nv_bfloat162* pv = reinterpret_cast<const __nv_bfloat162*>(&o);
-                const __nv_bfloat162* pd = reinterpret_cast<const __nv_bfloat162*>(&dpre[i8]);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const float2 f = __bfloat1622float2(pv[i]);
-                  const float2 d = __bfloat1622float2(pd[i]);
-                  v[2 * i] = f.x + beta * d.x;
-                  v[2 * i + 1] = f.y + beta * d.y;
-                }
-                o.x = pack_bf16(v[0], v[1]); o.y = pack_bf16(v[2], v[3]);
-                o.z = pack_bf16(v[4], v[5]); o.w = pack_bf16(v[6], v[7]);
-              }
-              *reinterpret_cast<uint4*>(Cb + goff + (long long)grow * args.ldc + gcol) = o;
-            }
-          }
-          if (mirror) {
-            // C[col][row] = C[row][col]: a lane gathers 8 rows of one staged column (16 bytes of the
-            // destination row), 4 lanes cover the 32 rows of the slab
-#pragma unroll
-            for (int i8 = 0; i8 < 8; ++i8) {
-              const int jc = i8 * 8 + (lane >> 2);          // staged column = destination row
-              const int r8 = (lane & 3) * 8;                // first of 8 staged rows = destination columns
-              const int drow = t.n_tile * BN + c + jc;
-              const int dcol = row0 + r8;
-              if (drow < args.N && dcol < args.M) {
-                __nv_bfloat16 e[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) e[i] = stg[r8 + i][jc];
-                *reinterpret_cast<uint4*>(Cb + goff + (long long)drow * args.ldc + dcol) =
-                    *reinterpret_cast<const uint4*>(e);
-              }
-            }
-          }
-          __syncwarp();
+      for (int c = 0; c < BN; c += 32) {
+        uint32_t r[32];
+        if (have_acc) {
+          tmem_ld_32x32(t_row + c, r);
+          tmem_ld_wait();
         }
-      } else if (!swiglu) {
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t r[32];
-          if (have_acc) {
-            tmem_ld_32x32(t_row + c, r);
-            tmem_ld_wait();
-          }
-          const int col = t.n_tile * BN + c;
-          if (row_ok && col < args.N) epilogue_store_chunk<float>(args, r, have_acc, coff, doff, col, scale, beta, 0);
-        }
-      } else {
-        __nv_bfloat16* H = reinterpret_cast<__nv_bfloat16*>(args.C);
-        __nv_bfloat16* G = reinterpret_cast<__nv_bfloat16*>(args.G_out);
-        __nv_bfloat16* U = reinterpret_cast<__nv_bfloat16*>(args.U_out);
-#pragma unroll 1
-        for (int c = 0; c < HALF_N; c += 32) {
-          uint32_t g[32], u[32];
-          if (have_acc) {
-            tmem_ld_32x32(t_row + c, g);
-            tmem_ld_32x32(t_row + HALF_N + c, u);
-            tmem_ld_wait();
-          }
-          const int col = t.n_tile * HALF_N + c;
-          if (row_ok && col < args.N) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (col + j >= args.N) break;
-              float gv[8], uv[8], hv[8];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                gv[i] = have_acc ? __uint_as_float(g[j + i]) : 0.f;
-                uv[i] = have_acc ? __uint_as_float(u[j + i]) : 0.f;
-                hv[i] = silu_f(gv[i]) * uv[i] * scale;
-              }
-              store8<__nv_bfloat16>(H + coff + col + j, hv);
-              if (G != nullptr) store8<__nv_bfloat16>(G + coff + col + j, gv);
-              if (U != nullptr) store8<__nv_bfloat16>(U + coff + col + j, uv);
-            }
-          }
-        }
+        const int col = t.n_tile * BN + c;
+        if (row_ok && col < args.N) epilogue_store_chunk_f32(args, r, have_acc, coff, doff, col, scale, beta);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (leader) mbar_arrive(&tmem_empty[acc]);
-        else mbar_arrive_cluster(map_to_cta(&tmem_empty[acc], 0));
-      }
+      release();
     }
   }
 
 teardown:
+  if (warp >= 2 && lane == 0) tma_store_wait_all();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                 // nothing of the peer may still point at this CTA's memory
@@ -918,30 +943,59 @@ static int make_operand_tmap(CUtensorMap* out, const void* base, int major, long
   return 0;
 }
 
+// Output tensor map (bf16): dims {N, rows, 1, G}.  Plain: box {64, 32}, 128B swizzle, the staging buffer of an epilogue
+// warp.  Transposed tiles of a symmetric product: box {32, 64} without swizzle.
+static int make_output_tmap(CUtensorMap* out, const void* base, long long rows, long long N, long long ld,
+                            long long gstride, int groups, bool transposed) {
+  TmapKey key{base, transposed ? 3 : 2, rows, N, ld, gstride, groups, 0};
+  {
+    std::lock_guard<std::mutex> lk(g_tmap_mutex);
+    auto it = g_tmap_cache.find(key);
+    if (it != g_tmap_cache.end()) {
+      *out = it->second;
+      return 0;
+    }
+  }
+  const long long gs = groups > 1 ? gstride : rows * ld;
+  const cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)rows, 1, (cuuint64_t)groups};
+  const cuuint64_t strides[3] = {(cuuint64_t)ld * 2, (cuuint64_t)rows * ld * 2, (cuuint64_t)gs * 2};
+  const cuuint32_t box[4] = {transposed ? 32u : 64u, transposed ? 64u : 32u, 1, 1};
+  const int rc = encode_bf16_4d(out, base, dims, strides, box,
+                                transposed ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc) return rc;
+  {
+    std::lock_guard<std::mutex> lk(g_tmap_mutex);
+    if (g_tmap_cache.size() > 4096) g_tmap_cache.clear();
+    g_tmap_cache[key] = *out;
+  }
+  return 0;
+}
+
 template <int BN, int AM, int BMj>
-static int launch_variant(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2, const GemmArgs& args,
-                          int grid, cudaStream_t stream) {
+static int launch_variant(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2, const CUtensorMap& tC,
+                          const CUtensorMap& tX, const CUtensorMap& tY, const GemmArgs& args, int grid,
+                          cudaStream_t stream) {
   constexpr int stage_bytes = A_STAGE_BYTES + BN * BK * 2;
-  int stages = (196 * 1024) / stage_bytes;      // leaves room for the 18 KB static staging buffer
+  int stages = (192 * 1024) / stage_bytes;      // operand ring beside the 32 KB of output staging
   if (stages > 8) stages = 8;
-  const int smem = stages * stage_bytes + 1024;
+  const int smem = stages * stage_bytes + OUT_STAGE_BYTES + 1024;
   auto kern = umma_gemm_kernel<BN, AM, BMj>;
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
     attr_set = true;
   }
-  kern<<<grid, NUM_THREADS, smem, stream>>>(tA, tB, tB2, args, stages);
+  kern<<<grid, NUM_THREADS, smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
 template <int BN, int AM, int BMj>
 static int launch_pair_variant(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2,
-                               const GemmArgs& args, long long pair_tiles, int sms, cudaStream_t stream) {
+                               const CUtensorMap& tC, const CUtensorMap& tX, const CUtensorMap& tY, const GemmArgs& args, long long pair_tiles, int sms, cudaStream_t stream) {
   constexpr int stage_bytes = A_STAGE_BYTES + (BN / 2) * BK * 2;
-  int stages = (196 * 1024) / stage_bytes;
+  int stages = (192 * 1024) / stage_bytes;
   if (stages > 8) stages = 8;
-  const int smem = stages * stage_bytes + 1024;
+  const int smem = stages * stage_bytes + OUT_STAGE_BYTES + 1024;
   auto kern = umma_gemm_pair_kernel<BN, AM, BMj>;
   static int max_clusters = 0;
   if (max_clusters == 0) {
@@ -960,7 +1014,7 @@ static int launch_pair_variant(const CUtensorMap& tA, const CUtensorMap& tB, con
   }
   long long pairs = pair_tiles < max_clusters ? pair_tiles : max_clusters;
   if (pairs < 1) pairs = 1;
-  kern<<<(unsigned)(2 * pairs), NUM_THREADS, smem, stream>>>(tA, tB, tB2, args, stages);
+  kern<<<(unsigned)(2 * pairs), NUM_THREADS, smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
@@ -1065,6 +1119,16 @@ extern "C" int kmoe_gemm(const KmoeGemmDesc* d, cudaStream_t stream) {
   } else {
     tB2 = tB;
   }
+  // outputs that leave by TMA stores: everything but fp32 results and per-row destinations
+  CUtensorMap tC = tA, tX = tA, tY = tA;
+  if (!d->out_f32 && d->c_row_ptr == nullptr) {
+    const int c_groups = (int)groups;
+    rc = make_output_tmap(&tC, d->C, d->M, d->N, d->ldc, d->c_gstride, c_groups, false);
+    if (!rc && swiglu && d->G_out) rc = make_output_tmap(&tX, d->G_out, d->M, d->N, d->ldc, d->c_gstride, c_groups, false);
+    if (!rc && swiglu && d->U_out) rc = make_output_tmap(&tY, d->U_out, d->M, d->N, d->ldc, d->c_gstride, c_groups, false);
+    if (!rc && d->sym_upper && pair) rc = make_output_tmap(&tX, d->C, d->M, d->N, d->ldc, d->c_gstride, c_groups, true);
+    if (rc) return rc;
+  }
   const int n_per_tile = swiglu ? BN / 2 : BN;
   long long total = tm_tiles * ((d->N + n_per_tile - 1) / n_per_tile) * groups;
   if (d->sym_upper) {
@@ -1077,8 +1141,8 @@ extern "C" int kmoe_gemm(const KmoeGemmDesc* d, cudaStream_t stream) {
   if (grid < 1) grid = 1;
 
   int lrc = 0;
-#define KMOE_LAUNCH_PAIR(BN_, AM_, BM_) lrc = launch_pair_variant<BN_, AM_, BM_>(tA, tB, tB2, a, total, sms, stream)
-#define KMOE_LAUNCH(BN_, AM_, BM_) lrc = launch_variant<BN_, AM_, BM_>(tA, tB, tB2, a, grid, stream)
+#define KMOE_LAUNCH_PAIR(BN_, AM_, BM_) lrc = launch_pair_variant<BN_, AM_, BM_>(tA, tB, tB2, tC, tX, tY, a, total, sms, stream)
+#define KMOE_LAUNCH(BN_, AM_, BM_) lrc = launch_variant<BN_, AM_, BM_>(tA, tB, tB2, tC, tX, tY, a, grid, stream)
   if (pair && BN == 256) {
     if (d->a_major == 0 && d->b_major == 0) KMOE_LAUNCH_PAIR(256, 0, 0);
     else if (d->a_major == 0 && d->b_major == 1) KMOE_LAUNCH_PAIR(256, 0, 1);

@@ -1,4 +1,4 @@
-// Host-side helper: encode a rank-4 bf16 TMA tensor map with 128-byte swizzle through the
+// Host-side helper: encode a rank-4 bf16 TMA tensor map (128-byte swizzle unless told otherwise) through the
 // driver entry point (resolved at run time, so nothing links against libcuda).
 #pragma once
 #include <cuda.h>
@@ -27,7 +27,7 @@ inline EncodeTiledFn get_encode_fn() {
 
 // dims/box innermost first; strides in bytes for dims 1..3.  Returns 0 or a negative code.
 inline int encode_bf16_4d(CUtensorMap* out, const void* base, const cuuint64_t dims[4], const cuuint64_t strides[3],
-                          const cuuint32_t box[4]) {
+                          const cuuint32_t box[4], CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   EncodeTiledFn enc = get_encode_fn();
   if (enc == nullptr) return -10;
   for (int i = 0; i < 3; ++i)
@@ -35,7 +35,7 @@ inline int encode_bf16_4d(CUtensorMap* out, const void* base, const cuuint64_t d
   if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return -13;
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -14;
 }

@@ -127,3 +127,31 @@ def test_loss_vocabulary(B, S, d, V, chunk):
     assert abs(total.item() - ref.item()) < 2e-3 * abs(ref.item())
     for g, w in zip(got, want):
         assert _rel(g, w) < EXPERT_TOL
+
+
+@pytest.mark.parametrize("M,N,G", [(1, 8, 1), (33, 72, 2), (130, 72, 3), (257, 264, 2), (300, 520, 2)])
+@pytest.mark.parametrize("addends", [0, 1, 2])
+def test_output_edges_stay_inside(M, N, G, addends):
+    """Results leave by TMA stores of 32 x 64 blocks: nothing past column N, row M or between the groups is written."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    if addends == 2 and M <= 128:
+        pytest.skip("the second addend exists in the CTA-pair kernel only")
+    K, pitch = 96, N + 24
+    a, b = _rand(G, M, K), _rand(G, N, K)
+    D, D2 = _rand(G, M + 5, pitch), _rand(G, M + 5, pitch)
+    out = torch.full((G, M + 5, pitch), 3.0, dtype=torch.bfloat16, device="cuda")
+    kw = {}
+    if addends:
+        kw.update(D=D, beta=0.5, ldd=pitch)
+    if addends == 2:
+        kw.update(D2=D2, beta2=-1.5)
+    c.gemm(a, b, out, mode=c.BATCHED, groups=G, M=M, N=N, Kd=K, lda=K, ldb=K, ldc=pitch, a_gs=M * K, b_gs=N * K,
+           c_gs=(M + 5) * pitch, **kw)
+    c.check_status()
+    ref = torch.bmm(a.double(), b.double().transpose(1, 2))
+    if addends:
+        ref = ref + 0.5 * D[:, :M, :N].double()
+    if addends == 2:
+        ref = ref - 1.5 * D2[:, :M, :N].double()
+    assert _rel(out[:, :M, :N], ref) < ONE_ROUNDING
+    assert (out[:, M:] == 3.0).all() and (out[:, :, N:] == 3.0).all()
