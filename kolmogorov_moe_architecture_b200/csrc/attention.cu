@@ -294,7 +294,6 @@ teardown:
 // other tile's warpgroup is in its softmax; 128-key steps halve the number of barrier round trips per key.
 constexpr int F2_KEYS = 128;
 constexpr int F2_THREADS = 320;
-constexpr int F2_TILE_BYTES = 2 * PANEL_BYTES;     // 128 rows x 128 bf16 columns, two 64-column panels
 
 // 2^x on the FMA pipe (x <= ~10): round-to-nearest split x = n + f, f in [-0.5, 0.5], cubic for 2^f, exponent
 // added in integer.  Relative error ~1e-4, far below the bf16 rounding of P.  Used for a share of the
@@ -314,7 +313,9 @@ template <int D>
 __global__ void __launch_bounds__(F2_THREADS, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const AttnArgs a) {
-  static_assert(D == 128, "two-tile forward is written for head_dim 128");
+  static_assert(D == 64 || D == 128, "head_dim is one or two 64-column panels");
+  constexpr int NP = D / 64;
+  constexpr int TILE_BYTES = NP * PANEL_BYTES;       // 128 rows x D bf16 columns in 64-column panels
   constexpr uint32_t IDESC_S = make_idesc_f16(128, F2_KEYS, 1, KMOE_MAJOR_K, KMOE_MAJOR_K);
   constexpr uint32_t IDESC_PV = make_idesc_f16(128, D, 1, KMOE_MAJOR_K, KMOE_MAJOR_MN);
   constexpr uint32_t TMEM_COLS = 512;
@@ -323,8 +324,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;                           // 2 tiles
-  uint8_t* sK = sQ + 2 * F2_TILE_BYTES;         // 2 stages
-  uint8_t* sV = sK + 2 * F2_TILE_BYTES;         // 2 stages
+  uint8_t* sK = sQ + 2 * TILE_BYTES;         // 2 stages
+  uint8_t* sV = sK + 2 * TILE_BYTES;         // 2 stages
   __shared__ uint64_t q_full, k_full[2], v_full[2], k_empty[2], v_empty[2], s_full[2], p_full[2], pv_done[2];
   __shared__ uint32_t tmem_slot;
 
@@ -367,32 +368,32 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one() && nblk > 0) {
-      mbar_expect_tx(&q_full, 2 * F2_TILE_BYTES);
+      mbar_expect_tx(&q_full, 2 * TILE_BYTES);
 #pragma unroll
       for (int t = 0; t < 2; ++t)
 #pragma unroll
-        for (int p = 0; p < 2; ++p)
-          tma_load_4d(sQ + t * F2_TILE_BYTES + p * PANEL_BYTES, &tmQ, &q_full, p * 64, h, q0 + t * 128, b);
+        for (int p = 0; p < NP; ++p)
+          tma_load_4d(sQ + t * TILE_BYTES + p * PANEL_BYTES, &tmQ, &q_full, p * 64, h, q0 + t * 128, b);
       for (int j = 0; j < nblk; ++j) {
         const int st = j & 1;
         const uint32_t par = ((j >> 1) & 1) ^ 1;
         if (!mbar_wait(&k_empty[st], par)) { atomicExch(a.status, 31); goto teardown; }
-        mbar_expect_tx(&k_full[st], F2_TILE_BYTES);
+        mbar_expect_tx(&k_full[st], TILE_BYTES);
 #pragma unroll
-        for (int p = 0; p < 2; ++p)
-          tma_load_4d(sK + st * F2_TILE_BYTES + p * PANEL_BYTES, &tmK, &k_full[st], p * 64, hkv, (jlo + j) * F2_KEYS, b);
+        for (int p = 0; p < NP; ++p)
+          tma_load_4d(sK + st * TILE_BYTES + p * PANEL_BYTES, &tmK, &k_full[st], p * 64, hkv, (jlo + j) * F2_KEYS, b);
         if (!mbar_wait(&v_empty[st], par)) { atomicExch(a.status, 32); goto teardown; }
-        mbar_expect_tx(&v_full[st], F2_TILE_BYTES);
+        mbar_expect_tx(&v_full[st], TILE_BYTES);
 #pragma unroll
-        for (int p = 0; p < 2; ++p)
-          tma_load_4d(sV + st * F2_TILE_BYTES + p * PANEL_BYTES, &tmV, &v_full[st], p * 64, hkv, (jlo + j) * F2_KEYS, b);
+        for (int p = 0; p < NP; ++p)
+          tma_load_4d(sV + st * TILE_BYTES + p * PANEL_BYTES, &tmV, &v_full[st], p * 64, hkv, (jlo + j) * F2_KEYS, b);
       }
     }
   } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one() && nblk > 0) {
       auto issue_S = [&](int t, int j) {
-        const uint32_t qa = smem_u32(sQ + t * F2_TILE_BYTES), ka = smem_u32(sK + (j & 1) * F2_TILE_BYTES);
+        const uint32_t qa = smem_u32(sQ + t * TILE_BYTES), ka = smem_u32(sK + (j & 1) * TILE_BYTES);
 #pragma unroll
         for (int k4 = 0; k4 < D / 16; ++k4) {
           const uint32_t off = (k4 >> 2) * PANEL_BYTES + (k4 & 3) * 32;
@@ -420,7 +421,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           if (j >= nb[t]) continue;
           if (!mbar_wait(&p_full[t], j & 1)) { atomicExch(a.status, 37); goto teardown; }
           tc_fence_after();
-          const uint32_t va = smem_u32(sV + st * F2_TILE_BYTES);
+          const uint32_t va = smem_u32(sV + st * TILE_BYTES);
 #pragma unroll
           for (int k4 = 0; k4 < F2_KEYS / 16; ++k4)   // A = P_t from tensor memory: 16 keys = 8 packed columns
             umma_f16_ts(tmem + COL_O + t * 128, tmem + COL_S + t * 128 + k4 * 8,
@@ -570,31 +571,42 @@ struct AttnBwdArgs {
   const int* doc_start;  // optional (B, S), see AttnArgs
 };
 
-// delta[b,h,s] = sum_d dO * O.  One warp per (b,s,h) row.
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                  float* __restrict__ delta, int B, int S, int H, int D) {
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const long long rows = (long long)B * S * H;
-  for (long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; row < rows; row += warps) {
-    const int h = (int)(row % H);
-    const long long bs = row / H;
-    const int s_ = (int)(bs % S);
-    const int b = (int)(bs / S);
-    float acc = 0.f;
-    for (int c = lane * 8; c < D; c += 256) {
-      uint4 r1 = *reinterpret_cast<const uint4*>(o + row * D + c);
-      uint4 r2 = *reinterpret_cast<const uint4*>(d_o + row * D + c);
-      const __nv_bfloat162* p1 = reinterpret_cast<const __nv_bfloat162*>(&r1);
-      const __nv_bfloat162* p2 = reinterpret_cast<const __nv_bfloat162*>(&r2);
+// delta[b,h,s] = sum_d dO * O.  D / 8 lanes per (b,s,h) row (one 16-byte vector of each operand per lane) and four rows
+// per lane in flight: the kernel only has to keep enough loads outstanding to stream O and dO once.  B = 4, S = 2048,
+// 16 x 128: 34.3 us with one row per warp and pass (half of the lanes without work), 14.6 us this way, 10.3 us at
+// the copy rate.
+template <int D>
+__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o,
+                                                         const __nv_bfloat16* __restrict__ d_o,
+                                                         float* __restrict__ delta, long long rows, int S, int H) {
+  constexpr int LPR = D / 8, RPB = 256 / LPR, U = 4;
+  const int sub = threadIdx.x % LPR, r_in = threadIdx.x / LPR;
+  const long long row0 = (long long)blockIdx.x * (RPB * U) + r_in;
+  uint4 x[U], y[U];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float2 f1 = __bfloat1622float2(p1[i]), f2 = __bfloat1622float2(p2[i]);
-        acc += f1.x * f2.x + f1.y * f2.y;
-      }
+  for (int u = 0; u < U; ++u) {
+    const long long row = row0 + u * RPB;
+    const bool ok = row < rows;
+    x[u] = ok ? __ldg(reinterpret_cast<const uint4*>(o + row * D) + sub) : make_uint4(0, 0, 0, 0);
+    y[u] = ok ? __ldg(reinterpret_cast<const uint4*>(d_o + row * D) + sub) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long row = row0 + u * RPB;
+    const __nv_bfloat162* p1 = reinterpret_cast<const __nv_bfloat162*>(&x[u]);
+    const __nv_bfloat162* p2 = reinterpret_cast<const __nv_bfloat162*>(&y[u]);
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f1 = __bfloat1622float2(p1[i]), f2 = __bfloat1622float2(p2[i]);
+      acc += f1.x * f2.x + f1.y * f2.y;
     }
-    acc = warp_sum(acc);
-    if (lane == 0) delta[((size_t)b * H + h) * S + s_] = acc;
+#pragma unroll
+    for (int k = LPR / 2; k > 0; k >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
+    if (sub == 0 && row < rows) {
+      const long long bs = row / H;
+      delta[((bs / S) * H + row % H) * S + bs % S] = acc;
+    }
   }
 }
 
@@ -1017,7 +1029,7 @@ teardown:
   if (warp == 5) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
 }
 
-// ------------------------------------------------- backward for head_dim 128: 128 x 128 steps, P and dS in TMEM
+// ------------------------------------------------- backward: 128 x 128 steps, P and dS in TMEM
 // Both kernels below keep the structure of the two-tile forward: 8 softmax warps (two warpgroups that split the
 // 128 columns of an accumulator in halves; thread = accumulator row), warp 8 is the TMA producer, warp 9 issues
 // the MMAs.  The bf16 operands made by the threads (P^T and dS^T for dK/dV, dS for dQ) are written as packed
@@ -1026,16 +1038,17 @@ teardown:
 // two chains that the tensor pipe interleaves: S -> P (exponentials) and dP -> dS (needs P, kept in
 // registers); while the threads are in one chain the pipe executes the MMAs of the other.
 constexpr int B2_THREADS = 320;
-constexpr int B2_TILE_BYTES = 2 * PANEL_BYTES;     // 128 rows x 128 bf16 columns
 constexpr int DKV2_Q_STAGES = 2;                   // a third stage would not fit beside K, V, two dO stages and the statistics
 
 // dK, dV of one (128-key block, KV head, batch): loops over the query heads of the group and over the
 // 128-query blocks at or after the key block.  TMEM: S^T | dP^T | dV | dK, 128 columns each.
+template <int D>
 __global__ void __launch_bounds__(B2_THREADS, 1)
 attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                      const AttnBwdArgs a) {
-  constexpr int D = 128;
+  constexpr int NP = D / 64;
+  constexpr int TILE_BYTES = NP * PANEL_BYTES;       // 128 rows x D bf16 columns
   constexpr int NQ = DKV2_Q_STAGES;
   constexpr uint32_t IDESC_ST = make_idesc_f16(128, 128, 1, KMOE_MAJOR_K, KMOE_MAJOR_K);
   constexpr uint32_t IDESC_ACC = make_idesc_f16(128, D, 1, KMOE_MAJOR_K, KMOE_MAJOR_MN);
@@ -1044,11 +1057,11 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
-  uint8_t* sV = sK + B2_TILE_BYTES;
+  uint8_t* sV = sK + TILE_BYTES;
   // Q is held until the dK MMAs of its step, the last of the step;
   // dO is released by the dV MMAs in mid-step.
-  uint8_t* sQ = sV + B2_TILE_BYTES;             // NQ stages (with the row statistics)
-  uint8_t* sdO = sQ + NQ * B2_TILE_BYTES;        // 2 stages
+  uint8_t* sQ = sV + TILE_BYTES;             // NQ stages (with the row statistics)
+  uint8_t* sdO = sQ + NQ * TILE_BYTES;        // 2 stages
   __shared__ uint64_t kv_full, q_full[NQ], q_empty[NQ], stat_full[NQ], do_full[2], do_empty[2];
   __shared__ uint64_t st_full, dpt_full, p_full, ds_full, acc_full;
   __shared__ uint32_t tmem_slot;
@@ -1090,9 +1103,9 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (warp == 8) {
     // ------------------------------------------------------------------ producer: tiles by TMA, row statistics
     if (elect_one()) {
-      mbar_expect_tx(&kv_full, 2 * B2_TILE_BYTES);
+      mbar_expect_tx(&kv_full, 2 * TILE_BYTES);
 #pragma unroll
-      for (int p = 0; p < 2; ++p) {
+      for (int p = 0; p < NP; ++p) {
         tma_load_4d(sK + p * PANEL_BYTES, &tmK, &kv_full, p * 64, hkv, k0, b);
         tma_load_4d(sV + p * PANEL_BYTES, &tmV, &kv_full, p * 64, hkv, k0, b);
       }
@@ -1106,10 +1119,10 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (!mbar_wait(&q_empty[qs], ((it / NQ) & 1) ^ 1)) { if (lane == 0) atomicExch(a.status, 41); goto teardown; }
       __syncwarp();
       if (elect_one()) {
-        mbar_expect_tx(&q_full[qs], B2_TILE_BYTES);
+        mbar_expect_tx(&q_full[qs], TILE_BYTES);
 #pragma unroll
-        for (int p = 0; p < 2; ++p)
-          tma_load_4d(sQ + qs * B2_TILE_BYTES + p * PANEL_BYTES, &tmQ, &q_full[qs], p * 64, h, qrow, b);
+        for (int p = 0; p < NP; ++p)
+          tma_load_4d(sQ + qs * TILE_BYTES + p * PANEL_BYTES, &tmQ, &q_full[qs], p * 64, h, qrow, b);
       }
       __syncwarp();
 #pragma unroll
@@ -1126,10 +1139,10 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (!mbar_wait(&do_empty[os], ((it >> 1) & 1) ^ 1)) { if (lane == 0) atomicExch(a.status, 40); goto teardown; }
       __syncwarp();
       if (elect_one()) {
-        mbar_expect_tx(&do_full[os], B2_TILE_BYTES);
+        mbar_expect_tx(&do_full[os], TILE_BYTES);
 #pragma unroll
-        for (int p = 0; p < 2; ++p)
-          tma_load_4d(sdO + os * B2_TILE_BYTES + p * PANEL_BYTES, &tmdO, &do_full[os], p * 64, h, qrow, b);
+        for (int p = 0; p < NP; ++p)
+          tma_load_4d(sdO + os * TILE_BYTES + p * PANEL_BYTES, &tmdO, &do_full[os], p * 64, h, qrow, b);
       }
       __syncwarp();
     }
@@ -1165,7 +1178,7 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       umma_commit(&dpt_full);
       for (int it = 0; it < niter; ++it) {
         const int qs = it % NQ, qn = (it + 1) % NQ, os = it & 1, on = os ^ 1;
-        const uint32_t qa = smem_u32(sQ + qs * B2_TILE_BYTES), da = smem_u32(sdO + os * B2_TILE_BYTES);
+        const uint32_t qa = smem_u32(sQ + qs * TILE_BYTES), da = smem_u32(sdO + os * TILE_BYTES);
         // chain 1: P^T(it) -> dV, then S^T(it + 1) over the same columns (in order behind the dV MMAs)
         if (!mbar_wait(&p_full, it & 1)) { atomicExch(a.status, 44); goto teardown; }
         tc_fence_after();
@@ -1174,7 +1187,7 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (it + 1 < niter) {
           if (!mbar_wait(&q_full[qn], ((it + 1) / NQ) & 1)) { atomicExch(a.status, 45); goto teardown; }
           tc_fence_after();
-          issue_t(COL_ST, ka, smem_u32(sQ + qn * B2_TILE_BYTES));
+          issue_t(COL_ST, ka, smem_u32(sQ + qn * TILE_BYTES));
           umma_commit(&st_full);
         }
         // chain 2: dS^T(it) -> dK, then dP^T(it + 1)
@@ -1185,7 +1198,7 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (it + 1 < niter) {
           if (!mbar_wait(&do_full[on], ((it + 1) >> 1) & 1)) { atomicExch(a.status, 45); goto teardown; }
           tc_fence_after();
-          issue_t(COL_DPT, va, smem_u32(sdO + on * B2_TILE_BYTES));
+          issue_t(COL_DPT, va, smem_u32(sdO + on * TILE_BYTES));
           umma_commit(&dpt_full);
         }
       }
@@ -1267,13 +1280,13 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tc_fence_after();
     }
     const bool row_ok = kj < a.S;
-    const size_t off = (((size_t)b * a.S + (row_ok ? kj : 0)) * a.Hkv + hkv) * D + cb;
+    const size_t off = (((size_t)b * a.S + (row_ok ? kj : 0)) * a.Hkv + hkv) * D + wg * (D / 2);
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
       __nv_bfloat16* drow = (which == 0 ? a.dv : a.dk) + off;
-      const uint32_t col0 = (which == 0 ? COL_DV : COL_DK) + cb;
+      const uint32_t col0 = (which == 0 ? COL_DV : COL_DK) + wg * (D / 2);
 #pragma unroll 1
-      for (int c = 0; c < 64; c += 32) {
+      for (int c = 0; c < D / 2; c += 32) {
         uint32_t v[32];
         if (niter > 0) {
           tmem_ld_32x32(tmem + lane_base + col0 + c, v);
@@ -1304,11 +1317,13 @@ teardown:
 // dQ of one (128-query block, head, batch): loops over the 128-key blocks the block can see.
 // TMEM: S | dP (two buffers, step parity) | dQ, 128 columns each.  S and dP of step j + 1 are issued as soon as
 // the threads have read S of step j into registers, a whole thread phase ahead of their use.
+template <int D>
 __global__ void __launch_bounds__(B2_THREADS, 1)
 attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     const AttnBwdArgs a) {
-  constexpr int D = 128;
+  constexpr int NP = D / 64;
+  constexpr int TILE_BYTES = NP * PANEL_BYTES;       // 128 rows x D bf16 columns
   constexpr uint32_t IDESC_S = make_idesc_f16(128, 128, 1, KMOE_MAJOR_K, KMOE_MAJOR_K);
   constexpr uint32_t IDESC_DQ = make_idesc_f16(128, D, 1, KMOE_MAJOR_K, KMOE_MAJOR_MN);
   constexpr uint32_t TMEM_COLS = 512, COL_S = 0, COL_DP = 128, COL_DQ = 384;   // dP buffer b at COL_DP + 128 b
@@ -1316,10 +1331,10 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
-  uint8_t* sdO = sQ + B2_TILE_BYTES;
+  uint8_t* sdO = sQ + TILE_BYTES;
   // K is held until the dQ MMAs of its step: a third stage lets the load of step j + 1 start a whole step ahead
-  uint8_t* sK = sdO + B2_TILE_BYTES;            // 3 stages
-  uint8_t* sV = sK + 3 * B2_TILE_BYTES;         // 2 stages
+  uint8_t* sK = sdO + TILE_BYTES;            // 3 stages
+  uint8_t* sV = sK + 3 * TILE_BYTES;         // 2 stages
   __shared__ uint64_t qdo_full, k_full[3], v_full[2], k_empty[3], v_empty[2], s_full, s_free, dp_full[2], ds_full[2], dq_full;
   __shared__ uint32_t tmem_slot;
 
@@ -1351,24 +1366,24 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   if (warp == 8) {
     if (elect_one() && nblk > 0) {
-      mbar_expect_tx(&qdo_full, 2 * B2_TILE_BYTES);
+      mbar_expect_tx(&qdo_full, 2 * TILE_BYTES);
 #pragma unroll
-      for (int p = 0; p < 2; ++p) {
+      for (int p = 0; p < NP; ++p) {
         tma_load_4d(sQ + p * PANEL_BYTES, &tmQ, &qdo_full, p * 64, h, q0, b);
         tma_load_4d(sdO + p * PANEL_BYTES, &tmdO, &qdo_full, p * 64, h, q0, b);
       }
       for (int j = 0; j < nblk; ++j) {
         const int st = j & 1, ks = j % 3;
         if (!mbar_wait(&k_empty[ks], ((j / 3) & 1) ^ 1)) { atomicExch(a.status, 51); goto teardown; }
-        mbar_expect_tx(&k_full[ks], B2_TILE_BYTES);
+        mbar_expect_tx(&k_full[ks], TILE_BYTES);
 #pragma unroll
-        for (int p = 0; p < 2; ++p)
-          tma_load_4d(sK + ks * B2_TILE_BYTES + p * PANEL_BYTES, &tmK, &k_full[ks], p * 64, hkv, (jlo + j) * ATT_BLK, b);
+        for (int p = 0; p < NP; ++p)
+          tma_load_4d(sK + ks * TILE_BYTES + p * PANEL_BYTES, &tmK, &k_full[ks], p * 64, hkv, (jlo + j) * ATT_BLK, b);
         if (!mbar_wait(&v_empty[st], ((j >> 1) & 1) ^ 1)) { atomicExch(a.status, 52); goto teardown; }
-        mbar_expect_tx(&v_full[st], B2_TILE_BYTES);
+        mbar_expect_tx(&v_full[st], TILE_BYTES);
 #pragma unroll
-        for (int p = 0; p < 2; ++p)
-          tma_load_4d(sV + st * B2_TILE_BYTES + p * PANEL_BYTES, &tmV, &v_full[st], p * 64, hkv, (jlo + j) * ATT_BLK, b);
+        for (int p = 0; p < NP; ++p)
+          tma_load_4d(sV + st * TILE_BYTES + p * PANEL_BYTES, &tmV, &v_full[st], p * 64, hkv, (jlo + j) * ATT_BLK, b);
       }
     }
   } else if (warp == 9) {
@@ -1403,9 +1418,9 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           // whose dS(j - 1) the dQ MMAs of step j - 1 (earlier in this pipe) have consumed.
           if (!mbar_wait(&s_free, j & 1)) { atomicExch(a.status, 60); goto teardown; }
           tc_fence_after();
-          issue_t(COL_S, qa, smem_u32(sK + kn * B2_TILE_BYTES));
+          issue_t(COL_S, qa, smem_u32(sK + kn * TILE_BYTES));
           umma_commit(&s_full);
-          issue_t(COL_DP + nx * 128, da, smem_u32(sV + nx * B2_TILE_BYTES));
+          issue_t(COL_DP + nx * 128, da, smem_u32(sV + nx * TILE_BYTES));
           umma_commit(&dp_full[nx]);
           umma_commit(&v_empty[nx]);
         }
@@ -1415,7 +1430,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tc_fence_after();
         // dQ += dS K_j with dS (128 queries x 128 keys, packed bf16) in the step's dP buffer: keys 0-63 in its
         // first 32 columns, keys 64-127 in the 32 columns from column 64
-        const uint32_t ka = smem_u32(sK + ks * B2_TILE_BYTES);
+        const uint32_t ka = smem_u32(sK + ks * TILE_BYTES);
 #pragma unroll
         for (int k4 = 0; k4 < ATT_BLK / 16; ++k4)
           umma_f16_ts(tmem + COL_DQ, tmem + COL_DP + st * 128 + (k4 >> 2) * 64 + (k4 & 3) * 8,
@@ -1495,12 +1510,12 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (!mbar_wait(&dq_full, 0)) { if (lane == 0) atomicExch(a.status, 59); goto teardown; }
       tc_fence_after();
     }
-    __nv_bfloat16* drow = a.dq + (((size_t)b * a.S + (row_ok ? qi : 0)) * a.H + h) * D + cb;
+    __nv_bfloat16* drow = a.dq + (((size_t)b * a.S + (row_ok ? qi : 0)) * a.H + h) * D + wg * (D / 2);
 #pragma unroll 1
-    for (int c = 0; c < 64; c += 32) {
+    for (int c = 0; c < D / 2; c += 32) {
       uint32_t v[32];
       if (nblk > 0) {
-        tmem_ld_32x32(tmem + lane_base + COL_DQ + cb + c, v);
+        tmem_ld_32x32(tmem + lane_base + COL_DQ + wg * (D / 2) + c, v);
         tmem_ld_wait();
       } else {
 #pragma unroll
@@ -1553,10 +1568,11 @@ static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const C
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
+template <int D>
 static int launch_attn_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a,
                             cudaStream_t st) {
-  const int smem = 6 * F2_TILE_BYTES + 1024;
-  auto kern = attn_fwd2_kernel<128>;
+  const int smem = 6 * (D / 64) * PANEL_BYTES + 1024;
+  auto kern = attn_fwd2_kernel<D>;
   static bool attr = false;
   if (!attr) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
@@ -1584,10 +1600,10 @@ extern "C" int kmoe_attn_fwd(const void* q, const void* k, const void* v, void* 
     const char* e = getenv("KMOE_ATTN_FWD2");
     fwd2 = (e != nullptr && e[0] == '0') ? 0 : 1;
   }
-  if (D == 128 && fwd2 == 1) {
+  if (fwd2 == 1) {
     if ((rc = make_bshd_tmap(&tk, k, B, S, Hkv, D, F2_KEYS))) return rc;
     if ((rc = make_bshd_tmap(&tv, v, B, S, Hkv, D, F2_KEYS))) return rc;
-    return launch_attn_fwd2(tq, tk, tv, a, st);
+    return D == 128 ? launch_attn_fwd2<128>(tq, tk, tv, a, st) : launch_attn_fwd2<64>(tq, tk, tv, a, st);
   }
   if ((rc = make_bshd_tmap(&tk, k, B, S, Hkv, D, FWD_BN))) return rc;
   if ((rc = make_bshd_tmap(&tv, v, B, S, Hkv, D, FWD_BN))) return rc;
@@ -1623,28 +1639,28 @@ static int launch_attn_bwd(const void* q, const void* k, const void* v, const vo
   // head_dim 128: 128 x 128 steps with P / dS in tensor memory.  KMOE_ATTN_BWD2=0 keeps the 64-wide kernels,
   // =dq / =dkv moves only that kernel.
   static int bwd2 = -1;
-  constexpr int smem2 = 7 * B2_TILE_BYTES + 1024, smem_dkv2 = (4 + DKV2_Q_STAGES) * B2_TILE_BYTES + 1024;
+  constexpr int smem2 = 7 * NP * PANEL_BYTES + 1024, smem_dkv2 = (4 + DKV2_Q_STAGES) * NP * PANEL_BYTES + 1024;
   if (bwd2 < 0) {
     const char* e = getenv("KMOE_ATTN_BWD2");
     int mode = 3;
     if (e != nullptr && e[0] == '0') mode = 0;
     else if (e != nullptr && e[0] == 'd' && e[1] == 'q') mode = 1;
     else if (e != nullptr && e[0] == 'd' && e[1] == 'k') mode = 2;
-    if (D == 128 && mode != 0) {
-      if (cudaFuncSetAttribute(attn_bwd_dq2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) !=
+    if (mode != 0) {
+      if (cudaFuncSetAttribute(attn_bwd_dq2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) !=
               cudaSuccess ||
-          cudaFuncSetAttribute(attn_bwd_dkv2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dkv2) !=
+          cudaFuncSetAttribute(attn_bwd_dkv2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dkv2) !=
               cudaSuccess)
         return -20;
     }
     bwd2 = mode;
   }
-  if (D == 128 && (bwd2 & 1))
-    attn_bwd_dq2_kernel<<<dim3(a.H, a.B, nb), B2_THREADS, smem2, st>>>(tq128, tdo128, tk128, tv128, a);
+  if (bwd2 & 1)
+    attn_bwd_dq2_kernel<D><<<dim3(a.H, a.B, nb), B2_THREADS, smem2, st>>>(tq128, tdo128, tk128, tv128, a);
   else
     k1<<<dim3(nb, a.H, a.B), ATT_THREADS, smem_dq, st>>>(tq128, tdo128, tk64, tv64, a);
-  if (D == 128 && (bwd2 & 2))
-    attn_bwd_dkv2_kernel<<<dim3(a.Hkv, a.B, nb), B2_THREADS, smem_dkv2, st>>>(tq128, tdo128, tk128, tv128, a);
+  if (bwd2 & 2)
+    attn_bwd_dkv2_kernel<D><<<dim3(a.Hkv, a.B, nb), B2_THREADS, smem_dkv2, st>>>(tq128, tdo128, tk128, tv128, a);
   else
     k2<<<dim3(nb, a.Hkv, a.B), ATT_THREADS, smem_dkv, st>>>(tq64, tdo64, tk128, tv128, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
@@ -1658,7 +1674,14 @@ extern "C" int kmoe_attn_bwd(const void* q, const void* k, const void* v, const 
   using namespace kmoe;
   if (D != 64 && D != 128) return -1;
   if (H % Hkv) return -2;
-  attn_delta_kernel<<<148 * 4, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, B, S, H, D);
+  const long long rows = (long long)B * S * H;
+  if (rows == 0) return 0;
+  const int rows_per_block = 4 * 256 / (D / 8);
+  const unsigned dgrid = (unsigned)((rows + rows_per_block - 1) / rows_per_block);
+  if (D == 128)
+    attn_delta_kernel<128><<<dgrid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, rows, S, H);
+  else
+    attn_delta_kernel<64><<<dgrid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, rows, S, H);
   AttnBwdArgs a{B, S, H, Hkv, scale, scale * 1.4426950408889634f, lse, delta, (__nv_bfloat16*)dq,
                 (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, status, doc_start};
   return D == 128 ? launch_attn_bwd<128>(q, k, v, d_o, a, st) : launch_attn_bwd<64>(q, k, v, d_o, a, st);
