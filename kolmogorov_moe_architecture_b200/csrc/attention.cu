@@ -5,20 +5,18 @@
 // lse [B, H, S] fp32 (natural log).  Query head h reads KV head h / (H / Hkv) directly -
 // K and V are never expanded to H heads.
 //
-// head_dim 128 (the model's): 320-thread CTAs - eight softmax warps in two warpgroups, a TMA producer warp, an
-// MMA warp - and 128-key / 128-query steps.
+// head_dim 64 and 128, 320-thread CTAs - eight softmax warps in two warpgroups, a TMA producer warp, an MMA warp - and
+// 128-key / 128-query steps.
 //   forward   attn_fwd2_kernel: two 128-query tiles per CTA, one per warpgroup; S = Q K^T in TMEM, the score row
 //             is read into registers once, P is written as packed bf16 over the S columns and feeds O += P V as
-//             the A operand from tensor memory; O is rescaled only when the row maximum grew by more than 2^8.
-//   backward  attn_bwd_dq2_kernel (loop over key blocks of a query block) and attn_bwd_dkv2_kernel (loop over
-//             the query heads of the group and their query blocks for a key block); both recompute P from the
-//             saved lse (no atomics, deterministic); the warpgroups split the 128 columns of an accumulator in
-//             halves; P^T / dS^T / dS are packed over consumed accumulator columns and enter the next MMA from
-//             tensor memory.
-// head_dim 64 keeps the earlier kernels (attn_fwd_kernel, attn_bwd_dq_kernel, attn_bwd_dkv_kernel): 192-thread
-// CTAs, one softmax warpgroup (thread = row), 64-wide steps, P / dS staged through swizzled shared memory.
-// In the head_dim-128 kernels the tile index is the slowest grid dimension, so the heavy tiles of all heads run
-// first.
+//             the A operand from tensor memory; O stays in TMEM and is rescaled only when the row maximum grew by
+//             more than 2^8.
+//   backward  attn_stats_kernel (row statistics), attn_bwd_dq2_kernel (loop over key blocks of a query block) and
+//             attn_bwd_dkv2_kernel (loop over the query heads of the group and their query blocks for a key block);
+//             both recompute P from the saved lse (no atomics, deterministic); the warpgroups split the 128 columns of
+//             an accumulator in halves; P^T / dS^T / dS are packed over consumed accumulator columns and enter the next
+//             MMA from tensor memory.
+// The tile index is the slowest grid dimension, so the heavy tiles of all heads run first.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -35,7 +33,6 @@ namespace kmoe {
 
 constexpr int ATT_BLK = 128;             // query rows per CTA and keys per step
 constexpr int PANEL_BYTES = ATT_BLK * 128;  // one 64-column bf16 panel of a 128-row tile
-constexpr int ATT_THREADS = 192;
 
 struct AttnArgs {
   int B, S, H, Hkv;
@@ -48,239 +45,7 @@ struct AttnArgs {
   const int* doc_start;
 };
 
-// Byte offset of the 16-byte chunk holding (row, col..col+7) in a K-major 128B-swizzled tile
-// made of 64-column panels.
-__device__ __forceinline__ uint32_t swz_kmajor(int row, int col) {
-  const int panel = col >> 6;
-  const int chunk = (col & 63) >> 3;
-  return panel * PANEL_BYTES + row * 128 + ((chunk ^ (row & 7)) << 4);
-}
-
-// 16-byte chunk offset inside a [rows x 64] K-major swizzled panel
-__device__ __forceinline__ uint32_t swz64(int row, int col) { return row * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4); }
-
-constexpr int FWD_BN = 64;                         // keys per forward step
-constexpr int FWD_KPANEL = FWD_BN * 128;           // 64 key rows x 64 bf16 columns
 constexpr float RESCALE_THRESHOLD = 8.0f;          // log2 units: rescale O only when the row max grew by > 2^8
-
-// Forward.  O stays in TMEM across the whole KV loop (the PV MMA accumulates into it); the running
-// maximum used for the exponent is only advanced - and O rescaled in place - when the true row
-// maximum has grown by more than RESCALE_THRESHOLD, so most steps never touch O.  64-key steps keep
-// the footprint at 112 KB of shared memory and 256 TMEM columns: two CTAs share an SM and the
-// softmax of one overlaps the MMAs of the other.
-template <int D>
-__global__ void __launch_bounds__(ATT_THREADS, 2)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                const __grid_constant__ CUtensorMap tmV, const AttnArgs a) {
-  constexpr int NP = D / 64;
-  constexpr int QTILE = NP * PANEL_BYTES;       // 128 query rows
-  constexpr int KTILE = NP * FWD_KPANEL;        // 64 key rows
-  constexpr uint32_t IDESC_S = make_idesc_f16(128, FWD_BN, 1, KMOE_MAJOR_K, KMOE_MAJOR_K);
-  constexpr uint32_t IDESC_PV = make_idesc_f16(128, D, 1, KMOE_MAJOR_K, KMOE_MAJOR_MN);
-  constexpr uint32_t TMEM_COLS = 256;
-  constexpr uint32_t COL_S0 = 0, COL_O = 128;
-
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sK = sQ + QTILE;             // 2 stages
-  uint8_t* sV = sK + 2 * KTILE;         // 2 stages
-  uint8_t* sP = sV + 2 * KTILE;         // 128 x 64 bf16, one K-major panel
-  __shared__ uint64_t q_full, k_full[2], v_full[2], k_empty[2], v_empty[2], s_full[2], s_free[2], p_full, pv_full;
-  __shared__ uint32_t tmem_slot;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qb = gridDim.x - 1 - blockIdx.x;  // heavy (late) query blocks first
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int hkv = h / (a.H / a.Hkv);
-  const int q0 = qb * ATT_BLK;
-  const int kmax = min(q0 + ATT_BLK, a.S);
-  // packed documents: key blocks that end before the document of the block's first query are invisible to
-  // every row of the block (document starts do not decrease along the sequence) and are not visited at all
-  const int jlo = a.doc_start != nullptr ? a.doc_start[(size_t)b * a.S + q0] / FWD_BN : 0;
-  const int nblk = (kmax + FWD_BN - 1) / FWD_BN - jlo;       // j below counts visited blocks; key block = jlo + j
-
-  if (threadIdx.x == 0) {
-    mbar_init(&q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1);
-      mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 128);
-    }
-    mbar_init(&p_full, 128);
-    mbar_init(&pv_full, 1);
-    mbar_fence_init();
-    prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV);
-  }
-  if (warp == 5) {
-    tmem_alloc(&tmem_slot, TMEM_COLS);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_slot;
-
-  if (warp == 4) {
-    if (elect_one()) {
-      mbar_expect_tx(&q_full, QTILE);
-#pragma unroll
-      for (int p = 0; p < NP; ++p) tma_load_4d(sQ + p * PANEL_BYTES, &tmQ, &q_full, p * 64, h, q0, b);
-      for (int j = 0; j < nblk; ++j) {
-        const int st = j & 1;
-        const uint32_t par = ((j >> 1) & 1) ^ 1;
-        if (!mbar_wait(&k_empty[st], par)) { atomicExch(a.status, 11); goto teardown; }
-        mbar_expect_tx(&k_full[st], KTILE);
-#pragma unroll
-        for (int p = 0; p < NP; ++p)
-          tma_load_4d(sK + st * KTILE + p * FWD_KPANEL, &tmK, &k_full[st], p * 64, hkv, (jlo + j) * FWD_BN, b);
-        if (!mbar_wait(&v_empty[st], par)) { atomicExch(a.status, 12); goto teardown; }
-        mbar_expect_tx(&v_full[st], KTILE);
-#pragma unroll
-        for (int p = 0; p < NP; ++p)
-          tma_load_4d(sV + st * KTILE + p * FWD_KPANEL, &tmV, &v_full[st], p * 64, hkv, (jlo + j) * FWD_BN, b);
-      }
-    }
-  } else if (warp == 5) {
-    if (elect_one()) {
-      auto issue_S = [&](int j) -> bool {
-        const int st = j & 1;
-        if (!mbar_wait(&k_full[st], (j >> 1) & 1)) return false;
-        if (!mbar_wait(&s_free[st], ((j >> 1) & 1) ^ 1)) return false;
-        tc_fence_after();
-        const uint32_t qa = smem_u32(sQ), ka = smem_u32(sK + st * KTILE);
-#pragma unroll
-        for (int k4 = 0; k4 < D / 16; ++k4) {
-          const uint32_t aoff = (k4 >> 2) * PANEL_BYTES + (k4 & 3) * 32;
-          const uint32_t boff = (k4 >> 2) * FWD_KPANEL + (k4 & 3) * 32;
-          umma_f16(tmem + COL_S0 + st * FWD_BN, make_smem_desc_sw128(qa + aoff, 16, 1024),
-                   make_smem_desc_sw128(ka + boff, 16, 1024), IDESC_S, k4 > 0);
-        }
-        umma_commit(&s_full[st]);
-        umma_commit(&k_empty[st]);
-        return true;
-      };
-      if (!mbar_wait(&q_full, 0)) { atomicExch(a.status, 13); goto teardown; }
-      if (!issue_S(0)) { atomicExch(a.status, 14); goto teardown; }
-      for (int j = 0; j < nblk; ++j) {
-        if (j + 1 < nblk && !issue_S(j + 1)) { atomicExch(a.status, 15); goto teardown; }
-        const int st = j & 1;
-        if (!mbar_wait(&v_full[st], (j >> 1) & 1)) { atomicExch(a.status, 16); goto teardown; }
-        if (!mbar_wait(&p_full, j & 1)) { atomicExch(a.status, 17); goto teardown; }
-        tc_fence_after();
-        const uint32_t pa = smem_u32(sP), va = smem_u32(sV + st * KTILE);
-#pragma unroll
-        for (int k4 = 0; k4 < FWD_BN / 16; ++k4)
-          umma_f16(tmem + COL_O, make_smem_desc_sw128(pa + k4 * 32, 16, 1024),
-                   make_smem_desc_sw128(va + k4 * 16 * 128, FWD_KPANEL, 1024), IDESC_PV, (j > 0 || k4 > 0));
-        umma_commit(&pv_full);
-        umma_commit(&v_empty[st]);
-      }
-    }
-  } else {
-    // ----------------------------------------------------------- softmax warps
-    const int r = warp * 32 + lane;                 // query row within the block
-    const int qi = q0 + r;
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-    float m_used = -INFINITY, l = 0.f;
-    const int qstart = (a.doc_start != nullptr && qi < a.S) ? a.doc_start[(size_t)b * a.S + qi] : 0;
-    for (int j = 0; j < nblk; ++j) {
-      const int st = j & 1;
-      if (!mbar_wait(&s_full[st], (j >> 1) & 1)) { if (lane == 0) atomicExch(a.status, 18); goto teardown; }
-      tc_fence_after();
-      const uint32_t ts = tmem + lane_base + COL_S0 + st * FWD_BN;
-      const int k0 = (jlo + j) * FWD_BN;
-      const bool need_mask = (k0 + FWD_BN > q0) || (k0 + FWD_BN > a.S) || (k0 < qstart);
-      uint32_t sv[FWD_BN];
-      {
-        uint32_t (&lo)[32] = *reinterpret_cast<uint32_t (*)[32]>(&sv[0]);
-        uint32_t (&hi)[32] = *reinterpret_cast<uint32_t (*)[32]>(&sv[32]);
-        tmem_ld_32x32(ts, lo);
-        tmem_ld_32x32(ts + 32, hi);
-        tmem_ld_wait();
-      }
-      tc_fence_before();
-      mbar_arrive(&s_free[st]);          // S_j is in registers: its TMEM buffer may be overwritten
-      float mx = -INFINITY;
-#pragma unroll
-      for (int i = 0; i < FWD_BN; ++i) {
-        float s = __uint_as_float(sv[i]) * a.scale_log2;
-        if (need_mask && (k0 + i > qi || k0 + i >= a.S || k0 + i < qstart)) s = -INFINITY;
-        sv[i] = __float_as_uint(s);
-        mx = fmaxf(mx, s);
-      }
-      const bool grow = mx > m_used + RESCALE_THRESHOLD;      // always true on the first step
-      const float m_new = grow ? mx : m_used;
-      const float alpha = grow ? exp2f(m_used - m_new) : 1.f;
-      // a row that has not met a visible key yet (its document starts in a later block) has m_new = -inf
-      const float m_exp = (m_new == -INFINITY) ? 0.f : m_new;
-      float rs = 0.f;
-      uint32_t pk[FWD_BN / 2];
-#pragma unroll
-      for (int i = 0; i < FWD_BN; i += 2) {
-        const float p0 = exp2f(__uint_as_float(sv[i]) - m_exp), p1 = exp2f(__uint_as_float(sv[i + 1]) - m_exp);
-        rs += p0 + p1;
-        pk[i >> 1] = pack_bf16(p0, p1);
-      }
-      l = l * alpha + rs;
-      m_used = m_new;
-      if (j > 0) {
-        // PV_{j-1} must have retired before P is overwritten or O is rescaled
-        if (!mbar_wait(&pv_full, (j - 1) & 1)) { if (lane == 0) atomicExch(a.status, 19); goto teardown; }
-        tc_fence_after();
-        if (__any_sync(0xffffffffu, grow)) {
-#pragma unroll
-          for (int c = 0; c < D; c += 32) {
-            uint32_t v[32];
-            tmem_ld_32x32(tmem + lane_base + COL_O + c, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-            tmem_st_32x32(tmem + lane_base + COL_O + c, v);
-          }
-          tmem_st_wait();
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < FWD_BN; c += 8)
-        *reinterpret_cast<uint4*>(sP + swz64(r, c)) = make_uint4(pk[c / 2], pk[c / 2 + 1], pk[c / 2 + 2], pk[c / 2 + 3]);
-      fence_async_smem();
-      tc_fence_before();
-      mbar_arrive(&p_full);
-    }
-    if (!mbar_wait(&pv_full, (nblk - 1) & 1)) { if (lane == 0) atomicExch(a.status, 20); goto teardown; }
-    tc_fence_after();
-    const bool row_ok = qi < a.S;
-    const float inv = 1.f / l;
-    __nv_bfloat16* orow = a.out + (((size_t)b * a.S + (row_ok ? qi : 0)) * a.H + h) * D;
-#pragma unroll
-    for (int c = 0; c < D; c += 32) {
-      uint32_t v[32];
-      tmem_ld_32x32(tmem + lane_base + COL_O + c, v);
-      tmem_ld_wait();
-      if (row_ok) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 8)
-          *reinterpret_cast<uint4*>(orow + c + i) =
-              make_uint4(pack_bf16(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv),
-                         pack_bf16(__uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv),
-                         pack_bf16(__uint_as_float(v[i + 4]) * inv, __uint_as_float(v[i + 5]) * inv),
-                         pack_bf16(__uint_as_float(v[i + 6]) * inv, __uint_as_float(v[i + 7]) * inv));
-      }
-    }
-    if (row_ok) a.lse[((size_t)b * a.H + h) * a.S + qi] = (m_used + log2f(l)) * 0.6931471805599453f;
-    tc_fence_before();
-  }
-
-teardown:
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 5) {
-    tc_fence_after();
-    tmem_dealloc(tmem, TMEM_COLS);
-  }
-}
-
 
 // ------------------------------------------------------------ forward, two query tiles per CTA
 // One CTA per SM owns 256 query rows as two 128-row tiles, each with its own softmax warpgroup, S and O
@@ -556,14 +321,12 @@ teardown:
 // ------------------------------------------------------------------- backward
 namespace kmoe {
 
-constexpr int BWD_SUB = 64;                       // keys (dQ kernel) / queries (dK/dV kernel) per step
-constexpr int SUBPANEL_BYTES = BWD_SUB * 128;     // 64 rows x 64 bf16 columns
-
 struct AttnBwdArgs {
   int B, S, H, Hkv;
   float scale, scale_log2;
-  const float* lse;     // [B,H,S]
-  const float* delta;   // [B,H,S]  rowsum(dO * O)
+  int Sp;               // S rounded up to whole 128-row blocks: pitch of the row statistics
+  const float* nlse;    // [B,H,Sp]  -lse * log2(e): the exponent of P is s * scale_log2 + this
+  const float* ndelta;  // [B,H,Sp]  -rowsum(dO * O) * scale: dS = P * (dP * scale + this)
   __nv_bfloat16* dq;    // [B,S,H,D]
   __nv_bfloat16* dk;    // [B,S,Hkv,D]
   __nv_bfloat16* dv;
@@ -571,28 +334,40 @@ struct AttnBwdArgs {
   const int* doc_start;  // optional (B, S), see AttnArgs
 };
 
-// delta[b,h,s] = sum_d dO * O.  D / 8 lanes per (b,s,h) row (one 16-byte vector of each operand per lane) and four rows
-// per lane in flight: the kernel only has to keep enough loads outstanding to stream O and dO once.  B = 4, S = 2048,
-// 16 x 128: 34.3 us with one row per warp and pass (half of the lanes without work), 14.6 us this way, 10.3 us at
-// the copy rate.
+// Row statistics of the backward pass, in the form and place its kernels want them: one row of Sp = whole 128-row
+// blocks per (b, h), so that a block's 128 values are one aligned 512-byte bulk copy; positions past S hold zeros.
+//   nlse = -lse * log2(e),  ndelta = -scale * sum_d dO * O
+// D / 8 lanes per (b, s, h) row (one 16-byte vector of each operand per lane) and four rows per lane in flight: the
+// kernel only has to keep enough loads outstanding to stream O and dO once.  B = 4, S = 2048, 16 x 128: 34.3 us with one
+// row per warp and pass (half of the lanes without work), 17.1 us this way, 10.3 us at the copy rate.
 template <int D>
-__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o,
+__global__ void __launch_bounds__(256) attn_stats_kernel(const __nv_bfloat16* __restrict__ o,
                                                          const __nv_bfloat16* __restrict__ d_o,
-                                                         float* __restrict__ delta, long long rows, int S, int H) {
+                                                         const float* __restrict__ lse, float* __restrict__ nlse,
+                                                         float* __restrict__ ndelta, long long rows, int S, int Sp, int H,
+                                                         float scale) {
   constexpr int LPR = D / 8, RPB = 256 / LPR, U = 4;
   const int sub = threadIdx.x % LPR, r_in = threadIdx.x / LPR;
-  const long long row0 = (long long)blockIdx.x * (RPB * U) + r_in;
+  const long long row0 = (long long)blockIdx.x * (RPB * U) + r_in;      // rows of the padded (B, Sp, H)
   uint4 x[U], y[U];
+  long long at[U];        // place in [B, H, Sp]
+  float ls[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const long long row = row0 + u * RPB;
-    const bool ok = row < rows;
-    x[u] = ok ? __ldg(reinterpret_cast<const uint4*>(o + row * D) + sub) : make_uint4(0, 0, 0, 0);
-    y[u] = ok ? __ldg(reinterpret_cast<const uint4*>(d_o + row * D) + sub) : make_uint4(0, 0, 0, 0);
+    const int h = (int)(row % H);
+    const long long bs = row / H;
+    const int s_ = (int)(bs % Sp);
+    const long long b = bs / Sp;
+    const bool ok = row < rows && s_ < S;
+    const long long src = ((b * S + s_) * H + h) * D;
+    x[u] = ok ? __ldg(reinterpret_cast<const uint4*>(o + src) + sub) : make_uint4(0, 0, 0, 0);
+    y[u] = ok ? __ldg(reinterpret_cast<const uint4*>(d_o + src) + sub) : make_uint4(0, 0, 0, 0);
+    at[u] = row < rows ? (b * H + h) * Sp + s_ : -1;
+    ls[u] = (ok && sub == 0) ? __ldg(lse + (b * H + h) * S + s_) : 0.f;
   }
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    const long long row = row0 + u * RPB;
     const __nv_bfloat162* p1 = reinterpret_cast<const __nv_bfloat162*>(&x[u]);
     const __nv_bfloat162* p2 = reinterpret_cast<const __nv_bfloat162*>(&y[u]);
     float acc = 0.f;
@@ -603,430 +378,11 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
     }
 #pragma unroll
     for (int k = LPR / 2; k > 0; k >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
-    if (sub == 0 && row < rows) {
-      const long long bs = row / H;
-      delta[((bs / S) * H + row % H) * S + bs % S] = acc;
+    if (sub == 0 && at[u] >= 0) {
+      nlse[at[u]] = -ls[u] * 1.4426950408889634f;
+      ndelta[at[u]] = -acc * scale;
     }
   }
-}
-
-
-// dQ for one (128-query block, head, batch): dQ = sum_j dS_j K_j, dS = P * (dO V^T - delta) * scale
-template <int D>
-__global__ void __launch_bounds__(ATT_THREADS, 1)
-attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
-                   const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                   const AttnBwdArgs a) {
-  constexpr int NP = D / 64;
-  constexpr int QTILE = NP * PANEL_BYTES;       // 128 rows
-  constexpr int KTILE = NP * SUBPANEL_BYTES;    // 64 rows
-  constexpr uint32_t IDESC_S = make_idesc_f16(128, BWD_SUB, 1, KMOE_MAJOR_K, KMOE_MAJOR_K);
-  constexpr uint32_t IDESC_DQ = make_idesc_f16(128, D, 1, KMOE_MAJOR_K, KMOE_MAJOR_MN);
-  // S and dP are double buffered in TMEM (buffer = block parity): the MMAs of block j+1 run while the
-  // threads turn block j into dS, and the dQ MMA of block j runs under the softmax of block j+1.
-  constexpr uint32_t TMEM_COLS = 512, COL_S = 0, COL_DP = 64, COL_BUF = 128, COL_DQ = 256;
-
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sdO = sQ + QTILE;
-  uint8_t* sK = sdO + QTILE;          // 2 stages
-  uint8_t* sV = sK + 2 * KTILE;       // 2 stages
-  uint8_t* sdS = sV + 2 * KTILE;      // 128 x 64 bf16
-  __shared__ uint64_t qdo_full, k_full[2], v_full[2], k_empty[2], v_empty[2], sdp_full[2], ds_full, ds_free, dq_full;
-  __shared__ uint32_t tmem_slot;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qb = gridDim.x - 1 - blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int hkv = h / (a.H / a.Hkv);
-  const int q0 = qb * ATT_BLK;
-  const int kmax = min(q0 + ATT_BLK, a.S);
-  const int jlo = a.doc_start != nullptr ? a.doc_start[(size_t)b * a.S + q0] / BWD_SUB : 0;   // see the forward kernel
-  const int nblk = (kmax + BWD_SUB - 1) / BWD_SUB - jlo;
-
-  if (threadIdx.x == 0) {
-    mbar_init(&qdo_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
-    }
-    mbar_init(&sdp_full[0], 1); mbar_init(&sdp_full[1], 1);
-    mbar_init(&ds_full, 128); mbar_init(&ds_free, 1); mbar_init(&dq_full, 1);
-    mbar_fence_init();
-  }
-  if (warp == 5) { tmem_alloc(&tmem_slot, TMEM_COLS); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_slot;
-
-  if (warp == 4) {
-    if (elect_one()) {
-      mbar_expect_tx(&qdo_full, 2 * QTILE);
-#pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        tma_load_4d(sQ + p * PANEL_BYTES, &tmQ, &qdo_full, p * 64, h, q0, b);
-        tma_load_4d(sdO + p * PANEL_BYTES, &tmdO, &qdo_full, p * 64, h, q0, b);
-      }
-      for (int j = 0; j < nblk; ++j) {
-        const int st = j & 1;
-        const uint32_t par = ((j >> 1) & 1) ^ 1;
-        if (!mbar_wait(&k_empty[st], par)) { atomicExch(a.status, 21); goto teardown; }
-        mbar_expect_tx(&k_full[st], KTILE);
-#pragma unroll
-        for (int p = 0; p < NP; ++p)
-          tma_load_4d(sK + st * KTILE + p * SUBPANEL_BYTES, &tmK, &k_full[st], p * 64, hkv, (jlo + j) * BWD_SUB, b);
-        if (!mbar_wait(&v_empty[st], par)) { atomicExch(a.status, 22); goto teardown; }
-        mbar_expect_tx(&v_full[st], KTILE);
-#pragma unroll
-        for (int p = 0; p < NP; ++p)
-          tma_load_4d(sV + st * KTILE + p * SUBPANEL_BYTES, &tmV, &v_full[st], p * 64, hkv, (jlo + j) * BWD_SUB, b);
-      }
-    }
-  } else if (warp == 5) {
-    if (elect_one()) {
-      if (!mbar_wait(&qdo_full, 0)) { atomicExch(a.status, 23); goto teardown; }
-      const uint32_t qa = smem_u32(sQ), da = smem_u32(sdO);
-      // S_j = Q K_j^T and dP_j = dO V_j^T into TMEM buffer j & 1
-      auto issue_sdp = [&](int j) -> bool {
-        const int st = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait(&k_full[st], ph) || !mbar_wait(&v_full[st], ph)) return false;
-        tc_fence_after();
-        const uint32_t ka = smem_u32(sK + st * KTILE), va = smem_u32(sV + st * KTILE);
-        const uint32_t tb = tmem + st * COL_BUF;
-#pragma unroll
-        for (int k4 = 0; k4 < D / 16; ++k4) {
-          const uint32_t aoff = (k4 >> 2) * PANEL_BYTES + (k4 & 3) * 32;
-          const uint32_t boff = (k4 >> 2) * SUBPANEL_BYTES + (k4 & 3) * 32;
-          umma_f16(tb + COL_S, make_smem_desc_sw128(qa + aoff, 16, 1024), make_smem_desc_sw128(ka + boff, 16, 1024),
-                   IDESC_S, k4 > 0);
-        }
-#pragma unroll
-        for (int k4 = 0; k4 < D / 16; ++k4) {
-          const uint32_t aoff = (k4 >> 2) * PANEL_BYTES + (k4 & 3) * 32;
-          const uint32_t boff = (k4 >> 2) * SUBPANEL_BYTES + (k4 & 3) * 32;
-          umma_f16(tb + COL_DP, make_smem_desc_sw128(da + aoff, 16, 1024), make_smem_desc_sw128(va + boff, 16, 1024),
-                   IDESC_S, k4 > 0);
-        }
-        umma_commit(&sdp_full[st]);
-        umma_commit(&v_empty[st]);
-        return true;
-      };
-      if (nblk > 0 && !issue_sdp(0)) { atomicExch(a.status, 24); goto teardown; }
-      for (int j = 0; j < nblk; ++j) {
-        const int st = j & 1;
-        // buffer (j+1)&1 was last read for block j-1, whose dS arrival was awaited in the previous iteration
-        if (j + 1 < nblk && !issue_sdp(j + 1)) { atomicExch(a.status, 24); goto teardown; }
-        if (!mbar_wait(&ds_full, j & 1)) { atomicExch(a.status, 25); goto teardown; }
-        tc_fence_after();
-        const uint32_t sa = smem_u32(sdS);
-        const uint32_t ka = smem_u32(sK + st * KTILE);
-#pragma unroll
-        for (int k4 = 0; k4 < BWD_SUB / 16; ++k4)
-          umma_f16(tmem + COL_DQ, make_smem_desc_sw128(sa + k4 * 32, 16, 1024),
-                   make_smem_desc_sw128(ka + k4 * 16 * 128, SUBPANEL_BYTES, 1024), IDESC_DQ, (j > 0 || k4 > 0));
-        umma_commit(&ds_free);
-        umma_commit(&k_empty[st]);
-      }
-      umma_commit(&dq_full);
-    }
-  } else {
-    const int r = warp * 32 + lane;
-    const int qi = q0 + r;
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-    const bool row_ok = qi < a.S;
-    const size_t stat = ((size_t)b * a.H + h) * a.S + (row_ok ? qi : 0);
-    const float lse2 = a.lse[stat] * 1.4426950408889634f;
-    const float dlt = a.delta[stat];
-    const int qstart = (a.doc_start != nullptr && row_ok) ? a.doc_start[(size_t)b * a.S + qi] : 0;
-    for (int j = 0; j < nblk; ++j) {
-      if (!mbar_wait(&sdp_full[j & 1], (j >> 1) & 1)) { if (lane == 0) atomicExch(a.status, 26); goto teardown; }
-      const uint32_t tbuf = tmem + lane_base + (j & 1) * COL_BUF;
-      tc_fence_after();
-      const int k0 = (jlo + j) * BWD_SUB;
-      // only blocks that touch the diagonal, the sequence end or a document start need per-element tests; the
-      // tests live in their own branch, off the common path (instruction-cache footprint)
-      const bool need_mask = (k0 + BWD_SUB > q0) || (k0 + BWD_SUB > a.S) || (k0 < qstart) || !row_ok;
-      uint32_t ds_packed[BWD_SUB / 2];
-#pragma unroll
-      for (int c = 0; c < BWD_SUB; c += 32) {        // two chunks: unrolled so the packed results stay in registers
-        uint32_t sv[32], dv_[32];
-        tmem_ld_32x32(tbuf + COL_S + c, sv);
-        tmem_ld_32x32(tbuf + COL_DP + c, dv_);
-        tmem_ld_wait();
-        if (need_mask) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int kj = k0 + c + i;
-            if ((kj > qi) || (kj >= a.S) || !row_ok || (kj < qstart)) sv[i] = 0xff800000u;   // -inf: p = 0
-          }
-        }
-        uint32_t* dsp = &ds_packed[c >> 1];
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float p0 = exp2f(fmaf(__uint_as_float(sv[i]), a.scale_log2, -lse2));
-          const float p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), a.scale_log2, -lse2));
-          dsp[i >> 1] = pack_bf16(p0 * (__uint_as_float(dv_[i]) - dlt) * a.scale,
-                                  p1 * (__uint_as_float(dv_[i + 1]) - dlt) * a.scale);
-        }
-      }
-      tc_fence_before();
-      if (!mbar_wait(&ds_free, (j & 1) ^ 1)) { if (lane == 0) atomicExch(a.status, 27); goto teardown; }
-#pragma unroll
-      for (int c = 0; c < BWD_SUB; c += 8)
-        *reinterpret_cast<uint4*>(sdS + swz64(r, c)) =
-            make_uint4(ds_packed[c / 2], ds_packed[c / 2 + 1], ds_packed[c / 2 + 2], ds_packed[c / 2 + 3]);
-      fence_async_smem();
-      mbar_arrive(&ds_full);
-    }
-    if (!mbar_wait(&dq_full, 0)) { if (lane == 0) atomicExch(a.status, 28); goto teardown; }
-    tc_fence_after();
-    __nv_bfloat16* drow = a.dq + (((size_t)b * a.S + (row_ok ? qi : 0)) * a.H + h) * D;
-#pragma unroll
-    for (int c = 0; c < D; c += 32) {
-      uint32_t v[32];
-      tmem_ld_32x32(tmem + lane_base + COL_DQ + c, v);
-      tmem_ld_wait();
-      if (row_ok) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 8)
-          *reinterpret_cast<uint4*>(drow + c + i) =
-              make_uint4(pack_bf16(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
-                         pack_bf16(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])),
-                         pack_bf16(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5])),
-                         pack_bf16(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7])));
-      }
-    }
-    tc_fence_before();
-  }
-teardown:
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 5) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
-}
-
-// dK, dV for one (128-key block, KV head, batch): loops over the query heads of the group and the
-// 64-query blocks at or after the key block.
-template <int D>
-__global__ void __launch_bounds__(ATT_THREADS, 1)
-attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
-                    const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                    const AttnBwdArgs a) {
-  constexpr int NP = D / 64;
-  constexpr int KTILE = NP * PANEL_BYTES;       // 128 key rows
-  constexpr int QTILE = NP * SUBPANEL_BYTES;    // 64 query rows
-  constexpr uint32_t IDESC_ST = make_idesc_f16(128, BWD_SUB, 1, KMOE_MAJOR_K, KMOE_MAJOR_K);
-  constexpr uint32_t IDESC_ACC = make_idesc_f16(128, D, 1, KMOE_MAJOR_K, KMOE_MAJOR_MN);
-  // S^T and dP^T are double buffered in TMEM (buffer = iteration parity) so that the MMAs of iteration it+1
-  // run while the threads turn iteration it into P^T / dS^T, and the dV / dK MMAs run under the next softmax.
-  constexpr uint32_t TMEM_COLS = 512, COL_ST = 0, COL_DPT = 64, COL_BUF = 128, COL_DV = 256, COL_DK = 384;
-
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sK = smem;
-  uint8_t* sV = sK + KTILE;
-  uint8_t* sQ = sV + KTILE;            // 2 stages
-  uint8_t* sdO = sQ + 2 * QTILE;       // 2 stages
-  uint8_t* sPT = sdO + 2 * QTILE;      // 128 x 64
-  uint8_t* sdST = sPT + ATT_BLK * 128; // 128 x 64
-  __shared__ uint64_t kv_full, q_full[2], q_empty[2], st_full[2], pds_full, pds_free, acc_full;
-  __shared__ uint32_t tmem_slot;
-  __shared__ float s_lse[BWD_SUB], s_delta[BWD_SUB];
-  __shared__ int s_start[BWD_SUB];
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kb = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
-  const int G = a.H / a.Hkv;
-  const int k0 = kb * ATT_BLK;
-  const int qblk0 = k0 / BWD_SUB;
-  const int qblk1 = (a.S + BWD_SUB - 1) / BWD_SUB;
-  int per_head = qblk1 - qblk0;
-  if (a.doc_start != nullptr) {
-    // packed documents: once a query block starts in a document that begins after this key block's last key,
-    // it and all later query blocks cannot see the block (document starts do not decrease along the sequence)
-    const int klast = min(k0 + ATT_BLK, a.S) - 1;
-    for (int i = 1; i < per_head; ++i) {
-      if (a.doc_start[(size_t)b * a.S + (qblk0 + i) * BWD_SUB] > klast) { per_head = i; break; }
-    }
-  }
-  const int niter = per_head * G;
-
-  if (threadIdx.x == 0) {
-    mbar_init(&kv_full, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
-    mbar_init(&st_full[0], 1); mbar_init(&st_full[1], 1);
-    mbar_init(&pds_full, 128); mbar_init(&pds_free, 1); mbar_init(&acc_full, 1);
-    mbar_fence_init();
-  }
-  if (warp == 5) { tmem_alloc(&tmem_slot, TMEM_COLS); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_slot;
-
-  if (warp == 4) {
-    if (elect_one()) {
-      mbar_expect_tx(&kv_full, 2 * KTILE);
-#pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        tma_load_4d(sK + p * PANEL_BYTES, &tmK, &kv_full, p * 64, hkv, k0, b);
-        tma_load_4d(sV + p * PANEL_BYTES, &tmV, &kv_full, p * 64, hkv, k0, b);
-      }
-      for (int it = 0; it < niter; ++it) {
-        const int st = it & 1;
-        const int h = hkv * G + it / per_head;
-        const int qrow = (qblk0 + it % per_head) * BWD_SUB;
-        if (!mbar_wait(&q_empty[st], ((it >> 1) & 1) ^ 1)) { atomicExch(a.status, 31); goto teardown; }
-        mbar_expect_tx(&q_full[st], 2 * QTILE);
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          tma_load_4d(sQ + st * QTILE + p * SUBPANEL_BYTES, &tmQ, &q_full[st], p * 64, h, qrow, b);
-          tma_load_4d(sdO + st * QTILE + p * SUBPANEL_BYTES, &tmdO, &q_full[st], p * 64, h, qrow, b);
-        }
-      }
-    }
-  } else if (warp == 5) {
-    if (elect_one()) {
-      if (!mbar_wait(&kv_full, 0)) { atomicExch(a.status, 32); goto teardown; }
-      const uint32_t ka = smem_u32(sK), va = smem_u32(sV);
-      // S^T = K Q^T and dP^T = V dO^T of iteration `it` into TMEM buffer it & 1
-      auto issue_st = [&](int it) -> bool {
-        const int st = it & 1;
-        if (!mbar_wait(&q_full[st], (it >> 1) & 1)) return false;
-        tc_fence_after();
-        const uint32_t qa = smem_u32(sQ + st * QTILE), da = smem_u32(sdO + st * QTILE);
-        const uint32_t tb = tmem + st * COL_BUF;
-#pragma unroll
-        for (int k4 = 0; k4 < D / 16; ++k4) {
-          const uint32_t aoff = (k4 >> 2) * PANEL_BYTES + (k4 & 3) * 32;
-          const uint32_t boff = (k4 >> 2) * SUBPANEL_BYTES + (k4 & 3) * 32;
-          umma_f16(tb + COL_ST, make_smem_desc_sw128(ka + aoff, 16, 1024), make_smem_desc_sw128(qa + boff, 16, 1024),
-                   IDESC_ST, k4 > 0);
-        }
-#pragma unroll
-        for (int k4 = 0; k4 < D / 16; ++k4) {
-          const uint32_t aoff = (k4 >> 2) * PANEL_BYTES + (k4 & 3) * 32;
-          const uint32_t boff = (k4 >> 2) * SUBPANEL_BYTES + (k4 & 3) * 32;
-          umma_f16(tb + COL_DPT, make_smem_desc_sw128(va + aoff, 16, 1024),
-                   make_smem_desc_sw128(da + boff, 16, 1024), IDESC_ST, k4 > 0);
-        }
-        umma_commit(&st_full[st]);
-        return true;
-      };
-      if (niter > 0 && !issue_st(0)) { atomicExch(a.status, 33); goto teardown; }
-      for (int it = 0; it < niter; ++it) {
-        const int st = it & 1;
-        // TMEM buffer (it+1)&1 was last read for iteration it-1, whose P^T/dS^T arrival was awaited last time;
-        // the Q/dO stage (it+1)&1 is handed back by q_empty after the accumulation MMAs of iteration it-1
-        if (it + 1 < niter && !issue_st(it + 1)) { atomicExch(a.status, 33); goto teardown; }
-        if (!mbar_wait(&pds_full, it & 1)) { atomicExch(a.status, 34); goto teardown; }
-        tc_fence_after();
-        const uint32_t qa = smem_u32(sQ + st * QTILE), da = smem_u32(sdO + st * QTILE);
-        const uint32_t pa = smem_u32(sPT), sa = smem_u32(sdST);
-#pragma unroll
-        for (int k4 = 0; k4 < BWD_SUB / 16; ++k4) {
-          umma_f16(tmem + COL_DV, make_smem_desc_sw128(pa + k4 * 32, 16, 1024),
-                   make_smem_desc_sw128(da + k4 * 16 * 128, SUBPANEL_BYTES, 1024), IDESC_ACC, (it > 0 || k4 > 0));
-          umma_f16(tmem + COL_DK, make_smem_desc_sw128(sa + k4 * 32, 16, 1024),
-                   make_smem_desc_sw128(qa + k4 * 16 * 128, SUBPANEL_BYTES, 1024), IDESC_ACC, (it > 0 || k4 > 0));
-        }
-        umma_commit(&pds_free);
-        umma_commit(&q_empty[st]);
-      }
-      umma_commit(&acc_full);
-    }
-  } else {
-    const int r = warp * 32 + lane;     // key row
-    const int kj = k0 + r;
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-    for (int it = 0; it < niter; ++it) {
-      const int h = hkv * G + it / per_head;
-      const int qrow = (qblk0 + it % per_head) * BWD_SUB;
-      // stage lse / delta of the 64 queries (previous iteration's readers are past their loop:
-      // they arrived on pds_full after their last read, and this point is after waiting st_full)
-      if (!mbar_wait(&st_full[it & 1], (it >> 1) & 1)) { if (lane == 0) atomicExch(a.status, 35); goto teardown; }
-      const uint32_t tbuf = tmem + lane_base + (it & 1) * COL_BUF;
-      tc_fence_after();
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (r < BWD_SUB) {
-        const int qi = qrow + r;
-        const size_t si = ((size_t)b * a.H + h) * a.S + (qi < a.S ? qi : 0);
-        s_lse[r] = a.lse[si] * 1.4426950408889634f;
-        s_delta[r] = a.delta[si];
-        s_start[r] = (a.doc_start != nullptr && qi < a.S) ? a.doc_start[(size_t)b * a.S + qi] : 0;
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      uint32_t pt[BWD_SUB / 2], dst[BWD_SUB / 2];
-      // per-element tests only for query blocks that touch this key block's diagonal, the sequence end or a
-      // document boundary (s_start > first key of the block); the tests live in their own branch
-      bool need_mask = (qrow < k0 + ATT_BLK) || (qrow + BWD_SUB > a.S) || (k0 + ATT_BLK > a.S);
-      if (a.doc_start != nullptr) need_mask = need_mask || (s_start[BWD_SUB - 1] > k0);
-#pragma unroll
-      for (int c = 0; c < BWD_SUB; c += 32) {        // two chunks: unrolled so the packed results stay in registers
-        uint32_t sv[32], dv_[32];
-        tmem_ld_32x32(tbuf + COL_ST + c, sv);
-        tmem_ld_32x32(tbuf + COL_DPT + c, dv_);
-        tmem_ld_wait();
-        if (need_mask) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int qi = qrow + c + i;
-            if ((kj > qi) || (qi >= a.S) || (kj >= a.S) || (kj < s_start[c + i])) sv[i] = 0xff800000u;   // p = 0
-          }
-        }
-        uint32_t* ptp = &pt[c >> 1];
-        uint32_t* dsp = &dst[c >> 1];
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float p0 = exp2f(fmaf(__uint_as_float(sv[i]), a.scale_log2, -s_lse[c + i]));
-          const float p1 = exp2f(fmaf(__uint_as_float(sv[i + 1]), a.scale_log2, -s_lse[c + i + 1]));
-          ptp[i >> 1] = pack_bf16(p0, p1);
-          dsp[i >> 1] = pack_bf16(p0 * (__uint_as_float(dv_[i]) - s_delta[c + i]) * a.scale,
-                                  p1 * (__uint_as_float(dv_[i + 1]) - s_delta[c + i + 1]) * a.scale);
-        }
-      }
-      tc_fence_before();
-      if (!mbar_wait(&pds_free, (it & 1) ^ 1)) { if (lane == 0) atomicExch(a.status, 36); goto teardown; }
-#pragma unroll
-      for (int c = 0; c < BWD_SUB; c += 8) {
-        *reinterpret_cast<uint4*>(sPT + swz64(r, c)) = make_uint4(pt[c / 2], pt[c / 2 + 1], pt[c / 2 + 2], pt[c / 2 + 3]);
-        *reinterpret_cast<uint4*>(sdST + swz64(r, c)) =
-            make_uint4(dst[c / 2], dst[c / 2 + 1], dst[c / 2 + 2], dst[c / 2 + 3]);
-      }
-      fence_async_smem();
-      mbar_arrive(&pds_full);
-    }
-    if (!mbar_wait(&acc_full, 0)) { if (lane == 0) atomicExch(a.status, 37); goto teardown; }
-    tc_fence_after();
-    const bool row_ok = kj < a.S;
-    const size_t off = (((size_t)b * a.S + (row_ok ? kj : 0)) * a.Hkv + hkv) * D;
-#pragma unroll
-    for (int which = 0; which < 2; ++which) {
-      __nv_bfloat16* drow = (which == 0 ? a.dv : a.dk) + off;
-      const uint32_t col0 = which == 0 ? COL_DV : COL_DK;
-#pragma unroll
-      for (int c = 0; c < D; c += 32) {
-        uint32_t v[32];
-        tmem_ld_32x32(tmem + lane_base + col0 + c, v);
-        tmem_ld_wait();
-        if (row_ok) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 8)
-            *reinterpret_cast<uint4*>(drow + c + i) =
-                make_uint4(pack_bf16(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
-                           pack_bf16(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])),
-                           pack_bf16(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5])),
-                           pack_bf16(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7])));
-        }
-      }
-    }
-    tc_fence_before();
-  }
-teardown:
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 5) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
 }
 
 // ------------------------------------------------- backward: 128 x 128 steps, P and dS in TMEM
@@ -1038,15 +394,29 @@ teardown:
 // two chains that the tensor pipe interleaves: S -> P (exponentials) and dP -> dS (needs P, kept in
 // registers); while the threads are in one chain the pipe executes the MMAs of the other.
 constexpr int B2_THREADS = 320;
-constexpr int DKV2_Q_STAGES = 2;                   // a third stage would not fit beside K, V, two dO stages and the statistics
+constexpr int DKV2_Q_STAGES = 3;
+// Shared memory of the dK/dV kernel: K, V, three Q and two dO tiles, the row statistics and the barriers.  At head_dim
+// 128 this is all of an SM's 227 KB but 400 bytes, so the dynamic segment (there is no static one) must start on a 1 KB
+// boundary by itself; the kernel checks that.
+template <int D>
+constexpr int dkv2_smem_bytes() { return 7 * (D / 64) * PANEL_BYTES + 5 * 512 + 256; }
 
 // dK, dV of one (128-key block, KV head, batch): loops over the query heads of the group and over the
 // 128-query blocks at or after the key block.  TMEM: S^T | dP^T | dV | dK, 128 columns each.
+//
+// The loads of a step (Q and its ndelta, dO and its nlse) are TMA / bulk copies issued by one thread.  Q is held until
+// the dK MMAs, the last of a step: with two stages (and the statistics loaded by the producer warp itself) the loads of
+// step i + 2 started a load latency before their use, which cost 0.3 us
+// per step (4x2048x16/4: 142 -> 123 us).
+//
+// The key blocks of a KV head are few when the batch is small, and the first of them visits every query block of every
+// head of the group.  A cluster of `split` CTAs shares a key block then, each taking 1 / split of the group's heads;
+// the partial sums meet in shared memory (fp32, fixed order) and each CTA stores its share of the rows.
 template <int D>
 __global__ void __launch_bounds__(B2_THREADS, 1)
 attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                     const AttnBwdArgs a) {
+                     const AttnBwdArgs a, const int split) {
   constexpr int NP = D / 64;
   constexpr int TILE_BYTES = NP * PANEL_BYTES;       // 128 rows x D bf16 columns
   constexpr int NQ = DKV2_Q_STAGES;
@@ -1054,24 +424,30 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   constexpr uint32_t IDESC_ACC = make_idesc_f16(128, D, 1, KMOE_MAJOR_K, KMOE_MAJOR_MN);
   constexpr uint32_t TMEM_COLS = 512, COL_ST = 0, COL_DPT = 128, COL_DV = 256, COL_DK = 384;
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
   uint8_t* sK = smem;
   uint8_t* sV = sK + TILE_BYTES;
-  // Q is held until the dK MMAs of its step, the last of the step;
-  // dO is released by the dV MMAs in mid-step.
-  uint8_t* sQ = sV + TILE_BYTES;             // NQ stages (with the row statistics)
-  uint8_t* sdO = sQ + NQ * TILE_BYTES;        // 2 stages
-  __shared__ uint64_t kv_full, q_full[NQ], q_empty[NQ], stat_full[NQ], do_full[2], do_empty[2];
-  __shared__ uint64_t st_full, dpt_full, p_full, ds_full, acc_full;
-  __shared__ uint32_t tmem_slot;
-  __shared__ __align__(16) float s_lse[NQ][128], s_delta[NQ][128];   // -lse * log2(e), -delta * scale
-  __shared__ __align__(16) int s_start[NQ][128];
+  uint8_t* sQ = sV + TILE_BYTES;                 // NQ stages
+  uint8_t* sdO = sQ + NQ * TILE_BYTES;           // 2 stages, released by the dV MMAs in mid-step
+  float(*s_ndelta)[128] = reinterpret_cast<float(*)[128]>(sdO + 2 * TILE_BYTES);   // one row per Q stage
+  float(*s_nlse)[128] = s_ndelta + NQ;                                             // one row per dO stage
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_nlse + 2);
+  uint64_t &kv_full = bars[0], &st_full = bars[1], &dpt_full = bars[2], &p_full = bars[3], &ds_full = bars[4],
+           &acc_full = bars[5];
+  uint64_t *q_full = bars + 6, *q_empty = bars + 9, *do_full = bars + 12, *do_empty = bars + 14;
+  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 16);
+  constexpr int PART_PITCH = 2 * D + 4;          // fp32 row of partial sums: conflict-free float4 rows
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (smem_u32(smem) & 1023u) {                  // never: see dkv2_smem_bytes
+    if (threadIdx.x == 0) atomicExch(a.status, 61);
+    return;
+  }
   // the key block is the slowest grid dimension: the heavy (early) key blocks of all heads are scheduled first
-  const int kb = blockIdx.z, hkv = blockIdx.x, b = blockIdx.y;
-  const int G = a.H / a.Hkv;
+  const int kb = blockIdx.z, hkv = blockIdx.x / split, part = blockIdx.x % split, b = blockIdx.y;
+  const int G = a.H / a.Hkv / split;             // query heads of this CTA
+  const int h0 = hkv * (a.H / a.Hkv) + part * G;
   const int k0 = kb * ATT_BLK;
   const int qblk1 = (a.S + ATT_BLK - 1) / ATT_BLK;
   int per_head = qblk1 - kb;
@@ -1087,7 +463,7 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   if (threadIdx.x == 0) {
     mbar_init(&kv_full, 1);
-    for (int i = 0; i < NQ; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); mbar_init(&stat_full[i], 32); }
+    for (int i = 0; i < NQ; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1); }
     mbar_init(&st_full, 1); mbar_init(&dpt_full, 1);
     mbar_init(&p_full, 256); mbar_init(&ds_full, 256); mbar_init(&acc_full, 1);
@@ -1101,50 +477,39 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const uint32_t tmem = tmem_slot;
 
   if (warp == 8) {
-    // ------------------------------------------------------------------ producer: tiles by TMA, row statistics
+    // ------------------------------------------------------------------ producer
     if (elect_one()) {
-      mbar_expect_tx(&kv_full, 2 * TILE_BYTES);
-#pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        tma_load_4d(sK + p * PANEL_BYTES, &tmK, &kv_full, p * 64, hkv, k0, b);
-        tma_load_4d(sV + p * PANEL_BYTES, &tmV, &kv_full, p * 64, hkv, k0, b);
-      }
-    }
-    __syncwarp();
-    for (int it = 0; it < niter; ++it) {
-      const int qs = it % NQ, os = it & 1;
-      const int h = hkv * G + it / per_head;
-      const int qrow = (kb + it % per_head) * ATT_BLK;
-      // the Q stage (tile and statistics) is free once the dK MMAs of step it - 3 have completed
-      if (!mbar_wait(&q_empty[qs], ((it / NQ) & 1) ^ 1)) { if (lane == 0) atomicExch(a.status, 41); goto teardown; }
-      __syncwarp();
-      if (elect_one()) {
-        mbar_expect_tx(&q_full[qs], TILE_BYTES);
+      auto load_q = [&](int it) {
+        const int qs = it % NQ, h = h0 + it / per_head, qrow = (kb + it % per_head) * ATT_BLK;
+        mbar_expect_tx(&q_full[qs], TILE_BYTES + 512);
 #pragma unroll
         for (int p = 0; p < NP; ++p)
           tma_load_4d(sQ + qs * TILE_BYTES + p * PANEL_BYTES, &tmQ, &q_full[qs], p * 64, h, qrow, b);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = lane + 32 * i;
-        const int qi = qrow + r;
-        const size_t si = ((size_t)b * a.H + h) * a.S + (qi < a.S ? qi : 0);
-        s_lse[qs][r] = -a.lse[si] * 1.4426950408889634f;       // the exponent is s * scale_log2 + this
-        s_delta[qs][r] = -a.delta[si] * a.scale;                // dS = P * (dP * scale + this)
-        s_start[qs][r] = (a.doc_start != nullptr && qi < a.S) ? a.doc_start[(size_t)b * a.S + qi] : 0;
-      }
-      mbar_arrive(&stat_full[qs]);
-      // the dO stage is free once the dV MMAs of step it - 2 have completed
-      if (!mbar_wait(&do_empty[os], ((it >> 1) & 1) ^ 1)) { if (lane == 0) atomicExch(a.status, 40); goto teardown; }
-      __syncwarp();
-      if (elect_one()) {
-        mbar_expect_tx(&do_full[os], TILE_BYTES);
+        bulk_load(s_ndelta[qs], a.ndelta + ((size_t)b * a.H + h) * a.Sp + qrow, 512, &q_full[qs]);
+      };
+      auto load_do = [&](int it) {
+        const int os = it & 1, h = h0 + it / per_head, qrow = (kb + it % per_head) * ATT_BLK;
+        mbar_expect_tx(&do_full[os], TILE_BYTES + 512);
 #pragma unroll
         for (int p = 0; p < NP; ++p)
           tma_load_4d(sdO + os * TILE_BYTES + p * PANEL_BYTES, &tmdO, &do_full[os], p * 64, h, qrow, b);
+        bulk_load(s_nlse[os], a.nlse + ((size_t)b * a.H + h) * a.Sp + qrow, 512, &do_full[os]);
+      };
+      mbar_expect_tx(&kv_full, 2 * TILE_BYTES);
+#pragma unroll
+      for (int p = 0; p < NP; ++p) tma_load_4d(sK + p * PANEL_BYTES, &tmK, &kv_full, p * 64, hkv, k0, b);
+      if (niter > 0) load_q(0);
+#pragma unroll
+      for (int p = 0; p < NP; ++p) tma_load_4d(sV + p * PANEL_BYTES, &tmV, &kv_full, p * 64, hkv, k0, b);
+      if (niter > 0) load_do(0);
+      for (int it = 1; it < niter; ++it) {
+        // the Q stage is free once the dK MMAs of step it - 3 have completed, the dO stage once the dV MMAs of step
+        // it - 2 have (those come first)
+        if (!mbar_wait(&q_empty[it % NQ], ((it / NQ) & 1) ^ 1)) { atomicExch(a.status, 41); goto finish; }
+        load_q(it);
+        if (!mbar_wait(&do_empty[it & 1], ((it >> 1) & 1) ^ 1)) { atomicExch(a.status, 40); goto finish; }
+        load_do(it);
       }
-      __syncwarp();
     }
   } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA issuer
@@ -1167,12 +532,12 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           umma_f16_ts(tmem + acc, tmem + col + (k4 >> 2) * 64 + (k4 & 3) * 8,
                       make_smem_desc_sw128(y_base + k4 * 16 * 128, PANEL_BYTES, 1024), IDESC_ACC, (!first || k4 > 0));
       };
-      if (!mbar_wait(&kv_full, 0)) { atomicExch(a.status, 42); goto teardown; }
-      if (!mbar_wait(&q_full[0], 0)) { atomicExch(a.status, 43); goto teardown; }
+      if (!mbar_wait(&kv_full, 0)) { atomicExch(a.status, 42); goto finish; }
+      if (!mbar_wait(&q_full[0], 0)) { atomicExch(a.status, 43); goto finish; }
       tc_fence_after();
       issue_t(COL_ST, ka, smem_u32(sQ));
       umma_commit(&st_full);
-      if (!mbar_wait(&do_full[0], 0)) { atomicExch(a.status, 43); goto teardown; }
+      if (!mbar_wait(&do_full[0], 0)) { atomicExch(a.status, 43); goto finish; }
       tc_fence_after();
       issue_t(COL_DPT, va, smem_u32(sdO));
       umma_commit(&dpt_full);
@@ -1180,23 +545,23 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const int qs = it % NQ, qn = (it + 1) % NQ, os = it & 1, on = os ^ 1;
         const uint32_t qa = smem_u32(sQ + qs * TILE_BYTES), da = smem_u32(sdO + os * TILE_BYTES);
         // chain 1: P^T(it) -> dV, then S^T(it + 1) over the same columns (in order behind the dV MMAs)
-        if (!mbar_wait(&p_full, it & 1)) { atomicExch(a.status, 44); goto teardown; }
+        if (!mbar_wait(&p_full, it & 1)) { atomicExch(a.status, 44); goto finish; }
         tc_fence_after();
         issue_acc(COL_DV, COL_ST, da, it == 0);
         umma_commit(&do_empty[os]);
         if (it + 1 < niter) {
-          if (!mbar_wait(&q_full[qn], ((it + 1) / NQ) & 1)) { atomicExch(a.status, 45); goto teardown; }
+          if (!mbar_wait(&q_full[qn], ((it + 1) / NQ) & 1)) { atomicExch(a.status, 45); goto finish; }
           tc_fence_after();
           issue_t(COL_ST, ka, smem_u32(sQ + qn * TILE_BYTES));
           umma_commit(&st_full);
         }
         // chain 2: dS^T(it) -> dK, then dP^T(it + 1)
-        if (!mbar_wait(&ds_full, it & 1)) { atomicExch(a.status, 46); goto teardown; }
+        if (!mbar_wait(&ds_full, it & 1)) { atomicExch(a.status, 46); goto finish; }
         tc_fence_after();
         issue_acc(COL_DK, COL_DPT, qa, it == 0);
         umma_commit(&q_empty[qs]);
         if (it + 1 < niter) {
-          if (!mbar_wait(&do_full[on], ((it + 1) >> 1) & 1)) { atomicExch(a.status, 45); goto teardown; }
+          if (!mbar_wait(&do_full[on], ((it + 1) >> 1) & 1)) { atomicExch(a.status, 45); goto finish; }
           tc_fence_after();
           issue_t(COL_DPT, va, smem_u32(sdO + on * TILE_BYTES));
           umma_commit(&dpt_full);
@@ -1215,14 +580,16 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t t_dp = tmem + lane_base + COL_DPT + cb;
     const uint64_t sl2 = pack_f32x2(a.scale_log2, a.scale_log2), sc2 = pack_f32x2(a.scale, a.scale);
     for (int it = 0; it < niter; ++it) {
-      const int st = it % NQ;
+      const int qs = it % NQ, os = it & 1;
       const int qrow = (kb + it % per_head) * ATT_BLK;
-      if (!mbar_wait(&stat_full[st], (it / NQ) & 1)) { if (lane == 0) atomicExch(a.status, 47); goto teardown; }
-      if (!mbar_wait(&st_full, it & 1)) { if (lane == 0) atomicExch(a.status, 48); goto teardown; }
+      int last_start = 0;                          // document start of the block's last query
+      if (a.doc_start != nullptr) last_start = __ldg(a.doc_start + (size_t)b * a.S + min(qrow + ATT_BLK, a.S) - 1);
+      if (!mbar_wait(&do_full[os], (it >> 1) & 1)) { if (lane == 0) atomicExch(a.status, 47); goto finish; }
+      if (!mbar_wait(&st_full, it & 1)) { if (lane == 0) atomicExch(a.status, 48); goto finish; }
       tc_fence_after();
       // per-element tests only for steps that touch the diagonal, the sequence end or a document boundary
-      bool need_mask = (qrow < k0 + ATT_BLK) || (qrow + ATT_BLK > a.S) || (k0 + ATT_BLK > a.S);
-      if (a.doc_start != nullptr) need_mask = need_mask || (s_start[st][ATT_BLK - 1] > k0);
+      const bool need_mask =
+          (qrow < k0 + ATT_BLK) || (qrow + ATT_BLK > a.S) || (k0 + ATT_BLK > a.S) || (last_start > k0);
       uint64_t p2[32];                             // P of this thread's 64 queries, fp32 pairs
       {
         uint32_t sv[64];
@@ -1233,14 +600,15 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
           for (int i = 0; i < 64; ++i) {
             const int qi = qrow + cb + i;
-            if ((kj > qi) || (qi >= a.S) || (kj >= a.S) || (kj < s_start[st][cb + i])) sv[i] = 0xff800000u;  // p = 0
+            const int start = (last_start > k0 && qi < a.S) ? __ldg(a.doc_start + (size_t)b * a.S + qi) : 0;
+            if ((kj > qi) || (qi >= a.S) || (kj >= a.S) || (kj < start)) sv[i] = 0xff800000u;  // p = 0
           }
         }
         uint32_t pk[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), sl2,
-                                       *reinterpret_cast<const uint64_t*>(&s_lse[st][cb + 2 * i]));
+                                       *reinterpret_cast<const uint64_t*>(&s_nlse[os][cb + 2 * i]));
           float x0, x1;
           unpack_f32x2(x, x0, x1);
           const float e0 = ex2_approx(x0), e1 = ex2_approx(x1);
@@ -1252,7 +620,8 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&p_full);
-      if (!mbar_wait(&dpt_full, it & 1)) { if (lane == 0) atomicExch(a.status, 49); goto teardown; }
+      if (!mbar_wait(&q_full[qs], (it / NQ) & 1)) { if (lane == 0) atomicExch(a.status, 47); goto finish; }
+      if (!mbar_wait(&dpt_full, it & 1)) { if (lane == 0) atomicExch(a.status, 49); goto finish; }
       tc_fence_after();
       {
         uint32_t dv_[64];
@@ -1264,7 +633,7 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int i = 0; i < 32; ++i) {
           // dS = P * (dP - delta) * scale = P * (dP * scale - delta * scale)
           const uint64_t t = fma_f32x2(pack_f32x2(__uint_as_float(dv_[2 * i]), __uint_as_float(dv_[2 * i + 1])), sc2,
-                                       *reinterpret_cast<const uint64_t*>(&s_delta[st][cb + 2 * i]));
+                                       *reinterpret_cast<const uint64_t*>(&s_ndelta[qs][cb + 2 * i]));
           float d0, d1;
           unpack_f32x2(mul_f32x2(p2[i], t), d0, d1);
           pk[i] = pack_bf16(d0, d1);
@@ -1276,39 +645,88 @@ attn_bwd_dkv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       mbar_arrive(&ds_full);
     }
     if (niter > 0) {
-      if (!mbar_wait(&acc_full, 0)) { if (lane == 0) atomicExch(a.status, 50); goto teardown; }
+      if (!mbar_wait(&acc_full, 0)) { if (lane == 0) atomicExch(a.status, 50); goto finish; }
       tc_fence_after();
     }
-    const bool row_ok = kj < a.S;
-    const size_t off = (((size_t)b * a.S + (row_ok ? kj : 0)) * a.Hkv + hkv) * D + wg * (D / 2);
+    if (split == 1) {
+      const bool row_ok = kj < a.S;
+      const size_t off = (((size_t)b * a.S + (row_ok ? kj : 0)) * a.Hkv + hkv) * D + wg * (D / 2);
 #pragma unroll
-    for (int which = 0; which < 2; ++which) {
-      __nv_bfloat16* drow = (which == 0 ? a.dv : a.dk) + off;
-      const uint32_t col0 = (which == 0 ? COL_DV : COL_DK) + wg * (D / 2);
+      for (int which = 0; which < 2; ++which) {
+        __nv_bfloat16* drow = (which == 0 ? a.dv : a.dk) + off;
+        const uint32_t col0 = (which == 0 ? COL_DV : COL_DK) + wg * (D / 2);
 #pragma unroll 1
-      for (int c = 0; c < D / 2; c += 32) {
-        uint32_t v[32];
-        if (niter > 0) {
-          tmem_ld_32x32(tmem + lane_base + col0 + c, v);
-          tmem_ld_wait();
-        } else {
+        for (int c = 0; c < D / 2; c += 32) {
+          uint32_t v[32];
+          if (niter > 0) {
+            tmem_ld_32x32(tmem + lane_base + col0 + c, v);
+            tmem_ld_wait();
+          } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = 0u;
+            for (int i = 0; i < 32; ++i) v[i] = 0u;
+          }
+          if (row_ok) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 8)
+              *reinterpret_cast<uint4*>(drow + c + i) =
+                  make_uint4(pack_bf16(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
+                             pack_bf16(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])),
+                             pack_bf16(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5])),
+                             pack_bf16(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7])));
+          }
         }
-        if (row_ok) {
+      }
+    } else {
+      // every MMA has completed and every load was consumed: the tiles' memory takes the fp32 rows [dV | dK]
+      float* prow = reinterpret_cast<float*>(smem) + r * PART_PITCH + wg * (D / 2);
 #pragma unroll
-          for (int i = 0; i < 32; i += 8)
-            *reinterpret_cast<uint4*>(drow + c + i) =
-                make_uint4(pack_bf16(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
-                           pack_bf16(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])),
-                           pack_bf16(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5])),
-                           pack_bf16(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7])));
+      for (int which = 0; which < 2; ++which) {
+#pragma unroll 1
+        for (int c = 0; c < D / 2; c += 32) {
+          uint32_t v[32];
+          if (niter > 0) {
+            tmem_ld_32x32(tmem + lane_base + (which == 0 ? COL_DV : COL_DK) + wg * (D / 2) + c, v);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = 0u;
+          }
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<uint4*>(prow + which * D + c + i) = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
         }
       }
     }
     tc_fence_before();
   }
-teardown:
+finish:
+  if (split > 1) {
+    // also on the way out after a wait that ran out: the peers' memory must stay mapped until all have read it
+    __syncthreads();
+    __syncwarp();
+    cluster_sync_all();
+    const int rows = ATT_BLK / split;
+    for (int i = threadIdx.x; i < rows * (2 * D / 8); i += B2_THREADS) {
+      const int rr = part * rows + i / (2 * D / 8), c = (i % (2 * D / 8)) * 8;
+      const float* mine = reinterpret_cast<const float*>(smem) + rr * PART_PITCH + c;
+      float s8[8];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) s8[x] = 0.f;
+      for (int p = 0; p < split; ++p) {
+        const uint32_t addr = map_to_cta(mine, p);
+        float4 v0 = ld_cluster_f4(addr), v1 = ld_cluster_f4(addr + 16);
+        s8[0] += v0.x; s8[1] += v0.y; s8[2] += v0.z; s8[3] += v0.w;
+        s8[4] += v1.x; s8[5] += v1.y; s8[6] += v1.z; s8[7] += v1.w;
+      }
+      if (k0 + rr < a.S) {
+        __nv_bfloat16* dst = (c < D ? a.dv : a.dk) + (((size_t)b * a.S + k0 + rr) * a.Hkv + hkv) * D + (c % D);
+        *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16(s8[0], s8[1]), pack_bf16(s8[2], s8[3]),
+                                                    pack_bf16(s8[4], s8[5]), pack_bf16(s8[6], s8[7]));
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 9) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
@@ -1447,13 +865,12 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int qi = q0 + r;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const bool row_ok = qi < a.S;
-    const size_t stat = ((size_t)b * a.H + h) * a.S + (row_ok ? qi : 0);
-    const float lse2 = a.lse[stat] * 1.4426950408889634f;
-    const float dlt = a.delta[stat];
+    const size_t stat = ((size_t)b * a.H + h) * a.Sp + qi;          // qi < Sp always
+    const float nl = a.nlse[stat], nd = a.ndelta[stat];
     const int qstart = (a.doc_start != nullptr && row_ok) ? a.doc_start[(size_t)b * a.S + qi] : 0;
     const uint32_t t_s = tmem + lane_base + COL_S + cb;
-    const uint64_t sl2 = pack_f32x2(a.scale_log2, a.scale_log2), nlse = pack_f32x2(-lse2, -lse2);
-    const uint64_t sc2 = pack_f32x2(a.scale, a.scale), nds = pack_f32x2(-dlt * a.scale, -dlt * a.scale);
+    const uint64_t sl2 = pack_f32x2(a.scale_log2, a.scale_log2), nlse = pack_f32x2(nl, nl);
+    const uint64_t sc2 = pack_f32x2(a.scale, a.scale), nds = pack_f32x2(nd, nd);
     for (int j = 0; j < nblk; ++j) {
       if (!mbar_wait(&s_full, j & 1)) { if (lane == 0) atomicExch(a.status, 57); goto teardown; }
       tc_fence_after();
@@ -1553,22 +970,6 @@ static int make_bshd_tmap(CUtensorMap* out, const void* base, int B, int S, int 
 }
 
 template <int D>
-static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a,
-                           cudaStream_t st) {
-  constexpr int NP = D / 64;
-  const int smem = NP * PANEL_BYTES + 4 * NP * FWD_KPANEL + ATT_BLK * 128 + 1024;
-  auto kern = attn_fwd_kernel<D>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
-    attr = true;
-  }
-  dim3 grid((a.S + ATT_BLK - 1) / ATT_BLK, a.H, a.B);
-  kern<<<grid, ATT_THREADS, smem, st>>>(tq, tk, tv, a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
-}
-
-template <int D>
 static int launch_attn_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a,
                             cudaStream_t st) {
   const int smem = 6 * (D / 64) * PANEL_BYTES + 1024;
@@ -1591,98 +992,91 @@ extern "C" int kmoe_attn_fwd(const void* q, const void* k, const void* v, void* 
   if (D != 64 && D != 128) return -1;
   if (H % Hkv) return -2;
   CUtensorMap tq, tk, tv;
-  int rc = make_bshd_tmap(&tq, q, B, S, H, D, ATT_BLK);
-  if (rc) return rc;
+  int rc;
+  if ((rc = make_bshd_tmap(&tq, q, B, S, H, D, ATT_BLK))) return rc;
+  if ((rc = make_bshd_tmap(&tk, k, B, S, Hkv, D, F2_KEYS))) return rc;
+  if ((rc = make_bshd_tmap(&tv, v, B, S, Hkv, D, F2_KEYS))) return rc;
   AttnArgs a{B, S, H, Hkv, scale * 1.4426950408889634f, (__nv_bfloat16*)out, lse, status, doc_start};
-  // head_dim 128: two query tiles per CTA, 128-key steps (KMOE_ATTN_FWD2=0 keeps the one-tile kernel)
-  static int fwd2 = -1;
-  if (fwd2 < 0) {
-    const char* e = getenv("KMOE_ATTN_FWD2");
-    fwd2 = (e != nullptr && e[0] == '0') ? 0 : 1;
-  }
-  if (fwd2 == 1) {
-    if ((rc = make_bshd_tmap(&tk, k, B, S, Hkv, D, F2_KEYS))) return rc;
-    if ((rc = make_bshd_tmap(&tv, v, B, S, Hkv, D, F2_KEYS))) return rc;
-    return D == 128 ? launch_attn_fwd2<128>(tq, tk, tv, a, st) : launch_attn_fwd2<64>(tq, tk, tv, a, st);
-  }
-  if ((rc = make_bshd_tmap(&tk, k, B, S, Hkv, D, FWD_BN))) return rc;
-  if ((rc = make_bshd_tmap(&tv, v, B, S, Hkv, D, FWD_BN))) return rc;
-  return D == 128 ? launch_attn_fwd<128>(tq, tk, tv, a, st) : launch_attn_fwd<64>(tq, tk, tv, a, st);
+  return D == 128 ? launch_attn_fwd2<128>(tq, tk, tv, a, st) : launch_attn_fwd2<64>(tq, tk, tv, a, st);
 }
 
 namespace kmoe {
+
+// CTAs that share a key block of the dK/dV kernel: 1, 2 or 4 out of the heads of the group.  Time is counted in steps:
+// the first key block's CTA needs group * nb of them, divided by the split; an SM gets its share of all steps plus about
+// eight for each CTA that it runs (prologue, epilogue, the sum over the cluster).  Measured us for 1 / 2 / 4 CTAs
+// (head_dim 128 unless noted): 4x2048x16/4 123 / 154 / 224, 2x2048x16/4 114 / 78 / 115, 1x2048x16/4 110 / 64 / 58,
+// 4x1024x12/3 64 / 45 / 66, 1x777x12/3 61 / 37 / 27, 8x1021x12/3x64 68 / 79 / 109, 1x64x8/2x64 16 / 14 / 12.
+static int dkv_split(int nb, int Hkv, int B, int group, int sms) {
+  const double ctas = (double)nb * Hkv * B / sms, steps = ctas * group * (nb + 1) / 2.0;
+  int best = 1;
+  double best_t = 1e30;
+  for (int s = 1; s <= 4 && group % s == 0; s *= 2) {
+    const double longest = (double)group * nb / s, share = steps + 8.0 * ctas * s;
+    const double t = longest > share ? longest : share;
+    if (t < best_t) { best_t = t; best = s; }
+  }
+  return best;
+}
+
 template <int D>
 static int launch_attn_bwd(const void* q, const void* k, const void* v, const void* d_o, const AttnBwdArgs& a,
                            cudaStream_t st) {
-  CUtensorMap tq128, tdo128, tk64, tv64, tq64, tdo64, tk128, tv128;
+  CUtensorMap tq, tdo, tk, tv;
   int rc;
-  if ((rc = make_bshd_tmap(&tq128, q, a.B, a.S, a.H, D, 128))) return rc;
-  if ((rc = make_bshd_tmap(&tdo128, d_o, a.B, a.S, a.H, D, 128))) return rc;
-  if ((rc = make_bshd_tmap(&tk64, k, a.B, a.S, a.Hkv, D, 64))) return rc;
-  if ((rc = make_bshd_tmap(&tv64, v, a.B, a.S, a.Hkv, D, 64))) return rc;
-  if ((rc = make_bshd_tmap(&tq64, q, a.B, a.S, a.H, D, 64))) return rc;
-  if ((rc = make_bshd_tmap(&tdo64, d_o, a.B, a.S, a.H, D, 64))) return rc;
-  if ((rc = make_bshd_tmap(&tk128, k, a.B, a.S, a.Hkv, D, 128))) return rc;
-  if ((rc = make_bshd_tmap(&tv128, v, a.B, a.S, a.Hkv, D, 128))) return rc;
-  constexpr int NP = D / 64;
-  const int smem_dq = 2 * NP * PANEL_BYTES + 4 * NP * SUBPANEL_BYTES + ATT_BLK * 128 + 1024;
-  const int smem_dkv = 2 * NP * PANEL_BYTES + 4 * NP * SUBPANEL_BYTES + 2 * ATT_BLK * 128 + 1024;
-  auto k1 = attn_bwd_dq_kernel<D>;
-  auto k2 = attn_bwd_dkv_kernel<D>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dq) != cudaSuccess) return -20;
-    if (cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dkv) != cudaSuccess) return -20;
-    attr = true;
+  if ((rc = make_bshd_tmap(&tq, q, a.B, a.S, a.H, D, ATT_BLK))) return rc;
+  if ((rc = make_bshd_tmap(&tdo, d_o, a.B, a.S, a.H, D, ATT_BLK))) return rc;
+  if ((rc = make_bshd_tmap(&tk, k, a.B, a.S, a.Hkv, D, ATT_BLK))) return rc;
+  if ((rc = make_bshd_tmap(&tv, v, a.B, a.S, a.Hkv, D, ATT_BLK))) return rc;
+  constexpr int smem_dq = 7 * (D / 64) * PANEL_BYTES + 1024, smem_dkv = dkv2_smem_bytes<D>();
+  static int sms = 0;
+  if (sms == 0) {
+    if (cudaFuncSetAttribute(attn_bwd_dq2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dq) != cudaSuccess ||
+        cudaFuncSetAttribute(attn_bwd_dkv2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dkv) != cudaSuccess)
+      return -20;
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    sms = n > 0 ? n : 148;
   }
   const int nb = (a.S + ATT_BLK - 1) / ATT_BLK;
-  // head_dim 128: 128 x 128 steps with P / dS in tensor memory.  KMOE_ATTN_BWD2=0 keeps the 64-wide kernels,
-  // =dq / =dkv moves only that kernel.
-  static int bwd2 = -1;
-  constexpr int smem2 = 7 * NP * PANEL_BYTES + 1024, smem_dkv2 = (4 + DKV2_Q_STAGES) * NP * PANEL_BYTES + 1024;
-  if (bwd2 < 0) {
-    const char* e = getenv("KMOE_ATTN_BWD2");
-    int mode = 3;
-    if (e != nullptr && e[0] == '0') mode = 0;
-    else if (e != nullptr && e[0] == 'd' && e[1] == 'q') mode = 1;
-    else if (e != nullptr && e[0] == 'd' && e[1] == 'k') mode = 2;
-    if (mode != 0) {
-      if (cudaFuncSetAttribute(attn_bwd_dq2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) !=
-              cudaSuccess ||
-          cudaFuncSetAttribute(attn_bwd_dkv2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dkv2) !=
-              cudaSuccess)
-        return -20;
-    }
-    bwd2 = mode;
-  }
-  if (bwd2 & 1)
-    attn_bwd_dq2_kernel<D><<<dim3(a.H, a.B, nb), B2_THREADS, smem2, st>>>(tq128, tdo128, tk128, tv128, a);
-  else
-    k1<<<dim3(nb, a.H, a.B), ATT_THREADS, smem_dq, st>>>(tq128, tdo128, tk64, tv64, a);
-  if (bwd2 & 2)
-    attn_bwd_dkv2_kernel<D><<<dim3(a.Hkv, a.B, nb), B2_THREADS, smem_dkv2, st>>>(tq128, tdo128, tk128, tv128, a);
-  else
-    k2<<<dim3(nb, a.Hkv, a.B), ATT_THREADS, smem_dkv, st>>>(tq64, tdo64, tk128, tv128, a);
+  attn_bwd_dq2_kernel<D><<<dim3(a.H, a.B, nb), B2_THREADS, smem_dq, st>>>(tq, tdo, tk, tv, a);
+  const int split = dkv_split(nb, a.Hkv, a.B, a.H / a.Hkv, sms);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(a.Hkv * split), (unsigned)a.B, (unsigned)nb);
+  cfg.blockDim = dim3(B2_THREADS);
+  cfg.dynamicSmemBytes = smem_dkv;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)split; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, attn_bwd_dkv2_kernel<D>, tq, tdo, tk, tv, a, split) != cudaSuccess) return -21;
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 }  // namespace kmoe
 
-// delta is scratch of B*H*S floats.
+// stats is scratch of 2 * B * H * Sp floats, Sp = S rounded up to 128.
 extern "C" int kmoe_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
-                             const float* lse, float* delta, void* dq, void* dk, void* dv, int B, int S, int H,
+                             const float* lse, float* stats, void* dq, void* dk, void* dv, int B, int S, int H,
                              int Hkv, int D, float scale, const int* doc_start, int* status, cudaStream_t st) {
   using namespace kmoe;
   if (D != 64 && D != 128) return -1;
   if (H % Hkv) return -2;
-  const long long rows = (long long)B * S * H;
+  const int Sp = (S + ATT_BLK - 1) / ATT_BLK * ATT_BLK;
+  const long long rows = (long long)B * Sp * H;
   if (rows == 0) return 0;
+  float *nlse = stats, *ndelta = stats + rows;
   const int rows_per_block = 4 * 256 / (D / 8);
-  const unsigned dgrid = (unsigned)((rows + rows_per_block - 1) / rows_per_block);
+  const unsigned grid = (unsigned)((rows + rows_per_block - 1) / rows_per_block);
   if (D == 128)
-    attn_delta_kernel<128><<<dgrid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, rows, S, H);
+    attn_stats_kernel<128><<<grid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, lse, nlse, ndelta,
+                                                 rows, S, Sp, H, scale);
   else
-    attn_delta_kernel<64><<<dgrid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, delta, rows, S, H);
-  AttnBwdArgs a{B, S, H, Hkv, scale, scale * 1.4426950408889634f, lse, delta, (__nv_bfloat16*)dq,
+    attn_stats_kernel<64><<<grid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, lse, nlse, ndelta,
+                                                rows, S, Sp, H, scale);
+  AttnBwdArgs a{B, S, H, Hkv, scale, scale * 1.4426950408889634f, Sp, nlse, ndelta, (__nv_bfloat16*)dq,
                 (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, status, doc_start};
   return D == 128 ? launch_attn_bwd<128>(q, k, v, d_o, a, st) : launch_attn_bwd<64>(q, k, v, d_o, a, st);
 }

@@ -466,9 +466,9 @@ std::tuple<Tensor, Tensor, Tensor> attn_bwd(const Tensor& q, const Tensor& k, co
   TORCH_CHECK(d_o.is_contiguous() && o.is_contiguous());
   const int B = q.size(0), S = q.size(1), H = q.size(2), D = q.size(3), Hkv = k.size(2);
   Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
-  Tensor delta = at::empty({B, H, S}, lse.options());
+  Tensor stats = at::empty({2, B, H, (S + 127) / 128 * 128}, lse.options());
   check(kmoe_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr<float>(),
-                      delta.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, S, H, Hkv, D,
+                      stats.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, S, H, Hkv, D,
                       (float)scale, doc_ptr(doc_start, B, S), status.data_ptr<int>(), cur_stream()), "attn_bwd");
   return {dq, dk, dv};
 }
