@@ -301,11 +301,22 @@ std::tuple<Tensor, Tensor, Tensor> conv1d_bwd(const Tensor& x, const Tensor& w, 
   return {dx, dw, db};
 }
 
+// B / C of the scan: [B,S,N], both bf16 or both fp32, rows of equal pitch
+inline void check_scan_bc(const Tensor& Bm, const Tensor& Cm) {
+  TORCH_CHECK(Bm.is_cuda() && Bm.scalar_type() == Cm.scalar_type() && Bm.dim() == 3 && Cm.dim() == 3 &&
+              (Bm.scalar_type() == at::kBFloat16 || Bm.scalar_type() == at::kFloat) && row_stride(Bm) == row_stride(Cm),
+              "B and C must be bf16 or fp32 [B,S,N] tensors of one layout");
+}
+inline void need_aligned(const Tensor& t, const char* n) {
+  TORCH_CHECK(t.numel() == 0 || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0, n, " must be 16-byte aligned");
+}
+
 std::tuple<Tensor, Tensor, Tensor> scan_fwd(const Tensor& u, const Tensor& delta, const OptT& z, const Tensor& A,
                                             const Tensor& Bm, const Tensor& Cm, const OptT& D, const OptT& dt_bias,
                                             bool softplus, bool save) {
   c10::cuda::CUDAGuard guard(u.device());
-  need_bf16(u, "u"); need_bf16(delta, "delta"); need_f32(A, "A"); need_f32(Bm, "B"); need_f32(Cm, "C");
+  need_bf16(u, "u"); need_bf16(delta, "delta"); need_f32(A, "A"); check_scan_bc(Bm, Cm);
+  need_aligned(u, "u"); need_aligned(delta, "delta"); need_aligned(A, "A");
   // A [C,N], or [G,C,N] with G parameter sets over the batch (D, dt_bias [G,C] then)
   TORCH_CHECK(u.is_contiguous() && delta.is_contiguous() && u.dim() == 3 && A.is_contiguous());
   const int B = u.size(0), S = u.size(1), C = u.size(2), N = A.size(-1);
@@ -313,14 +324,14 @@ std::tuple<Tensor, Tensor, Tensor> scan_fwd(const Tensor& u, const Tensor& delta
   TORCH_CHECK(A.size(-2) == C && B % G == 0, "A does not match u");
   Tensor out = at::empty_like(u);
   const int nch = (S + kmoe_scan_chunk() - 1) / kmoe_scan_chunk();
-  Tensor ckpt = save ? at::empty({B, nch, N, C}, A.options()) : at::empty({0}, A.options());
+  Tensor ckpt = save ? at::empty({B, nch, C, N}, A.options()) : at::empty({0}, A.options());
   const int P = kmoe_scan_segments(B, S, C);
   Tensor seg = P > 1 ? at::empty({B, P, N + 1, C}, A.options()) : at::empty({0}, A.options());
   const bool has_z = z.has_value() && z->defined();
-  if (has_z) need_bf16(*z, "z");
+  if (has_z) { need_bf16(*z, "z"); need_aligned(*z, "z"); }
   check(kmoe_scan_fwd(u.data_ptr(), delta.data_ptr(), has_z ? z->data_ptr() : nullptr, A.data_ptr<float>(),
-                      Bm.data_ptr<float>(), Cm.data_ptr<float>(), (const float*)ptr_or_null(D),
-                      (const float*)ptr_or_null(dt_bias), out.data_ptr(), save ? ckpt.data_ptr<float>() : nullptr,
+                      Bm.data_ptr(), Cm.data_ptr(), row_stride(Bm), Bm.scalar_type() == at::kBFloat16,
+                      (const float*)ptr_or_null(D), (const float*)ptr_or_null(dt_bias), out.data_ptr(), save ? ckpt.data_ptr<float>() : nullptr,
                       P > 1 ? seg.data_ptr<float>() : nullptr, B, S, C, N, has_z ? row_stride(*z) : 0,
                       softplus ? 1 : 0, G, cur_stream()), "scan_fwd");
   return {out, ckpt, seg};
@@ -330,7 +341,7 @@ std::vector<Tensor> scan_bwd(const Tensor& u, const Tensor& delta, const OptT& z
                              const Tensor& Cm, const OptT& D, const OptT& dt_bias, const Tensor& dout,
                              const Tensor& ckpt, const Tensor& seg, bool softplus) {
   c10::cuda::CUDAGuard guard(u.device());
-  need_bf16(dout, "dout");
+  need_bf16(dout, "dout"); need_aligned(dout, "dout"); check_scan_bc(Bm, Cm);
   TORCH_CHECK(dout.is_contiguous());
   const int B = u.size(0), S = u.size(1), C = u.size(2), N = A.size(-1);
   const int G = A.dim() == 3 ? (int)A.size(0) : 1;
@@ -344,10 +355,10 @@ std::vector<Tensor> scan_bwd(const Tensor& u, const Tensor& delta, const OptT& z
   Tensor dbias = at::zeros_like(dD);
   const int P = kmoe_scan_segments(B, S, C);
   TORCH_CHECK(P == 1 || seg.numel() == (int64_t)B * P * (N + 1) * C, "segment scratch of the forward pass expected");
-  Tensor gseg = P > 1 ? at::empty({B, P, N, C}, f32) : at::empty({0}, f32);
+  Tensor gseg = P > 1 ? at::empty({B, P, C, N}, f32) : at::empty({0}, f32);
   check(kmoe_scan_bwd(u.data_ptr(), delta.data_ptr(), has_z ? z->data_ptr() : nullptr, A.data_ptr<float>(),
-                      Bm.data_ptr<float>(), Cm.data_ptr<float>(), (const float*)ptr_or_null(D),
-                      (const float*)ptr_or_null(dt_bias), dout.data_ptr(), ckpt.data_ptr<float>(),
+                      Bm.data_ptr(), Cm.data_ptr(), row_stride(Bm), Bm.scalar_type() == at::kBFloat16,
+                      (const float*)ptr_or_null(D), (const float*)ptr_or_null(dt_bias), dout.data_ptr(), ckpt.data_ptr<float>(),
                       P > 1 ? seg.data_ptr<float>() : nullptr, P > 1 ? gseg.data_ptr<float>() : nullptr, du.data_ptr(),
                       dd.data_ptr(), has_z ? dz.data_ptr() : nullptr, C, dA.data_ptr<float>(), dB.data_ptr<float>(),
                       dC.data_ptr<float>(), dD.data_ptr<float>(), dbias.data_ptr<float>(), B, S, C, N,

@@ -511,11 +511,26 @@ def causal_conv1d(x, weight, bias, activation=True):
     return _Conv1d.apply(x, weight, bias, bool(activation))
 
 
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t`` itself when its first element sits on a 16-byte boundary, else a copy that does."""
+    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
+def _scan_bc(Bm, Cm):
+    """B and C the way the scan kernel reads them: bf16 column slices of one projection as they are, anything else as
+    contiguous fp32."""
+    if all(_bf16(t) and _rows_ok(t) and t.data_ptr() % 16 == 0 for t in (Bm, Cm)) and Bm.stride(-2) == Cm.stride(-2):
+        return Bm, Cm
+    return Bm.float().contiguous(), Cm.float().contiguous()
+
+
 class _Scan(torch.autograd.Function):
     @staticmethod
     def forward(ctx, u, delta, A, Bm, Cm, D, z, dt_bias, softplus):
-        Af = A.float().contiguous()
-        Bf, Cf = Bm.float().contiguous(), Cm.float().contiguous()
+        u, delta = _aligned(u), _aligned(delta)
+        z = _aligned(z) if z is not None else None
+        Af = _aligned(A.float().contiguous())
+        Bf, Cf = _scan_bc(Bm, Cm)
         Df = D.float().contiguous() if D is not None else None
         bf = dt_bias.float().contiguous() if dt_bias is not None else None
         need = any(ctx.needs_input_grad)
@@ -530,8 +545,8 @@ class _Scan(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         u, delta, z, Af, Bf, Cf, Df, bf, ckpt, seg = ctx.saved_tensors
-        du, dd, dz, dA, dB, dC, dD, dbias = K.scan_bwd(u, delta, z, Af, Bf, Cf, Df, bf, dout.contiguous(),
-                                                       ckpt, seg, ctx.softplus)
+        du, dd, dz, dA, dB, dC, dD, dbias = K.scan_bwd(u, delta, z, Af, Bf, Cf, Df, bf,
+                                                       _aligned(dout.contiguous()), ckpt, seg, ctx.softplus)
         _count(2 if seg.numel() else 1)
         a_dt, b_dt, c_dt, d_dt, bias_dt = ctx.dtypes
         return (du, dd, dA.to(a_dt), dB.to(b_dt), dC.to(c_dt), dD.to(d_dt) if Df is not None else None,

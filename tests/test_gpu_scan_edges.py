@@ -1,0 +1,59 @@
+"""Selective scan where its schedule changes: one and several segments, chunks and channel blocks that end early, B and C as
+column slices of a projection (bf16) and as fp32, with and without gate, bias and skip."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# Results and activation gradients are rounded to bf16 once (1.7e-3 in the 2-norm); ex2.approx and the 32-bit sums add less.
+TOL = 4e-3
+
+
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm().clamp(min=1e-30)).item()
+
+
+def _ref(u, dt, A, Bm, Cm, D, z, bias, softplus):
+    d = dt if bias is None else dt + bias
+    d = torch.nn.functional.softplus(d) if softplus else d
+    h = torch.zeros(u.shape[0], u.shape[2], 16, dtype=u.dtype, device=u.device)
+    ys = []
+    for t in range(u.shape[1]):
+        h = torch.exp(d[:, t, :, None] * A) * h + (d[:, t] * u[:, t])[..., None] * Bm[:, t, None, :]
+        ys.append((h * Cm[:, t, None, :]).sum(-1))
+    y = torch.stack(ys, 1)
+    y = y if D is None else y + u * D
+    return y if z is None else y * torch.nn.functional.silu(z)
+
+
+@pytest.mark.parametrize("B,S,C,form,gate", [
+    (1, 1, 8, "slice", True), (2, 7, 72, "float", True), (1, 8, 64, "slice", False), (3, 9, 136, "slice", True),
+    (1, 65, 200, "slice", True), (1, 333, 1536, "slice", True), (2, 517, 64, "float", False), (4, 130, 4096, "slice", True)])
+def test_segments_chunks_layouts(B, S, C, form, gate):
+    from kolmogorov_moe_architecture_b200 import ops
+    torch.manual_seed(S + C)
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    u, dt, xz = bf(B, S, C), bf(B, S, C) * 0.5, bf(B, S, 2 * C)
+    proj = bf(B, S, 24 + 32)
+    Bm, Cm = proj[..., 24:40], proj[..., 40:]
+    if form == "float":
+        Bm, Cm = Bm.float(), Cm.float()
+    A = -torch.exp(torch.randn(C, 16, device="cuda") * 0.5)
+    D = torch.randn(C, device="cuda") if gate else None
+    bias = torch.randn(C, device="cuda") if gate else None
+    z = xz[..., C:] if gate else None
+    dt = dt if gate else dt.abs()
+    go = bf(B, S, C)
+    args = [u, dt, A, Bm, Cm, D, z, bias]
+    on = [t for t in args if t is not None]
+    for t in on:
+        t.requires_grad_(True)
+    y = ops.selective_scan(*args, gate)
+    got = (y, *torch.autograd.grad(y, on, go))
+    with torch.no_grad():
+        assert torch.equal(ops.selective_scan(*args, gate), y)
+    ref_args = [None if t is None else t.detach().double().requires_grad_(True) for t in args]
+    yr = _ref(*ref_args, gate)
+    want = (yr, *torch.autograd.grad(yr, [t for t in ref_args if t is not None], go.double()))
+    for g, w in zip(got, want):
+        assert _rel(g, w) < TOL
