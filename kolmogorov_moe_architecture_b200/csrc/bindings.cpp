@@ -296,7 +296,7 @@ std::tuple<Tensor, Tensor, Tensor> conv1d_bwd(const Tensor& x, const Tensor& w, 
   Tensor dw = at::zeros_like(w);
   Tensor db = w.dim() == 3 ? at::zeros({G, C}, w.options()) : at::zeros({C}, w.options());
   check(kmoe_conv1d_bwd(x.data_ptr(), w.data_ptr<float>(), (const float*)ptr_or_null(bias), dy.data_ptr(),
-                        dx.data_ptr(), dw.data_ptr<float>(), db.data_ptr<float>(), B, S, C, row_stride(x),
+                        dx.data_ptr(), dw.data_ptr<float>(), db.data_ptr<float>(), B, S, C, row_stride(x), C,
                         act ? 1 : 0, G, cur_stream()), "conv1d_bwd");
   return {dx, dw, db};
 }

@@ -162,7 +162,8 @@ int kmoe_swiglu_bwd(const void* g, const void* u, const void* dh, void* dg, void
 int kmoe_conv1d_fwd(const void* x, const float* w, const float* bias, void* y, int B, int S, int C, long long ldx,
                     int act, int groups, cudaStream_t st);
 int kmoe_conv1d_bwd(const void* x, const float* w, const float* bias, const void* dy, void* dx, float* dw,
-                    float* dbias, int B, int S, int C, long long ldx, int act, int groups, cudaStream_t st);
+                    float* dbias, int B, int S, int C, long long ldx, long long lddx, int act, int groups,
+                    cudaStream_t st);
 // Selective scan.  The sequence is processed in kmoe_scan_segments(B, S, C) parallel segments.
 //   Bm, Cm: [B, S, N] with rows ldbc elements apart, bf16 (bc_bf16 != 0) or fp32, rows 16-byte aligned.
 //   ckpt (forward, optional): [B, ceil(S / kmoe_scan_chunk()), C, N] floats, the state before every chunk.

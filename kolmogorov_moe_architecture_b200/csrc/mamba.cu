@@ -11,90 +11,192 @@
 namespace kmoe {
 
 __device__ __forceinline__ float bf2f(__nv_bfloat16 v) { return __bfloat162float(v); }
-__device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf(-x)); }
 
 // ------------------------------------------------------------------ conv1d
 // y[b,t,c] = act(bias[c] + sum_j w[c,j] * x[b, t-(W-1)+j, c]),  W = 4
-constexpr int CONV_T = 64;  // time steps per thread
+// A thread owns V neighbouring channels (two where rows are 4-byte aligned: a warp then moves whole 128-byte lines) and
+// CONV_T steps, a CTA eight such stretches.  Both directions stream their operands once; what counts is to have enough
+// loads in flight, so the rows of a batch of steps are requested, unconditionally (rows past the end repeat the last
+// one), before the first of them is looked at.
+// 4 x 2048 x 4096: forward 37.7 -> 36.6 us (20.5 at the copy rate), backward 132.5 -> 88.8 us (30.8) against one
+// channel, 64 steps and one row at a time per thread.
+constexpr int CONV_T = 32;      // time steps per thread
+constexpr int CONV_WARPS = 8;
 
-__global__ void conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
-                                  const float* __restrict__ bias, __nv_bfloat16* __restrict__ y, int S, int C,
-                                  long long ldx, int act, int bpg) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
+template <int V>
+struct ConvVec;
+template <>
+struct ConvVec<1> {
+  using Raw = unsigned short;
+  __device__ static __forceinline__ Raw load(const __nv_bfloat16* p) { return __ldg(reinterpret_cast<const Raw*>(p)); }
+  __device__ static __forceinline__ void widen(Raw r, float (&v)[1]) { v[0] = __uint_as_float((uint32_t)r << 16); }
+  __device__ static __forceinline__ void store(__nv_bfloat16* p, const float (&v)[1]) { *p = __float2bfloat16(v[0]); }
+};
+template <>
+struct ConvVec<2> {
+  using Raw = uint32_t;
+  __device__ static __forceinline__ Raw load(const __nv_bfloat16* p) { return __ldg(reinterpret_cast<const Raw*>(p)); }
+  __device__ static __forceinline__ void widen(Raw r, float (&v)[2]) {
+    v[0] = __uint_as_float(r << 16);
+    v[1] = __uint_as_float(r & 0xffff0000u);
+  }
+  __device__ static __forceinline__ void store(__nv_bfloat16* p, const float (&v)[2]) {
+    *reinterpret_cast<uint32_t*>(p) = pack_bf16(v[0], v[1]);
+  }
+};
+
+template <int V>
+__global__ void __launch_bounds__(32 * CONV_WARPS)
+conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+                  __nv_bfloat16* __restrict__ y, int S, int C, long long ldx, int act, int bpg) {
+  const int c = (blockIdx.x * 32 + (threadIdx.x & 31)) * V;
+  const int t0 = (blockIdx.y * CONV_WARPS + (threadIdx.x >> 5)) * CONV_T;
+  if (c >= C || t0 >= S) return;
   const int b = blockIdx.z;
-  const int t0 = blockIdx.y * CONV_T;
   const int pc = (b / bpg) * C + c;   // parameter row: batch entries [g*bpg, (g+1)*bpg) use parameter set g
-  const float w0 = w[pc * 4 + 0], w1 = w[pc * 4 + 1], w2 = w[pc * 4 + 2], w3 = w[pc * 4 + 3];
-  const float bs = bias ? bias[pc] : 0.f;
+  float wv[V][4], bs[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) wv[k][j] = w[(size_t)(pc + k) * 4 + j];
+    bs[k] = bias ? bias[pc + k] : 0.f;
+  }
   const __nv_bfloat16* xb = x + (size_t)b * S * ldx + c;
   __nv_bfloat16* yb = y + (size_t)b * S * C + c;
-  float x0 = t0 >= 3 ? bf2f(xb[(size_t)(t0 - 3) * ldx]) : 0.f;
-  float x1 = t0 >= 2 ? bf2f(xb[(size_t)(t0 - 2) * ldx]) : 0.f;
-  float x2 = t0 >= 1 ? bf2f(xb[(size_t)(t0 - 1) * ldx]) : 0.f;
-  const int t1 = min(t0 + CONV_T, S);
-#pragma unroll 4
-  for (int t = t0; t < t1; ++t) {
-    const float x3 = bf2f(xb[(size_t)t * ldx]);
-    float v = bs + w0 * x0 + w1 * x1 + w2 * x2 + w3 * x3;
-    if (act) v = silu_f(v);
-    yb[(size_t)t * C] = __float2bfloat16(v);
-    x0 = x1; x1 = x2; x2 = x3;
+  float win[3][V];                    // x[t-3], x[t-2], x[t-1]
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) win[j][k] = 0.f;
+    if (t0 - 3 + j >= 0) ConvVec<V>::widen(ConvVec<V>::load(xb + (size_t)(t0 - 3 + j) * ldx), win[j]);
+  }
+  constexpr int BATCH = 8;
+#pragma unroll 1
+  for (int tb = t0; tb < min(t0 + CONV_T, S); tb += BATCH) {
+    typename ConvVec<V>::Raw raw[BATCH];
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i) raw[i] = ConvVec<V>::load(xb + (size_t)min(tb + i, S - 1) * ldx);
+    float xv[BATCH][V];
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i) ConvVec<V>::widen(raw[i], xv[i]);
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i) {
+      float o[V];
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const float x0 = i > 2 ? xv[i - 3][k] : win[i][k], x1 = i > 1 ? xv[i - 2][k] : win[i + 1][k],
+                    x2 = i > 0 ? xv[i - 1][k] : win[2][k];
+        const float v = bs[k] + wv[k][0] * x0 + wv[k][1] * x1 + wv[k][2] * x2 + wv[k][3] * xv[i][k];
+        o[k] = act ? silu_f(v) : v;
+      }
+      if (tb + i < S) ConvVec<V>::store(yb + (size_t)(tb + i) * C, o);
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int k = 0; k < V; ++k) win[j][k] = xv[BATCH - 3 + j][k];
   }
 }
 
-// dx, and atomically accumulated dw [C,4], dbias [C] (fp32, zeroed by the caller).
-__global__ void conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
-                                  const float* __restrict__ bias, const __nv_bfloat16* __restrict__ dy,
-                                  __nv_bfloat16* __restrict__ dx, float* __restrict__ dw, float* __restrict__ dbias,
-                                  int S, int C, long long ldx, int act, int bpg) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
+// dx (rows lddx apart), and atomically accumulated dw [C,4], dbias [C] (fp32, zeroed by the caller; one addition per
+// channel and CTA).
+template <int V>
+__global__ void __launch_bounds__(32 * CONV_WARPS)
+conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+                  const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
+                  float* __restrict__ dbias, int S, int C, long long ldx, long long lddx, int act, int bpg) {
+  __shared__ float sums[CONV_WARPS][5 * V][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = (blockIdx.x * 32 + lane) * V;
+  const int t0 = (blockIdx.y * CONV_WARPS + warp) * CONV_T;
   const int b = blockIdx.z;
-  const int t0 = blockIdx.y * CONV_T;
   const int pc = (b / bpg) * C + c;
-  const float w0 = w[pc * 4 + 0], w1 = w[pc * 4 + 1], w2 = w[pc * 4 + 2], w3 = w[pc * 4 + 3];
-  const float bs = bias ? bias[pc] : 0.f;
-  const __nv_bfloat16* xb = x + (size_t)b * S * ldx + c;
-  const __nv_bfloat16* gb = dy + (size_t)b * S * C + c;
-  __nv_bfloat16* dxb = dx + (size_t)b * S * C + c;
-  float x0 = t0 >= 3 ? bf2f(xb[(size_t)(t0 - 3) * ldx]) : 0.f;
-  float x1 = t0 >= 2 ? bf2f(xb[(size_t)(t0 - 2) * ldx]) : 0.f;
-  float x2 = t0 >= 1 ? bf2f(xb[(size_t)(t0 - 1) * ldx]) : 0.f;
-  float p0 = 0.f, p1 = 0.f, p2 = 0.f;  // dpre[t-3], dpre[t-2], dpre[t-1]
-  float aw0 = 0.f, aw1 = 0.f, aw2 = 0.f, aw3 = 0.f, ab = 0.f;
-  const int t_own_end = min(t0 + CONV_T, S);
-  const int t_end = t0 + CONV_T + 3;  // dx[t] needs dpre up to t+3
-  for (int t = t0; t < t_end; ++t) {
-    float p3 = 0.f, x3 = 0.f;
-    if (t < S) {
-      x3 = bf2f(xb[(size_t)t * ldx]);
-      const float pre = bs + w0 * x0 + w1 * x1 + w2 * x2 + w3 * x3;
-      float g = bf2f(gb[(size_t)t * C]);
-      if (act) {
-        const float sg = sigmoid_f(pre);
-        g *= sg * (1.f + pre * (1.f - sg));
+  float acc[V][5];                    // dw[0..3], dbias
+#pragma unroll
+  for (int k = 0; k < V; ++k)
+#pragma unroll
+    for (int j = 0; j < 5; ++j) acc[k][j] = 0.f;
+  if (c < C && t0 < S) {
+    float wv[V][4], bs[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) wv[k][j] = w[(size_t)(pc + k) * 4 + j];
+      bs[k] = bias ? bias[pc + k] : 0.f;
+    }
+    const __nv_bfloat16* xb = x + (size_t)b * S * ldx + c;
+    const __nv_bfloat16* gb = dy + (size_t)b * S * C + c;
+    __nv_bfloat16* dxb = dx + (size_t)b * S * lddx + c;
+    const int t_own = min(t0 + CONV_T, S);
+    float xw[3][V], pw[3][V];         // x[t-3 .. t-1], dpre[t-3 .. t-1]; the dpre window starts empty, which is exact:
+#pragma unroll                        // dx[td >= t0] never reads dpre[< t0]
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) xw[j][k] = pw[j][k] = 0.f;
+      if (t0 - 3 + j >= 0) ConvVec<V>::widen(ConvVec<V>::load(xb + (size_t)(t0 - 3 + j) * ldx), xw[j]);
+    }
+    constexpr int BATCH = 7;          // CONV_T + 3 steps in all: dx[t] needs dpre up to t + 3
+    static_assert((CONV_T + 3) % BATCH == 0, "whole batches");
+#pragma unroll 1
+    for (int tb = t0; tb < t0 + CONV_T + 3; tb += BATCH) {
+      typename ConvVec<V>::Raw xr[BATCH], gr[BATCH];
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) {
+        const int t = min(tb + i, S - 1);
+        xr[i] = ConvVec<V>::load(xb + (size_t)t * ldx);
+        gr[i] = ConvVec<V>::load(gb + (size_t)t * C);
       }
-      p3 = g;
-      if (t < t_own_end) {
-        aw0 += g * x0; aw1 += g * x1; aw2 += g * x2; aw3 += g * x3; ab += g;
+#pragma unroll
+      for (int i = 0; i < BATCH; ++i) {
+        float o[V], xv[V], gv[V];
+        ConvVec<V>::widen(xr[i], xv);
+        ConvVec<V>::widen(gr[i], gv);
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          const float x0 = xw[0][k], x1 = xw[1][k], x2 = xw[2][k], x3 = xv[k];
+          float g = tb + i < S ? gv[k] : 0.f;
+          if (act) {
+            const float pre = bs[k] + wv[k][0] * x0 + wv[k][1] * x1 + wv[k][2] * x2 + wv[k][3] * x3;
+            const float sg = sigmoid_f(pre);
+            g *= sg * (1.f + pre * (1.f - sg));
+          }
+          if (tb + i < t_own) {
+            acc[k][0] += g * x0; acc[k][1] += g * x1; acc[k][2] += g * x2; acc[k][3] += g * x3; acc[k][4] += g;
+          }
+          // dx[t - 3] = w0 dpre[t] + w1 dpre[t-1] + w2 dpre[t-2] + w3 dpre[t-3]
+          o[k] = wv[k][0] * g + wv[k][1] * pw[2][k] + wv[k][2] * pw[1][k] + wv[k][3] * pw[0][k];
+          xw[0][k] = x1; xw[1][k] = x2; xw[2][k] = x3;
+          pw[0][k] = pw[1][k]; pw[1][k] = pw[2][k]; pw[2][k] = g;
+        }
+        const int td = tb + i - 3;
+        if (td >= t0 && td < t_own) ConvVec<V>::store(dxb + (size_t)td * lddx, o);
       }
     }
-    const int td = t - 3;  // dx[td] = w0 dpre[td+3] + w1 dpre[td+2] + w2 dpre[td+1] + w3 dpre[td]
-    if (td >= t0 && td < t_own_end) {
-      float v = w0 * p3 + w1 * p2 + w2 * p1 + w3 * p0;
-      dxb[(size_t)td * C] = __float2bfloat16(v);
-    }
-    x0 = x1; x1 = x2; x2 = x3;
-    p0 = p1; p1 = p2; p2 = p3;
   }
-  // the dpre window starts empty, which is exact: dx[td >= t0] never reads dpre[< t0]
-  atomicAdd(&dw[pc * 4 + 0], aw0);
-  atomicAdd(&dw[pc * 4 + 1], aw1);
-  atomicAdd(&dw[pc * 4 + 2], aw2);
-  atomicAdd(&dw[pc * 4 + 3], aw3);
-  if (dbias) atomicAdd(&dbias[pc], ab);
+#pragma unroll
+  for (int k = 0; k < V; ++k)
+#pragma unroll
+    for (int j = 0; j < 5; ++j) sums[warp][k * 5 + j][lane] = acc[k][j];
+  __syncthreads();
+  for (int i = threadIdx.x; i < 5 * V * 32; i += 32 * CONV_WARPS) {
+    const int kj = i / 32, l = i % 32, k = kj / 5, j = kj % 5, cc = (blockIdx.x * 32 + l) * V + k;
+    if (cc >= C) continue;
+    float v = 0.f;
+#pragma unroll
+    for (int q = 0; q < CONV_WARPS; ++q) v += sums[q][kj][l];
+    const size_t row = (size_t)(b / bpg) * C + cc;
+    if (j < 4) atomicAdd(&dw[row * 4 + j], v);
+    else if (dbias) atomicAdd(&dbias[row], v);
+  }
+}
+
+static bool conv_pairs(const void* a, const void* b, const void* c, int C, long long ld1, long long ld2) {
+  return C % 2 == 0 && ld1 % 2 == 0 && ld2 % 2 == 0 &&
+         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 3) == 0;
+}
+static dim3 conv_grid(int B, int S, int C, int v) {
+  return dim3((C + 32 * v - 1) / (32 * v), (S + CONV_T * CONV_WARPS - 1) / (CONV_T * CONV_WARPS), B);
 }
 
 }  // namespace kmoe
@@ -104,18 +206,23 @@ using namespace kmoe;
 extern "C" int kmoe_conv1d_fwd(const void* x, const float* w, const float* bias, void* y, int B, int S, int C,
                                long long ldx, int act, int groups, cudaStream_t st) {
   if (groups < 1 || B % groups) return -1;
-  dim3 grid((C + 127) / 128, (S + CONV_T - 1) / CONV_T, B);
-  conv1d_fwd_kernel<<<grid, 128, 0, st>>>((const __nv_bfloat16*)x, w, bias, (__nv_bfloat16*)y, S, C, ldx, act,
-                                          B / groups);
+  if (B == 0 || S == 0 || C == 0) return 0;
+  const bool two = conv_pairs(x, y, y, C, ldx, C);
+  auto kern = two ? conv1d_fwd_kernel<2> : conv1d_fwd_kernel<1>;
+  kern<<<conv_grid(B, S, C, two ? 2 : 1), 32 * CONV_WARPS, 0, st>>>((const __nv_bfloat16*)x, w, bias, (__nv_bfloat16*)y, S,
+                                                                    C, ldx, act, B / groups);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 extern "C" int kmoe_conv1d_bwd(const void* x, const float* w, const float* bias, const void* dy, void* dx, float* dw,
-                               float* dbias, int B, int S, int C, long long ldx, int act, int groups,
+                               float* dbias, int B, int S, int C, long long ldx, long long lddx, int act, int groups,
                                cudaStream_t st) {
   if (groups < 1 || B % groups) return -1;
-  dim3 grid((C + 127) / 128, (S + CONV_T - 1) / CONV_T, B);
-  conv1d_bwd_kernel<<<grid, 128, 0, st>>>((const __nv_bfloat16*)x, w, bias, (const __nv_bfloat16*)dy,
-                                          (__nv_bfloat16*)dx, dw, dbias, S, C, ldx, act, B / groups);
+  if (B == 0 || S == 0 || C == 0) return 0;
+  const bool two = conv_pairs(x, dy, dx, C, ldx, lddx);
+  auto kern = two ? conv1d_bwd_kernel<2> : conv1d_bwd_kernel<1>;
+  kern<<<conv_grid(B, S, C, two ? 2 : 1), 32 * CONV_WARPS, 0, st>>>((const __nv_bfloat16*)x, w, bias,
+                                                                    (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, dw, dbias,
+                                                                    S, C, ldx, lddx, act, B / groups);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
