@@ -998,6 +998,23 @@ def _head_weight_tensor(weights: tuple, device) -> torch.Tensor:
     return t
 
 
+def _loss_split(rows: int, d: int, V: int) -> int:
+    """Slices of the vocabulary in which the hidden states' gradient ``dlogits W`` is accumulated (fp32, summed once at
+    the end).  The product has few output tiles and a reduction of tens of thousands, so a last round of tiles that is
+    nearly empty costs a whole reduction: 4096 x 1536 is 96 tiles on 74 CTA pairs, two rounds for 1.3.  Slices shorten
+    the rounds; each one costs a pass over its fp32 tile per head (~3 % of a slice of 16 k, hence the term per slice)."""
+    pairs = 74
+    tiles = -(-rows // 256) * -(-d // 256)
+    best, best_t = 1, 1e30
+    for parts in range(1, 7):
+        if parts > 1 and V // parts < 8192:
+            break
+        t = -(-tiles * parts // pairs) / parts + 0.03 * parts * tiles / pairs * (parts > 1)
+        if t < best_t - 0.05:
+            best, best_t = parts, t
+    return best
+
+
 class _MTPLoss(torch.autograd.Function):
     """Per head: logits chunk = H W^T (tcgen05 GEMM) -> CE kernel writes d logits in place ->
     dH += dlogits W and dW = dlogits^T H.  Gradients are produced during forward (scaled
@@ -1013,6 +1030,12 @@ class _MTPLoss(torch.autograd.Function):
         # ones, so neither needs a zero fill nor an addend read on its first use
         dH = torch.empty_like(h2) if need_grad else None
         dH_started = False
+        V0 = head_weights[0].shape[0]
+        parts = _loss_split(min(R, chunk_rows), d, V0) if need_grad and all(w.shape[0] == V0 for w in head_weights) else 1
+        if parts > 1:
+            kb, kl = _split_k_ranges(V0, parts, hidden.device)
+            parts = kb.numel()
+            acc32 = torch.empty(parts, R, d, dtype=torch.float32, device=hidden.device)
         dWs: List[Optional[torch.Tensor]] = []
         per = []
         for i, W in enumerate(head_weights):
@@ -1042,8 +1065,12 @@ class _MTPLoss(torch.autograd.Function):
                 _count()
                 loss_sum = loss_sum + rows.sum()
                 if need_grad:
-                    acc = dict(D=dH[r0:r1], beta=1.0) if dH_started else {}
-                    gemm(buf, Wc, dH[r0:r1], M=n, N=d, Kd=V, b_major=MAJ_MN, lda=pitch, ldb=d, ldc=d, **acc)
+                    dst, kw = dH[r0:r1], {}
+                    if parts > 1:
+                        dst = acc32[:, r0:r1]
+                        kw = dict(mode=BATCHED, groups=parts, k_begin=kb, k_len=kl, c_gs=R * d)
+                    acc = dict(D=dst, beta=1.0) if dH_started else {}
+                    gemm(buf, Wc, dst, M=n, N=d, Kd=V, b_major=MAJ_MN, lda=pitch, ldb=d, ldc=d, **acc, **kw)
                     acc = dict(D=dW, beta=1.0) if r0 > 0 else {}
                     gemm(buf, hc, dW, M=V, N=d, Kd=n, a_major=MAJ_MN, b_major=MAJ_MN, lda=pitch, ldb=d, ldc=d, **acc)
             dH_started = dH_started or need_grad
@@ -1051,6 +1078,9 @@ class _MTPLoss(torch.autograd.Function):
             dWs.append(dW)
         if need_grad and not dH_started:
             dH.zero_()
+        elif need_grad and parts > 1:
+            K.sum_partials(acc32, dH)
+            _count()
         per_t = torch.stack(per)
         total = (per_t * _head_weight_tensor(tuple(float(w) for w in weights), hidden.device)).sum()
         ctx.shape = (B, S, d)
@@ -1068,7 +1098,17 @@ class _MTPLoss(torch.autograd.Function):
         saved = ctx.saved_tensors
         dH, dWs = saved[0], saved[1:]
         B, S, d = ctx.shape
-        gh = (dH * g_total.to(dH.dtype)).view(B, S, d) if dH.numel() else None
+        g32 = g_total.reshape(1).float()
+
+        def scaled(t, dst=None):            # one vectorised pass, the factor read from the device
+            dst = torch.empty_like(t) if dst is None else dst
+            if dst.is_contiguous() and dst.data_ptr() % 16 == 0 and t.data_ptr() % 16 == 0:
+                K.scale_copy(t, dst, g32)
+                _count()
+            else:
+                torch.mul(t, g_total.to(t.dtype), out=dst)
+            return dst
+        gh = scaled(dH).view(B, S, d) if dH.numel() else None
         gws = []
         for W, w in zip(ctx.heads, dWs):
             if not w.numel():
@@ -1076,17 +1116,12 @@ class _MTPLoss(torch.autograd.Function):
                 continue
             sink = grad_sink(W) if W.is_contiguous() else None
             if sink is not None:
-                # scaled straight into the weight's slot of the flat gradient buffer: one pass instead of a
-                # multiplication into a new tensor plus the copy into the buffer
-                dst = sink[0]
-                if dst.is_contiguous() and dst.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
-                    K.scale_copy(w, dst, g_total.reshape(1).float())
-                else:
-                    torch.mul(w, g_total.to(w.dtype), out=dst)
+                # straight into the weight's slot of the flat gradient buffer, without a tensor and a copy between
+                scaled(w, sink[0])
                 sink[1]()
                 gws.append(None)
             else:
-                gws.append(w * g_total.to(w.dtype))
+                gws.append(scaled(w))
         return (gh, None, None, None, None, *gws)
 
 

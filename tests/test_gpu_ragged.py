@@ -155,3 +155,49 @@ def test_output_edges_stay_inside(M, N, G, addends):
         ref = ref - 1.5 * D2[:, :M, :N].double()
     assert _rel(out[:, :M, :N], ref) < ONE_ROUNDING
     assert (out[:, M:] == 3.0).all() and (out[:, :, N:] == 3.0).all()
+
+
+@pytest.mark.parametrize("R,V", [(3, 65), (5, 8), (7, 50257), (2, 114000), (2, 116000)])
+@pytest.mark.parametrize("grad", [True, False])
+def test_cross_entropy_rows(R, V, grad):
+    """Rows that fit shared memory and rows that do not (from 115200 entries), with a tail, ignored and large entries."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(V)
+    pitch = -(-V // 64) * 64
+    buf = torch.full((R, pitch), float("nan"), dtype=torch.bfloat16, device="cuda")
+    buf[:, :V] = (torch.randn(R, V, device="cuda") * 3).to(torch.bfloat16)
+    buf[0, V - 1] = 80.0
+    lab = torch.randint(0, V, (R,), device="cuda")
+    lab[1] = -100
+    lg = buf[:, :V].double()
+    ref = torch.nn.functional.cross_entropy(lg, lab, ignore_index=-100, reduction="none")
+    p = (torch.softmax(lg, -1) - torch.nn.functional.one_hot(lab.clamp(min=0), V)) * 0.37
+    p[1] = 0
+    rows = c.K.ce_fwd_bwd(buf[:, :V], lab, torch.full((1,), 0.37, device="cuda"), -100, grad)
+    assert (rows.double() - ref).abs().max() < 2e-5 * ref.abs().max()        # 32-bit sums
+    if grad:
+        assert _rel(buf[:, :V], p) < ONE_ROUNDING
+    else:
+        assert torch.equal(buf[:, :V].double(), lg)
+    assert buf[:, V:].isnan().all()
+
+
+@pytest.mark.parametrize("parts", [1, 2, 3])
+def test_loss_vocabulary_slices(parts, monkeypatch):
+    """The hidden states' gradient accumulated in vocabulary slices, several row chunks and heads."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    monkeypatch.setattr(cuda_ops, "_loss_split", lambda *a: parts)
+    torch.manual_seed(parts)
+    B, S, d, V = 2, 90, 128, 1003
+    h = _rand(B, S, d)
+    Ws = [_rand(V, d, scale=0.1) for _ in range(3)]
+    labels = torch.randint(0, V, (B, S), device="cuda")
+    leaves = [t.clone().requires_grad_() for t in (h, *Ws)]
+    total, _ = cuda_ops.mtp_cross_entropy(leaves[0], leaves[1:], labels, (0.5, 0.3, 0.2), chunk_rows=64)
+    got = torch.autograd.grad(total, leaves)
+    cuda_ops.check_status()
+    rl = [t.double().requires_grad_() for t in (h, *Ws)]
+    ref = sum(w * torch.nn.functional.cross_entropy((rl[0][:, : S - i - 1] @ W.t()).reshape(-1, V), labels[:, i + 1:].reshape(-1))
+              for i, (W, w) in enumerate(zip(rl[1:], (0.5, 0.3, 0.2))))
+    for g, w in zip(got, torch.autograd.grad(ref, rl)):
+        assert _rel(g, w) < EXPERT_TOL
