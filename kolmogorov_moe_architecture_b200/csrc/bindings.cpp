@@ -729,30 +729,38 @@ void gemm_mxfp8(const Tensor& A, const Tensor& sfa, const Tensor& B, const Tenso
 }
 
 // ------------------------------------------------------------- routing decisions
-std::vector<Tensor> route_topk_fwd(const Tensor& logits, int64_t k) {
+// logits fp32 or bf16 -> (weights in the logits' type, indices, aux, fp32 weights, lse, sums)
+std::vector<Tensor> route_topk_fwd(const Tensor& logits, int64_t k, double w_lb, double w_z) {
   c10::cuda::CUDAGuard guard(logits.device());
-  need_f32(logits, "logits");
-  TORCH_CHECK(logits.dim() == 2 && logits.is_contiguous());
+  const bool bf = logits.scalar_type() == at::kBFloat16;
+  TORCH_CHECK(logits.is_cuda() && (bf || logits.scalar_type() == at::kFloat) && logits.dim() == 2 && logits.is_contiguous(),
+              "logits must be contiguous fp32 or bf16 (T, E)");
   const int64_t T = logits.size(0), E = logits.size(1);
-  auto of = logits.options();
+  auto of = logits.options().dtype(at::kFloat);
   Tensor w = at::empty({T, k}, of), idx = at::empty({T, k}, of.dtype(at::kLong)), lse = at::empty({T}, of);
+  Tensor w_out = bf ? at::empty({T, k}, logits.options()) : w;
   Tensor acc = at::zeros({2 * E + 1}, of);   // [0,E) sum of probabilities, [E,2E) counts, [2E] sum lse^2
-  float* a = acc.data_ptr<float>();
-  check(kmoe_route_topk_fwd(logits.data_ptr<float>(), (int)T, (int)E, (int)k, w.data_ptr<float>(),
-                            (long long*)idx.data_ptr<int64_t>(), lse.data_ptr<float>(), a, a + E, a + 2 * E,
-                            cur_stream()), "route_topk_fwd");
-  return {w, idx, lse, acc};
+  Tensor aux = T > 0 ? at::empty({}, of) : at::zeros({}, of);
+  check(kmoe_route_topk_fwd(logits.data_ptr(), bf, (int)T, (int)E, (int)k, w.data_ptr<float>(),
+                            bf ? w_out.data_ptr() : nullptr, (long long*)idx.data_ptr<int64_t>(), lse.data_ptr<float>(),
+                            acc.data_ptr<float>(), aux.data_ptr<float>(), (float)w_lb, (float)w_z, cur_stream()),
+        "route_topk_fwd");
+  return {w_out, idx, aux, w, lse, acc};
 }
 
+// dw in the logits' type; returns dlogits in the logits' type
 Tensor route_topk_bwd(const Tensor& logits, const Tensor& lse, const Tensor& idx, const Tensor& w, const OptT& dw,
                       const Tensor& acc, const OptT& d_aux, double w_lb, double w_z) {
   c10::cuda::CUDAGuard guard(logits.device());
   const int64_t T = logits.size(0), E = logits.size(1), k = idx.size(1);
+  if (dw.has_value() && dw->defined())
+    TORCH_CHECK(dw->scalar_type() == logits.scalar_type() && dw->is_contiguous() && dw->numel() == T * k,
+                "dw must be contiguous and of the logits' type");
   Tensor dl = at::empty_like(logits);
-  check(kmoe_route_topk_bwd(logits.data_ptr<float>(), lse.data_ptr<float>(), (const long long*)idx.data_ptr<int64_t>(),
-                            w.data_ptr<float>(), (const float*)ptr_or_null(dw), acc.data_ptr<float>() + E,
-                            (const float*)ptr_or_null(d_aux), (float)w_lb, (float)w_z, (int)T, (int)E, (int)k,
-                            dl.data_ptr<float>(), cur_stream()), "route_topk_bwd");
+  check(kmoe_route_topk_bwd(logits.data_ptr(), logits.scalar_type() == at::kBFloat16, lse.data_ptr<float>(),
+                            (const long long*)idx.data_ptr<int64_t>(), w.data_ptr<float>(), ptr_or_null(dw),
+                            acc.data_ptr<float>() + E, (const float*)ptr_or_null(d_aux), (float)w_lb, (float)w_z, (int)T,
+                            (int)E, (int)k, dl.data_ptr(), cur_stream()), "route_topk_bwd");
   return dl;
 }
 

@@ -243,13 +243,14 @@ int kmoe_ep_move(const void* slots, void* packed, const int* meta_in, const int*
                  int dir, long long* row_ptr_out, cudaStream_t st);
 
 // ---------------------------------------------------------------------------- routing decisions
-// Token choice: softmax over E experts -> top-k -> renormalise; also accumulates (atomically, into
-// zero-initialised buffers) sum_t p[t, e], the number of assignments per expert and sum_t lse_t^2.
-int kmoe_route_topk_fwd(const float* logits, int T, int E, int k, float* w, long long* idx, float* lse, float* p_sum,
-                        float* counts, float* z_sum, cudaStream_t st);
-int kmoe_route_topk_bwd(const float* logits, const float* lse, const long long* idx, const float* w, const float* dw,
-                        const float* counts, const float* d_aux, float w_lb, float w_z, int T, int E, int k,
-                        float* dlogits, cudaStream_t st);
+// Token choice: softmax over E experts -> top-k -> renormalise; also accumulates (atomically, into the zero-initialised
+// acc[2 E + 1]) sum_t p[t, e], the number of assignments per expert and sum_t lse_t^2, and forms the auxiliary loss.
+// logits, w_out (the weights once more, optional), dw and dlogits are fp32 or bf16 (is_bf16).
+int kmoe_route_topk_fwd(const void* logits, int is_bf16, int T, int E, int k, float* w, void* w_out, long long* idx,
+                        float* lse, float* acc, float* aux, float w_lb, float w_z, cudaStream_t st);
+int kmoe_route_topk_bwd(const void* logits, int is_bf16, const float* lse, const long long* idx, const float* w,
+                        const void* dw, const float* counts, const float* d_aux, float w_lb, float w_z, int T, int E, int k,
+                        void* dlogits, cudaStream_t st);
 // Per-row top-k of a strided score matrix; row r starts at (r / rows_inner) * outer_stride +
 // (r % rows_inner) * row_stride and its S entries are col_stride apart.  mode 0: k largest scores,
 // indices ascending, softmax over the kept scores.  mode 1: softmax over the row, k largest

@@ -772,21 +772,20 @@ class _RouteTopK(torch.autograd.Function):
     def forward(ctx, logits, k, w_lb, w_z):
         shape = logits.shape
         E = shape[-1]
-        lf = logits.reshape(-1, E).float().contiguous()
-        T = lf.shape[0]
-        w, idx, lse, acc = K.route_topk_fwd(lf, k)
-        _count()
-        aux = (w_lb * E / (float(T) * T * k)) * (acc[:E] * acc[E:2 * E]).sum() + (w_z / T) * acc[2 * E]
+        lf = logits.reshape(-1, E)
+        lf = (lf if lf.dtype in (torch.bfloat16, torch.float32) else lf.float()).contiguous()
+        w_out, idx, aux, w, lse, acc = K.route_topk_fwd(lf, k, w_lb, w_z)
+        _count(2)
         ctx.save_for_backward(lf, lse, idx, w, acc)
         ctx.meta = (shape, logits.dtype, k, w_lb, w_z)
         ctx.mark_non_differentiable(idx)
-        return w.view(*shape[:-1], k).to(logits.dtype), idx.view(*shape[:-1], k), aux, acc[E:2 * E]
+        return w_out.view(*shape[:-1], k).to(logits.dtype), idx.view(*shape[:-1], k), aux, acc[E:2 * E]
 
     @staticmethod
     def backward(ctx, dw, _didx, daux, _dcounts):
         lf, lse, idx, w, acc = ctx.saved_tensors
         shape, dtype, k, w_lb, w_z = ctx.meta
-        dwf = dw.reshape(-1, k).float().contiguous() if dw is not None else None
+        dwf = dw.reshape(-1, k).to(lf.dtype).contiguous() if dw is not None else None
         da = daux.reshape(1).float().contiguous() if daux is not None else None
         dl = K.route_topk_bwd(lf, lse, idx, w, dwf, acc, da, w_lb, w_z)
         _count()

@@ -1,0 +1,76 @@
+"""Routing at its edges: one token, odd counts, all expert widths of a warp, bf16 and fp32 logits with ties; the plan with
+empty experts, dropped assignments and several warps' stretches; the combine with long, mostly empty slot lists."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 1, 1), (3, 4, 2), (97, 33, 3), (2500, 64, 2), (4097, 16, 8), (130, 128, 4)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_route(T, E, k, dtype):
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    torch.manual_seed(T)
+    logits = torch.randn(T, E, device="cuda").to(dtype)
+    logits[::3] = logits[::3].round()                                     # many ties
+    x = logits.clone().requires_grad_(True)
+    w, idx, aux, counts = cuda_ops.route_topk(x, k, 0.3, 0.1)
+    r = logits.double().requires_grad_(True)
+    ridx = torch.sort(r, dim=-1, descending=True, stable=True).indices[:, :k]
+    p = torch.softmax(r, -1)
+    rw = p.gather(1, ridx)
+    rw = rw / rw.sum(-1, keepdim=True)
+    rc = torch.bincount(ridx.reshape(-1), minlength=E)
+    raux = 0.3 * E * (rc / (T * k) * p.mean(0)).sum() + 0.1 * torch.logsumexp(r, -1).square().mean()
+    assert torch.equal(idx, ridx) and torch.equal(counts.long(), rc)       # whole numbers; the lower index wins a tie
+    gw = torch.randn(T, k, device="cuda").to(dtype)
+    got = torch.autograd.grad((w, aux), x, (gw, torch.ones_like(aux)))[0]
+    want = torch.autograd.grad((rw, raux), r, (gw.double(), torch.ones_like(raux)))[0]
+    tol = 4e-3 if dtype == torch.bfloat16 else 1e-5                        # one rounding of the result / 32-bit sums
+    assert (w.double() - rw).norm() <= tol * rw.norm()
+    assert abs(aux.item() - raux.item()) <= 1e-5 * abs(raux.item()) + 1e-12
+    # k = E: the weights are the softmax itself and its gradient cancels to the auxiliary part, hence the floor
+    assert (got.double() - want).norm() <= tol * want.norm() + 1e-6 * gw.double().norm()
+
+
+@pytest.mark.parametrize("n,E", [(1, 3), (31, 1), (1024, 16), (1025, 64), (12289, 33), (5000, 164)])
+@pytest.mark.parametrize("drop", [False, True])
+def test_plan(n, E, drop):
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    torch.manual_seed(n)
+    idx = torch.randint(0, max(1, E - 1), (n,), device="cuda")             # the last expert stays empty
+    keep = torch.rand(n, device="cuda") < 0.7 if drop else None
+    pos, row_src, counts, offsets, tile_group, meta = [t.cpu() for t in cuda_ops.K.moe_plan(idx, keep, E, 0)]
+    ids, kp = idx.cpu(), keep.cpu() if drop else torch.ones(n, dtype=torch.bool)
+    run, tiles = 0, []
+    want_rows = torch.full_like(row_src, -1)
+    want_pos = torch.full_like(pos, -1)
+    for e in range(E):
+        a = ((ids == e) & kp).nonzero().flatten()
+        assert counts[e] == a.numel() and offsets[e] == run
+        want_rows[run:run + a.numel()] = a.int()
+        want_pos[a] = torch.arange(run, run + a.numel(), dtype=torch.int32)
+        nt = -(-a.numel() // 128)
+        tiles += [e] * nt
+        run += nt * 128
+    assert offsets[E] == run and meta.tolist() == [len(tiles), run]
+    assert torch.equal(row_src, want_rows) and torch.equal(pos, want_pos)
+    assert tile_group.tolist() == tiles + [0] * (tile_group.numel() - len(tiles))
+
+
+@pytest.mark.parametrize("T,k,d", [(1, 1, 8), (37, 2, 264), (300, 16, 2048), (9, 40, 1096)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_combine(T, k, d, weighted):
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    torch.manual_seed(k)
+    rows = max(1, T * k // 3)
+    Y = torch.randn(rows, d, device="cuda").to(torch.bfloat16)
+    pos = torch.full((T * k,), -1, dtype=torch.int32, device="cuda")
+    at = torch.randperm(T * k, device="cuda")[:rows]
+    pos[at] = torch.arange(rows, dtype=torch.int32, device="cuda")
+    w = torch.rand(T * k, device="cuda") if weighted else None
+    out = cuda_ops.K.moe_combine(Y, pos, w, T, k)
+    scale = (w if weighted else torch.ones(T * k, device="cuda")).double()
+    ref = torch.zeros(T, d, dtype=torch.double, device="cuda")
+    ref.index_add_(0, at // k, Y.double() * scale[at, None])
+    assert (out.double() - ref).norm() <= 4e-3 * ref.norm()
