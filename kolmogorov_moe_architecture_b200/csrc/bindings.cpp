@@ -728,6 +728,221 @@ void gemm_mxfp8(const Tensor& A, const Tensor& sfa, const Tensor& B, const Tenso
   check(kmoe_gemm_mxfp8(&d, cur_stream()), "gemm_mxfp8");
 }
 
+// ------------------------------------------------------------------- whole passes
+// The forward and backward passes of the dense and expert layers as one operator call each: a call from Python costs about
+// as much as the launch it makes (15 us against 5), and these passes are made of up to eleven of them.
+struct Gemm {
+  KmoeGemmDesc d{};
+  Gemm(const Tensor& A, int a_major, int64_t lda, const Tensor& B, int b_major, int64_t ldb, const Tensor& C, int64_t ldc,
+       int64_t M, int64_t N, int64_t K, const Tensor& status) {
+    need_bf16(A, "A"); need_bf16(B, "B");
+    d.A = A.data_ptr(); d.B = B.data_ptr(); d.C = C.data_ptr();
+    d.groups = 1; d.M = (int)M; d.N = (int)N; d.K = (int)K;
+    d.a_major = a_major; d.b_major = b_major; d.lda = lda; d.ldb = ldb; d.ldc = ldc;
+    d.alpha = 1.f;
+    d.out_f32 = C.scalar_type() == at::kFloat ? 1 : 0;
+    d.status = status.data_ptr<int>();
+    d.num_sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  }
+  void run(const char* what) { check(kmoe_gemm(&d, cur_stream()), what); }
+};
+constexpr int KM = KMOE_MAJOR_K, MN = KMOE_MAJOR_MN;
+
+inline void need_rows(const Tensor& t, const char* n) {
+  need_bf16(t, n);
+  TORCH_CHECK(t.dim() == 2 && t.stride(1) == 1 && t.stride(0) % 8 == 0, n, " must be a matrix with dense rows of a pitch of 8 elements");
+}
+inline void need_weight(const Tensor& t, const char* n) {
+  need_bf16(t, n);
+  TORCH_CHECK(t.is_contiguous(), n, " must be contiguous");
+}
+
+Tensor linear_fwd(const Tensor& x, const Tensor& w, const Tensor& status) {
+  c10::cuda::CUDAGuard guard(x.device());
+  need_rows(x, "x"); need_weight(w, "w");
+  const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
+  TORCH_CHECK(w.dim() == 2 && w.size(1) == K, "w does not match x");
+  Tensor y = at::empty({M, N}, x.options());
+  Gemm(x, KM, x.stride(0), w, KM, K, y, N, M, N, K, status).run("linear_fwd");
+  return y;
+}
+
+std::vector<Tensor> linear_multi_fwd(const Tensor& x, const std::vector<Tensor>& ws, const Tensor& status) {
+  std::vector<Tensor> ys;
+  for (const auto& w : ws) ys.push_back(linear_fwd(x, w, status));
+  return ys;
+}
+
+// dW = dy^T x into `dst` (new when absent).  kb / kl: the rows in slices (fp32 partial results, one sum), for results of
+// few output tiles.
+Tensor wgrad_into(const Tensor& dy, const Tensor& x, const Tensor& w, const OptT& dst, const OptT& kb, const OptT& kl,
+                  const Tensor& status) {
+  const int64_t T = x.size(0), out_f = w.size(0), in_f = w.size(1);
+  Tensor dw = dst.has_value() && dst->defined() ? *dst : at::empty_like(w);
+  need_bf16(dw, "dW");
+  TORCH_CHECK(dw.dim() == 2 && dw.stride(1) == 1 && dw.size(0) == out_f && dw.size(1) == in_f, "dW does not match the weight");
+  const bool sliced = kb.has_value() && kb->defined();
+  if (!sliced) {
+    Gemm(dy, MN, dy.stride(0), x, MN, x.stride(0), dw, dw.stride(0), out_f, in_f, T, status).run("wgrad");
+    return dw;
+  }
+  TORCH_CHECK(dw.is_contiguous(), "a sliced dW must be contiguous");
+  const int64_t parts = kb->numel();
+  Tensor partial = at::empty({parts, out_f, in_f}, dw.options().dtype(at::kFloat));
+  Gemm g(dy, MN, dy.stride(0), x, MN, x.stride(0), partial, in_f, out_f, in_f, T, status);
+  g.d.mode = KMOE_GEMM_BATCHED; g.d.groups = (int)parts; g.d.c_gstride = out_f * in_f;
+  g.d.k_begin = kb->data_ptr<int>(); g.d.k_len = kl->data_ptr<int>();
+  g.run("wgrad");
+  check(kmoe_sum_partials(partial.data_ptr<float>(), dw.data_ptr(), (int)parts, out_f * in_f, cur_stream()), "sum_partials");
+  return dw;
+}
+
+// (dx, dW) of y = x W^T; either may be unwanted (undefined).  dx_acc: dx is added onto this tensor.
+std::tuple<Tensor, Tensor> linear_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, bool need_dx, const OptT& dx_acc,
+                                      bool need_dw, const OptT& dw_dst, const OptT& kb, const OptT& kl,
+                                      const Tensor& status) {
+  c10::cuda::CUDAGuard guard(x.device());
+  need_rows(dy, "dy"); need_rows(x, "x"); need_weight(w, "w");
+  const int64_t T = x.size(0), out_f = w.size(0), in_f = w.size(1);
+  TORCH_CHECK(x.size(1) == in_f && dy.size(0) == T && dy.size(1) == out_f, "shapes of dy, x and w do not match");
+  Tensor dx, dw;
+  if (need_dx) {
+    const bool acc = dx_acc.has_value() && dx_acc->defined();
+    dx = acc ? *dx_acc : at::empty({T, in_f}, dy.options());
+    Gemm g(dy, KM, dy.stride(0), w, MN, in_f, dx, dx.stride(0), T, in_f, out_f, status);
+    if (acc) { g.d.D = dx.data_ptr(); g.d.ldd = dx.stride(0); g.d.beta = 1.f; }
+    g.run("dgrad");
+  }
+  if (need_dw) dw = wgrad_into(dy, x, w, dw_dst, kb, kl, status);
+  return {dx, dw};
+}
+
+// y = w3(silu(w1 x) * (w2 x)); also the hidden activations and - when `save` - the two pre-activations
+std::tuple<Tensor, Tensor, Tensor, Tensor> dense_swiglu_fwd(const Tensor& x, const Tensor& w1, const Tensor& w2,
+                                                            const Tensor& w3, bool save, const Tensor& status) {
+  c10::cuda::CUDAGuard guard(x.device());
+  need_rows(x, "x"); need_weight(w1, "w1"); need_weight(w2, "w2"); need_weight(w3, "w3");
+  const int64_t T = x.size(0), d = x.size(1), f = w1.size(0), o = w3.size(0);
+  TORCH_CHECK(w1.size(1) == d && w2.sizes() == w1.sizes() && w3.size(1) == f, "weights do not match x");
+  Tensor H = at::empty({T, f}, x.options()), G, U;
+  if (save) { G = at::empty_like(H); U = at::empty_like(H); }
+  Gemm g(x, KM, x.stride(0), w1, KM, d, H, f, T, f, d, status);
+  g.d.epilogue = KMOE_EPI_SWIGLU; g.d.B2 = w2.data_ptr();
+  if (save) { g.d.G_out = G.data_ptr(); g.d.U_out = U.data_ptr(); }
+  g.run("gate_up");
+  Tensor y = at::empty({T, o}, x.options());
+  Gemm(H, KM, f, w3, KM, f, y, o, T, o, f, status).run("down");
+  return {y, H, G, U};
+}
+
+// kb1 / kl1 slice the weight gradients of w1 and w2, kb3 / kl3 that of w3
+std::tuple<Tensor, Tensor, Tensor, Tensor> dense_swiglu_bwd(const Tensor& dy, const Tensor& x, const Tensor& G,
+                                                            const Tensor& U, const OptT& H_in, const Tensor& w1,
+                                                            const Tensor& w2, const Tensor& w3, bool need_dx,
+                                                            const OptT& dst1, const OptT& dst2, const OptT& dst3,
+                                                            const OptT& kb1, const OptT& kl1, const OptT& kb3,
+                                                            const OptT& kl3, const Tensor& status) {
+  c10::cuda::CUDAGuard guard(x.device());
+  need_rows(dy, "dy"); need_rows(x, "x");
+  const int64_t T = x.size(0), d = x.size(1), f = w1.size(0), o = w3.size(0);
+  Tensor dH = at::empty({T, f}, dy.options());
+  Gemm(dy, KM, dy.stride(0), w3, MN, f, dH, f, T, f, o, status).run("dH");
+  Tensor dGU = swiglu_bwd_cat(G, U, dH, OptT());
+  const int64_t P = dGU.size(1) / 2;
+  Tensor dG = dGU.narrow(1, 0, f), dU = dGU.narrow(1, P, f), dx;
+  if (need_dx) {
+    dx = at::empty({T, d}, dy.options());
+    Gemm g(dGU, KM, 2 * P, w1, MN, d, dx, d, T, d, 2 * P, status);
+    g.d.B2 = w2.data_ptr(); g.d.k_split = (int)P; g.d.b_klen = (int)f;
+    g.run("dx");
+  }
+  Tensor H = H_in.has_value() && H_in->defined() ? *H_in : swiglu_fwd(G, U, OptT());
+  Tensor dw1 = wgrad_into(dG, x, w1, dst1, kb1, kl1, status), dw2 = wgrad_into(dU, x, w2, dst2, kb1, kl1, status);
+  Tensor dw3 = wgrad_into(dy, H, w3, dst3, kb3, kl3, status);
+  return {dx, dw1, dw2, dw3};
+}
+
+// Token-choice experts: (out, Xp, G, U, H, Y, wf, pos, row_src, counts, offsets, tile_group, meta); G and U only when `save`
+std::vector<Tensor> grouped_swiglu_fwd(const Tensor& x_in, const Tensor& w1, const Tensor& w2, const Tensor& w3,
+                                       const Tensor& idx, const OptT& keep, const Tensor& weights, bool save,
+                                       const Tensor& status) {
+  c10::cuda::CUDAGuard guard(x_in.device());
+  need_weight(w1, "w1"); need_weight(w2, "w2"); need_weight(w3, "w3");
+  const Tensor x = x_in.contiguous();
+  const int64_t T = x.size(0), d = x.size(1), E = w1.size(0), f = w1.size(2), k = idx.size(1);
+  auto plan = moe_plan(idx.reshape({-1}).contiguous(), keep, E, 0);
+  const Tensor &pos = plan[0], &row_src = plan[1], &tile_group = plan[4], &meta = plan[5];
+  const int64_t R = row_src.numel();
+  Tensor Xp = moe_gather_rows(x, row_src, OptT(), meta, k);
+  Tensor H = at::empty({R, f}, x.options()), G, U;
+  if (save) { G = at::empty_like(H); U = at::empty_like(H); }
+  auto grouped = [&](Gemm& g, int64_t gs) {
+    g.d.mode = KMOE_GEMM_GROUPED_M; g.d.groups = (int)E; g.d.b_gstride = gs;
+    g.d.tile_group = tile_group.data_ptr<int>(); g.d.num_m_tiles = meta.data_ptr<int>();
+  };
+  Gemm g1(Xp, KM, d, w1, MN, f, H, f, R, f, d, status);
+  grouped(g1, d * f);
+  g1.d.epilogue = KMOE_EPI_SWIGLU; g1.d.B2 = w2.data_ptr();
+  if (save) { g1.d.G_out = G.data_ptr(); g1.d.U_out = U.data_ptr(); }
+  g1.run("experts gate_up");
+  Tensor Y = at::empty({R, d}, x.options());
+  Gemm g2(H, KM, f, w3, MN, d, Y, d, R, d, f, status);
+  grouped(g2, f * d);
+  g2.run("experts down");
+  Tensor wf = weights.reshape({-1}).to(at::kFloat).contiguous();
+  Tensor out = moe_combine(Y, pos, wf, T, k);
+  return {out, Xp, G, U, H, Y, wf, pos, row_src, plan[2], plan[3], tile_group, meta};
+}
+
+// (dx, dw1, dw2, dw3, d weights in fp32); H undefined: recomputed
+std::vector<Tensor> grouped_swiglu_bwd(const Tensor& dout_in, const Tensor& Xp, const Tensor& G, const Tensor& U,
+                                       const OptT& H_in, const Tensor& Y, const Tensor& w1, const Tensor& w2,
+                                       const Tensor& w3, const Tensor& wf, const Tensor& pos, const Tensor& row_src,
+                                       const Tensor& counts, const Tensor& offsets, const Tensor& tile_group,
+                                       const Tensor& meta, int64_t k, const OptT& dst1, const OptT& dst2, const OptT& dst3,
+                                       const Tensor& status) {
+  c10::cuda::CUDAGuard guard(Xp.device());
+  const Tensor dout = dout_in.contiguous();
+  const int64_t T = dout.size(0), d = dout.size(1), E = w1.size(0), f = w1.size(2), R = row_src.numel();
+  const Tensor live = meta.narrow(0, 1, 1);
+  Tensor dYp = moe_gather_rows(dout, row_src, wf, meta, k);
+  Tensor dwts = moe_combine_dw(Y, dout, pos, k);
+  auto grouped = [&](Gemm& g, int64_t gs) {
+    g.d.mode = KMOE_GEMM_GROUPED_M; g.d.groups = (int)E; g.d.b_gstride = gs;
+    g.d.tile_group = tile_group.data_ptr<int>(); g.d.num_m_tiles = meta.data_ptr<int>();
+  };
+  Tensor dH = at::empty({R, f}, dout.options());
+  Gemm g1(dYp, KM, d, w3, KM, d, dH, f, R, f, d, status);
+  grouped(g1, f * d);
+  g1.run("experts dH");
+  Tensor dGU = swiglu_bwd_cat(G, U, dH, live);           // [dG | dU], one operand; P = f in whole 64-blocks
+  const int64_t P = dGU.size(1) / 2;
+  Tensor dG = dGU.narrow(1, 0, f), dU = dGU.narrow(1, P, f);
+  Tensor dXp = at::empty({R, d}, dout.options());
+  // dXp = dG W1^T + dU W2^T in one grouped GEMM: the reduction runs over [dG | dU] and [W1 | W2]
+  Gemm g2(dGU, KM, 2 * P, w1, KM, f, dXp, d, R, d, 2 * P, status);
+  grouped(g2, d * f);
+  g2.d.B2 = w2.data_ptr(); g2.d.k_split = (int)P; g2.d.b_klen = (int)f;
+  g2.run("experts dx");
+  Tensor dx = moe_combine(dXp, pos, OptT(), T, k);
+  Tensor H = H_in.has_value() && H_in->defined() ? *H_in : swiglu_fwd(G, U, live);
+  // weight gradients: per expert, reduction over its rows (the rows up to the next whole block are zeros)
+  auto wg = [&](const Tensor& A, int64_t lda, const Tensor& B, int64_t ldb, const Tensor& w, const OptT& dst, int64_t M,
+                int64_t N) {
+    Tensor dw = dst.has_value() && dst->defined() ? *dst : at::empty_like(w);
+    TORCH_CHECK(dw.is_contiguous() && dw.sizes() == w.sizes(), "an expert weight gradient must be laid out like its weight");
+    need_bf16(dw, "dW");
+    Gemm g(A, MN, lda, B, MN, ldb, dw, N, M, N, R, status);
+    g.d.mode = KMOE_GEMM_BATCHED; g.d.groups = (int)E; g.d.c_gstride = M * N;
+    g.d.k_begin = offsets.data_ptr<int>(); g.d.k_len = counts.data_ptr<int>();
+    g.run("experts wgrad");
+    return dw;
+  };
+  Tensor dw1 = wg(Xp, d, dG, 2 * P, w1, dst1, d, f), dw2 = wg(Xp, d, dU, 2 * P, w2, dst2, d, f);
+  Tensor dw3 = wg(H, f, dYp, d, w3, dst3, f, d);
+  return {dx, dw1, dw2, dw3, dwts};
+}
+
 // ------------------------------------------------------------- routing decisions
 // logits fp32 or bf16 -> (weights in the logits' type, indices, aux, fp32 weights, lse, sums)
 std::vector<Tensor> route_topk_fwd(const Tensor& logits, int64_t k, double w_lb, double w_z) {
@@ -853,6 +1068,13 @@ TORCH_LIBRARY(kmoe, m) {
   m.def("conv1d_bwd", &conv1d_bwd);
   m.def("scan_fwd", &scan_fwd);
   m.def("scan_bwd", &scan_bwd);
+  m.def("linear_fwd", &linear_fwd);
+  m.def("linear_multi_fwd", &linear_multi_fwd);
+  m.def("linear_bwd", &linear_bwd);
+  m.def("dense_swiglu_fwd", &dense_swiglu_fwd);
+  m.def("dense_swiglu_bwd", &dense_swiglu_bwd);
+  m.def("grouped_swiglu_fwd", &grouped_swiglu_fwd);
+  m.def("grouped_swiglu_bwd", &grouped_swiglu_bwd);
   m.def("moe_plan", &moe_plan);
   m.def("moe_capacity_mask", &moe_capacity_mask);
   m.def("moe_balanced_assign", &moe_balanced_assign);

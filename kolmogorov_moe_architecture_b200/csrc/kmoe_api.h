@@ -35,7 +35,8 @@ typedef struct KmoeGemmDesc {
   // *num_m_tiles (device) tiles are live.
   const int* tile_group;
   const int* num_m_tiles;
-  // BATCHED, optional ragged reduction range per group, in elements of K (multiples of 64).
+  // BATCHED, optional ragged reduction range per group, in elements of K: k_begin a multiple of 64, k_len rounded up to
+  // one (both operands must be finite there, and one of them zero past k_len).
   const int* k_begin;
   const int* k_len;
   int out_f32;

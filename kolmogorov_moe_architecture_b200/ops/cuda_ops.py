@@ -175,36 +175,31 @@ def _split_k_ranges(T: int, parts: int, device):
     return hit
 
 
-def _wgrad(dy: torch.Tensor, x2: torch.Tensor, w: torch.Tensor):
-    """dW = dy^T x2 into the weight's slot of the flat gradient buffer when one is registered (returns None
-    then), else into a new tensor.  Narrow results (router and projection matrices of a few output tiles) are
-    computed as slices of the token dimension in one batched launch, fp32 partial results, and summed."""
-    out_f, in_f = w.shape
-    T = x2.shape[0]
+def _wgrad_plan(w: torch.Tensor, T: int, device):
+    """(sink, destination, slice starts, slice lengths) of a weight gradient over T rows: the weight's slot of the flat
+    gradient buffer when one is registered; slices of the rows when the result is only a few output tiles (router and
+    projection matrices: fp32 partial results of one batched launch, summed)."""
     sink = grad_sink(w)
-    dst = sink[0] if sink is not None else torch.empty_like(w)
-    parts = split_k_parts(out_f, in_f, T) if (out_f * in_f) % 4 == 0 and dst.is_contiguous() else 1
-    out, extra = dst, {}
-    if parts > 1:
-        kb, kl = _split_k_ranges(T, parts, dy.device)
-        parts = kb.numel()
-        out = torch.empty(parts, out_f, in_f, dtype=torch.float32, device=dy.device)
-        extra = dict(mode=BATCHED, groups=parts, k_begin=kb, k_len=kl, c_gs=out_f * in_f)
-    if out_f % 64 == 0:
-        gemm(dy, x2, out, M=out_f, N=in_f, Kd=T, a_major=MAJ_MN, b_major=MAJ_MN, lda=dy.stride(0),
-             ldb=x2.stride(0), ldc=in_f if parts > 1 else dst.stride(0), **extra)
-    else:
-        # dy is too narrow to be read MN-major (rows of whole 64-element atoms): use its transpose, K-major
-        dyT = dy.t().contiguous()
-        gemm(dyT, x2, out, M=out_f, N=in_f, Kd=T, a_major=MAJ_K, b_major=MAJ_MN, lda=T, ldb=x2.stride(0),
-             ldc=in_f if parts > 1 else dst.stride(0), **extra)
-    if parts > 1:
-        K.sum_partials(out, dst)
-        _count()
+    dst = sink[0] if sink is not None else None
+    out_f, in_f = w.shape
+    if (out_f * in_f) % 4 == 0 and (dst is None or dst.is_contiguous()):
+        parts = split_k_parts(out_f, in_f, T)
+        if parts > 1:
+            return (sink, dst, *_split_k_ranges(T, parts, device))
+    return sink, dst, None, None
+
+
+def _linear_bwd(dy, x2, w, need_dx: bool, need_dw: bool, dx_acc=None):
+    """(dx, dW) of ``y = x2 w^T``; dW is None when it went to the flat gradient buffer."""
+    if not _rows_ok(dy):
+        dy = dy.contiguous()
+    sink, dst, kb, kl = _wgrad_plan(w, x2.shape[0], x2.device) if need_dw else (None, None, None, None)
+    dx, dw = K.linear_bwd(dy, x2, w, need_dx, dx_acc, need_dw, dst, kb, kl, status_tensor(x2.device))
+    _count(int(need_dx) + int(need_dw) + (kb is not None))
     if sink is not None:
         sink[1]()
-        return None
-    return dst
+        dw = None
+    return dx, dw
 
 
 class _Linear(torch.autograd.Function):
@@ -214,16 +209,13 @@ class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x2, w):
         ctx.save_for_backward(x2, w)
-        return mm_nt(x2, w)
+        _count()
+        return K.linear_fwd(x2, w, status_tensor(x2.device))
 
     @staticmethod
     def backward(ctx, dy):
         x2, w = ctx.saved_tensors
-        if not _rows_ok(dy):
-            dy = dy.contiguous()
-        dx = mm_nn(dy, w) if ctx.needs_input_grad[0] else None
-        dw = _wgrad(dy, x2, w) if ctx.needs_input_grad[1] else None
-        return dx, dw
+        return _linear_bwd(dy, x2, w, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
 
 
 class _RowDot(torch.autograd.Function):
@@ -272,7 +264,8 @@ class _LinearMulti(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x2, *ws):
         ctx.save_for_backward(x2, *ws)
-        return tuple(mm_nt(x2, w) for w in ws)
+        _count(len(ws))
+        return tuple(K.linear_multi_fwd(x2, ws, status_tensor(x2.device)))
 
     @staticmethod
     def backward(ctx, *dys):
@@ -283,14 +276,9 @@ class _LinearMulti(torch.autograd.Function):
             if dy is None:
                 dws.append(None)
                 continue
-            if not _rows_ok(dy):
-                dy = dy.contiguous()
-            if ctx.needs_input_grad[0]:
-                if dx is None:
-                    dx = mm_nn(dy, w)
-                else:
-                    mm_nn(dy, w, out=dx, D=dx, beta=1.0)
-            dws.append(_wgrad(dy, x2, w) if ctx.needs_input_grad[1 + i] else None)
+            got, dw = _linear_bwd(dy, x2, w, ctx.needs_input_grad[0], ctx.needs_input_grad[1 + i], dx)
+            dx = dx if got is None else got
+            dws.append(dw)
         return (dx, *dws)
 
 
@@ -312,15 +300,12 @@ class _DenseSwiGLU(torch.autograd.Function):
     gate and 128 up columns), the same kernels the experts use with a single group."""
 
     @staticmethod
-    def forward(ctx, x2, w1, w2, w3):
-        T, d = x2.shape
-        f = w1.shape[0]
-        H = torch.empty(T, f, dtype=x2.dtype, device=x2.device)
-        G, U = torch.empty_like(H), torch.empty_like(H)
-        gemm(x2, w1, H, B2=w2, G=G, U=U, epi=EPI_SWIGLU, M=T, N=f, Kd=d, lda=x2.stride(0), ldb=d, ldc=f)
-        y = mm_nt(H, w3)
-        keep_h = os.environ.get("KMOE_MOE_KEEP_H", "1") != "0"      # else H is recomputed in the backward pass
-        ctx.save_for_backward(x2, G, U, w1, w2, w3, *((H,) if keep_h else ()))
+    def forward(ctx, x2, w1, w2, w3, grad):
+        y, H, G, U = K.dense_swiglu_fwd(x2, w1, w2, w3, grad, status_tensor(x2.device))
+        _count(2)
+        if grad:
+            keep_h = os.environ.get("KMOE_MOE_KEEP_H", "1") != "0"      # else H is recomputed in the backward pass
+            ctx.save_for_backward(x2, G, U, w1, w2, w3, *((H,) if keep_h else ()))
         return y
 
     @staticmethod
@@ -328,26 +313,22 @@ class _DenseSwiGLU(torch.autograd.Function):
         x2, G, U, w1, w2, w3, *kept = ctx.saved_tensors
         if not _rows_ok(dy):
             dy = dy.contiguous()
-        dH = mm_nn(dy, w3)
-        T, f = dH.shape
-        d = w1.shape[1]
-        dGU = K.swiglu_bwd_cat(G, U, dH, None)              # [dG | dU], one (T, 2f) operand
-        dG, dU = dGU[:, :f], dGU[:, f:]
-        _count()
-        dx = None
-        if ctx.needs_input_grad[0]:
-            # dx = dG W1 + dU W2 as one GEMM whose reduction runs over [dG | dU] and [W1 ; W2]
-            dx = torch.empty(T, d, dtype=dy.dtype, device=dy.device)
-            gemm(dGU, w1, dx, B2=w2, M=T, N=d, Kd=2 * f, k_split=f, b_major=MAJ_MN, lda=2 * f, ldb=d, ldc=d)
-        if kept:
-            H = kept[0]
-        else:
-            H = K.swiglu_fwd(G, U, None)
-            _count()
-        dw1 = _wgrad(dG, x2, w1)
-        dw2 = _wgrad(dU, x2, w2)
-        dw3 = _wgrad(dy, H, w3)
-        return dx, dw1, dw2, dw3
+        T, dev = x2.shape[0], x2.device
+        s1, d1, kb1, kl1 = _wgrad_plan(w1, T, dev)
+        s2, d2, kb2, _ = _wgrad_plan(w2, T, dev)
+        s3, d3, kb3, kl3 = _wgrad_plan(w3, T, dev)
+        if (kb1 is None) != (kb2 is None):              # only one of the two destinations can take a sliced sum
+            kb1 = kl1 = None
+        dx, dw1, dw2, dw3 = K.dense_swiglu_bwd(dy, x2, G, U, kept[0] if kept else None, w1, w2, w3,
+                                               ctx.needs_input_grad[0], d1, d2, d3, kb1, kl1, kb3, kl3, status_tensor(dev))
+        _count(6)
+        out = []
+        for sink, dw in ((s1, dw1), (s2, dw2), (s3, dw3)):
+            if sink is not None:
+                sink[1]()
+                dw = None
+            out.append(dw)
+        return (dx, *out, None)
 
 
 def dense_swiglu(x, w1, w2, w3):
@@ -360,7 +341,8 @@ def dense_swiglu(x, w1, w2, w3):
           and f % 64 == 0 and d % 64 == 0)
     if not ok:
         return linear(swiglu(linear(x, w1), linear(x, w2)), w3)
-    return _DenseSwiGLU.apply(x2, w1, w2, w3).view(*lead, d)
+    grad = torch.is_grad_enabled() and (x2.requires_grad or w1.requires_grad or w2.requires_grad or w3.requires_grad)
+    return _DenseSwiGLU.apply(x2, w1, w2, w3, grad).view(*lead, d)
 
 
 # ------------------------------------------------------------------- RMSNorm
@@ -572,72 +554,36 @@ def attention(q, k, v, causal=True, doc_start=None):
 # ------------------------------------------------------------- MoE experts
 class _GroupedSwiGLU(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w1, w2, w3, idx, weights, keep):
-        T, d = x.shape
-        E, _, f = w1.shape
-        k = idx.shape[1]
-        idx_flat = idx.reshape(-1).contiguous()
-        pos, row_src, counts, offsets, tile_group, meta = K.moe_plan(idx_flat, keep.reshape(-1) if keep is not None else None, E, 0)
-        max_rows = row_src.numel()
-        xc = x.contiguous()
-        Xp = K.moe_gather_rows(xc, row_src, None, meta, k)
-        H = torch.empty(max_rows, f, dtype=x.dtype, device=x.device)
-        G, U = torch.empty_like(H), torch.empty_like(H)
-        nmt = meta[0:1]
-        gemm(Xp, w1, H, B2=w2, G=G, U=U, mode=GROUPED_M, epi=EPI_SWIGLU, M=max_rows, N=f, Kd=d, groups=E,
-             b_major=MAJ_MN, lda=d, ldb=f, ldc=f, b_gs=d * f, tile_group=tile_group, num_m_tiles=nmt)
-        Y = torch.empty(max_rows, d, dtype=x.dtype, device=x.device)
-        gemm(H, w3, Y, mode=GROUPED_M, M=max_rows, N=d, Kd=f, groups=E, b_major=MAJ_MN, lda=f, ldb=d, ldc=d,
-             b_gs=f * d, tile_group=tile_group, num_m_tiles=nmt)
-        wf = weights.reshape(-1).float().contiguous()
-        out = K.moe_combine(Y, pos, wf, T, k)
-        _count(3)
-        # The hidden activations H are kept for the weight gradient of the down projection unless
-        # KMOE_MOE_KEEP_H=0 (then they are recomputed from G and U in the backward pass: one more kernel per
-        # layer, rows x f bf16 less memory held between the passes).
-        keep_h = os.environ.get("KMOE_MOE_KEEP_H", "1") != "0"
-        ctx.save_for_backward(Xp, G, U, Y, w1, w2, w3, wf, pos, row_src, offsets, tile_group, meta,
-                              *((H,) if keep_h else ()))
-        ctx.dims = (T, d, E, f, k, max_rows)
-        ctx.wdtype = weights.dtype
+    def forward(ctx, x, w1, w2, w3, idx, weights, keep, grad=True):
+        (out, Xp, G, U, H, Y, wf, pos, row_src, counts, offsets, tile_group, meta) = K.grouped_swiglu_fwd(
+            x, w1, w2, w3, idx, keep.reshape(-1) if keep is not None else None, weights, grad, status_tensor(x.device))
+        _count(5)
+        if grad:
+            # The hidden activations H are kept for the weight gradient of the down projection unless
+            # KMOE_MOE_KEEP_H=0 (then they are recomputed from G and U in the backward pass: one more kernel per
+            # layer, rows x f bf16 less memory held between the passes).
+            keep_h = os.environ.get("KMOE_MOE_KEEP_H", "1") != "0"
+            ctx.save_for_backward(Xp, G, U, Y, w1, w2, w3, wf, pos, row_src, counts, offsets, tile_group, meta,
+                                  *((H,) if keep_h else ()))
+            ctx.k = idx.shape[1]
+            ctx.wdtype = weights.dtype
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        Xp, G, U, Y, w1, w2, w3, wf, pos, row_src, offsets, tile_group, meta, *kept = ctx.saved_tensors
-        T, d, E, f, k, max_rows = ctx.dims
-        dout = dout.contiguous()
-        nmt = meta[0:1]
-        dYp = K.moe_gather_rows(dout, row_src, wf, meta, k)
-        dwts = K.moe_combine_dw(Y, dout, pos, k).view(T, k).to(ctx.wdtype)
-        dH = torch.empty(max_rows, f, dtype=dout.dtype, device=dout.device)
-        gemm(dYp, w3, dH, mode=GROUPED_M, M=max_rows, N=f, Kd=d, groups=E, lda=d, ldb=d, ldc=f, b_gs=f * d,
-             tile_group=tile_group, num_m_tiles=nmt)
-        dGU = K.swiglu_bwd_cat(G, U, dH, meta[1:2])          # [dG | dU], one operand; P = f in whole 64-blocks
-        P = dGU.shape[1] // 2
-        dG, dU = dGU[:, :f], dGU[:, P:P + f]
-        dXp = torch.empty(max_rows, d, dtype=dout.dtype, device=dout.device)
-        # dXp = dG W1^T + dU W2^T in one grouped GEMM: the reduction runs over [dG | dU] and [W1 | W2]
-        gemm(dGU, w1, dXp, B2=w2, mode=GROUPED_M, M=max_rows, N=d, Kd=2 * P, k_split=P, b_klen=f, groups=E, lda=2 * P,
-             ldb=f, ldc=d, b_gs=d * f, tile_group=tile_group, num_m_tiles=nmt)
-        dx = K.moe_combine(dXp, pos, None, T, k)
-        # weight gradients: per expert, reduction over that expert's (padded) row range
-        kb = offsets[:E].contiguous()
-        kl = (offsets[1:] - offsets[:E]).contiguous()
-        H = kept[0] if kept else K.swiglu_fwd(G, U, meta[1:2])
+        Xp, G, U, Y, w1, w2, w3, wf, pos, row_src, counts, offsets, tile_group, meta, *kept = ctx.saved_tensors
         # weight gradients go straight to their place in the flat gradient buffer when one is registered
         sinks = [grad_sink(w) for w in (w1, w2, w3)]
-        dw1, dw2, dw3 = [s[0] if s is not None else torch.empty_like(w) for s, w in zip(sinks, (w1, w2, w3))]
-        common = dict(mode=BATCHED, groups=E, a_major=MAJ_MN, b_major=MAJ_MN, Kd=max_rows, k_begin=kb, k_len=kl)
-        gemm(Xp, dG, dw1, M=d, N=f, lda=d, ldb=2 * P, ldc=f, c_gs=d * f, **common)
-        gemm(Xp, dU, dw2, M=d, N=f, lda=d, ldb=2 * P, ldc=f, c_gs=d * f, **common)
-        gemm(H, dYp, dw3, M=f, N=d, lda=f, ldb=d, ldc=d, c_gs=f * d, **common)
-        _count(5)
+        dst = [s_[0] if s_ is not None else None for s_ in sinks]
+        dx, dw1, dw2, dw3, dwts = K.grouped_swiglu_bwd(dout, Xp, G, U, kept[0] if kept else None, Y, w1, w2, w3, wf, pos,
+                                                       row_src, counts, offsets, tile_group, meta, ctx.k, *dst,
+                                                       status_tensor(Xp.device))
+        _count(9)
         for s_ in sinks:
             if s_ is not None:
                 s_[1]()
         dw1, dw2, dw3 = [None if s_ is not None else g for s_, g in zip(sinks, (dw1, dw2, dw3))]
-        return dx, dw1, dw2, dw3, None, dwts, None
+        return dx, dw1, dw2, dw3, None, dwts.view(-1, ctx.k).to(ctx.wdtype), None, None
 
 
 def _expert_widths_ok(d: int, f: int) -> bool:
@@ -658,7 +604,8 @@ def grouped_swiglu(x, w1, w2, w3, idx, weights, keep=None, moe_dtype="bf16"):
     if moe_dtype == "mxfp8":
         from . import mxfp8
         return mxfp8.grouped_swiglu_mxfp8(x, w1, w2, w3, idx, weights, keep)
-    return _GroupedSwiGLU.apply(x, w1.contiguous(), w2.contiguous(), w3.contiguous(), idx, weights, keep)
+    grad = torch.is_grad_enabled() and any(t.requires_grad for t in (x, w1, w2, w3, weights))
+    return _GroupedSwiGLU.apply(x, w1.contiguous(), w2.contiguous(), w3.contiguous(), idx, weights, keep, grad)
 
 
 class _ExpertChoiceSwiGLU(torch.autograd.Function):
