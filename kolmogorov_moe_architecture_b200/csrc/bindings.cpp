@@ -943,6 +943,90 @@ std::vector<Tensor> grouped_swiglu_bwd(const Tensor& dout_in, const Tensor& Xp, 
   return {dx, dw1, dw2, dw3, dwts};
 }
 
+// The Mamba mixer between its in- and out-projection.  xz (B,S,2C): conv input | gate.
+// Forward: (y, conv output, x_dbl, delta, params, ckpt, seg)
+std::vector<Tensor> mamba_inner_fwd(const Tensor& xz, const Tensor& conv_w, const Tensor& conv_b, const Tensor& xp_w,
+                                    const Tensor& dt_w, const Tensor& dt_b, const Tensor& A_log, const Tensor& D, bool save,
+                                    const Tensor& status) {
+  c10::cuda::CUDAGuard guard(xz.device());
+  need_bf16(xz, "xz"); need_aligned(xz, "xz"); need_weight(xp_w, "x_proj"); need_weight(dt_w, "dt_proj");
+  const int64_t B = xz.size(0), S = xz.size(1), C = xz.size(2) / 2, T = B * S, R = dt_w.size(1), N = 16;
+  const bool bf = A_log.scalar_type() == at::kBFloat16;
+  for (const Tensor* p : {&conv_w, &conv_b, &dt_b, &A_log, &D})
+    TORCH_CHECK(p->is_cuda() && p->is_contiguous() && p->scalar_type() == A_log.scalar_type() &&
+                (bf || p->scalar_type() == at::kFloat), "mixer parameters must be contiguous and of one type");
+  TORCH_CHECK(xz.is_contiguous() && xz.dim() == 3 && C % 8 == 0 && R % 8 == 0 && conv_w.numel() == 4 * C &&
+              conv_b.numel() == C && dt_b.numel() == C && D.numel() == C && A_log.numel() == N * C &&
+              xp_w.size(0) == R + 2 * N && xp_w.size(1) == C && dt_w.size(0) == C, "mixer shapes do not match");
+  auto f32 = xz.options().dtype(at::kFloat);
+  Tensor params = at::empty({23 * C}, f32);
+  float* P = params.data_ptr<float>();
+  check(kmoe_mamba_params(A_log.data_ptr(), conv_w.data_ptr(), conv_b.data_ptr(), dt_b.data_ptr(), D.data_ptr(), bf, P, (int)C,
+                          cur_stream()), "mamba_params");
+  Tensor x = at::empty({T, C}, xz.options());
+  check(kmoe_conv1d_fwd(xz.data_ptr(), P + 16 * C, P + 20 * C, x.data_ptr(), (int)B, (int)S, (int)C, 2 * C, 1, 1,
+                        cur_stream()), "conv1d_fwd");
+  // like every projection: few rows of no multiple of 8 stay with the library
+  Tensor x_dbl = T % 8 == 0 ? linear_fwd(x, xp_w, status) : at::linear(x, xp_w);
+  const int64_t ld = R + 2 * N;
+  Tensor delta = at::empty({T, C}, xz.options());
+  Gemm(x_dbl, KM, ld, dt_w, KM, R, delta, C, T, C, R, status).run("dt_proj");
+  Tensor y = at::empty({T, C}, xz.options());
+  const char* xd = reinterpret_cast<const char*>(x_dbl.data_ptr());
+  const int nch = (int)((S + kmoe_scan_chunk() - 1) / kmoe_scan_chunk()), segs = kmoe_scan_segments((int)B, (int)S, (int)C);
+  Tensor ckpt = save ? at::empty({B, nch, C, N}, f32) : Tensor();
+  Tensor seg = segs > 1 ? at::empty({B * segs * (N + 1) * C}, f32) : at::empty({0}, f32);
+  const char* z = reinterpret_cast<const char*>(xz.data_ptr()) + 2 * C;
+  check(kmoe_scan_fwd(x.data_ptr(), delta.data_ptr(), z, P, xd + 2 * R, xd + 2 * (R + N), ld, 1, P + 22 * C, P + 21 * C,
+                      y.data_ptr(), save ? ckpt.data_ptr<float>() : nullptr, segs > 1 ? seg.data_ptr<float>() : nullptr,
+                      (int)B, (int)S, (int)C, (int)N, 2 * C, 1, 1, cur_stream()), "scan_fwd");
+  return {y.view({B, S, C}), x, x_dbl, delta, params, ckpt, seg};
+}
+
+// (dxz, d x_proj, d dt_proj, flat gradients of the small parameters in their own type: A_log | conv w | conv b | dt b | D)
+std::vector<Tensor> mamba_inner_bwd(const Tensor& dy_in, const Tensor& xz, const Tensor& x, const Tensor& x_dbl,
+                                    const Tensor& delta, const Tensor& params, const Tensor& ckpt, const Tensor& seg,
+                                    const Tensor& xp_w, const Tensor& dt_w, bool params_bf16, const OptT& xp_dst,
+                                    const OptT& xp_kb, const OptT& xp_kl, const OptT& dt_dst, const OptT& dt_kb,
+                                    const OptT& dt_kl, const Tensor& status) {
+  c10::cuda::CUDAGuard guard(xz.device());
+  Tensor dy = dy_in.contiguous();
+  if (reinterpret_cast<uintptr_t>(dy.data_ptr()) & 15) dy = dy.clone();
+  need_bf16(dy, "dy");
+  const int64_t B = xz.size(0), S = xz.size(1), C = xz.size(2) / 2, T = B * S, R = dt_w.size(1), N = 16, ld = R + 2 * N;
+  TORCH_CHECK(dy.numel() == T * C, "dy does not match");
+  auto f32 = xz.options().dtype(at::kFloat);
+  // everything that accumulates, zeroed together: the small parameters' gradients, dB, dC
+  Tensor acc = at::zeros({23 * C + 2 * T * N}, f32);
+  float *a = acc.data_ptr<float>(), *dB = a + 23 * C, *dC = dB + T * N;
+  const float* P = params.data_ptr<float>();
+  const char* xd = reinterpret_cast<const char*>(x_dbl.data_ptr());
+  char* z = reinterpret_cast<char*>(xz.data_ptr()) + 2 * C;
+  Tensor dxz = at::empty_like(xz), du = at::empty({T, C}, xz.options()), dd = at::empty({T, C}, xz.options());
+  const int segs = kmoe_scan_segments((int)B, (int)S, (int)C);
+  Tensor gseg = segs > 1 ? at::empty({B * segs * N * C}, f32) : Tensor();
+  check(kmoe_scan_bwd(x.data_ptr(), delta.data_ptr(), z, P, xd + 2 * R, xd + 2 * (R + N), ld, 1, P + 22 * C, P + 21 * C,
+                      dy.data_ptr(), ckpt.data_ptr<float>(), segs > 1 ? seg.data_ptr<float>() : nullptr,
+                      segs > 1 ? gseg.data_ptr<float>() : nullptr, du.data_ptr(), dd.data_ptr(),
+                      reinterpret_cast<char*>(dxz.data_ptr()) + 2 * C, 2 * C, a, dB, dC, a + 22 * C, a + 21 * C, (int)B,
+                      (int)S, (int)C, (int)N, 2 * C, 1, 1, cur_stream()), "scan_bwd");
+  Tensor dx_dbl = at::empty({T, ld}, xz.options());
+  Gemm(dd, KM, C, dt_w, MN, R, dx_dbl, ld, T, R, C, status).run("d dt");
+  check(kmoe_mamba_pack_bc(dB, dC, reinterpret_cast<char*>(dx_dbl.data_ptr()) + 2 * R, T, ld, cur_stream()), "pack_bc");
+  Tensor ddt = wgrad_into(dd, x_dbl.narrow(1, 0, R), dt_w, dt_dst, dt_kb, dt_kl, status);
+  {  // the conv output's gradient: what the scan left plus dx_dbl x_proj, added before the one rounding
+    Gemm g(dx_dbl, KM, ld, xp_w, MN, C, du, C, T, C, ld, status);
+    g.d.D = du.data_ptr(); g.d.ldd = C; g.d.beta = 1.f;
+    g.run("d x");
+  }
+  Tensor dxp = wgrad_into(dx_dbl, x, xp_w, xp_dst, xp_kb, xp_kl, status);
+  check(kmoe_conv1d_bwd(xz.data_ptr(), P + 16 * C, P + 20 * C, du.data_ptr(), dxz.data_ptr(), a + 16 * C, a + 20 * C, (int)B,
+                        (int)S, (int)C, 2 * C, 2 * C, 1, 1, cur_stream()), "conv1d_bwd");
+  Tensor dp = at::empty({23 * C}, params_bf16 ? xz.options() : f32);
+  check(kmoe_mamba_params_bwd(a, P, dp.data_ptr(), params_bf16, (int)C, cur_stream()), "mamba_params_bwd");
+  return {dxz, dxp, ddt, dp};
+}
+
 // ------------------------------------------------------------- routing decisions
 // logits fp32 or bf16 -> (weights in the logits' type, indices, aux, fp32 weights, lse, sums)
 std::vector<Tensor> route_topk_fwd(const Tensor& logits, int64_t k, double w_lb, double w_z) {
@@ -1075,6 +1159,8 @@ TORCH_LIBRARY(kmoe, m) {
   m.def("dense_swiglu_bwd", &dense_swiglu_bwd);
   m.def("grouped_swiglu_fwd", &grouped_swiglu_fwd);
   m.def("grouped_swiglu_bwd", &grouped_swiglu_bwd);
+  m.def("mamba_inner_fwd", &mamba_inner_fwd);
+  m.def("mamba_inner_bwd", &mamba_inner_bwd);
   m.def("moe_plan", &moe_plan);
   m.def("moe_capacity_mask", &moe_capacity_mask);
   m.def("moe_balanced_assign", &moe_balanced_assign);

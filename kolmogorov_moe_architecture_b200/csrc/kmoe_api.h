@@ -165,6 +165,13 @@ int kmoe_conv1d_fwd(const void* x, const float* w, const float* bias, void* y, i
 int kmoe_conv1d_bwd(const void* x, const float* w, const float* bias, const void* dy, void* dx, float* dw,
                     float* dbias, int B, int S, int C, long long ldx, long long lddx, int act, int groups,
                     cudaStream_t st);
+// Small parameters of a mixer with C channels (all bf16 or all fp32) <-> flat fp32 buffers of 23 C:
+// A = -exp(A_log) [C,16] | conv weight [C,4] | conv bias | dt bias | D;  the gradients of A_log are dA * A.
+int kmoe_mamba_params(const void* A_log, const void* conv_w, const void* conv_b, const void* dt_b, const void* D, int is_bf16,
+                      float* out, int C, cudaStream_t st);
+int kmoe_mamba_params_bwd(const float* acc, const float* params, void* out, int is_bf16, int C, cudaStream_t st);
+// fp32 dB, dC [rows, 16] -> 32 bf16 columns at `out`, rows `ld` elements apart
+int kmoe_mamba_pack_bc(const float* dB, const float* dC, void* out, long long rows, long long ld, cudaStream_t st);
 // Selective scan.  The sequence is processed in kmoe_scan_segments(B, S, C) parallel segments.
 //   Bm, Cm: [B, S, N] with rows ldbc elements apart, bf16 (bc_bf16 != 0) or fp32, rows 16-byte aligned.
 //   ckpt (forward, optional): [B, ceil(S / kmoe_scan_chunk()), C, N] floats, the state before every chunk.

@@ -191,6 +191,43 @@ conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
   }
 }
 
+// ------------------------------------------------------------------ parameters
+// The mixer's small parameters as the kernels read them, in one launch instead of a cast per tensor: flat fp32
+//   A = -exp(A_log) [C,16] | conv weight [C,4] | conv bias [C] | dt bias [C] | D [C]
+// Their gradients accumulate in a buffer of the same layout; the second kernel turns it into the parameters' type, with
+// dA_log = dA * A.
+template <typename T>
+__global__ void mamba_params_kernel(const T* __restrict__ A_log, const T* __restrict__ conv_w, const T* __restrict__ conv_b,
+                                    const T* __restrict__ dt_b, const T* __restrict__ D, float* __restrict__ out, int C) {
+  const int n = C * 23;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    float v;
+    if (i < 16 * C) v = (float)-exp((double)(float)A_log[i]);   // not the fast-math expf
+    else if (i < 20 * C) v = (float)conv_w[i - 16 * C];
+    else if (i < 21 * C) v = (float)conv_b[i - 20 * C];
+    else if (i < 22 * C) v = (float)dt_b[i - 21 * C];
+    else v = (float)D[i - 22 * C];
+    out[i] = v;
+  }
+}
+template <typename T>
+__global__ void mamba_params_bwd_kernel(const float* __restrict__ acc, const float* __restrict__ params,
+                                        T* __restrict__ out, int C) {
+  const int n = C * 23;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    out[i] = (T)(i < 16 * C ? acc[i] * params[i] : acc[i]);
+}
+// fp32 rows dB | dC (two [rows, 16] arrays) -> the last 32 columns of bf16 rows `ld` apart
+__global__ void mamba_pack_bc_kernel(const float* __restrict__ dB, const float* __restrict__ dC,
+                                     __nv_bfloat16* __restrict__ out, long long rows, long long ld) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < rows * 8; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i >> 3;
+    const int q = (int)(i & 7);
+    const float4 v = *reinterpret_cast<const float4*>((q < 4 ? dB : dC) + r * 16 + (q & 3) * 4);
+    *reinterpret_cast<uint2*>(out + r * ld + q * 4) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+  }
+}
+
 static bool conv_pairs(const void* a, const void* b, const void* c, int C, long long ld1, long long ld2) {
   return C % 2 == 0 && ld1 % 2 == 0 && ld2 % 2 == 0 &&
          ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 3) == 0;
@@ -224,5 +261,36 @@ extern "C" int kmoe_conv1d_bwd(const void* x, const float* w, const float* bias,
   kern<<<conv_grid(B, S, C, two ? 2 : 1), 32 * CONV_WARPS, 0, st>>>((const __nv_bfloat16*)x, w, bias,
                                                                     (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, dw, dbias,
                                                                     S, C, ldx, lddx, act, B / groups);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+extern "C" int kmoe_mamba_params(const void* A_log, const void* conv_w, const void* conv_b, const void* dt_b, const void* D,
+                                 int is_bf16, float* out, int C, cudaStream_t st) {
+  const int grid = (C * 23 + 255) / 256;
+  if (is_bf16)
+    mamba_params_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)A_log, (const __nv_bfloat16*)conv_w,
+                                                             (const __nv_bfloat16*)conv_b, (const __nv_bfloat16*)dt_b,
+                                                             (const __nv_bfloat16*)D, out, C);
+  else
+    mamba_params_kernel<float><<<grid, 256, 0, st>>>((const float*)A_log, (const float*)conv_w, (const float*)conv_b,
+                                                     (const float*)dt_b, (const float*)D, out, C);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+extern "C" int kmoe_mamba_params_bwd(const float* acc, const float* params, void* out, int is_bf16, int C, cudaStream_t st) {
+  const int grid = (C * 23 + 255) / 256;
+  if (is_bf16)
+    mamba_params_bwd_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(acc, params, (__nv_bfloat16*)out, C);
+  else
+    mamba_params_bwd_kernel<float><<<grid, 256, 0, st>>>(acc, params, (float*)out, C);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+extern "C" int kmoe_mamba_pack_bc(const float* dB, const float* dC, void* out, long long rows, long long ld,
+                                  cudaStream_t st) {
+  if (ld % 4 || (reinterpret_cast<uintptr_t>(out) & 7)) return -1;
+  if (rows <= 0) return 0;
+  const long long grid = (rows * 8 + 255) / 256;
+  mamba_pack_bc_kernel<<<(unsigned)(grid < 148 * 8 ? grid : 148 * 8), 256, 0, st>>>(dB, dC, (__nv_bfloat16*)out, rows, ld);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

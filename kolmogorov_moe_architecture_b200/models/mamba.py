@@ -48,8 +48,19 @@ class Mamba(nn.Module):
         self.D = nn.Parameter(torch.ones(self.d_inner))
         self.out_proj = Linear(self.d_inner, d_model, bias=False)
 
+    def _plain_projections(self) -> bool:
+        """x_proj is the layer this class made, unhooked: then its weight may be used without calling it."""
+        m = self.x_proj
+        return type(m) is Linear and m.bias is None and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks
+                                                             or m._backward_pre_hooks)
+
     def forward(self, hidden_states: torch.Tensor) -> torch.Tensor:
         xz = self.in_proj(hidden_states)
+        if self._plain_projections():
+            y = ops.mamba_inner(xz, self.conv1d.weight, self.conv1d.bias, self.x_proj.weight, self.dt_proj.weight,
+                                self.dt_proj.bias, self.A_log, self.D)
+            if y is not None:
+                return self.out_proj(y)
         x, z = xz.chunk(2, dim=-1)
         x = ops.causal_conv1d(x, self.conv1d.weight.squeeze(1), self.conv1d.bias, activation=True)
         x_dbl = self.x_proj(x)

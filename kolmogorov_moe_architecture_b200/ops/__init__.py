@@ -113,6 +113,15 @@ def selective_scan(u, delta, A, Bm, Cm, D, z, delta_bias, delta_softplus=True):
     return eager.selective_scan(u, delta, A, Bm, Cm, D, z, delta_bias, delta_softplus)
 
 
+def mamba_inner(xz, conv_w, conv_b, xp_w, dt_w, dt_b, A_log, D):
+    """Convolution, x_proj, dt_proj and scan of a Mamba mixer as one pass on the GPU path; None where that does not cover
+    the call (the caller then composes the single ops)."""
+    if not xz.is_cuda or not _use_cuda(xz):
+        return None
+    from . import cuda_ops
+    return cuda_ops.mamba_inner(xz, conv_w, conv_b, xp_w, dt_w, dt_b, A_log, D)
+
+
 def grouped_swiglu(x, w1, w2, w3, idx, weights, keep=None, moe_dtype="bf16"):
     if x.shape[0] == 0:
         return x * 0

@@ -545,6 +545,55 @@ def selective_scan(u, delta, A, Bm, Cm, D, z, delta_bias, delta_softplus=True):
     return _Scan.apply(u, delta, A, Bm, Cm, D, z, delta_bias, bool(delta_softplus))
 
 
+class _MambaInner(torch.autograd.Function):
+    """The mixer between its in- and out-projection as one node: convolution, x_proj, dt_proj, scan.  As separate nodes the
+    two halves of ``d xz`` were concatenated, the convolution output's two gradients added, B and C cast and every small
+    parameter converted by kernels of their own; here the backward kernels write where the next one reads."""
+
+    @staticmethod
+    def forward(ctx, xz, conv_w, conv_b, xp_w, dt_w, dt_b, A_log, D, grad):
+        y, x, x_dbl, delta, params, ckpt, seg = K.mamba_inner_fwd(xz, conv_w, conv_b, xp_w, dt_w, dt_b, A_log, D, grad,
+                                                                  status_tensor(xz.device))
+        _count(5 + int(seg.numel() > 0))
+        if grad:
+            ctx.save_for_backward(xz, x, x_dbl, delta, params, ckpt, seg, xp_w, dt_w)
+            ctx.small = [(p.shape, p.dtype) for p in (A_log, conv_w, conv_b, dt_b, D)]
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        xz, x, x_dbl, delta, params, ckpt, seg, xp_w, dt_w = ctx.saved_tensors
+        T, dev = x.shape[0], x.device
+        s1, d1, kb1, kl1 = _wgrad_plan(xp_w, T, dev)
+        s2, d2, kb2, kl2 = _wgrad_plan(dt_w, T, dev)
+        dxz, dxp, ddt, dp = K.mamba_inner_bwd(dy, xz, x, x_dbl, delta, params, ckpt, seg, xp_w, dt_w,
+                                              ctx.small[0][1] == torch.bfloat16, d1, kb1, kl1, d2, kb2, kl2,
+                                              status_tensor(dev))
+        _count(8 + int(seg.numel() > 0))
+        for sink in (s1, s2):
+            if sink is not None:
+                sink[1]()
+        sizes = [shape.numel() for shape, _ in ctx.small]
+        dA_log, dcw, dcb, ddb, dD = [g.view(shape) for g, (shape, _) in zip(dp.split(sizes), ctx.small)]
+        return (dxz, dcw, dcb, None if s1 is not None else dxp, None if s2 is not None else ddt, ddb, dA_log, dD, None)
+
+
+def mamba_inner(xz, conv_w, conv_b, xp_w, dt_w, dt_b, A_log, D):
+    """Output of the mixer's scan for its in-projection ``xz`` (B, S, 2C), or None when the fused pass does not cover the
+    call: bf16 activations and projections, 16 states, convolution width 4, C % 64 and dt_rank % 8, small parameters all of
+    one type (bf16 or fp32)."""
+    C2, R = xz.shape[-1], dt_w.shape[1]
+    small = (conv_w, conv_b, dt_b, A_log, D)
+    if not (_bf16(xz) and _bf16(xp_w) and _bf16(dt_w) and xz.numel() > 0 and C2 % 128 == 0 and R % 8 == 0 and R > 0
+            and conv_b is not None and conv_w.shape[-1] == 4 and A_log.dim() == 2 and A_log.shape[-1] == 16
+            and A_log.dtype in (torch.bfloat16, torch.float32)
+            and all(p.dtype == A_log.dtype and p.is_contiguous() for p in small)
+            and xp_w.is_contiguous() and dt_w.is_contiguous()):
+        return None
+    grad = torch.is_grad_enabled() and any(t.requires_grad for t in (xz, xp_w, dt_w, *small))
+    return _MambaInner.apply(_aligned(xz.contiguous()), conv_w, conv_b, xp_w, dt_w, dt_b, A_log, D, grad)
+
+
 # ----------------------------------------------------------------- attention
 def attention(q, k, v, causal=True, doc_start=None):
     from . import attention_cuda
