@@ -131,24 +131,25 @@ rmsnorm_fwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
   }
 }
 
-template <int NCH, bool WITH_DW>
-__global__ void __launch_bounds__(256, WITH_DW ? 1 : 2)
+// A lane carries 8 NCH column sums beside the row itself, so the blocks are small - four warps, three blocks per SM up to
+// 1536 columns, two above (168 registers would spill) - and the warps' column sums meet in shared memory without atomics.  Traffic bound: 8192 x 2048
+// with a residual gradient 41.8 us with 8-warp blocks (one per SM) and shared atomics, 29.4 us this way, 20.5 at the copy
+// rate; 4096 x 1536, which had three generic kernels, forward + backward 38.6 -> 23.8 us.
+constexpr int NORM_BWD_WARPS = 4;
+template <int NCH>
+__global__ void __launch_bounds__(32 * NORM_BWD_WARPS, NCH <= 6 ? 3 : 2)
 rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                         const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd,
                         __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows,
                         const __nv_bfloat16* __restrict__ dres) {
   constexpr int D = NCH * 256;
-  __shared__ float sacc[D];
+  __shared__ __align__(16) float sacc[NORM_BWD_WARPS][D];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (WITH_DW) {
-    for (int i = threadIdx.x; i < D; i += 256) sacc[i] = 0.f;
-    __syncthreads();
-  }
   const __nv_bfloat16* wl = w + lane * 8;          // re-read per row (first-level cache hits): saves 4 NCH registers
-  float acc[WITH_DW ? NCH * 8 : 1];
+  float acc[NCH * 8];
 #pragma unroll
-  for (int i = 0; i < (WITH_DW ? NCH * 8 : 1); ++i) acc[i] = 0.f;
-  for (int row = blockIdx.x * 8 + warp; row < rows; row += gridDim.x * 8) {
+  for (int i = 0; i < NCH * 8; ++i) acc[i] = 0.f;
+  for (int row = blockIdx.x * NORM_BWD_WARPS + warp; row < rows; row += gridDim.x * NORM_BWD_WARPS) {
     const size_t base = (size_t)row * D + lane * 8;
     uint4 xq[NCH], gq[NCH];
 #pragma unroll
@@ -167,7 +168,7 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         dot += gv[i] * wv[i] * xv[i];
-        if (WITH_DW) acc[j * 8 + i] += gv[i] * xv[i] * r;
+        acc[j * 8 + i] += gv[i] * xv[i] * r;
       }
     }
     dot = warp_sum(dot);
@@ -189,13 +190,18 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
       *reinterpret_cast<uint4*>(dx + base + j * 256) = pack8(o);
     }
   }
-  if (WITH_DW) {
 #pragma unroll
-    for (int j = 0; j < NCH; ++j)
+  for (int j = 0; j < NCH; ++j)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) atomicAdd(&sacc[j * 256 + lane * 8 + i], acc[j * 8 + i]);
-    __syncthreads();
-    for (int i = threadIdx.x; i < D; i += 256) partial[(size_t)blockIdx.x * D + i] = sacc[i];
+    for (int i = 0; i < 8; i += 4)
+      *reinterpret_cast<float4*>(&sacc[warp][j * 256 + lane * 8 + i]) =
+          make_float4(acc[j * 8 + i], acc[j * 8 + i + 1], acc[j * 8 + i + 2], acc[j * 8 + i + 3]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < D; i += 32 * NORM_BWD_WARPS) {
+    float s = sacc[0][i];
+#pragma unroll
+    for (int q = 1; q < NORM_BWD_WARPS; ++q) s += sacc[q][i];
+    partial[(size_t)blockIdx.x * D + i] = s;
   }
 }
 
@@ -471,16 +477,22 @@ extern "C" int kmoe_add_rmsnorm_fwd(const void* x, const void* addend, const voi
   const int block = 256, wpb = block / 32;
   int grid = (rows + wpb - 1) / wpb;
   if (grid > 148 * 8) grid = 148 * 8;
-  if (rows > 0 && (d == 256 || d == 512 || d == 1024 || d == 2048)) {
+  if (rows > 0 && d % 256 == 0 && d <= 2048) {
     const int g2 = grid > 148 * 4 ? 148 * 4 : grid;
 #define KMOE_FWD_ROWS(NCH)                                                                                        \
   rmsnorm_fwd_rows_kernel<NCH><<<g2, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w,              \
                                                    (__nv_bfloat16*)y, rstd, rows, eps,                            \
                                                    (const __nv_bfloat16*)addend, (__nv_bfloat16*)sum_out)
-    if (d == 2048) KMOE_FWD_ROWS(8);
-    else if (d == 1024) KMOE_FWD_ROWS(4);
-    else if (d == 512) KMOE_FWD_ROWS(2);
-    else KMOE_FWD_ROWS(1);
+    switch (d / 256) {
+      case 8: KMOE_FWD_ROWS(8); break;
+      case 7: KMOE_FWD_ROWS(7); break;
+      case 6: KMOE_FWD_ROWS(6); break;
+      case 5: KMOE_FWD_ROWS(5); break;
+      case 4: KMOE_FWD_ROWS(4); break;
+      case 3: KMOE_FWD_ROWS(3); break;
+      case 2: KMOE_FWD_ROWS(2); break;
+      default: KMOE_FWD_ROWS(1);
+    }
 #undef KMOE_FWD_ROWS
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
@@ -499,7 +511,7 @@ extern "C" int kmoe_rmsnorm_fwd(const void* x, const void* w, void* y, float* rs
 // rows per CTA and sweep, at most two CTAs per SM).
 extern "C" int kmoe_rmsnorm_bwd_num_partials(int rows) {
   int r = (rows + 7) / 8;
-  return r > 296 ? 296 : (r < 1 ? 1 : r);
+  return r > 444 ? 444 : (r < 1 ? 1 : r);        // three small blocks per SM
 }
 
 // `partial` is scratch of kmoe_rmsnorm_bwd_num_partials(rows) * d floats.
@@ -516,36 +528,29 @@ extern "C" int kmoe_rmsnorm_bwd_res(const void* x, const void* w, const void* dy
   const int block = 256, wpb = block / 32;
   int grid = (rows + wpb - 1) / wpb;
   if (grid > 148 * 8) grid = 148 * 8;
-  static int rows_mode = -1;      // KMOE_NORM_ROWS: 0 = generic kernels, 1 = one fused pass, 2 = register-resident dx + separate dw
+  static int rows_mode = -1;      // KMOE_NORM_ROWS: 0 = generic kernels, 1 = one fused pass for whole 256-column chunks
   if (rows_mode < 0) {
     const char* e = getenv("KMOE_NORM_ROWS");
     rows_mode = e != nullptr ? atoi(e) : 1;
   }
-  if (rows_mode != 0 && rows > 0 && (d == 256 || d == 512 || d == 1024 || d == 2048)) {
-    const int g2 = kmoe_rmsnorm_bwd_num_partials(rows);
-    const bool fused = rows_mode == 1;
-#define KMOE_BWD_ROWS(NCH)                                                                                        \
-  do {                                                                                                            \
-    if (fused)                                                                                                    \
-      rmsnorm_bwd_rows_kernel<NCH, true><<<g2, 256, 0, st>>>(                                                     \
-          (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)dy, rstd, (__nv_bfloat16*)dx,   \
-          partial, rows, (const __nv_bfloat16*)dres);                                                             \
-    else                                                                                                          \
-      rmsnorm_bwd_rows_kernel<NCH, false><<<grid > 148 * 4 ? 148 * 4 : grid, 256, 0, st>>>(                       \
-          (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)dy, rstd, (__nv_bfloat16*)dx,   \
-          partial, rows, (const __nv_bfloat16*)dres);                                                             \
-  } while (0)
-    if (d == 2048) KMOE_BWD_ROWS(8);
-    else if (d == 1024) KMOE_BWD_ROWS(4);
-    else if (d == 512) KMOE_BWD_ROWS(2);
-    else KMOE_BWD_ROWS(1);
-#undef KMOE_BWD_ROWS
-    int parts = g2;
-    if (!fused) {
-      parts = g2 > 64 ? 64 : g2;
-      rmsnorm_dw_kernel<<<dim3((d + 255) / 256, parts), 256, 0, st>>>((const __nv_bfloat16*)x,
-                                                                      (const __nv_bfloat16*)dy, rstd, partial, rows, d);
+  if (rows_mode != 0 && rows > 0 && d % 256 == 0 && d <= 2048) {
+    int parts = kmoe_rmsnorm_bwd_num_partials(rows);
+    if (d > 1536 && parts > 296) parts = 296;      // two blocks per SM
+#define KMOE_BWD_ROWS(NCH)                                                                                       \
+  rmsnorm_bwd_rows_kernel<NCH><<<parts, 32 * NORM_BWD_WARPS, 0, st>>>(                                           \
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)dy, rstd, (__nv_bfloat16*)dx, partial, rows, \
+      (const __nv_bfloat16*)dres)
+    switch (d / 256) {
+      case 8: KMOE_BWD_ROWS(8); break;
+      case 7: KMOE_BWD_ROWS(7); break;
+      case 6: KMOE_BWD_ROWS(6); break;
+      case 5: KMOE_BWD_ROWS(5); break;
+      case 4: KMOE_BWD_ROWS(4); break;
+      case 3: KMOE_BWD_ROWS(3); break;
+      case 2: KMOE_BWD_ROWS(2); break;
+      default: KMOE_BWD_ROWS(1);
     }
+#undef KMOE_BWD_ROWS
     colsum_partials_kernel<<<colsum_grid(d), 256, 0, st>>>(partial, (__nv_bfloat16*)dw_bf16, dw_f32, parts, d);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }

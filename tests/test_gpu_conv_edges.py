@@ -24,3 +24,23 @@ def test_conv(B, S, C, act, off):
     want = (yr, *torch.autograd.grad(yr, (xr, wr, br), go.double()))
     for g, r in zip(got, want):
         assert ((g.double() - r).norm() / r.norm().clamp(min=1e-30)).item() < TOL
+
+
+@pytest.mark.parametrize("T,d", [(1, 256), (7, 768), (33, 1280), (4097, 1536), (130, 1792), (3000, 2048), (5, 1600)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_norm_rows(T, d, residual):
+    """RMSNorm at every register-resident width, a generic one, few and many rows (one, some and all blocks)."""
+    from kolmogorov_moe_architecture_b200 import ops
+    torch.manual_seed(T)
+    mk = lambda: torch.randn(T, d, device="cuda").to(torch.bfloat16)
+    x, a, g, gh = mk().requires_grad_(True), mk(), mk(), mk()
+    w = torch.randn(d, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    h, y = ops.residual_rmsnorm(x, a if residual else None, w, 1e-5)
+    got = (h, y, *torch.autograd.grad((h, y), (x, w), (gh, g)))
+    xr, wr = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    hr = xr + a.double() if residual else xr * 1
+    hr = hr + (h.detach().double() - hr.detach())                         # the norm works on the rounded sum
+    yr = wr * hr * torch.rsqrt(hr.square().mean(-1, keepdim=True) + 1e-5)
+    want = (hr, yr, *torch.autograd.grad((hr, yr), (xr, wr), (gh.double(), g.double())))
+    for u, v in zip(got, want):
+        assert ((u.double() - v).norm() / v.norm()).item() < TOL
