@@ -62,13 +62,50 @@ struct GemmArgs {
 
 struct Tile {
   int m_tile, n_tile, g_a, g_b, g_c, k0, k_blocks;
+  int row;        // first output row
+  int rows_ok;    // CTA pair on the expert-padded schedule: 0 = the lower 128 rows belong to the next expert
 };
+
+// CTA pairs on the expert-padded schedule: two consecutive 128-row blocks of one expert make a 256-row tile, the last
+// block of an expert with an odd count a tile of which only the upper half is stored.  list[i] = first block of tile i,
+// bit 15 set when the second block is the same expert's.  Built by one warp of each CTA from the block -> expert table
+// (four loads in flight per lane), returns the number of tiles.
+constexpr int PAIR_LIST_MAX = 768;
+__device__ __forceinline__ int build_pair_list(const int* __restrict__ tile_group, int blocks, uint16_t* list, int lane) {
+  int tiles = 0, run = 0, prev = -1;                 // carried: first block of the current run, its expert
+  for (int base = 0; base < blocks; base += 128) {
+    int g[4], nx[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int b = base + j * 32 + lane;
+      g[j] = b < blocks ? __ldg(tile_group + b) : -2;
+      nx[j] = b + 1 < blocks ? __ldg(tile_group + b + 1) : -2;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int b = base + j * 32 + lane;
+      int before = __shfl_up_sync(0xffffffffu, g[j], 1);
+      if (lane == 0) before = prev;
+      const uint32_t starts = __ballot_sync(0xffffffffu, g[j] != before);
+      const uint32_t upto = starts & (0xffffffffu >> (31 - lane));
+      const int my_run = upto ? base + j * 32 + 31 - __clz(upto) : run;
+      const bool first = b < blocks && ((b - my_run) & 1) == 0;
+      const uint32_t emit = __ballot_sync(0xffffffffu, first);
+      if (first) list[tiles + __popc(emit & ((1u << lane) - 1))] = (uint16_t)(b | (nx[j] == g[j] ? 0x8000 : 0));
+      tiles += __popc(emit);
+      run = __shfl_sync(0xffffffffu, my_run, 31);
+      prev = __shfl_sync(0xffffffffu, g[j], 31);
+    }
+  }
+  return tiles;
+}
 
 __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Maps a linear work index to a tile of TM x BN outputs. Returns false past the end.
 template <int BN, int TM = BM>
-__device__ __forceinline__ bool get_tile(const GemmArgs& a, int idx, int num_m, int num_n, Tile& t) {
+__device__ __forceinline__ bool get_tile(const GemmArgs& a, int idx, int num_m, int num_n, Tile& t,
+                                         const uint16_t* pair_list = nullptr) {
   const int n_out = (a.epilogue == KMOE_EPI_SWIGLU) ? BN / 2 : BN;
   (void)n_out;
   int per_group = num_m * num_n;
@@ -108,8 +145,17 @@ __device__ __forceinline__ bool get_tile(const GemmArgs& a, int idx, int num_m, 
   }
   t.k0 = 0;
   t.k_blocks = ceil_div(a.K, BK);
+  t.row = t.m_tile * TM;
+  t.rows_ok = 1;
   if (a.mode == KMOE_GEMM_GROUPED_M) {
-    int e = a.tile_group[t.m_tile];
+    int block = t.m_tile;
+    if (TM == 2 * BM) {
+      const int entry = pair_list[t.m_tile];
+      block = entry & 0x7fff;
+      t.row = block * BM;
+      t.rows_ok = entry >> 15;
+    }
+    int e = a.tile_group[block];
     t.g_a = 0;
     t.g_b = e;
     t.g_c = 0;
@@ -656,9 +702,13 @@ teardown:
 //
 // Barriers: `full` lives in the leader and is credited by both CTAs' loads; `empty` and `tmem_full` exist in
 // both CTAs and are signalled by the leader's commits (multicast arrive); `tmem_empty` lives in the leader
-// and collects the epilogue warps of both CTAs.  DENSE and BATCHED schedules, all epilogues except per-row
-// destination addresses.
+// and collects the epilogue warps of both CTAs.  All schedules, all epilogues except per-row destination addresses.
 constexpr int PAIR_TM = 2 * BM;
+// Expert-padded schedule: blocks per expert (counting the padding) from which pairs are taken.  Up / down / dH products
+// in µs, pairs against single CTAs, at d = 2048, f = 2816: 2.6 live blocks per expert 459/234/235 against 434/219/226,
+// 4.6 blocks 351/180/178 against 343/175/185, 6.4 blocks 309/157/156 against 310/165/167, 12.4 blocks 268/132/135 against
+// 272/141/149.
+constexpr int GROUPED_PAIR_MIN = 7;
 
 template <int BN, int A_MAJOR, int B_MAJOR>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
@@ -680,6 +730,8 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   __shared__ uint64_t tmem_full[2];
   __shared__ uint64_t tmem_empty[2];
   __shared__ uint32_t tmem_base_slot;
+  __shared__ uint16_t pair_list[PAIR_LIST_MAX];
+  __shared__ int pair_list_len;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -705,6 +757,10 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     tmem_alloc_pair(&tmem_base_slot, TMEM_COLS);
     tmem_relinquish_pair();
   }
+  if (warp == 2 && args.mode == KMOE_GEMM_GROUPED_M) {
+    const int n = build_pair_list(args.tile_group, min(ceil_div(args.M, BM), *args.num_m_tiles), pair_list, lane);
+    if (lane == 0) pair_list_len = n;
+  }
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                 // the peer's barriers exist before anything is signalled across
@@ -713,7 +769,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
   const bool swiglu = args.epilogue == KMOE_EPI_SWIGLU;
   const int n_per_tile = swiglu ? BN / 2 : BN;
-  const int num_m = ceil_div(args.M, PAIR_TM);
+  const int num_m = args.mode == KMOE_GEMM_GROUPED_M ? pair_list_len : ceil_div(args.M, PAIR_TM);
   const int num_n = ceil_div(args.N, n_per_tile);
 
   if (warp == 0) {
@@ -722,8 +778,8 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       int s = 0;
       uint32_t ph = 0;
       Tile t;
-      for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t); idx += num_pairs) {
-        const int arow = t.m_tile * PAIR_TM + (int)rank * BM;
+      for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, pair_list); idx += num_pairs) {
+        const int arow = t.row + (int)rank * BM;
         for (int kb = 0; kb < t.k_blocks; ++kb) {
           if (!mbar_wait(&empty_bar[s], ph ^ 1)) {
             atomicExch(args.status, 11);
@@ -759,7 +815,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       uint32_t ph = 0;
       int it = 0;
       Tile t;
-      for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t); idx += num_pairs) {
+      for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, pair_list); idx += num_pairs) {
         const int acc = it & 1;
         const uint32_t acc_ph = (it >> 1) & 1;
         ++it;
@@ -802,12 +858,13 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     int it = 0;
     Tile t;
     OutStage out{smem + stages * STAGE_BYTES + q * 2 * OUT_BUF_BYTES, 0};
-    for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t); idx += num_pairs) {
+    for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, pair_list); idx += num_pairs) {
       const int acc = it & 1;
       const uint32_t acc_ph = (it >> 1) & 1;
       ++it;
       const bool have_acc = t.k_blocks > 0;
-      const int row0 = t.m_tile * PAIR_TM + (int)rank * BM + q * 32;
+      // rows of another expert: past the end, so that nothing is stored
+      const int row0 = leader || t.rows_ok ? t.row + (int)rank * BM + q * 32 : args.M;
       const int row = row0 + lane;
       const bool row_ok = row < args.M;
       float scale = args.alpha;
@@ -1057,11 +1114,15 @@ extern "C" int kmoe_gemm(const KmoeGemmDesc* d, cudaStream_t stream) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  // CTA-pair kernel (256-row tiles): every schedule except the expert-padded one (its row blocks are 128 high
-  // and neighbouring blocks may belong to different experts) and per-row destination addresses
-  const bool pair = pair_enabled() && d->mode != KMOE_GEMM_GROUPED_M && d->c_row_ptr == nullptr && d->M > BM;
+  // CTA-pair kernel (256-row tiles): everything except per-row destination addresses.  On the expert-padded schedule
+  // (128-row blocks) an expert with an odd number of blocks wastes half a tile, at most `groups` blocks in all, so the
+  // pair is taken from GROUPED_PAIR_MIN blocks per expert up.
+  const bool grouped_pair = d->mode == KMOE_GEMM_GROUPED_M && m_tiles <= PAIR_LIST_MAX &&
+                            m_tiles >= (long long)GROUPED_PAIR_MIN * d->groups;
+  const bool pair = pair_enabled() && (d->mode != KMOE_GEMM_GROUPED_M || grouped_pair) && d->c_row_ptr == nullptr &&
+                    d->M > BM;
   const int TM = pair ? PAIR_TM : BM;
-  const long long tm_tiles = (d->M + TM - 1) / TM;
+  const long long tm_tiles = pair && grouped_pair ? (m_tiles + d->groups) / 2 : (d->M + TM - 1) / TM;
   const int units = pair ? sms / 2 : sms;       // CTAs or CTA pairs that run at once
   // 256-wide tiles unless that would leave most of the machine idle.  A CTA pair on 256 x 128 tiles asks the L2
   // for about 1.5x the bytes per FLOP of a 256 x 256 tile and runs at nearly the same time per reduction block,

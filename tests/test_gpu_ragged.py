@@ -201,3 +201,49 @@ def test_loss_vocabulary_slices(parts, monkeypatch):
               for i, (W, w) in enumerate(zip(rl[1:], (0.5, 0.3, 0.2))))
     for g, w in zip(got, torch.autograd.grad(ref, rl)):
         assert _rel(g, w) < EXPERT_TOL
+
+
+@pytest.mark.parametrize("blocks,spare,d,f,swiglu", [
+    ((8, 7, 6), 0, 256, 384, True),           # 21 blocks for 3 experts: the first count that takes CTA pairs
+    ((14, 1, 0, 11), 2, 192, 328, True),      # one-block and empty experts, odd ends, spare blocks after the live ones
+    ((33, 2, 94), 3, 128, 264, False),        # runs across the 32- and 128-block steps of the tile list
+    ((0, 0), 16, 128, 256, False),            # nothing routed here
+    ((500, 267), 1, 64, 64, False),           # the longest list
+    ((500, 268), 1, 64, 64, False),           # one more: single CTAs
+])
+def test_expert_blocks_in_pairs(blocks, spare, d, f, swiglu):
+    """256-row tiles over 128-row expert blocks: each expert's blocks in twos, an odd last one alone.  The products have
+    one bf16 rounding on fp32 sums of at most 2 * 256 terms: |error| <= 2^-8 |y| + 512 * 2^-24 * sum |terms|; the SwiGLU
+    value adds the rounding of nothing else (it is formed from the fp32 accumulators)."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(5)
+    E, live = len(blocks), sum(blocks)
+    rows = (live + spare) * 128
+    group = [e for e, n in enumerate(blocks) for _ in range(n)]
+    tiles = torch.tensor(group + [0] * spare, dtype=torch.int32, device="cuda")
+    nmt = torch.tensor([live], dtype=torch.int32, device="cuda")
+    x = torch.randn(rows, d, device="cuda").bfloat16()
+    x[live * 128:] = float("nan")                                    # never part of a live result
+    w1, w2 = (torch.randn(E, d, f, device="cuda").mul(d ** -0.5).bfloat16() for _ in range(2))
+    out = torch.full((rows, f), 7.0, dtype=torch.bfloat16, device="cuda")
+    kw = dict(mode=c.GROUPED_M, M=rows, N=f, groups=E, b_major=c.MAJ_MN, ldb=f, ldc=f, b_gs=d * f, tile_group=tiles,
+              num_m_tiles=nmt)
+    if swiglu:
+        c.gemm(x, w1, out, B2=w2, epi=c.EPI_SWIGLU, Kd=d, lda=d, **kw)
+    else:
+        xx = torch.cat([x, x], dim=1)                                # [x | x] [w1 ; w2] as one split reduction
+        c.gemm(xx, w1, out, B2=w2, k_split=d, Kd=2 * d, lda=2 * d, **kw)
+    c.check_status()
+    assert bool((out[live * 128:] == 7.0).all())
+    first = 0
+    for e, n in enumerate(blocks):
+        xs, o = x[first * 128:(first + n) * 128].double(), out[first * 128:(first + n) * 128].double()
+        first += n
+        g, u = xs @ w1[e].double(), xs @ w2[e].double()
+        mag = xs.abs() @ w1[e].double().abs(), xs.abs() @ w2[e].double().abs()
+        if swiglu:
+            y = torch.nn.functional.silu(g) * u
+            slack = 512 * 2.0 ** -24 * (1.1 * mag[0] * u.abs() + mag[1] * g.abs()) + 2.0 ** -20 * y.abs()   # fast exp
+        else:
+            y, slack = g + u, 512 * 2.0 ** -24 * (mag[0] + mag[1])
+        assert bool(((o - y).abs() <= 2.0 ** -8 * y.abs() + slack + 1e-30).all())
