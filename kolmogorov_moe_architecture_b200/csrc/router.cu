@@ -195,142 +195,7 @@ route_topk_bwd_kernel(const T_* __restrict__ logits, const float* __restrict__ l
 }
 
 // ---------------------------------------------------------------------------- per-row top-k
-// One CTA per row.  keys: value descending, index ascending on ties.
-__device__ __forceinline__ bool key_before(float va, int ia, float vb, int ib) {
-  return va > vb || (va == vb && ia < ib);
-}
-
-__global__ void seq_topk_fwd_kernel(const float* __restrict__ scores, long long row_stride, long long col_stride,
-                                    int rows_inner, long long outer_stride, int S, int S2, int k, int mode,
-                                    long long* __restrict__ idx_out, float* __restrict__ w_out,
-                                    float* __restrict__ stat_out) {
-  extern __shared__ float sm[];
-  float* val = sm;                                   // [S2]
-  int* ind = reinterpret_cast<int*>(sm + S2);        // [S2]
-  __shared__ float red[32];
-  __shared__ float s_mx, s_den;
-  const int r = blockIdx.x;
-  const float* base = scores + (long long)(r / rows_inner) * outer_stride + (long long)(r % rows_inner) * row_stride;
-  float mx = -CUDART_INF_F;
-  for (int i = threadIdx.x; i < S2; i += blockDim.x) {
-    const float v = i < S ? base[(long long)i * col_stride] : -CUDART_INF_F;
-    val[i] = v;
-    ind[i] = i < S ? i : 0x7fffffff;
-    mx = fmaxf(mx, v);
-  }
-  if (mode == 1) {                                   // softmax statistics of the whole row
-    mx = warp_max(mx);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      float m = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : -CUDART_INF_F;
-      m = warp_max(m);
-      if (threadIdx.x == 0) s_mx = m;
-    }
-    __syncthreads();
-    float den = 0.f;
-    for (int i = threadIdx.x; i < S; i += blockDim.x) den += __expf(val[i] - s_mx);
-    den = warp_sum(den);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = den;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      float d = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.f;
-      d = warp_sum(d);
-      if (threadIdx.x == 0) s_den = d;
-    }
-  }
-  __syncthreads();
-  // bitonic sort, best key first
-  for (int size = 2; size <= S2; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < (S2 >> 1); i += blockDim.x) {
-        const int lo = 2 * i - (i & (stride - 1));
-        const int hi = lo + stride;
-        const bool up = (lo & size) == 0;
-        const float va = val[lo], vb = val[hi];
-        const int ia = ind[lo], ib = ind[hi];
-        const bool a_first = key_before(va, ia, vb, ib);
-        if (a_first != up) {
-          val[lo] = vb; val[hi] = va;
-          ind[lo] = ib; ind[hi] = ia;
-        }
-      }
-      __syncthreads();
-    }
-  }
-  if (mode == 1) {
-    // top-k probabilities, descending; renormalised over the kept ones (+1e-9 as the reference)
-    float part = 0.f;
-    for (int i = threadIdx.x; i < k; i += blockDim.x) part += __expf(val[i] - s_mx) / s_den;
-    part = warp_sum(part);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
-    __syncthreads();
-    float tot = 0.f;
-    for (int i = 0; i < (blockDim.x >> 5); ++i) tot += red[i];
-    for (int i = threadIdx.x; i < k; i += blockDim.x) {
-      idx_out[(size_t)r * k + i] = ind[i];
-      w_out[(size_t)r * k + i] = (__expf(val[i] - s_mx) / s_den) / (tot + 1e-9f);
-    }
-    if (threadIdx.x == 0) {
-      stat_out[(size_t)r * 3 + 0] = s_mx;
-      stat_out[(size_t)r * 3 + 1] = s_den;
-      stat_out[(size_t)r * 3 + 2] = tot;
-    }
-    return;
-  }
-  // mode 0: the k-th key is the threshold; kept positions are emitted in ascending index order
-  const float thr_v = val[k - 1];
-  const int thr_i = ind[k - 1];
-  const float top = val[0];
-  __syncthreads();
-  // flags over original positions, reusing `ind` as a prefix-sum array after reloading the scores
-  for (int i = threadIdx.x; i < S2; i += blockDim.x) {
-    const float v = i < S ? base[(long long)i * col_stride] : -CUDART_INF_F;
-    val[i] = v;
-    ind[i] = (i < S && !key_before(thr_v, thr_i, v, i)) ? 1 : 0;   // keep iff key(i) is not after the threshold
-  }
-  __syncthreads();
-  // inclusive scan (Hillis-Steele over S2 entries, ping-pong avoided by chunked sequential-per-thread scan)
-  __shared__ int chunk_sum[1024];
-  const int per = (S2 + blockDim.x - 1) / blockDim.x;
-  const int b0 = threadIdx.x * per;
-  int acc = 0;
-  for (int i = b0; i < min(b0 + per, S2); ++i) acc += ind[i];
-  chunk_sum[threadIdx.x] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int i = 0; i < blockDim.x; ++i) { const int c = chunk_sum[i]; chunk_sum[i] = run; run += c; }
-  }
-  __syncthreads();
-  float den = 0.f;
-  int o = chunk_sum[threadIdx.x];
-  for (int i = b0; i < min(b0 + per, S2); ++i) {
-    if (ind[i]) {
-      const float ex = __expf(val[i] - top);
-      idx_out[(size_t)r * k + o] = i;
-      w_out[(size_t)r * k + o] = ex;               // normalised below
-      den += ex;
-      ++o;
-    }
-  }
-  den = warp_sum(den);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = den;
-  __syncthreads();
-  float tot = 0.f;
-  for (int i = 0; i < (blockDim.x >> 5); ++i) tot += red[i];
-  __threadfence_block();
-  __syncthreads();
-  for (int i = threadIdx.x; i < k; i += blockDim.x) w_out[(size_t)r * k + i] /= tot;
-}
-
-// Mode 0 without a sort: the k-th best key of the row is found by a 4-pass radix selection over
-// order-preserving 32-bit images of the scores (256-bin histograms in shared memory), then one block-wide
-// prefix count places the kept positions in ascending order.  Same result as the sorting kernel above: keys
-// compare by value descending and index ascending, so of the scores equal to the threshold the lowest
-// positions are kept.  (The images order -0.0 below +0.0.)
+// Order-preserving 32-bit images of the scores.
 __device__ __forceinline__ uint32_t score_key(float v) {
   const uint32_t u = __float_as_uint(v);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
@@ -339,6 +204,121 @@ __device__ __forceinline__ float key_score(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k);
 }
 
+// Expert choice: the k largest of a row's softmax, best first, lowest position first among equals.  One CTA per row,
+// a bitonic sort of 64-bit keys (score image, position).  Bound by the latency of its 66 stages at S = 2048 (the grid is
+// sequences x experts, mostly less than one wave): a warp takes the strides up to 32 of 64 neighbouring keys in
+// registers, so 20 stages of the 66 go through shared memory and a block barrier.  64 rows of 1536, k = 96:
+// 23.7 -> 12.4 us.
+__device__ __forceinline__ unsigned long long sort_key(float v, int i) {
+  uint32_t k = score_key(v);
+  if (v == 0.f) k = 0x80000000u;                     // -0 ties with +0
+  if (v != v) k = 0xffffffffu;                       // NaN first, as torch.topk
+  return ((unsigned long long)k << 32) | (0xffffffffu - (uint32_t)i);
+}
+__device__ __forceinline__ unsigned long long sort_step(unsigned long long k, int i, int size, int stride) {
+  const unsigned long long o = __shfl_xor_sync(0xffffffffu, k, stride);
+  const bool keep_larger = ((i & stride) == 0) == ((i & size) == 0);
+  return (k > o) == keep_larger ? k : o;
+}
+
+__global__ void __launch_bounds__(1024)
+seq_topk_softmax_kernel(const float* __restrict__ scores, long long row_stride, long long col_stride, int rows_inner,
+                        long long outer_stride, int S, int S2, int k, long long* __restrict__ idx_out,
+                        float* __restrict__ w_out, float* __restrict__ stat_out) {
+  extern __shared__ unsigned long long key[];        // [S2], S2 a power of two >= 64; padding sorts last
+  __shared__ float red[32];
+  __shared__ float s_mx, s_den;
+  const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const float* base = scores + (long long)(r / rows_inner) * outer_stride + (long long)(r % rows_inner) * row_stride;
+  float mx = -CUDART_INF_F;
+  for (int i = threadIdx.x; i < S2; i += blockDim.x) {
+    const float v = i < S ? base[(long long)i * col_stride] : -CUDART_INF_F;
+    key[i] = i < S ? sort_key(v, i) : (unsigned long long)(0xffffffffu - (uint32_t)i);
+    mx = fmaxf(mx, v);
+  }
+  auto score = [&](int i) { return key_score((uint32_t)(key[i] >> 32)); };
+  // softmax statistics of the whole row
+  mx = warp_max(mx);
+  if (lane == 0) red[warp] = mx;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    float m = lane < warps ? red[lane] : -CUDART_INF_F;
+    m = warp_max(m);
+    if (lane == 0) s_mx = m;
+  }
+  __syncthreads();
+  float den = 0.f;
+  for (int i = threadIdx.x; i < S; i += blockDim.x) den += __expf(score(i) - s_mx);
+  den = warp_sum(den);
+  if (lane == 0) red[warp] = den;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    float d = lane < warps ? red[lane] : 0.f;
+    d = warp_sum(d);
+    if (lane == 0) s_den = d;
+  }
+  for (int size = 64; size <= S2; size <<= 1) {
+    for (int stride = size >> 1; stride >= 64; stride >>= 1) {
+      for (int i = threadIdx.x; i < (S2 >> 1); i += blockDim.x) {
+        const int lo = 2 * i - (i & (stride - 1));
+        const int hi = lo + stride;
+        const unsigned long long a = key[lo], b = key[hi];
+        if ((a > b) != ((lo & size) == 0)) {
+          key[lo] = b;
+          key[hi] = a;
+        }
+      }
+      __syncthreads();
+    }
+    for (int seg = warp * 64; seg < S2; seg += warps * 64) {
+      const int i0 = seg + lane, i1 = i0 + 32;
+      unsigned long long k0 = key[i0], k1 = key[i1];
+      if (size == 64) {
+        for (int sz = 2; sz <= 32; sz <<= 1)
+          for (int stride = sz >> 1; stride > 0; stride >>= 1) {
+            k0 = sort_step(k0, i0, sz, stride);
+            k1 = sort_step(k1, i1, sz, stride);
+          }
+      }
+      if ((k0 > k1) != ((i0 & size) == 0)) {
+        const unsigned long long t = k0;
+        k0 = k1;
+        k1 = t;
+      }
+#pragma unroll
+      for (int stride = 16; stride > 0; stride >>= 1) {
+        k0 = sort_step(k0, i0, size, stride);
+        k1 = sort_step(k1, i1, size, stride);
+      }
+      key[i0] = k0;
+      key[i1] = k1;
+    }
+    __syncthreads();
+  }
+  // top-k probabilities, descending; renormalised over the kept ones (+1e-9 as the reference)
+  float part = 0.f;
+  for (int i = threadIdx.x; i < k; i += blockDim.x) part += __expf(score(i) - s_mx) / s_den;
+  part = warp_sum(part);
+  if (lane == 0) red[warp] = part;
+  __syncthreads();
+  float tot = 0.f;
+  for (int i = 0; i < warps; ++i) tot += red[i];
+  for (int i = threadIdx.x; i < k; i += blockDim.x) {
+    idx_out[(size_t)r * k + i] = (long long)(0xffffffffu - (uint32_t)key[i]);
+    w_out[(size_t)r * k + i] = (__expf(score(i) - s_mx) / s_den) / (tot + 1e-9f);
+  }
+  if (threadIdx.x == 0) {
+    stat_out[(size_t)r * 3 + 0] = s_mx;
+    stat_out[(size_t)r * 3 + 1] = s_den;
+    stat_out[(size_t)r * 3 + 2] = tot;
+  }
+}
+
+// Mode 0 without a sort: the k-th best key of the row is found by a 4-pass radix selection over
+// order-preserving 32-bit images of the scores (256-bin histograms in shared memory), then one block-wide
+// prefix count places the kept positions in ascending order.  Keys compare by value
+// descending and index ascending, so of the scores equal to the threshold the lowest
+// positions are kept.  (The images order -0.0 below +0.0.)
 __global__ void __launch_bounds__(1024)
 seq_topk_select_kernel(const float* __restrict__ scores, long long row_stride, long long col_stride, int rows_inner,
                        long long outer_stride, int S, int k, long long* __restrict__ idx_out,
@@ -560,13 +540,14 @@ extern "C" int kmoe_route_topk_bwd(const void* logits, int is_bf16, const float*
 extern "C" int kmoe_seq_topk_fwd(const float* scores, long long row_stride, long long col_stride, int rows_inner,
                                  long long outer_stride, int rows, int S, int k, int mode, long long* idx, float* w,
                                  float* stat, cudaStream_t st) {
-  const int S2 = next_pow2(S < 2 ? 2 : S);
+  const int S2 = next_pow2(S < 64 ? 64 : S);
   if (k < 1 || k > S || S2 > 16384) return -1;
   if (rows == 0) return 0;
   const size_t smem = (size_t)S2 * 8;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(seq_topk_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 8) != cudaSuccess)
+    if (cudaFuncSetAttribute(seq_topk_softmax_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 8) !=
+        cudaSuccess)
       return -3;
     if (cudaFuncSetAttribute(seq_topk_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4) !=
         cudaSuccess)
@@ -578,8 +559,8 @@ extern "C" int kmoe_seq_topk_fwd(const float* scores, long long row_stride, long
                                                               outer_stride, S, k, idx, w);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
-  seq_topk_fwd_kernel<<<rows, 1024, smem, st>>>(scores, row_stride, col_stride, rows_inner, outer_stride, S, S2, k,
-                                                mode, idx, w, stat);
+  seq_topk_softmax_kernel<<<rows, 1024, smem, st>>>(scores, row_stride, col_stride, rows_inner, outer_stride, S, S2, k,
+                                                    idx, w, stat);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -74,3 +74,34 @@ def test_combine(T, k, d, weighted):
     ref = torch.zeros(T, d, dtype=torch.double, device="cuda")
     ref.index_add_(0, at // k, Y.double() * scale[at, None])
     assert (out.double() - ref).norm() <= 4e-3 * ref.norm()
+
+
+@pytest.mark.parametrize("S,k", [(1, 1), (2, 1), (33, 33), (64, 5), (65, 64), (129, 17), (1536, 96), (16384, 700)])
+def test_softmax_topk(S, k):
+    """Order and positions are exact: larger first, lower position first among equals, -0 equal to +0."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    torch.manual_seed(S)
+    B, E = 2, 3
+    logits = torch.randn(B, S, E, device="cuda")
+    logits[0, :, 0] = (logits[0, :, 0] * 2).round() / 2                    # ties, both zeros
+    logits[0, ::2, 1] = float("-inf")                                      # masked positions (the last expert has none)
+    if S > 2:
+        logits[1, :, 2] = torch.tensor([0.0, -0.0], device="cuda").repeat(S)[:S]
+    w, tok = cuda_ops.expert_choice_route(logits, k)
+    x = logits.transpose(1, 2).double()
+    order = torch.sort(x, dim=-1, descending=True, stable=True).indices[..., :k]
+    assert torch.equal(tok, order)
+    p = torch.softmax(x, -1).gather(-1, order)
+    ref = p / (p.sum(-1, keepdim=True) + 1e-9)
+    ok = torch.isfinite(ref).all(-1)                                       # S = 1: a row of -inf alone has no softmax
+    # 32-bit sums of at most 16384 exponentials with a relative error of 2^-21 each (the fast exponential at |x| < 20)
+    assert ((w.double() - ref).abs() <= 1e-5 * ref + 1e-30)[ok].all()
+
+
+@pytest.mark.parametrize("at", [0, 40])
+def test_softmax_topk_keeps_positions_valid_with_nan(at):
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    logits = torch.randn(1, 50, 1, device="cuda")
+    logits[0, at, 0] = -float("nan")
+    _, tok = cuda_ops.expert_choice_route(logits, 50)
+    assert tok[0, 0, 0] == at and torch.equal(tok.sort(dim=-1).values[0, 0], torch.arange(50, device="cuda"))
