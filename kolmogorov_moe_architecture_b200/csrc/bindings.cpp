@@ -437,6 +437,41 @@ Tensor moe_combine(const Tensor& Y, const Tensor& pos, const OptT& w, int64_t T,
   return out;
 }
 
+// (dY, dw): C > 0 = expert choice, dw in (sequence, expert, pick) order
+std::tuple<Tensor, Tensor> moe_gather_dw(const Tensor& dout, const Tensor& row_src, const Tensor& w, const Tensor& Y,
+                                         const Tensor& meta, const Tensor& pos, int64_t k, int64_t B, int64_t C) {
+  c10::cuda::CUDAGuard guard(dout.device());
+  need_bf16(dout, "dout"); need_bf16(Y, "Y");
+  TORCH_CHECK(dout.is_contiguous() && dout.dim() == 2 && Y.is_contiguous() && Y.dim() == 2 && Y.size(1) == dout.size(1) &&
+              Y.size(0) == row_src.numel() && w.scalar_type() == at::kFloat && w.is_contiguous() &&
+              w.numel() == pos.numel(), "combine backward: shapes do not match");
+  const int max_rows = row_src.numel(), d = dout.size(1), n = pos.numel();
+  TORCH_CHECK(C == 0 || max_rows == B * k * C, "combine backward: rows do not match the picks");
+  Tensor dY = at::empty({max_rows, d}, dout.options());
+  Tensor dw = at::empty({C > 0 ? max_rows : n}, dout.options().dtype(at::kFloat));
+  check(kmoe_moe_gather_dw(dout.data_ptr(), row_src.data_ptr<int>(), w.data_ptr<float>(), Y.data_ptr(),
+                           meta.data_ptr<int>(), pos.data_ptr<int>(), dY.data_ptr(), dw.data_ptr<float>(), max_rows, n, d,
+                           (int)k, (int)B, (int)C, cur_stream()), "moe_gather_dw");
+  return {dY, dw};
+}
+
+// tok, wts (B, E, C) -> (row_src, pos, weight, meta)
+std::tuple<Tensor, Tensor, Tensor, Tensor> moe_choice_plan(const Tensor& tok, const Tensor& wts, int64_t S, int64_t T,
+                                                           const Tensor& status) {
+  c10::cuda::CUDAGuard guard(tok.device());
+  TORCH_CHECK(tok.is_cuda() && tok.dim() == 3 && wts.is_cuda() && wts.sizes() == tok.sizes(),
+              "expert choice: tokens and weights, both (sequences, experts, picks)");
+  const Tensor tk = tok.to(at::kLong).contiguous(), wf = wts.to(at::kFloat).contiguous();
+  const int64_t B = tok.size(0), E = tok.size(1), C = tok.size(2);
+  auto i32 = tok.options().dtype(at::kInt);
+  Tensor row_src = at::empty({B * E * C}, i32), pos = at::empty({T * E}, i32), meta = at::empty({2}, i32);
+  Tensor weight = at::empty({T * E}, wf.options());
+  check(kmoe_moe_choice_plan((const long long*)tk.data_ptr<int64_t>(), wf.data_ptr<float>(), row_src.data_ptr<int>(),
+                             pos.data_ptr<int>(), weight.data_ptr<float>(), meta.data_ptr<int>(), (int)B, (int)E, (int)C,
+                             (int)S, (int)T, status.data_ptr<int>(), cur_stream()), "moe_choice_plan");
+  return {row_src, pos, weight, meta};
+}
+
 Tensor moe_combine_dw(const Tensor& Y, const Tensor& dout, const Tensor& pos, int64_t k) {
   c10::cuda::CUDAGuard guard(Y.device());
   need_bf16(Y, "Y"); need_bf16(dout, "dout");
@@ -905,8 +940,7 @@ std::vector<Tensor> grouped_swiglu_bwd(const Tensor& dout_in, const Tensor& Xp, 
   const Tensor dout = dout_in.contiguous();
   const int64_t T = dout.size(0), d = dout.size(1), E = w1.size(0), f = w1.size(2), R = row_src.numel();
   const Tensor live = meta.narrow(0, 1, 1);
-  Tensor dYp = moe_gather_rows(dout, row_src, wf, meta, k);
-  Tensor dwts = moe_combine_dw(Y, dout, pos, k);
+  auto [dYp, dwts] = moe_gather_dw(dout, row_src, wf, Y, meta, pos, k, 0, 0);
   auto grouped = [&](Gemm& g, int64_t gs) {
     g.d.mode = KMOE_GEMM_GROUPED_M; g.d.groups = (int)E; g.d.b_gstride = gs;
     g.d.tile_group = tile_group.data_ptr<int>(); g.d.num_m_tiles = meta.data_ptr<int>();
@@ -1167,6 +1201,8 @@ TORCH_LIBRARY(kmoe, m) {
   m.def("moe_gather_rows", &moe_gather_rows);
   m.def("moe_combine", &moe_combine);
   m.def("moe_combine_dw", &moe_combine_dw);
+  m.def("moe_gather_dw", &moe_gather_dw);
+  m.def("moe_choice_plan", &moe_choice_plan);
   m.def("ce_fwd_bwd", &ce_fwd_bwd);
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);

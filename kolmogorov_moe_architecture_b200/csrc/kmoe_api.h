@@ -204,6 +204,14 @@ int kmoe_moe_gather_rows(const void* src, const int* row_src, const float* assig
 int kmoe_moe_combine(const void* Y, const int* pos, const float* w, void* out, int T, int k, int d, cudaStream_t st);
 int kmoe_moe_combine_dw(const void* Y, const void* dout, const int* pos, float* dw, int n, int k, int d,
                         cudaStream_t st);
+// dY[row] = w[row_src[row]] * dout[row_src[row] / k] and dw, the weights' gradients: one per assignment (n of them; pos
+// gives those without a row), or with C > 0 in (sequence, expert, pick) order for B sequences and C picks (pos unused)
+int kmoe_moe_gather_dw(const void* dout, const int* row_src, const float* w, const void* Y, const int* meta,
+                       const int* pos, void* dY, float* dw, int max_rows, int n, int d, int k, int B, int C,
+                       cudaStream_t st);
+// expert choice (tok, wts: B x E x C, T = B * S tokens): row_src [E * B * C], pos [T * E], weight [T * E], meta [2]
+int kmoe_moe_choice_plan(const long long* tok, const float* wts, int* row_src, int* pos, float* weight, int* meta, int B,
+                         int E, int C, int S, int T, int* status, cudaStream_t st);
 
 // ----------------------------------------------------------------------- attention
 // Causal GQA flash attention. q/out/dq [B,S,H,D], k/v/dk/dv [B,S,Hkv,D] bf16; lse [B,H,S] fp32; D in {64,128}.

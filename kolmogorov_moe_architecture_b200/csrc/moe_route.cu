@@ -209,59 +209,164 @@ __global__ void moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ src, co
   }
 }
 
-// out[t] = sum_k w[t,k] * Y[pos[t,k]]   (pos < 0 skipped; w null = 1).  One warp per token.  The lanes fetch the token's
-// positions and weights together, then all rows that exist are read with four 16-byte loads per lane in flight; expert
-// choice calls this with k = experts and mostly empty slots.  6144 x 2048, two rows each: 26 -> 16 us.
+// out[t] = sum_k w[t,k] * Y[pos[t,k]]   (pos < 0 skipped; w null = 1).  Bound by memory latency: one warp per 512 columns
+// of a token, two rows of it in flight (a lane holds four 16-byte loads), added in slot order.  Expert choice calls this
+// with k = experts and mostly empty slots, a few tokens having many; a whole row per warp made those the tail of the
+// launch.  6144 x 2048: two rows each 16.4 -> 15.1 us (26 with one load per lane), one row each among 16 slots 20.7 ->
+// 13.5 us.
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const __nv_bfloat16* __restrict__ Y, const int* __restrict__ pos, const float* __restrict__ w,
                    __nv_bfloat16* __restrict__ out, int T, int k, int d) {
-  constexpr int U = 4;
+  constexpr int U = 2;
   const int vec = d / 8;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
+  const int chunks = (vec + 32 * U - 1) / (32 * U);
+  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
-  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < T; t += warps) {
-    for (int v0 = 0; v0 < vec; v0 += 32 * U) {
-      float acc[U][8];
+  for (long long wi = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; wi < (long long)T * chunks; wi += warps) {
+    const int t = (int)(wi / chunks);
+    const int v0 = (int)(wi - (long long)t * chunks) * 32 * U + lane;
+    float acc[U][8];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[u][i] = 0.f;
-      for (int j0 = 0; j0 < k; j0 += 32) {
-        const int pj = j0 + lane < k ? pos[(size_t)t * k + j0 + lane] : -1;
-        const float wj = (w != nullptr && j0 + lane < k) ? w[(size_t)t * k + j0 + lane] : 1.f;
-        for (unsigned m = __ballot_sync(0xffffffffu, pj >= 0); m != 0; m &= m - 1) {
-          const int j = __ffs(m) - 1;
-          const int p = __shfl_sync(0xffffffffu, pj, j);
-          const float s = __shfl_sync(0xffffffffu, wj, j);
-          const uint4* row = reinterpret_cast<const uint4*>(Y + (size_t)p * d);
-          uint4 r[U];
+      for (int i = 0; i < 8; ++i) acc[u][i] = 0.f;
+    for (int j0 = 0; j0 < k; j0 += 32) {
+      const int pj = j0 + lane < k ? pos[(size_t)t * k + j0 + lane] : -1;
+      const float wj = (w != nullptr && pj >= 0) ? w[(size_t)t * k + j0 + lane] : 1.f;
+      unsigned m = __ballot_sync(0xffffffffu, pj >= 0);
+      while (m != 0) {
+        int p[2];
+        float s[2];
+        uint4 r[2][U];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int j = m != 0 ? __ffs(m) - 1 : -1;
+          m &= m - 1;
+          p[q] = __shfl_sync(0xffffffffu, pj, j & 31);
+          s[q] = __shfl_sync(0xffffffffu, wj, j & 31);
+          if (j < 0) p[q] = -1;
 #pragma unroll
           for (int u = 0; u < U; ++u) {
-            const int v = v0 + u * 32 + lane;
-            r[u] = v < vec ? __ldg(row + v) : make_uint4(0, 0, 0, 0);
+            const int v = v0 + u * 32;
+            r[q][u] = p[q] >= 0 && v < vec ? __ldg(reinterpret_cast<const uint4*>(Y + (size_t)p[q] * d) + v)
+                                           : make_uint4(0, 0, 0, 0);
           }
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (p[q] < 0) break;
 #pragma unroll
           for (int u = 0; u < U; ++u) {
-            const __nv_bfloat162* q = reinterpret_cast<const __nv_bfloat162*>(&r[u]);
+            const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&r[q][u]);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const float2 f = __bfloat1622float2(q[i]);
-              acc[u][2 * i] += s * f.x;
-              acc[u][2 * i + 1] += s * f.y;
+              const float2 f = __bfloat1622float2(b[i]);
+              acc[u][2 * i] += s[q] * f.x;
+              acc[u][2 * i + 1] += s[q] * f.y;
             }
           }
         }
       }
+    }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int v = v0 + u * 32 + lane;
-        if (v < vec)
-          *reinterpret_cast<uint4*>(out + (size_t)t * d + v * 8) =
-              make_uint4(pack_bf16(acc[u][0], acc[u][1]), pack_bf16(acc[u][2], acc[u][3]), pack_bf16(acc[u][4], acc[u][5]),
-                         pack_bf16(acc[u][6], acc[u][7]));
+    for (int u = 0; u < U; ++u) {
+      const int v = v0 + u * 32;
+      if (v < vec)
+        *reinterpret_cast<uint4*>(out + (size_t)t * d + v * 8) =
+            make_uint4(pack_bf16(acc[u][0], acc[u][1]), pack_bf16(acc[u][2], acc[u][3]), pack_bf16(acc[u][4], acc[u][5]),
+                       pack_bf16(acc[u][6], acc[u][7]));
+    }
+  }
+}
+
+// Backward of the weighted combine in one pass over the rows: dY[row] = w[a] * dout[t] and dw = <dout[t], Y[row]>, with
+// a = row_src[row] and t = a / k.  Bound by memory; as two kernels dout's rows were read twice and the dot products ran
+// over k slots per token although only the rows exist.  One warp per row, four loads of each side in flight.
+// dw is written at a (assignments without a row: 0), or, where C > 0 (expert choice: B sequences, C picks each, rows in
+// (expert, sequence, pick) order), at (sequence, expert, pick).
+// Against the two kernels: 12288 rows of 2048 33.5 -> 22.5 us, 6144 rows among 16 slots 35 -> 14.8 us.
+__global__ void __launch_bounds__(256)
+moe_gather_dw_kernel(const __nv_bfloat16* __restrict__ dout, const int* __restrict__ row_src, const float* __restrict__ w,
+                     const __nv_bfloat16* __restrict__ Y, const int* __restrict__ meta, const int* __restrict__ pos,
+                     __nv_bfloat16* __restrict__ dY, float* __restrict__ dw, int max_rows, int n, int d, int k, int B,
+                     int C) {
+  constexpr int U = 4;
+  const int live_rows = min(meta[1], max_rows);
+  const int vec = d / 8;
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < live_rows; row += warps) {
+    const int a = row_src[row];
+    uint4* orow = reinterpret_cast<uint4*>(dY + (size_t)row * d);
+    float dot = 0.f;
+    if (a < 0) {
+      for (int v = lane; v < vec; v += 32) orow[v] = make_uint4(0, 0, 0, 0);
+    } else {
+      const uint4* grow = reinterpret_cast<const uint4*>(dout + (size_t)(a / k) * d);
+      const uint4* yrow = reinterpret_cast<const uint4*>(Y + (size_t)row * d);
+      const float s = w[a];
+      for (int v0 = lane; v0 < vec; v0 += 32 * U) {
+        uint4 g[U], y[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int v = v0 + u * 32;
+          g[u] = v < vec ? __ldg(grow + v) : make_uint4(0, 0, 0, 0);
+          y[u] = v < vec ? __ldg(yrow + v) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int v = v0 + u * 32;
+          if (v >= vec) break;
+          __nv_bfloat162* q1 = reinterpret_cast<__nv_bfloat162*>(&g[u]);
+          const __nv_bfloat162* q2 = reinterpret_cast<const __nv_bfloat162*>(&y[u]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 f = __bfloat1622float2(q1[i]), h = __bfloat1622float2(q2[i]);
+            dot += f.x * h.x + f.y * h.y;
+            q1[i] = __floats2bfloat162_rn(f.x * s, f.y * s);
+          }
+          orow[v] = g[u];
+        }
+      }
+      dot = warp_sum(dot);
+    }
+    if (lane == 0) {
+      if (C > 0) {
+        const int e = row / (B * C), b = row / C - e * B;
+        dw[((size_t)b * k + e) * C + row % C] = dot;
+      } else if (a >= 0) {
+        dw[a] = dot;
       }
     }
   }
+  if (C == 0)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+      if (pos[i] < 0) dw[i] = 0.f;
+}
+
+// Expert choice in the bookkeeping of token choice with k = E: row (e, b, c) holds token b * S + tok[b][e][c] of the T
+// tokens.  row_src[row] = assignment t * E + e, pos[assignment] = row (preset to -1), weight[assignment] = wts[b][e][c];
+// the weights of assignments without a row are never read.  A token outside [0, T) leaves its row empty and sets the
+// status.  One launch in place of a dozen elementwise and indexing ones.
+__global__ void moe_choice_plan_kernel(const long long* __restrict__ tok, const float* __restrict__ wts,
+                                       int* __restrict__ row_src, int* __restrict__ pos, float* __restrict__ weight,
+                                       int* __restrict__ meta, int B, int E, int C, int S, int T,
+                                       int* __restrict__ status) {
+  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+  if (row < 2) meta[row] = E * B * C;
+  if (row >= E * B * C) return;
+  const int e = row / (B * C), b = row / C - e * B, c = row % C;
+  const size_t src = ((size_t)b * E + e) * C + c;
+  const long long t = tok[src] + (long long)b * S;
+  if (t < 0 || t >= T) {
+    row_src[row] = -1;
+    atomicExch(status, 31);
+    return;
+  }
+  const int a = (int)t * E + e;
+  row_src[row] = a;
+  pos[a] = row;
+  weight[a] = wts[src];
 }
 
 // dw[t,k] = <dout[t], Y[pos[t,k]]>.  One warp per assignment.
@@ -357,9 +462,30 @@ extern "C" int kmoe_moe_combine(const void* Y, const int* pos, const float* w, v
                                 cudaStream_t st) {
   if (d % 8) return -1;
   if (T <= 0) return 0;
-  const int grid = (T + 7) / 8;
-  moe_combine_kernel<<<grid < 148 * 8 ? grid : 148 * 8, 256, 0, st>>>((const __nv_bfloat16*)Y, pos, w, (__nv_bfloat16*)out,
-                                                                      T, k, d);
+  const long long units = (long long)T * ((d / 8 + 63) / 64);
+  const int grid = (int)((units + 7) / 8 < 148 * 8 ? (units + 7) / 8 : 148 * 8);
+  moe_combine_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)Y, pos, w, (__nv_bfloat16*)out, T, k, d);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+extern "C" int kmoe_moe_gather_dw(const void* dout, const int* row_src, const float* w, const void* Y, const int* meta,
+                                  const int* pos, void* dY, float* dw, int max_rows, int n, int d, int k, int B, int C,
+                                  cudaStream_t st) {
+  if (d % 8 || k < 1 || (C == 0 && pos == nullptr)) return -1;
+  if (max_rows <= 0) return 0;
+  const int grid = (max_rows + 7) / 8;
+  moe_gather_dw_kernel<<<grid < 148 * 8 ? grid : 148 * 8, 256, 0, st>>>((const __nv_bfloat16*)dout, row_src, w,
+                                                                        (const __nv_bfloat16*)Y, meta, pos,
+                                                                        (__nv_bfloat16*)dY, dw, max_rows, n, d, k, B, C);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+extern "C" int kmoe_moe_choice_plan(const long long* tok, const float* wts, int* row_src, int* pos, float* weight,
+                                    int* meta, int B, int E, int C, int S, int T, int* status, cudaStream_t st) {
+  if ((long long)T * E > 0x7fffffff || (long long)B * E * C > 0x7fffff00) return -1;
+  if (cudaMemsetAsync(pos, 0xff, (size_t)T * E * sizeof(int), st) != cudaSuccess) return -2;
+  const int rows = B * E * C;
+  moe_choice_plan_kernel<<<(rows + 255) / 256, 256, 0, st>>>(tok, wts, row_src, pos, weight, meta, B, E, C, S, T, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -673,15 +673,7 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
         f = w1.shape[2]
         BC = B * C
         dev = x2.device
-        t_glob = tok + (torch.arange(B, device=dev) * S).view(B, 1, 1)             # token row in x2
-        a = t_glob * E + torch.arange(E, device=dev).view(1, E, 1)                 # assignment id = t * E + e
-        a_rows = a.permute(1, 0, 2).reshape(-1)                                     # rows ordered (e, b, c)
-        row_src = a_rows.to(torch.int32)
-        pos = torch.full((T * E,), -1, dtype=torch.int32, device=dev)
-        pos[a_rows] = torch.arange(E * BC, dtype=torch.int32, device=dev)
-        wdense = torch.zeros(T * E, dtype=torch.float32, device=dev)
-        wdense[a_rows] = wts.permute(1, 0, 2).reshape(-1).float()
-        meta = torch.full((2,), E * BC, dtype=torch.int32, device=dev)          # [1] = live rows
+        row_src, pos, wdense, meta = K.moe_choice_plan(tok, wts, S, T, status_tensor(dev))   # rows ordered (e, b, c)
         Xg = K.moe_gather_rows(x2.contiguous(), row_src, None, meta, E)
         H = torch.empty(E * BC, f, dtype=x2.dtype, device=dev)
         G, U = torch.empty_like(H), torch.empty_like(H)
@@ -691,19 +683,20 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
         gemm(H, w3, Y, mode=BATCHED, groups=E, M=BC, N=d, Kd=f, b_major=MAJ_MN, lda=f, ldb=d, ldc=d,
              a_gs=BC * f, b_gs=f * d, c_gs=BC * d)
         out = K.moe_combine(Y, pos, wdense, T, E)
-        _count(2)
-        ctx.save_for_backward(Xg, G, U, Y, w1, w2, w3, wdense, pos, row_src, meta, a)
-        ctx.dims = (T, d, E, f, BC)
+        _count(3)
+        keep_h = os.environ.get("KMOE_MOE_KEEP_H", "1") != "0"                    # as in _GroupedSwiGLU
+        ctx.save_for_backward(Xg, G, U, Y, w1, w2, w3, wdense, pos, row_src, meta, *((H,) if keep_h else ()))
+        ctx.dims = (T, d, E, f, B, C)
         ctx.wdtype = wts.dtype
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        Xg, G, U, Y, w1, w2, w3, wdense, pos, row_src, meta, a = ctx.saved_tensors
-        T, d, E, f, BC = ctx.dims
-        dout = dout.contiguous()
-        dY = K.moe_gather_rows(dout, row_src, wdense, meta, E)
-        dwts = K.moe_combine_dw(Y, dout, pos, E)[a].to(ctx.wdtype)                  # (B, E, C)
+        Xg, G, U, Y, w1, w2, w3, wdense, pos, row_src, meta, *kept = ctx.saved_tensors
+        T, d, E, f, B, C = ctx.dims
+        BC = B * C
+        dY, dwts = K.moe_gather_dw(dout.contiguous(), row_src, wdense, Y, meta, pos, E, B, C)
+        dwts = dwts.view(B, E, C).to(ctx.wdtype)
         dH = torch.empty(E * BC, f, dtype=dout.dtype, device=dout.device)
         gemm(dY, w3, dH, mode=BATCHED, groups=E, M=BC, N=f, Kd=d, lda=d, ldb=d, ldc=f,
              a_gs=BC * d, b_gs=f * d, c_gs=BC * f)
@@ -714,7 +707,7 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
         gemm(dGU, w1, dXg, B2=w2, mode=BATCHED, groups=E, M=BC, N=d, Kd=2 * P, k_split=P, b_klen=f, lda=2 * P, ldb=f,
              ldc=d, a_gs=BC * 2 * P, b_gs=d * f, c_gs=BC * d)
         dx = K.moe_combine(dXg, pos, None, T, E)
-        H = K.swiglu_fwd(G, U, None)
+        H = kept[0] if kept else K.swiglu_fwd(G, U, None)
         sinks = [grad_sink(w) for w in (w1, w2, w3)]
         dw1, dw2, dw3 = [s_[0] if s_ is not None else torch.empty_like(w) for s_, w in zip(sinks, (w1, w2, w3))]
         common = dict(mode=BATCHED, groups=E, a_major=MAJ_MN, b_major=MAJ_MN, Kd=BC)

@@ -243,8 +243,8 @@ class _GroupedSwiGLUMX(torch.autograd.Function):
         nmt, live = meta[0:1], meta[1:2]
         dout = dout.contiguous()
         grp = dict(mode=C.GROUPED_M, groups=E, b_grouped=True, tile_group=tile_group, num_m_tiles=nmt)
-        dYp = K.moe_gather_rows(dout, row_src, wf, meta, k)
-        dwts = K.moe_combine_dw(Y, dout, pos, k).view(T, k).to(ctx.wdtype)
+        dYp, dwts = K.moe_gather_dw(dout, row_src, wf, Y, meta, pos, k, 0, 0)
+        dwts = dwts.view(T, k).to(ctx.wdtype)
         dYq, sdY = quant_rows(dYp, live_rows=live)
         W3r, s3r = _weight_quant(w3, "rows")                  # (E, f, d): reduction over d
         dH = torch.empty(R, f, dtype=dout.dtype, device=dout.device)

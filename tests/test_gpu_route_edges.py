@@ -105,3 +105,53 @@ def test_softmax_topk_keeps_positions_valid_with_nan(at):
     logits[0, at, 0] = -float("nan")
     _, tok = cuda_ops.expert_choice_route(logits, 50)
     assert tok[0, 0, 0] == at and torch.equal(tok.sort(dim=-1).values[0, 0], torch.arange(50, device="cuda"))
+
+
+@pytest.mark.parametrize("T,k,d", [(1, 1, 8), (37, 2, 264), (200, 4, 2048), (65, 3, 1032)])
+def test_gather_with_weight_gradient(T, k, d):
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    torch.manual_seed(d)
+    E = 5
+    idx = torch.randint(0, E, (T * k,), device="cuda")
+    keep = torch.rand(T * k, device="cuda") < 0.7
+    pos, row_src, _, _, _, meta = cuda_ops.K.moe_plan(idx, keep, E, 0)
+    rows = row_src.numel()
+    Y = torch.randn(rows, d, device="cuda").bfloat16()
+    Y[row_src < 0] = float("nan")                                          # never read
+    dout, w = torch.randn(T, d, device="cuda").bfloat16(), torch.rand(T * k, device="cuda")
+    dY, dw = cuda_ops.K.moe_gather_dw(dout, row_src, w, Y, meta, pos, k, 0, 0)
+    live = int(meta[1])
+    a = row_src[:live].long()
+    ref = torch.where((a >= 0)[:, None], dout[a.clamp(min=0) // k].float() * w[a.clamp(min=0), None], 0.0).bfloat16()
+    assert torch.equal(dY[:live], ref)                                     # one product, one rounding
+    p = pos.long()
+    prod = torch.where((p >= 0)[:, None], dout.double().repeat_interleave(k, 0) * Y[p.clamp(min=0)].double(), 0.0)
+    # products of bf16 are exact in 32 bits; a sum of d of them
+    assert ((dw.double() - prod.sum(-1)).abs() <= d * 2.0 ** -24 * prod.abs().sum(-1)).all()
+
+
+@pytest.mark.parametrize("B,S,E,C,d", [(1, 1, 1, 1, 8), (3, 50, 4, 13, 264), (2, 300, 33, 300, 136)])
+def test_choice_bookkeeping(B, S, E, C, d):
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    torch.manual_seed(S)
+    T = B * S
+    tok = torch.stack([torch.randperm(S, device="cuda")[:C] for _ in range(B * E)]).view(B, E, C)
+    wts = torch.rand(B, C, E, device="cuda").transpose(1, 2)               # strided
+    status = cuda_ops.status_tensor(tok.device)
+    row_src, pos, weight, meta = cuda_ops.K.moe_choice_plan(tok.int(), wts, S, T, status)
+    a = ((tok + torch.arange(B, device="cuda").view(B, 1, 1) * S) * E + torch.arange(E, device="cuda").view(1, E, 1))
+    rows = a.permute(1, 0, 2).reshape(-1)
+    want = torch.full((T * E,), -1, dtype=torch.int32, device="cuda")
+    want[rows] = torch.arange(rows.numel(), dtype=torch.int32, device="cuda")
+    assert torch.equal(row_src.long(), rows) and torch.equal(pos, want) and meta.tolist() == [rows.numel()] * 2
+    assert torch.equal(weight[a], wts)
+    Y, dout = torch.randn(rows.numel(), d, device="cuda").bfloat16(), torch.randn(T, d, device="cuda").bfloat16()
+    _, dw = cuda_ops.K.moe_gather_dw(dout, row_src, weight, Y, meta, pos, E, B, C)
+    prod = dout[rows // E].double() * Y.double()
+    bound = (d * 2.0 ** -24 * prod.abs().sum(-1)).view(E, B, C).transpose(0, 1)
+    assert ((dw.view(B, E, C).double() - prod.sum(-1).view(E, B, C).transpose(0, 1)).abs() <= bound).all()
+    tok[0, 0, 0] = T + 7                                                   # outside: an empty row and an error
+    row_src, *_ = cuda_ops.K.moe_choice_plan(tok, wts, S, T, status)
+    assert row_src[0] == -1
+    with pytest.raises(RuntimeError, match="status 31"):
+        cuda_ops.check_status()
