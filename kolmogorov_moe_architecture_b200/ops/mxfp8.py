@@ -13,6 +13,7 @@ without ever casting to an fp8 dtype (reference: moe_arch/model/fp8_moe.py:247-2
 from __future__ import annotations
 
 import torch
+from torch.multiprocessing.reductions import StorageWeakRef
 
 E4M3_MAX = 448.0
 BLOCK = 32
@@ -171,8 +172,9 @@ def linear_mx(x: torch.Tensor, w: torch.Tensor, bias=None) -> torch.Tensor:
 
 # Quantised copies of the expert weights are kept until the weights change, so a step with several
 # micro-batches (or forward + backward of one) quantises each orientation once.  A copy is valid while the
-# tensor's autograd version and the global epoch are unchanged; code that rewrites parameters through raw
-# device pointers (the fused optimizer / all-gather kernels) calls ``invalidate_weight_cache``.
+# weight's storage is alive and the tensor's autograd version and the global epoch are unchanged (an address alone
+# says nothing: freed memory is handed out again); code that rewrites parameters through raw device pointers (the
+# fused optimizer / all-gather kernels) calls ``invalidate_weight_cache``.
 _WCACHE: dict = {}
 _EPOCH = [0]
 
@@ -188,12 +190,16 @@ def _weight_quant(w: torch.Tensor, orient: str):
     if os.environ.get("KMOE_MXFP8_WEIGHT_CACHE", "1") != "1":
         return quant_cols(w) if orient == "cols" else quant_rows(w)
     key = (w.data_ptr(), tuple(w.shape), orient)
+    home = StorageWeakRef(w.untyped_storage())
     stamp = (w._version, _EPOCH[0])
     hit = _WCACHE.get(key)
-    if hit is not None and hit[0] == stamp:
+    if hit is not None and hit[0] == stamp and hit[2] == home and not hit[2].expired():
         return hit[1]
+    if hit is None:                                            # a weight not seen before: let go of freed ones' copies
+        for k in [k for k, v in list(_WCACHE.items()) if v[2].expired()]:
+            _WCACHE.pop(k, None)
     val = quant_cols(w) if orient == "cols" else quant_rows(w)
-    _WCACHE[key] = (stamp, val)
+    _WCACHE[key] = (stamp, val, home)
     return val
 
 
