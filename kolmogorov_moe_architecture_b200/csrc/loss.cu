@@ -4,7 +4,8 @@
 // logits = H W^T (tcgen05 GEMM), then this kernel turns the chunk into
 // d(loss)/d(logits) in place while producing the per-row losses, then two more
 // GEMMs consume the gradient chunk.  The chunk is the only (rows, V) tensor that
-// ever exists.  One CTA per row; fp32 online max / sum-exp; second pass hits L2.
+// ever exists.  One CTA per row, fp32 max / sum-exp; a row that fits in shared memory
+// is read once (ce_fwd_bwd_row_kernel), a longer one twice, the second time from L2.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
