@@ -7,7 +7,7 @@
 //
 // head_dim 64 and 128, 320-thread CTAs - eight softmax warps in two warpgroups, a TMA producer warp, an MMA warp - and
 // 128-key / 128-query steps.
-//   forward   attn_fwd2_kernel: two 128-query tiles per CTA, one per warpgroup; S = Q K^T in TMEM, the score row
+//   forward   attn_fwd2_kernel: one or two 128-query tiles per CTA, one per warpgroup; S = Q K^T in TMEM, the score row
 //             is read into registers once, P is written as packed bf16 over the S columns and feeds O += P V as
 //             the A operand from tensor memory; O stays in TMEM and is rescaled only when the row maximum grew by
 //             more than 2^8.
@@ -43,13 +43,14 @@ struct AttnArgs {
   // optional (B, S): first position of the packed document that contains each position; a query then sees
   // only keys k with doc_start[q] <= k <= q (block-diagonal causal mask of packed sequences)
   const int* doc_start;
+  int q_tiles;       // forward: 128-query tiles per CTA, 1 or 2
 };
 
 constexpr float RESCALE_THRESHOLD = 8.0f;          // log2 units: rescale O only when the row max grew by > 2^8
 
 // ------------------------------------------------------------ forward, two query tiles per CTA
-// One CTA per SM owns 256 query rows as two 128-row tiles, each with its own softmax warpgroup, S and O
-// accumulators (4 x 128 TMEM columns in all) and barriers; both tiles share the K/V tiles of a 128-key step.
+// One CTA per SM owns 256 query rows as two 128-row tiles (or 128 rows as one, where the grid is small), each with its
+// own softmax warpgroup, S and O accumulators (4 x 128 TMEM columns in all) and barriers; both tiles share the K/V tiles of a 128-key step.
 //   warps 0-3 / 4-7  softmax of tile 0 / 1 (thread = query row)
 //   warp 8           TMA producer: Q tiles once, K_j / V_j into 2-stage rings
 //   warp 9           MMA issuer: S_t = Q_t K_j^T (128 x 128 x 128), O_t += P_t V_j with P_t read from TMEM
@@ -99,7 +100,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int qb = gridDim.z - 1 - blockIdx.z;
   const int h = blockIdx.x, b = blockIdx.y;
   const int hkv = h / (a.H / a.Hkv);
-  const int q0 = qb * 256;
+  const int q0 = qb * 128 * a.q_tiles;
   // packed documents: key blocks that end before the document of the CTA's first query are invisible to all rows
   const int jlo = a.doc_start != nullptr ? a.doc_start[(size_t)b * a.S + q0] / F2_KEYS : 0;
   // visited key blocks per tile (causal): tile t sees keys < min(q0 + 128 (t + 1), S)
@@ -107,7 +108,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
     const int kmax = min(q0 + 128 * (t + 1), a.S);
-    nb[t] = (q0 + 128 * t < a.S) ? max((kmax + F2_KEYS - 1) / F2_KEYS - jlo, 0) : 0;
+    nb[t] = (t < a.q_tiles && q0 + 128 * t < a.S) ? max((kmax + F2_KEYS - 1) / F2_KEYS - jlo, 0) : 0;
   }
   const int nblk = max(nb[0], nb[1]);
 
@@ -133,9 +134,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one() && nblk > 0) {
-      mbar_expect_tx(&q_full, 2 * TILE_BYTES);
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
+      mbar_expect_tx(&q_full, a.q_tiles * TILE_BYTES);
+      for (int t = 0; t < a.q_tiles; ++t)
 #pragma unroll
         for (int p = 0; p < NP; ++p)
           tma_load_4d(sQ + t * TILE_BYTES + p * PANEL_BYTES, &tmQ, &q_full, p * 64, h, q0 + t * 128, b);
@@ -969,8 +969,13 @@ static int make_bshd_tmap(CUtensorMap* out, const void* base, int B, int S, int 
   return encode_bf16_4d(out, base, dims, strides, box);
 }
 
+// Query tiles per CTA.  Two tiles keep the tensor pipe busier but slow each other down: a lone tile takes a key block in
+// about 0.85 of a pair's time.  So one tile per CTA while all tiles run at once on the 148 SMs, and up to 4/3 of that where
+// the causal mask makes enough of them short.  Forward us, two / one: 1x149x16 10.9 / 8.9, 1x777x12 20.2 / 17.6, 1x1536x12
+// 32.4 / 27.7, 2x777x12 (1.1 waves) 21.7 / 18.5, 1x2048x12x64 (1.3) 34.5 / 29.0; beyond: 2x1002x16 (1.7) 24.9 / 26.5,
+// 8x256x16 (1.7) 13.2 / 16.9, 4x1024x12 (2.6) 31.6 / 40.9.
 template <int D>
-static int launch_attn_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a,
+static int launch_attn_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, AttnArgs a,
                             cudaStream_t st) {
   const int smem = 6 * (D / 64) * PANEL_BYTES + 1024;
   auto kern = attn_fwd2_kernel<D>;
@@ -979,7 +984,11 @@ static int launch_attn_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const 
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
     attr = true;
   }
-  dim3 grid(a.H, a.B, (a.S + 255) / 256);
+  const int blocks = (a.S + 127) / 128;
+  const long long tiles = (long long)a.H * a.B * blocks;
+  a.q_tiles = tiles <= 148 || (blocks >= 6 && 3 * tiles <= 4 * 148) ? 1 : 2;
+  const int rows = 128 * a.q_tiles;
+  dim3 grid(a.H, a.B, (a.S + rows - 1) / rows);
   kern<<<grid, F2_THREADS, smem, st>>>(tq, tk, tv, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
@@ -996,7 +1005,7 @@ extern "C" int kmoe_attn_fwd(const void* q, const void* k, const void* v, void* 
   if ((rc = make_bshd_tmap(&tq, q, B, S, H, D, ATT_BLK))) return rc;
   if ((rc = make_bshd_tmap(&tk, k, B, S, Hkv, D, F2_KEYS))) return rc;
   if ((rc = make_bshd_tmap(&tv, v, B, S, Hkv, D, F2_KEYS))) return rc;
-  AttnArgs a{B, S, H, Hkv, scale * 1.4426950408889634f, (__nv_bfloat16*)out, lse, status, doc_start};
+  AttnArgs a{B, S, H, Hkv, scale * 1.4426950408889634f, (__nv_bfloat16*)out, lse, status, doc_start, 2};
   return D == 128 ? launch_attn_fwd2<128>(tq, tk, tv, a, st) : launch_attn_fwd2<64>(tq, tk, tv, a, st);
 }
 

@@ -49,3 +49,21 @@ def test_blocks_groups_documents(B, S, H, Hkv, docs, D):
         assert (g.double() - w).norm().item() <= TOL * max(scale, 1e-3 * w.numel() ** 0.5)
     for g, h in zip(got[1:], again):
         assert torch.equal(g, h)                       # fixed order of every sum
+
+
+@pytest.mark.parametrize("B,S,H,Hkv,docs", [
+    (1, 1, 1, 1, 0), (1, 1152, 16, 4, 0), (1, 1200, 16, 4, 3), (1, 1281, 18, 6, 0),   # one wave of single tiles and beyond it
+    (8, 300, 16, 4, 0), (3, 700, 16, 4, 4), (25, 640, 2, 1, 0)])                   # pairs, an odd last tile
+@pytest.mark.parametrize("D", [64, 128])
+def test_query_tiles_per_cta(B, S, H, Hkv, docs, D):
+    from kolmogorov_moe_architecture_b200 import ops
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops, eager
+    torch.manual_seed(S)
+    q, k, v = (torch.randn(B, S, n, D, device="cuda").to(torch.bfloat16) for n in (H, Hkv, Hkv))
+    ds = None
+    if docs:
+        ds = eager.doc_start_from_ids(torch.sort(torch.randint(0, docs, (B, S), device="cuda"), dim=1).values)
+    out = ops.attention(q, k, v, doc_start=ds)
+    cuda_ops.check_status()
+    ref = _ref(q.float(), k.float(), v.float(), ds)
+    assert ((out.float() - ref).norm() / ref.norm()).item() < TOL
