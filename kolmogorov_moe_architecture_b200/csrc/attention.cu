@@ -63,7 +63,9 @@ constexpr int F2_THREADS = 320;
 
 // 2^x on the FMA pipe (x <= ~10): round-to-nearest split x = n + f, f in [-0.5, 0.5], cubic for 2^f, exponent
 // added in integer.  Relative error ~1e-4, far below the bf16 rounding of P.  Used for a share of the
-// exponentials so that the MUFU pipe (16 per clock and SM) is not the only limit of the softmax.
+// exponentials of 128-wide heads so that the MUFU pipe (16 per clock and SM) is not the only limit of the softmax.  64-wide
+// heads take MUFU alone: with the share their saved row sums were off by up to 2e-4 (now 1e-6); 4x2048x16 78.0 -> 80.7 us,
+// 8x1021x12 43.3 -> 43.5 us.
 __device__ __forceinline__ float ex2_fma(float x) {
   x = fmaxf(x, -125.f);
   const float t = x + 12582912.f;                   // 1.5 * 2^23: the integer part lands in the low mantissa bits
@@ -264,9 +266,9 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         for (int i = 0; i < 32; i += 2) {
           float x0, x1;
           unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[c + i]), __uint_as_float(v[c + i + 1])), sc2, nm2), x0, x1);
-          // every fourth pair on the FMA pipe, the rest on MUFU
-          const float p0 = ((i & 6) == 6) ? ex2_fma(x0) : ex2_approx(x0);
-          const float p1 = ((i & 6) == 6) ? ex2_fma(x1) : ex2_approx(x1);
+          // head_dim 128: every fourth pair on the FMA pipe, the rest on MUFU
+          const float p0 = (D == 128 && (i & 6) == 6) ? ex2_fma(x0) : ex2_approx(x0);
+          const float p1 = (D == 128 && (i & 6) == 6) ? ex2_fma(x1) : ex2_approx(x1);
           rsum = add_f32x2(rsum, pack_f32x2(p0, p1));
           pk[i >> 1] = pack_bf16(p0, p1);
         }

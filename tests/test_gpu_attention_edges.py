@@ -67,3 +67,17 @@ def test_query_tiles_per_cta(B, S, H, Hkv, docs, D):
     cuda_ops.check_status()
     ref = _ref(q.float(), k.float(), v.float(), ds)
     assert ((out.float() - ref).norm() / ref.norm()).item() < TOL
+
+
+@pytest.mark.parametrize("S,H", [(256, 2), (1021, 4)])
+def test_row_sums_of_64_wide_heads_are_32_bit(S, H):
+    """The saved log-sum-exp: scores of 64 bf16 products each summed in fp32 (below 64 * 2^-24 * 8 for scores below 8) and
+    exponentials within 2^-21, the sum in fp32 - 2^-15 covers all of it ten times over; the mean is ten times closer."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(S)
+    q, k, v = (torch.randn(1, S, H, 64, device="cuda").bfloat16() for _ in range(3))
+    _, lse = c.K.attn_fwd(q, k, v, 0.125, None, c.status_tensor(q.device))
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) * 0.125
+    s = s.masked_fill(torch.triu(torch.ones(S, S, dtype=torch.bool, device="cuda"), 1), float("-inf"))
+    err = lse.double() - torch.logsumexp(s, -1)
+    assert err.abs().max() < 2.0 ** -15 and err.mean().abs() < 2.0 ** -18
