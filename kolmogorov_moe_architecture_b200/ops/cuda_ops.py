@@ -1006,14 +1006,14 @@ def _loss_split(rows: int, d: int, V: int) -> int:
 class _MTPLoss(torch.autograd.Function):
     """Per head: logits chunk = H W^T (tcgen05 GEMM) -> CE kernel writes d logits in place ->
     dH += dlogits W and dW = dlogits^T H.  Gradients are produced during forward (scaled
-    for an upstream gradient of 1) and rescaled in backward."""
+    for an upstream gradient of 1) and rescaled in backward; without ``grad`` only the loss is computed."""
 
     @staticmethod
-    def forward(ctx, hidden, labels, weights, ignore_index, chunk_rows, *head_weights):
+    def forward(ctx, hidden, labels, weights, ignore_index, chunk_rows, grad, *head_weights):
         B, S, d = hidden.shape
         R = B * S
         h2 = hidden.reshape(R, d).contiguous()
-        need_grad = ctx.needs_input_grad[0] or any(ctx.needs_input_grad[5:])
+        need_grad = grad                # not ctx.needs_input_grad: that is True for parameters under no_grad as well
         # dH and dW are written by the first GEMM that contributes to them (beta = 0) and accumulated by the later
         # ones, so neither needs a zero fill nor an addend read on its first use
         dH = torch.empty_like(h2) if need_grad else None
@@ -1110,7 +1110,7 @@ class _MTPLoss(torch.autograd.Function):
                 gws.append(None)
             else:
                 gws.append(scaled(w))
-        return (gh, None, None, None, None, *gws)
+        return (gh, None, None, None, None, None, *gws)
 
 
 def mtp_cross_entropy(hidden, head_weights: Sequence[torch.Tensor], labels, weights, ignore_index=-100,
@@ -1122,7 +1122,8 @@ def mtp_cross_entropy(hidden, head_weights: Sequence[torch.Tensor], labels, weig
     if not ok:
         _fallback("mtp_cross_entropy", f"dtype {hidden.dtype} d={d} V={V}")
         return eager.mtp_cross_entropy(hidden, head_weights, labels, weights, ignore_index)
-    return _MTPLoss.apply(hidden, labels, tuple(weights), ignore_index, chunk_rows, *head_weights)
+    grad = torch.is_grad_enabled() and any(t.requires_grad for t in (hidden, *head_weights))
+    return _MTPLoss.apply(hidden, labels, tuple(weights), ignore_index, chunk_rows, grad, *head_weights)
 
 
 # ------------------------------------------------------------ Newton-Schulz

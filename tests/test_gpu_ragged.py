@@ -262,3 +262,28 @@ def test_expert_blocks_in_pairs(blocks, spare, d, f, swiglu):
         else:
             y, slack = g + u, 512 * 2.0 ** -24 * (mag[0] + mag[1])
         assert bool(((o - y).abs() <= 2.0 ** -8 * y.abs() + slack + 1e-30).all())
+
+
+@pytest.mark.parametrize("V", [1003, 1024])
+def test_loss_without_gradients_makes_none(V):
+    """An evaluation pass: per head the logits' product and the row kernel, and no gradient buffers."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(V)
+    h = _rand(2, 40, 128).requires_grad_()
+    Ws = [torch.nn.Parameter(_rand(V, 128, scale=0.1)) for _ in range(3)]
+    labels = torch.randint(0, V, (2, 40), device="cuda")
+
+    def run():
+        n = c.LAUNCHES["count"]
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        held = torch.cuda.memory_allocated()
+        total, per = c.mtp_cross_entropy(h, Ws, labels, (0.5, 0.3, 0.2))
+        return total, c.LAUNCHES["count"] - n, torch.cuda.max_memory_allocated() - held
+    with torch.no_grad():
+        run()
+        total, launches, peak = run()
+    assert launches == 6 and not total.requires_grad
+    assert peak < 2 * 80 * (V + 64) * 2            # two logits buffers at most; the heads' dW alone are more than that
+    with_grad, launches, _ = run()
+    assert launches > 6 and torch.equal(with_grad.detach(), total)
