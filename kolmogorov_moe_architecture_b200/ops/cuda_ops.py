@@ -508,20 +508,20 @@ def _scan_bc(Bm, Cm):
 
 class _Scan(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, u, delta, A, Bm, Cm, D, z, dt_bias, softplus):
+    def forward(ctx, u, delta, A, Bm, Cm, D, z, dt_bias, softplus, grad):
         u, delta = _aligned(u), _aligned(delta)
         z = _aligned(z) if z is not None else None
         Af = _aligned(A.float().contiguous())
         Bf, Cf = _scan_bc(Bm, Cm)
         Df = D.float().contiguous() if D is not None else None
         bf = dt_bias.float().contiguous() if dt_bias is not None else None
-        need = any(ctx.needs_input_grad)
-        out, ckpt, seg = K.scan_fwd(u, delta, z, Af, Bf, Cf, Df, bf, softplus, need)
+        out, ckpt, seg = K.scan_fwd(u, delta, z, Af, Bf, Cf, Df, bf, softplus, grad)
         _count(2 if seg.numel() else 1)
-        ctx.save_for_backward(u, delta, z, Af, Bf, Cf, Df, bf, ckpt, seg)
-        ctx.softplus = softplus
-        ctx.dtypes = (A.dtype, Bm.dtype, Cm.dtype, D.dtype if D is not None else None,
-                      dt_bias.dtype if dt_bias is not None else None)
+        if grad:
+            ctx.save_for_backward(u, delta, z, Af, Bf, Cf, Df, bf, ckpt, seg)
+            ctx.softplus = softplus
+            ctx.dtypes = (A.dtype, Bm.dtype, Cm.dtype, D.dtype if D is not None else None,
+                          dt_bias.dtype if dt_bias is not None else None)
         return out
 
     @staticmethod
@@ -532,7 +532,7 @@ class _Scan(torch.autograd.Function):
         _count(2 if seg.numel() else 1)
         a_dt, b_dt, c_dt, d_dt, bias_dt = ctx.dtypes
         return (du, dd, dA.to(a_dt), dB.to(b_dt), dC.to(c_dt), dD.to(d_dt) if Df is not None else None,
-                dz if z is not None else None, dbias.to(bias_dt) if bf is not None else None, None)
+                dz if z is not None else None, dbias.to(bias_dt) if bf is not None else None, None, None)
 
 
 def selective_scan(u, delta, A, Bm, Cm, D, z, delta_bias, delta_softplus=True):
@@ -542,7 +542,8 @@ def selective_scan(u, delta, A, Bm, Cm, D, z, delta_bias, delta_softplus=True):
     u, delta = u.contiguous(), delta.contiguous()
     if z is not None and not _rows_ok(z):
         z = z.contiguous()
-    return _Scan.apply(u, delta, A, Bm, Cm, D, z, delta_bias, bool(delta_softplus))
+    grad = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (u, delta, A, Bm, Cm, D, z, delta_bias))
+    return _Scan.apply(u, delta, A, Bm, Cm, D, z, delta_bias, bool(delta_softplus), grad)
 
 
 class _MambaInner(torch.autograd.Function):

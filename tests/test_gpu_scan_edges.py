@@ -57,3 +57,28 @@ def test_segments_chunks_layouts(B, S, C, form, gate):
     want = (yr, *torch.autograd.grad(yr, [t for t in ref_args if t is not None], go.double()))
     for g, w in zip(got, want):
         assert _rel(g, w) < TOL
+
+
+def test_no_checkpoints_without_gradients():
+    """Under no_grad the state before every chunk (16 fp32 values per channel and 8 steps, four times the output) is not kept."""
+    from kolmogorov_moe_architecture_b200 import ops
+    torch.manual_seed(0)
+    B, S, C = 2, 512, 1024
+    mk = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    u, dt, z, Bm, Cm = mk(B, S, C), mk(B, S, C), mk(B, S, C), mk(B, S, 16), mk(B, S, 16)
+    A = torch.nn.Parameter(-torch.rand(C, 16, device="cuda") - 0.5)
+    D, bias = (torch.nn.Parameter(torch.randn(C, device="cuda")) for _ in range(2))
+    peaks = []
+    for enabled in (False, True):
+        with torch.set_grad_enabled(enabled):
+            for _ in range(2):
+                out = None
+                torch.cuda.synchronize()
+                held = torch.cuda.memory_allocated()
+                torch.cuda.reset_peak_memory_stats()
+                out = ops.selective_scan(u, dt, A, Bm, Cm, D, z, bias)
+                peak = torch.cuda.max_memory_allocated() - held
+        peaks.append((peak, out.detach().clone()))
+    checkpoints = 4 * B * (S // 8) * C * 16
+    assert torch.equal(peaks[0][1], peaks[1][1])
+    assert peaks[0][0] < peaks[1][0] - checkpoints // 2
