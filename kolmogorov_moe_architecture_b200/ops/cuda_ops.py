@@ -667,7 +667,7 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
     no atomics).  Reference: moe_arch/model/moe.py:533-673 (gather + bmm + Triton scatter)."""
 
     @staticmethod
-    def forward(ctx, x2, w1, w2, w3, wts, tok, S):
+    def forward(ctx, x2, w1, w2, w3, wts, tok, S, grad):
         # x2 (B*S, d); wts, tok (B, E, C); w1, w2 (E, d, f); w3 (E, f, d)
         T, d = x2.shape
         B, E, C = tok.shape
@@ -677,7 +677,7 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
         row_src, pos, wdense, meta = K.moe_choice_plan(tok, wts, S, T, status_tensor(dev))   # rows ordered (e, b, c)
         Xg = K.moe_gather_rows(x2.contiguous(), row_src, None, meta, E)
         H = torch.empty(E * BC, f, dtype=x2.dtype, device=dev)
-        G, U = torch.empty_like(H), torch.empty_like(H)
+        G, U = (torch.empty_like(H), torch.empty_like(H)) if grad else (None, None)
         gemm(Xg, w1, H, B2=w2, G=G, U=U, mode=BATCHED, groups=E, epi=EPI_SWIGLU, M=BC, N=f, Kd=d, b_major=MAJ_MN,
              lda=d, ldb=f, ldc=f, a_gs=BC * d, b_gs=d * f, c_gs=BC * f)
         Y = torch.empty(E * BC, d, dtype=x2.dtype, device=dev)
@@ -685,10 +685,11 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
              a_gs=BC * f, b_gs=f * d, c_gs=BC * d)
         out = K.moe_combine(Y, pos, wdense, T, E)
         _count(3)
-        keep_h = os.environ.get("KMOE_MOE_KEEP_H", "1") != "0"                    # as in _GroupedSwiGLU
-        ctx.save_for_backward(Xg, G, U, Y, w1, w2, w3, wdense, pos, row_src, meta, *((H,) if keep_h else ()))
-        ctx.dims = (T, d, E, f, B, C)
-        ctx.wdtype = wts.dtype
+        if grad:
+            keep_h = os.environ.get("KMOE_MOE_KEEP_H", "1") != "0"                # as in _GroupedSwiGLU
+            ctx.save_for_backward(Xg, G, U, Y, w1, w2, w3, wdense, pos, row_src, meta, *((H,) if keep_h else ()))
+            ctx.dims = (T, d, E, f, B, C)
+            ctx.wdtype = wts.dtype
         return out
 
     @staticmethod
@@ -720,7 +721,7 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
             if s_ is not None:
                 s_[1]()
         dw1, dw2, dw3 = [None if s_ is not None else g for s_, g in zip(sinks, (dw1, dw2, dw3))]
-        return dx, dw1, dw2, dw3, dwts, None, None
+        return dx, dw1, dw2, dw3, dwts, None, None, None
 
 
 def expert_choice_swiglu(x, w1, w2, w3, wts, tok):
@@ -731,8 +732,9 @@ def expert_choice_swiglu(x, w1, w2, w3, wts, tok):
     if not ok:
         _fallback("expert_choice_swiglu", f"dtype {x.dtype}/{w1.dtype} d={d} f={f}")
         return eager.expert_choice_swiglu(x, w1, w2, w3, wts, tok)
+    grad = torch.is_grad_enabled() and any(t.requires_grad for t in (x, w1, w2, w3, wts))
     out = _ExpertChoiceSwiGLU.apply(x.reshape(B * S, d), w1.contiguous(), w2.contiguous(), w3.contiguous(), wts,
-                                    tok, S)
+                                    tok, S, grad)
     return out.view(B, S, d)
 
 

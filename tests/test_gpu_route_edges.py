@@ -155,3 +155,26 @@ def test_choice_bookkeeping(B, S, E, C, d):
     assert row_src[0] == -1
     with pytest.raises(RuntimeError, match="status 31"):
         cuda_ops.check_status()
+
+
+def test_expert_choice_keeps_nothing_without_gradients():
+    """Under no_grad the pre-activations (two rows x f bf16 buffers) are neither formed nor kept."""
+    from kolmogorov_moe_architecture_b200 import ops
+    torch.manual_seed(0)
+    B, S, d, f, E, C = 2, 256, 64, 1024, 4, 128
+    x = torch.randn(B, S, d, device="cuda").bfloat16()
+    ws = [torch.nn.Parameter((torch.randn(*s, device="cuda") * 0.1).bfloat16()) for s in ((E, d, f), (E, d, f), (E, f, d))]
+    w, tok = ops.expert_choice_route(torch.randn(B, S, E, device="cuda"), C)
+    got = []
+    for enabled in (False, True):
+        with torch.set_grad_enabled(enabled):
+            for _ in range(2):
+                out = None
+                torch.cuda.synchronize()
+                held = torch.cuda.memory_allocated()
+                torch.cuda.reset_peak_memory_stats()
+                out = ops.expert_choice_swiglu(x, *ws, w, tok)
+                peak = torch.cuda.max_memory_allocated() - held
+        got.append((peak, out.detach().clone()))
+    assert torch.equal(got[0][1], got[1][1])
+    assert got[0][0] <= got[1][0] - 2 * (E * B * C * f * 2)
