@@ -989,12 +989,12 @@ def _head_weight_tensor(weights: tuple, device) -> torch.Tensor:
     return t
 
 
-def _loss_split(rows: int, d: int, V: int) -> int:
+def _loss_split(rows: int, d: int, V: int, sms: int = 148) -> int:
     """Slices of the vocabulary in which the hidden states' gradient ``dlogits W`` is accumulated (fp32, summed once at
     the end).  The product has few output tiles and a reduction of tens of thousands, so a last round of tiles that is
     nearly empty costs a whole reduction: 4096 x 1536 is 96 tiles on 74 CTA pairs, two rounds for 1.3.  Slices shorten
     the rounds; each one costs a pass over its fp32 tile per head (~3 % of a slice of 16 k, hence the term per slice)."""
-    pairs = 74
+    pairs = sms // 2
     tiles = -(-rows // 256) * -(-d // 256)
     best, best_t = 1, 1e30
     for parts in range(1, 7):
@@ -1020,58 +1020,60 @@ class _MTPLoss(torch.autograd.Function):
         # dH and dW are written by the first GEMM that contributes to them (beta = 0) and accumulated by the later
         # ones, so neither needs a zero fill nor an addend read on its first use
         dH = torch.empty_like(h2) if need_grad else None
-        dH_started = False
         V0 = head_weights[0].shape[0]
-        parts = _loss_split(min(R, chunk_rows), d, V0) if need_grad and all(w.shape[0] == V0 for w in head_weights) else 1
+        parts = 1
+        if need_grad and all(w.shape[0] == V0 for w in head_weights):
+            sms = torch.cuda.get_device_properties(hidden.device).multi_processor_count
+            parts = _loss_split(min(R, chunk_rows), d, V0, sms)
         if parts > 1:
             kb, kl = _split_k_ranges(V0, parts, hidden.device)
             parts = kb.numel()
-            acc32 = torch.empty(parts, R, d, dtype=torch.float32, device=hidden.device)
-        dWs: List[Optional[torch.Tensor]] = []
-        per = []
+            acc32 = torch.empty(parts * min(R, chunk_rows) * d, dtype=torch.float32, device=hidden.device)
+        heads = []                          # (index, weight, labels, gradient scale)
+        dWs: List[Optional[torch.Tensor]] = [None] * len(head_weights)
+        n_valid, loss_sum = [], []
         for i, W in enumerate(head_weights):
-            V = W.shape[0]
             shift = i + 1
+            loss_sum.append(torch.zeros((), dtype=torch.float32, device=hidden.device))
             if shift >= S:
-                per.append(torch.zeros((), dtype=torch.float32, device=hidden.device))
-                dWs.append(None)
+                n_valid.append(None)
                 continue
             lab = torch.full((B, S), ignore_index, dtype=torch.long, device=hidden.device)
             lab[:, : S - shift] = labels[:, shift:]
             lab = lab.reshape(R)
-            n_valid = (lab != ignore_index).sum().clamp(min=1).float()
-            gscale = (float(weights[i]) / n_valid).reshape(1).contiguous()
+            n_valid.append((lab != ignore_index).sum().clamp(min=1).float())
             Wc = W.contiguous()
-            dW = torch.empty_like(Wc) if need_grad else None
-            loss_sum = torch.zeros((), dtype=torch.float32, device=hidden.device)
-            pitch = -(-V // 64) * 64        # whole 16-byte rows for TMA whatever the vocabulary (50257)
-            for r0 in range(0, R, chunk_rows):
-                r1 = min(R, r0 + chunk_rows)
-                n = r1 - r0
-                hc = h2[r0:r1]
+            dWs[i] = torch.empty_like(Wc) if need_grad else None
+            heads.append((i, Wc, lab, (float(weights[i]) / n_valid[i]).reshape(1).contiguous()))
+        # row chunks outside, heads inside: what is held beside the results is one chunk's logits and accumulators
+        for r0 in range(0, R, chunk_rows):
+            r1 = min(R, r0 + chunk_rows)
+            n = r1 - r0
+            hc = h2[r0:r1]
+            for first, (i, Wc, lab, gscale) in enumerate(heads):
+                V = Wc.shape[0]
+                pitch = -(-V // 64) * 64        # whole 16-byte rows for TMA whatever the vocabulary (50257)
                 buf = torch.empty(n, pitch, dtype=h2.dtype, device=h2.device)
                 # N in whole output vectors: the columns past V are products with rows of W that read as zero
                 gemm(hc, Wc, buf, M=n, N=-(-V // 8) * 8, Kd=d, lda=d, ldb=d, ldc=pitch, b_rows=V)
                 rows = K.ce_fwd_bwd(buf[:, :V], lab[r0:r1].contiguous(), gscale, ignore_index, need_grad)
                 _count()
-                loss_sum = loss_sum + rows.sum()
+                loss_sum[i] = loss_sum[i] + rows.sum()
                 if need_grad:
                     dst, kw = dH[r0:r1], {}
                     if parts > 1:
-                        dst = acc32[:, r0:r1]
-                        kw = dict(mode=BATCHED, groups=parts, k_begin=kb, k_len=kl, c_gs=R * d)
-                    acc = dict(D=dst, beta=1.0) if dH_started else {}
+                        dst = acc32[:parts * n * d].view(parts, n, d)
+                        kw = dict(mode=BATCHED, groups=parts, k_begin=kb, k_len=kl, c_gs=n * d)
+                    acc = dict(D=dst, beta=1.0) if first > 0 else {}
                     gemm(buf, Wc, dst, M=n, N=d, Kd=V, b_major=MAJ_MN, lda=pitch, ldb=d, ldc=d, **acc, **kw)
-                    acc = dict(D=dW, beta=1.0) if r0 > 0 else {}
-                    gemm(buf, hc, dW, M=V, N=d, Kd=n, a_major=MAJ_MN, b_major=MAJ_MN, lda=pitch, ldb=d, ldc=d, **acc)
-            dH_started = dH_started or need_grad
-            per.append(loss_sum / n_valid)
-            dWs.append(dW)
-        if need_grad and not dH_started:
+                    acc = dict(D=dWs[i], beta=1.0) if r0 > 0 else {}
+                    gemm(buf, hc, dWs[i], M=V, N=d, Kd=n, a_major=MAJ_MN, b_major=MAJ_MN, lda=pitch, ldb=d, ldc=d, **acc)
+            if need_grad and heads and parts > 1:
+                K.sum_partials(dst, dH[r0:r1])
+                _count()
+        if need_grad and not heads:
             dH.zero_()
-        elif need_grad and parts > 1:
-            K.sum_partials(acc32, dH)
-            _count()
+        per = [s_ if n is None else s_ / n for s_, n in zip(loss_sum, n_valid)]
         per_t = torch.stack(per)
         total = (per_t * _head_weight_tensor(tuple(float(w) for w in weights), hidden.device)).sum()
         ctx.shape = (B, S, d)

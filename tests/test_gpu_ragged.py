@@ -287,3 +287,24 @@ def test_loss_without_gradients_makes_none(V):
     assert peak < 2 * 80 * (V + 64) * 2            # two logits buffers at most; the heads' dW alone are more than that
     with_grad, launches, _ = run()
     assert launches > 6 and torch.equal(with_grad.detach(), total)
+
+
+def test_loss_memory_is_bounded_by_the_row_chunk(monkeypatch):
+    """Beside the gradients themselves the loss holds one chunk's logits and fp32 accumulators, whatever the row count."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    monkeypatch.setattr(c, "_loss_split", lambda *a: 3)
+    torch.manual_seed(0)
+    B, S, d, V, chunk = 4, 4096, 256, 1003, 512
+    h = _rand(B, S, d).requires_grad_()
+    Ws = [_rand(V, d, scale=0.1).requires_grad_() for _ in range(2)]
+    labels = torch.randint(0, V, (B, S), device="cuda")
+    for _ in range(2):
+        total = None
+        torch.cuda.synchronize()
+        held = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        total, _ = c.mtp_cross_entropy(h, Ws, labels, (0.5, 0.5), chunk_rows=chunk)
+        peak = torch.cuda.max_memory_allocated() - held
+    results = 2 * B * S * d + 2 * 2 * V * d                          # dH and the dW
+    small = 2 * 2 * chunk * (V + 64) + 4 * 3 * chunk * d             # two logits buffers, three slices of a chunk
+    assert peak < results + small + 4 * 8 * B * S + (1 << 20)        # label copies
