@@ -16,6 +16,7 @@ from typing import Tuple
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules import module as _module
 
 from .. import ops
 from .linear import Linear
@@ -49,10 +50,13 @@ class Mamba(nn.Module):
         self.out_proj = Linear(self.d_inner, d_model, bias=False)
 
     def _plain_projections(self) -> bool:
-        """x_proj is the layer this class made, unhooked: then its weight may be used without calling it."""
+        """x_proj is the layer this class made and nothing listens to its calls - no hook of its own or of all modules, no
+        ``forward`` set on the instance: then its weight may be used without calling it."""
         m = self.x_proj
-        return type(m) is Linear and m.bias is None and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks
-                                                             or m._backward_pre_hooks)
+        hooks = (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks, m._backward_pre_hooks,
+                 _module._global_forward_hooks, _module._global_forward_pre_hooks, _module._global_backward_hooks,
+                 _module._global_backward_pre_hooks)
+        return type(m) is Linear and "forward" not in m.__dict__ and m.bias is None and not any(hooks)
 
     def forward(self, hidden_states: torch.Tensor) -> torch.Tensor:
         xz = self.in_proj(hidden_states)

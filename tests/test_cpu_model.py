@@ -310,3 +310,39 @@ def test_input_validation_mode_accepts_what_the_model_itself_produces(kw, monkey
         m(torch.zeros(1, 33, dtype=torch.long))
     with pytest.raises(IndexError, match="position_ids: value 32"):
         m(ids, position_ids=torch.arange(1, 33).expand(2, 32))
+
+
+@pytest.mark.parametrize("how", ["instance forward", "global forward hook", "global pre-hook", "global backward hook", "hook"])
+def test_the_one_pass_mixer_steps_aside_for_whoever_watches_its_projection(how, monkeypatch):
+    """The one-pass mixer reads x_proj's weight without calling the module; anything that sees the module's calls must
+    still see them."""
+    from torch.nn.modules import module as M
+    from kolmogorov_moe_architecture_b200 import ops
+    from kolmogorov_moe_architecture_b200.models.mamba import Mamba
+    m = Mamba(32)
+    monkeypatch.setattr(ops, "mamba_inner", lambda *a: pytest.fail("the projection was passed by"))
+    seen = []
+    see = lambda mod, *a: seen.append(mod) if mod is m.x_proj else None
+    if how == "instance forward":
+        plain = m.x_proj.forward
+        m.x_proj.forward = lambda x: (seen.append(m.x_proj), plain(x))[1]
+        handle = None
+    else:
+        handle = {"global forward hook": M.register_module_forward_hook, "global pre-hook": M.register_module_forward_pre_hook,
+                  "global backward hook": M.register_module_full_backward_hook,
+                  "hook": m.x_proj.register_forward_hook}[how](see)
+    try:
+        m(torch.randn(1, 5, 32)).sum().backward()
+    finally:
+        if handle is not None:
+            handle.remove()
+    assert len(seen) == 1
+
+
+def test_the_one_pass_mixer_is_offered_an_unwatched_projection(monkeypatch):
+    from kolmogorov_moe_architecture_b200 import ops
+    from kolmogorov_moe_architecture_b200.models.mamba import Mamba
+    calls = []
+    monkeypatch.setattr(ops, "mamba_inner", lambda *a: calls.append(a))
+    Mamba(32)(torch.randn(1, 5, 32))
+    assert len(calls) == 1
