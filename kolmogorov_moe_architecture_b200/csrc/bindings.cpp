@@ -1017,12 +1017,12 @@ std::vector<Tensor> mamba_inner_fwd(const Tensor& xz, const Tensor& conv_w, cons
   return {y.view({B, S, C}), x, x_dbl, delta, params, ckpt, seg};
 }
 
-// (dxz, d x_proj, d dt_proj, flat gradients of the small parameters in their own type: A_log | conv w | conv b | dt b | D)
+// (dxz, d x_proj and d dt_proj where wanted, flat gradients of the small parameters in their own type: A_log | conv w | conv b | dt b | D)
 std::vector<Tensor> mamba_inner_bwd(const Tensor& dy_in, const Tensor& xz, const Tensor& x, const Tensor& x_dbl,
                                     const Tensor& delta, const Tensor& params, const Tensor& ckpt, const Tensor& seg,
-                                    const Tensor& xp_w, const Tensor& dt_w, bool params_bf16, const OptT& xp_dst,
-                                    const OptT& xp_kb, const OptT& xp_kl, const OptT& dt_dst, const OptT& dt_kb,
-                                    const OptT& dt_kl, const Tensor& status) {
+                                    const Tensor& xp_w, const Tensor& dt_w, bool params_bf16, bool need_xp, const OptT& xp_dst,
+                                    const OptT& xp_kb, const OptT& xp_kl, bool need_dt, const OptT& dt_dst,
+                                    const OptT& dt_kb, const OptT& dt_kl, const Tensor& status) {
   c10::cuda::CUDAGuard guard(xz.device());
   Tensor dy = dy_in.contiguous();
   if (reinterpret_cast<uintptr_t>(dy.data_ptr()) & 15) dy = dy.clone();
@@ -1047,13 +1047,14 @@ std::vector<Tensor> mamba_inner_bwd(const Tensor& dy_in, const Tensor& xz, const
   Tensor dx_dbl = at::empty({T, ld}, xz.options());
   Gemm(dd, KM, C, dt_w, MN, R, dx_dbl, ld, T, R, C, status).run("d dt");
   check(kmoe_mamba_pack_bc(dB, dC, reinterpret_cast<char*>(dx_dbl.data_ptr()) + 2 * R, T, ld, cur_stream()), "pack_bc");
-  Tensor ddt = wgrad_into(dd, x_dbl.narrow(1, 0, R), dt_w, dt_dst, dt_kb, dt_kl, status);
+  Tensor ddt, dxp;
+  if (need_dt) ddt = wgrad_into(dd, x_dbl.narrow(1, 0, R), dt_w, dt_dst, dt_kb, dt_kl, status);
   {  // the conv output's gradient: what the scan left plus dx_dbl x_proj, added before the one rounding
     Gemm g(dx_dbl, KM, ld, xp_w, MN, C, du, C, T, C, ld, status);
     g.d.D = du.data_ptr(); g.d.ldd = C; g.d.beta = 1.f;
     g.run("d x");
   }
-  Tensor dxp = wgrad_into(dx_dbl, x, xp_w, xp_dst, xp_kb, xp_kl, status);
+  if (need_xp) dxp = wgrad_into(dx_dbl, x, xp_w, xp_dst, xp_kb, xp_kl, status);
   check(kmoe_conv1d_bwd(xz.data_ptr(), P + 16 * C, P + 20 * C, du.data_ptr(), dxz.data_ptr(), a + 16 * C, a + 20 * C, (int)B,
                         (int)S, (int)C, 2 * C, 2 * C, 1, 1, cur_stream()), "conv1d_bwd");
   Tensor dp = at::empty({23 * C}, params_bf16 ? xz.options() : f32);

@@ -565,18 +565,20 @@ class _MambaInner(torch.autograd.Function):
     def backward(ctx, dy):
         xz, x, x_dbl, delta, params, ckpt, seg, xp_w, dt_w = ctx.saved_tensors
         T, dev = x.shape[0], x.device
-        s1, d1, kb1, kl1 = _wgrad_plan(xp_w, T, dev)
-        s2, d2, kb2, kl2 = _wgrad_plan(dt_w, T, dev)
+        need1, need2 = ctx.needs_input_grad[3], ctx.needs_input_grad[4]     # a frozen projection's sink gets nothing
+        s1, d1, kb1, kl1 = _wgrad_plan(xp_w, T, dev) if need1 else (None,) * 4
+        s2, d2, kb2, kl2 = _wgrad_plan(dt_w, T, dev) if need2 else (None,) * 4
         dxz, dxp, ddt, dp = K.mamba_inner_bwd(dy, xz, x, x_dbl, delta, params, ckpt, seg, xp_w, dt_w,
-                                              ctx.small[0][1] == torch.bfloat16, d1, kb1, kl1, d2, kb2, kl2,
-                                              status_tensor(dev))
-        _count(8 + int(seg.numel() > 0))
+                                              ctx.small[0][1] == torch.bfloat16, need1, d1, kb1, kl1, need2, d2, kb2,
+                                              kl2, status_tensor(dev))
+        _count(6 + need1 + need2 + int(seg.numel() > 0))
         for sink in (s1, s2):
             if sink is not None:
                 sink[1]()
         sizes = [shape.numel() for shape, _ in ctx.small]
         dA_log, dcw, dcb, ddb, dD = [g.view(shape) for g, (shape, _) in zip(dp.split(sizes), ctx.small)]
-        return (dxz, dcw, dcb, None if s1 is not None else dxp, None if s2 is not None else ddt, ddb, dA_log, dD, None)
+        return (dxz, dcw, dcb, dxp if need1 and s1 is None else None, ddt if need2 and s2 is None else None, ddb, dA_log, dD,
+                None)
 
 
 def mamba_inner(xz, conv_w, conv_b, xp_w, dt_w, dt_b, A_log, D):

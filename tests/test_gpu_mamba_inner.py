@@ -38,3 +38,28 @@ def test_one_pass_equals_single_ops(B, S, d, small, monkeypatch):
     # the same quantities with fewer roundings to bf16 in between (1.7e-3 each): a handful of them in quadrature
     for a, b in zip(one, many):
         assert a.shape == b.shape and a.dtype == b.dtype and _rel(a, b) < 1e-2
+
+
+@pytest.mark.parametrize("frozen", ["x_proj", "dt_proj"])
+def test_a_frozen_projection_gets_no_gradient(frozen):
+    """With destinations registered for both weights, only the trained one's is written and committed."""
+    from kolmogorov_moe_architecture_b200.models.mamba import Mamba
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        m = Mamba(128).to(torch.bfloat16)
+    views, done = {}, []
+    ws = {"x_proj": m.x_proj.weight, "dt_proj": m.dt_proj.weight}
+    try:
+        for n, w in ws.items():
+            views[n] = torch.full_like(w, 7.0)
+            cuda_ops.register_grad_sink(w, views[n], lambda p, n=n: done.append(n))
+        ws[frozen].requires_grad_(False)
+        x = torch.randn(2, 24, 128, device="cuda").to(torch.bfloat16)
+        m(x).float().square().mean().backward()
+    finally:
+        for w in ws.values():
+            cuda_ops._GRAD_SINKS.pop(w.data_ptr(), None)
+    (trained,) = set(ws) - {frozen}
+    assert done == [trained]
+    assert (views[frozen] == 7.0).all() and not (views[trained] == 7.0).any()
