@@ -139,6 +139,11 @@ def _bf16(t: torch.Tensor) -> bool:
     return t.dtype == torch.bfloat16
 
 
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t`` itself when its first element sits on a 16-byte boundary, else a copy that does."""
+    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
 # -------------------------------------------------------------------- Linear
 def _linear_ok(x2: torch.Tensor, w: torch.Tensor) -> bool:
     """Shapes the GEMM covers for all three products of a linear layer: the input width is a whole number
@@ -493,11 +498,6 @@ def causal_conv1d(x, weight, bias, activation=True):
     return _Conv1d.apply(x, weight, bias, bool(activation))
 
 
-def _aligned(t: torch.Tensor) -> torch.Tensor:
-    """``t`` itself when its first element sits on a 16-byte boundary, else a copy that does."""
-    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
-
-
 def _scan_bc(Bm, Cm):
     """B and C the way the scan kernel reads them: bf16 column slices of one projection as they are, anything else as
     contiguous fp32."""
@@ -583,15 +583,15 @@ class _MambaInner(torch.autograd.Function):
 
 def mamba_inner(xz, conv_w, conv_b, xp_w, dt_w, dt_b, A_log, D):
     """Output of the mixer's scan for its in-projection ``xz`` (B, S, 2C), or None when the fused pass does not cover the
-    call: bf16 activations and projections, 16 states, convolution width 4, C % 64 and dt_rank % 8, small parameters all of
-    one type (bf16 or fp32)."""
+    call: bf16 activations and projections (on 16-byte boundaries, which the single ops at an odd token count do not need), 16
+    states, convolution width 4, C % 64 and dt_rank % 8, small parameters all of one type (bf16 or fp32)."""
     C2, R = xz.shape[-1], dt_w.shape[1]
     small = (conv_w, conv_b, dt_b, A_log, D)
     if not (_bf16(xz) and _bf16(xp_w) and _bf16(dt_w) and xz.numel() > 0 and C2 % 128 == 0 and R % 8 == 0 and R > 0
             and conv_b is not None and conv_w.shape[-1] == 4 and A_log.dim() == 2 and A_log.shape[-1] == 16
             and A_log.dtype in (torch.bfloat16, torch.float32)
             and all(p.dtype == A_log.dtype and p.is_contiguous() for p in small)
-            and xp_w.is_contiguous() and dt_w.is_contiguous()):
+            and xp_w.is_contiguous() and dt_w.is_contiguous() and xp_w.data_ptr() % 16 == 0 and dt_w.data_ptr() % 16 == 0):
         return None
     grad = torch.is_grad_enabled() and any(t.requires_grad for t in (xz, xp_w, dt_w, *small))
     return _MambaInner.apply(_aligned(xz.contiguous()), conv_w, conv_b, xp_w, dt_w, dt_b, A_log, D, grad)
@@ -627,7 +627,7 @@ class _GroupedSwiGLU(torch.autograd.Function):
         # weight gradients go straight to their place in the flat gradient buffer when one is registered
         sinks = [grad_sink(w) for w in (w1, w2, w3)]
         dst = [s_[0] if s_ is not None else None for s_ in sinks]
-        dx, dw1, dw2, dw3, dwts = K.grouped_swiglu_bwd(dout, Xp, G, U, kept[0] if kept else None, Y, w1, w2, w3, wf, pos,
+        dx, dw1, dw2, dw3, dwts = K.grouped_swiglu_bwd(_aligned(dout.contiguous()), Xp, G, U, kept[0] if kept else None, Y, w1, w2, w3, wf, pos,
                                                        row_src, counts, offsets, tile_group, meta, ctx.k, *dst,
                                                        status_tensor(Xp.device))
         _count(9)
@@ -653,11 +653,13 @@ def grouped_swiglu(x, w1, w2, w3, idx, weights, keep=None, moe_dtype="bf16"):
     if not ok:
         _fallback("grouped_swiglu", f"dtype {x.dtype}/{w1.dtype} d={d} f={f}")
         return eager.grouped_swiglu(x, w1, w2, w3, idx, weights, keep)
+    # the gather reads 16-byte vectors, TMA starts on 16-byte boundaries
+    x, w1, w2, w3 = (_aligned(t.contiguous()) for t in (x, w1, w2, w3))
     if moe_dtype == "mxfp8":
         from . import mxfp8
         return mxfp8.grouped_swiglu_mxfp8(x, w1, w2, w3, idx, weights, keep)
     grad = torch.is_grad_enabled() and any(t.requires_grad for t in (x, w1, w2, w3, weights))
-    return _GroupedSwiGLU.apply(x, w1.contiguous(), w2.contiguous(), w3.contiguous(), idx, weights, keep, grad)
+    return _GroupedSwiGLU.apply(x, w1, w2, w3, idx, weights, keep, grad)
 
 
 class _ExpertChoiceSwiGLU(torch.autograd.Function):
@@ -677,7 +679,7 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
         BC = B * C
         dev = x2.device
         row_src, pos, wdense, meta = K.moe_choice_plan(tok, wts, S, T, status_tensor(dev))   # rows ordered (e, b, c)
-        Xg = K.moe_gather_rows(x2.contiguous(), row_src, None, meta, E)
+        Xg = K.moe_gather_rows(x2, row_src, None, meta, E)
         H = torch.empty(E * BC, f, dtype=x2.dtype, device=dev)
         G, U = (torch.empty_like(H), torch.empty_like(H)) if grad else (None, None)
         gemm(Xg, w1, H, B2=w2, G=G, U=U, mode=BATCHED, groups=E, epi=EPI_SWIGLU, M=BC, N=f, Kd=d, b_major=MAJ_MN,
@@ -699,7 +701,7 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
         Xg, G, U, Y, w1, w2, w3, wdense, pos, row_src, meta, *kept = ctx.saved_tensors
         T, d, E, f, B, C = ctx.dims
         BC = B * C
-        dY, dwts = K.moe_gather_dw(dout.contiguous(), row_src, wdense, Y, meta, pos, E, B, C)
+        dY, dwts = K.moe_gather_dw(_aligned(dout.contiguous()), row_src, wdense, Y, meta, pos, E, B, C)
         dwts = dwts.view(B, E, C).to(ctx.wdtype)
         dH = torch.empty(E * BC, f, dtype=dout.dtype, device=dout.device)
         gemm(dY, w3, dH, mode=BATCHED, groups=E, M=BC, N=f, Kd=d, lda=d, ldb=d, ldc=f,
@@ -734,9 +736,9 @@ def expert_choice_swiglu(x, w1, w2, w3, wts, tok):
     if not ok:
         _fallback("expert_choice_swiglu", f"dtype {x.dtype}/{w1.dtype} d={d} f={f}")
         return eager.expert_choice_swiglu(x, w1, w2, w3, wts, tok)
-    grad = torch.is_grad_enabled() and any(t.requires_grad for t in (x, w1, w2, w3, wts))
-    out = _ExpertChoiceSwiGLU.apply(x.reshape(B * S, d), w1.contiguous(), w2.contiguous(), w3.contiguous(), wts,
-                                    tok, S, grad)
+    x2, w1, w2, w3 = (_aligned(t.contiguous()) for t in (x.reshape(B * S, d), w1, w2, w3))      # as in grouped_swiglu
+    grad = torch.is_grad_enabled() and any(t.requires_grad for t in (x2, w1, w2, w3, wts))
+    out = _ExpertChoiceSwiGLU.apply(x2, w1, w2, w3, wts, tok, S, grad)
     return out.view(B, S, d)
 
 
@@ -1017,7 +1019,7 @@ class _MTPLoss(torch.autograd.Function):
     def forward(ctx, hidden, labels, weights, ignore_index, chunk_rows, grad, *head_weights):
         B, S, d = hidden.shape
         R = B * S
-        h2 = hidden.reshape(R, d).contiguous()
+        h2 = _aligned(hidden.reshape(R, d).contiguous())
         need_grad = grad                # not ctx.needs_input_grad: that is True for parameters under no_grad as well
         # dH and dW are written by the first GEMM that contributes to them (beta = 0) and accumulated by the later
         # ones, so neither needs a zero fill nor an addend read on its first use
@@ -1044,7 +1046,7 @@ class _MTPLoss(torch.autograd.Function):
             lab[:, : S - shift] = labels[:, shift:]
             lab = lab.reshape(R)
             n_valid.append((lab != ignore_index).sum().clamp(min=1).float())
-            Wc = W.contiguous()
+            Wc = _aligned(W.contiguous())
             dWs[i] = torch.empty_like(Wc) if need_grad else None
             heads.append((i, Wc, lab, (float(weights[i]) / n_valid[i]).reshape(1).contiguous()))
         # row chunks outside, heads inside: what is held beside the results is one chunk's logits and accumulators

@@ -308,3 +308,50 @@ def test_loss_memory_is_bounded_by_the_row_chunk(monkeypatch):
     results = 2 * B * S * d + 2 * 2 * V * d                          # dH and the dW
     small = 2 * 2 * chunk * (V + 64) + 4 * 3 * chunk * d             # two logits buffers, three slices of a chunk
     assert peak < results + small + 4 * 8 * B * S + (1 << 20)        # label copies
+
+
+def _off(t):
+    """The same values at an address that is a multiple of 2 bytes only."""
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    v = buf[1:].view(t.shape)
+    v.copy_(t)
+    assert v.data_ptr() % 4 == 2
+    return v
+
+
+@pytest.mark.parametrize("f", [72, 128])
+@pytest.mark.parametrize("which", ["tokens", "experts"])
+def test_expert_operands_off_the_16_byte_grid(which, f):
+    """Inputs, weights and the incoming gradient as views that start anywhere: the same bits as aligned copies give."""
+    from kolmogorov_moe_architecture_b200 import ops
+    from kolmogorov_moe_architecture_b200.ops import eager
+    torch.manual_seed(f)
+    B, S, d, E, k = 1, 40, 64, 3, 2
+    x, ws, go = _rand(B, S, d), _expert_case(E, d, f), _rand(B, S, d)
+    if which == "tokens":
+        wts, idx = eager.topk_softmax_route(torch.randn(S, E, device="cuda"), k)
+        run = lambda x, *w: ops.grouped_swiglu(x.view(S, d), *w, idx, wts).view(B, S, d)
+    else:
+        wts, tok = eager.expert_choice_route(torch.randn(B, S, E, device="cuda"), 14)
+        run = lambda x, *w: ops.expert_choice_swiglu(x, *w, wts, tok)
+
+    def results(move):
+        leaves = [move(t).requires_grad_() for t in (x, *ws)]
+        out = run(*leaves)
+        return (out, *torch.autograd.grad(out, leaves, move(go)))
+    for a, b in zip(results(lambda t: t.clone()), results(_off)):
+        assert torch.equal(a, b)
+
+
+def test_loss_operands_off_the_16_byte_grid():
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(0)
+    h, W = _rand(2, 20, 64), _rand(131, 64, scale=0.1)
+    labels = torch.randint(0, 131, (2, 20), device="cuda")
+
+    def results(move):
+        leaves = [move(t).requires_grad_() for t in (h, W)]
+        total, _ = c.mtp_cross_entropy(leaves[0], [leaves[1]], labels, (1.0,))
+        return (total, *torch.autograd.grad(total, leaves))
+    for a, b in zip(results(lambda t: t.clone()), results(_off)):
+        assert torch.equal(a, b)
