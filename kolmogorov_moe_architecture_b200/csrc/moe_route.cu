@@ -346,24 +346,23 @@ moe_gather_dw_kernel(const __nv_bfloat16* __restrict__ dout, const int* __restri
 
 // Expert choice in the bookkeeping of token choice with k = E: row (e, b, c) holds token b * S + tok[b][e][c] of the T
 // tokens.  row_src[row] = assignment t * E + e, pos[assignment] = row (preset to -1), weight[assignment] = wts[b][e][c];
-// the weights of assignments without a row are never read.  A token outside [0, T) leaves its row empty and sets the
-// status.  One launch in place of a dozen elementwise and indexing ones.
+// the weights of assignments without a row are never read.  A token outside [0, S) leaves its row empty and sets status
+// 310.  One launch in place of a dozen elementwise and indexing ones.
 __global__ void moe_choice_plan_kernel(const long long* __restrict__ tok, const float* __restrict__ wts,
                                        int* __restrict__ row_src, int* __restrict__ pos, float* __restrict__ weight,
-                                       int* __restrict__ meta, int B, int E, int C, int S, int T,
-                                       int* __restrict__ status) {
+                                       int* __restrict__ meta, int B, int E, int C, int S, int* __restrict__ status) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row < 2) meta[row] = E * B * C;
   if (row >= E * B * C) return;
   const int e = row / (B * C), b = row / C - e * B, c = row % C;
   const size_t src = ((size_t)b * E + e) * C + c;
-  const long long t = tok[src] + (long long)b * S;
-  if (t < 0 || t >= T) {
+  const long long t = tok[src];
+  if (t < 0 || t >= S) {
     row_src[row] = -1;
-    atomicExch(status, 31);
+    atomicExch(status, 310);
     return;
   }
-  const int a = (int)t * E + e;
+  const int a = ((int)t + b * S) * E + e;
   row_src[row] = a;
   pos[a] = row;
   weight[a] = wts[src];
@@ -482,10 +481,11 @@ extern "C" int kmoe_moe_gather_dw(const void* dout, const int* row_src, const fl
 
 extern "C" int kmoe_moe_choice_plan(const long long* tok, const float* wts, int* row_src, int* pos, float* weight,
                                     int* meta, int B, int E, int C, int S, int T, int* status, cudaStream_t st) {
+  if ((long long)B * S != T) return -3;
   if ((long long)T * E > 0x7fffffff || (long long)B * E * C > 0x7fffff00) return -1;
   if (cudaMemsetAsync(pos, 0xff, (size_t)T * E * sizeof(int), st) != cudaSuccess) return -2;
   const int rows = B * E * C;
-  moe_choice_plan_kernel<<<(rows + 255) / 256, 256, 0, st>>>(tok, wts, row_src, pos, weight, meta, B, E, C, S, T, status);
+  moe_choice_plan_kernel<<<(rows + 255) / 256, 256, 0, st>>>(tok, wts, row_src, pos, weight, meta, B, E, C, S, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -45,13 +45,18 @@ def status_tensor(device) -> torch.Tensor:
     return t
 
 
+# Status codes that report bad input; every other one is a bounded wait that ran out.
+_INPUT_STATUS = {310: "an expert-choice token index outside its sequence"}
+
+
 def check_status(device=None) -> None:
-    """Raise if any kernel since the last check gave up on a bounded wait.  Synchronises."""
+    """Raise if any kernel since the last check gave up on a bounded wait or met bad input.  Synchronises."""
     for key, t in list(_STATUS.items()):
         v = int(t.item())
         if v != 0:
             t.zero_()
-            raise RuntimeError(f"kmoe kernel on cuda:{key} reported wait-timeout status {v}")
+            what = f"status {v} ({_INPUT_STATUS[v]})" if v in _INPUT_STATUS else f"wait-timeout status {v}"
+            raise RuntimeError(f"kmoe kernel on cuda:{key} reported {what}")
 
 
 # Destinations for weight gradients, registered by the sharded data-parallel wrapper: parameter address ->

@@ -157,6 +157,20 @@ def test_choice_bookkeeping(B, S, E, C, d):
         cuda_ops.check_status()
 
 
+@pytest.mark.parametrize("bad", [-1, 20, 45])
+def test_a_token_outside_its_sequence_is_an_error(bad):
+    """Also in the first sequence of a batch, where the index would name a row of the next one."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    B, S, E, C = 2, 20, 2, 3
+    tok = torch.arange(C, device="cuda").repeat(B, E, 1)
+    tok[0, 1, 2] = bad
+    status = cuda_ops.status_tensor(tok.device)
+    row_src, pos, *_ = cuda_ops.K.moe_choice_plan(tok, torch.ones(B, E, C, device="cuda"), S, B * S, status)
+    assert row_src[B * C + 2] == -1 and (row_src >= 0).sum() == B * E * C - 1 and (pos >= 0).sum() == B * E * C - 1
+    with pytest.raises(RuntimeError, match="token index outside its sequence"):
+        cuda_ops.check_status()
+
+
 def test_expert_choice_keeps_nothing_without_gradients():
     """Under no_grad the pre-activations (two rows x f bf16 buffers) are neither formed nor kept."""
     from kolmogorov_moe_architecture_b200 import ops
