@@ -981,11 +981,8 @@ static int launch_attn_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const 
                             cudaStream_t st) {
   const int smem = 6 * (D / 64) * PANEL_BYTES + 1024;
   auto kern = attn_fwd2_kernel<D>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
-    attr = true;
-  }
+  static SmemLimit limit;
+  if (!limit.raise(kern, smem)) return -20;
   const int blocks = (a.S + 127) / 128;
   const long long tiles = (long long)a.H * a.B * blocks;
   a.q_tiles = tiles <= 148 || (blocks >= 6 && 3 * tiles <= 4 * 148) ? 1 : 2;
@@ -1040,11 +1037,10 @@ static int launch_attn_bwd(const void* q, const void* k, const void* v, const vo
   if ((rc = make_bshd_tmap(&tk, k, a.B, a.S, a.Hkv, D, ATT_BLK))) return rc;
   if ((rc = make_bshd_tmap(&tv, v, a.B, a.S, a.Hkv, D, ATT_BLK))) return rc;
   constexpr int smem_dq = 7 * (D / 64) * PANEL_BYTES + 1024, smem_dkv = dkv2_smem_bytes<D>();
+  static SmemLimit limit_dq, limit_dkv;
+  if (!limit_dq.raise(attn_bwd_dq2_kernel<D>, smem_dq) || !limit_dkv.raise(attn_bwd_dkv2_kernel<D>, smem_dkv)) return -20;
   static int sms = 0;
   if (sms == 0) {
-    if (cudaFuncSetAttribute(attn_bwd_dq2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dq) != cudaSuccess ||
-        cudaFuncSetAttribute(attn_bwd_dkv2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dkv) != cudaSuccess)
-      return -20;
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);

@@ -386,12 +386,8 @@ extern "C" int kmoe_gemm_mxfp8(const KmoeMxGemmDesc* d, cudaStream_t stream) {
   int grid = (int)(total < sms ? total : sms);
   if (grid < 1) grid = 1;
   const int smem = STAGES * STAGE_BYTES + 1024;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(mxfp8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return -20;
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  if (!limit.raise(mxfp8_gemm_kernel, smem)) return -20;
   mxfp8_gemm_kernel<<<grid, NUM_THREADS, smem, stream>>>(tA, tB, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }

@@ -1037,26 +1037,25 @@ static int launch_variant(const CUtensorMap& tA, const CUtensorMap& tB, const CU
   if (stages > 8) stages = 8;
   const int smem = stages * stage_bytes + OUT_STAGE_BYTES + 1024;
   auto kern = umma_gemm_kernel<BN, AM, BMj>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  if (!limit.raise(kern, smem)) return -20;
   kern<<<grid, NUM_THREADS, smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
 template <int BN, int AM, int BMj>
 static int launch_pair_variant(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2,
-                               const CUtensorMap& tC, const CUtensorMap& tX, const CUtensorMap& tY, const GemmArgs& args, long long pair_tiles, int sms, cudaStream_t stream) {
+                               const CUtensorMap& tC, const CUtensorMap& tX, const CUtensorMap& tY,
+                               const GemmArgs& args, long long pair_tiles, int sms, cudaStream_t stream) {
   constexpr int stage_bytes = A_STAGE_BYTES + (BN / 2) * BK * 2;
   int stages = (192 * 1024) / stage_bytes;
   if (stages > 8) stages = 8;
   const int smem = stages * stage_bytes + OUT_STAGE_BYTES + 1024;
   auto kern = umma_gemm_pair_kernel<BN, AM, BMj>;
+  static SmemLimit limit;
+  if (!limit.raise(kern, smem)) return -20;
   static int max_clusters = 0;
   if (max_clusters == 0) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -20;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * (sms / 2)));
     cfg.blockDim = dim3(NUM_THREADS);

@@ -222,13 +222,8 @@ extern "C" int kmoe_ce_fwd_bwd(void* logits, const long long* labels, float* los
   if (R <= 0) return 0;
   const int row_bytes = (V * 2 + 15) / 16 * 16;
   if (row_bytes <= kmoe::CE_ROW_MAX && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
-    static bool attr = false;
-    if (!attr) {
-      if (cudaFuncSetAttribute(kmoe::ce_fwd_bwd_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kmoe::CE_ROW_MAX) != cudaSuccess)
-        return -3;
-      attr = true;
-    }
+    static kmoe::SmemLimit limit;
+    if (!limit.raise(kmoe::ce_fwd_bwd_row_kernel, kmoe::CE_ROW_MAX)) return -3;
     kmoe::ce_fwd_bwd_row_kernel<<<R, kmoe::CE_ROW_THREADS, row_bytes, st>>>((__nv_bfloat16*)logits, labels, loss_rows,
                                                                             grad_scale, V, ld, ignore_index, write_grad);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;

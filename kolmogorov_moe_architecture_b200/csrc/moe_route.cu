@@ -410,12 +410,8 @@ extern "C" int kmoe_moe_plan(const long long* idx, const unsigned char* keep, in
                              int* meta, cudaStream_t st) {
   const size_t smem = ((size_t)PLAN_WARPS * E + E + 1) * sizeof(int);
   if (smem > 200 * 1024 || E >= 0xffff) return -1;
-  static size_t attr_set = 0;
-  if (smem > 48 * 1024 && smem > attr_set) {
-    if (cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return -3;
-    attr_set = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024 && !limit.raise(moe_plan_kernel, smem)) return -3;
   moe_plan_kernel<<<1, 32 * PLAN_WARPS, smem, st>>>(idx, keep, n, E, max_rows, expert_base, pos, row_src, counts, offsets,
                                                     tile_group, meta);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -425,13 +421,8 @@ extern "C" int kmoe_moe_capacity_mask(const long long* idx, int n, int E, int ca
                                       cudaStream_t st) {
   const size_t smem = (size_t)PLAN_THREADS * E * sizeof(int);
   if (smem > 200 * 1024) return -1;
-  static size_t attr_set = 0;
-  if (smem > 48 * 1024 && smem > attr_set) {
-    if (cudaFuncSetAttribute(moe_capacity_mask_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return -3;
-    attr_set = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024 && !limit.raise(moe_capacity_mask_kernel, smem)) return -3;
   moe_capacity_mask_kernel<<<1, PLAN_THREADS, smem, st>>>(idx, n, E, cap, keep);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

@@ -11,11 +11,33 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #ifndef KMOE_SPIN_LIMIT
 #define KMOE_SPIN_LIMIT (1u << 22)
 #endif
 
 namespace kmoe {
+
+// Host side: allows a kernel `bytes` of dynamic shared memory, once per device (the limit belongs to the kernel on one
+// device, so a process that uses a second one has to raise it there too).  One object per kernel, kept in static storage;
+// threads that meet in the first call store the same value.
+class SmemLimit {
+  static constexpr int MAX_DEVICES = 64;
+  std::atomic<int> have_[MAX_DEVICES] = {};
+
+ public:
+  template <class Kernel>
+  bool raise(Kernel kern, size_t bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const bool known = dev >= 0 && dev < MAX_DEVICES;
+    if (known && have_[dev].load(std::memory_order_relaxed) >= (int)bytes) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+    if (known) have_[dev].store((int)bytes, std::memory_order_relaxed);
+    return true;
+  }
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -544,16 +544,8 @@ extern "C" int kmoe_seq_topk_fwd(const float* scores, long long row_stride, long
   if (k < 1 || k > S || S2 > 16384) return -1;
   if (rows == 0) return 0;
   const size_t smem = (size_t)S2 * 8;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(seq_topk_softmax_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 8) !=
-        cudaSuccess)
-      return -3;
-    if (cudaFuncSetAttribute(seq_topk_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4) !=
-        cudaSuccess)
-      return -3;
-    attr_set = true;
-  }
+  static SmemLimit limit_sort, limit_select;
+  if (!limit_sort.raise(seq_topk_softmax_kernel, 16384 * 8) || !limit_select.raise(seq_topk_select_kernel, 16384 * 4)) return -3;
   if (mode == 0) {      // kept positions in ascending order: selection instead of a sort
     seq_topk_select_kernel<<<rows, 1024, (size_t)S * 4, st>>>(scores, row_stride, col_stride, rows_inner,
                                                               outer_stride, S, k, idx, w);
@@ -569,12 +561,8 @@ extern "C" int kmoe_seq_topk_bwd(const float* scores, long long row_stride, long
                                  const float* w, const float* dw, const float* stat, float* dscores, cudaStream_t st) {
   if (S > 16384) return -1;
   if (rows == 0) return 0;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(seq_topk_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4) != cudaSuccess)
-      return -3;
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  if (!limit.raise(seq_topk_bwd_kernel, 16384 * 4)) return -3;
   seq_topk_bwd_kernel<<<rows, 512, (size_t)S * 4, st>>>(scores, row_stride, col_stride, rows_inner, outer_stride, S, k,
                                                         mode, idx, w, dw, stat, dscores);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

@@ -336,3 +336,31 @@ def test_loss_curve_one_gpu_equals_n_gpus(tmp_path, n):
         curves[ranks] = json.loads([l for l in r.stdout.splitlines() if l.startswith("CURVE")][0][6:])
     for a, b in zip(curves[1], curves[n]):
         assert abs(a - b) < 2e-2 * abs(a), (curves[1], curves[n])
+
+
+def test_one_process_may_use_a_second_gpu():
+    """Kernels that need more than 48 KB of shared memory ask for it on every device they are launched on."""
+    if not torch.cuda.is_available() or torch.cuda.device_count() < 2:
+        pytest.skip("needs 2 GPUs")
+    from kolmogorov_moe_architecture_b200 import ops
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    got = []
+    for dev in ("cuda:0", "cuda:1"):
+        g = torch.Generator().manual_seed(0)
+        mk = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).bfloat16().to(dev).requires_grad_()
+        with torch.cuda.device(dev):
+            h, W = mk(2, 200, 128), mk(50257, 128, scale=0.1)
+            labels = torch.randint(0, 50257, (2, 200), generator=g).to(dev)
+            total, _ = cuda_ops.mtp_cross_entropy(h, [W], labels, (1.0,))
+            x, ws = mk(300, 128), [mk(3, *s, scale=0.1) for s in ((128, 72), (128, 72), (72, 128))]
+            wts, idx, aux, _ = ops.route_topk(mk(300, 3), 2, 0.01, 0.001)
+            y = ops.grouped_swiglu(x, *ws, idx, wts)
+            q, k, v = mk(1, 300, 4, 64), mk(1, 300, 2, 64), mk(1, 300, 2, 64)
+            o = ops.attention(q, k, v)
+            w, tok = ops.expert_choice_route(mk(1, 300, 3), 120)
+            loss = total + y.float().mean() + o.float().mean() + aux + w.float().mean()
+            got.append([loss, *torch.autograd.grad(loss, [h, W, x, *ws, q, k, v])])
+            torch.cuda.synchronize(dev)
+    cuda_ops.check_status()
+    for a, b in zip(*got):
+        assert torch.allclose(a.float().cpu(), b.float().cpu(), rtol=1e-2, atol=1e-6)
