@@ -8,6 +8,7 @@ the GPU tests set so that a kernel path cannot be skipped unnoticed.
 """
 from __future__ import annotations
 
+import functools
 import os
 from typing import List, Optional, Sequence
 
@@ -147,6 +148,22 @@ def _bf16(t: torch.Tensor) -> bool:
 def _aligned(t: torch.Tensor) -> torch.Tensor:
     """``t`` itself when its first element sits on a 16-byte boundary, else a copy that does."""
     return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
+def _first_order(backward):
+    """For a backward pass whose gradients carry no graph: under ``create_graph`` they get a node that raises when they are
+    differentiated again, so that a penalty on them cannot quietly leave out its own gradient.
+    (``once_differentiable`` does so only where the incoming gradient itself requires one.)"""
+    @functools.wraps(backward)
+    def run(ctx, *grads):
+        again = torch.is_grad_enabled()
+        with torch.no_grad():
+            out = backward(ctx, *grads)
+        if not again:
+            return out
+        stop = torch._C._functions.DelayedError(b"kmoe: no second derivative of this operator on CUDA", len(out))
+        return stop(*[t if t is None else t.detach().requires_grad_() for t in out])
+    return run
 
 
 # -------------------------------------------------------------------- Linear
@@ -627,6 +644,7 @@ class _GroupedSwiGLU(torch.autograd.Function):
         return out
 
     @staticmethod
+    @_first_order
     def backward(ctx, dout):
         Xp, G, U, Y, w1, w2, w3, wf, pos, row_src, counts, offsets, tile_group, meta, *kept = ctx.saved_tensors
         # weight gradients go straight to their place in the flat gradient buffer when one is registered
@@ -702,6 +720,7 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
         return out
 
     @staticmethod
+    @_first_order
     def backward(ctx, dout):
         Xg, G, U, Y, w1, w2, w3, wdense, pos, row_src, meta, *kept = ctx.saved_tensors
         T, d, E, f, B, C = ctx.dims
@@ -1096,6 +1115,7 @@ class _MTPLoss(torch.autograd.Function):
         return total, per_t
 
     @staticmethod
+    @_first_order
     def backward(ctx, g_total, _g_per):
         saved = ctx.saved_tensors
         dH, dWs = saved[0], saved[1:]

@@ -355,3 +355,23 @@ def test_loss_operands_off_the_16_byte_grid():
         return (total, *torch.autograd.grad(total, leaves))
     for a, b in zip(results(lambda t: t.clone()), results(_off)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("which", ["loss", "tokens", "experts"])
+def test_a_second_derivative_is_refused(which):
+    """The kernels' gradients carry no graph.  A penalty on them raises instead of quietly leaving out its own gradient."""
+    from kolmogorov_moe_architecture_b200 import ops
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c, eager
+    torch.manual_seed(0)
+    x = _rand(1, 24, 64).requires_grad_()
+    if which == "loss":
+        y, _ = c.mtp_cross_entropy(x, [_rand(131, 64, scale=0.1)], torch.randint(0, 131, (1, 24), device="cuda"), (1.0,))
+    elif which == "tokens":
+        wts, idx = eager.topk_softmax_route(torch.randn(24, 3, device="cuda"), 2)
+        y = ops.grouped_swiglu(x.view(24, 64), *_expert_case(3, 64, 72), idx, wts).float().sum()
+    else:
+        wts, tok = eager.expert_choice_route(torch.randn(1, 24, 3, device="cuda"), 8)
+        y = ops.expert_choice_swiglu(x, *_expert_case(3, 64, 72), wts, tok).float().sum()
+    (g,) = torch.autograd.grad(y, x, create_graph=True)
+    with pytest.raises(RuntimeError, match="no second derivative"):
+        (x.float().square().sum() + g.float().square().sum()).backward()
