@@ -1,5 +1,5 @@
-"""The mixer as one pass against the composition of the single ops and against 64 bits: odd token counts, narrow dt ranks,
-several segments, small parameters in bf16 and fp32."""
+"""The mixer as one pass against the composition of the single ops and against plain torch in 64 bits: odd token counts,
+narrow dt ranks, several segments, small parameters in bf16 and fp32."""
 import pytest
 import torch
 
@@ -38,6 +38,42 @@ def test_one_pass_equals_single_ops(B, S, d, small, monkeypatch):
     # the same quantities with fewer roundings to bf16 in between (1.7e-3 each): a handful of them in quadrature
     for a, b in zip(one, many):
         assert a.shape == b.shape and a.dtype == b.dtype and _rel(a, b) < 1e-2
+
+
+def _mixer64(m, x, p):
+    """The mixer's definition in plain torch; ``p`` holds the parameters by name."""
+    B, S, _ = x.shape
+    F, R = torch.nn.functional, m.dt_rank
+    u, z = F.linear(x, p["in_proj.weight"]).chunk(2, dim=-1)
+    u = F.silu(F.conv1d(u.transpose(1, 2), p["conv1d.weight"], p["conv1d.bias"], padding=3, groups=u.shape[-1])[..., :S].transpose(1, 2))
+    dt, Bm, Cm = F.linear(u, p["x_proj.weight"]).split([R, 16, 16], dim=-1)
+    dt = F.softplus(F.linear(dt, p["dt_proj.weight"], p["dt_proj.bias"]))
+    A, h, ys = -torch.exp(p["A_log"]), u.new_zeros(B, u.shape[-1], 16), []
+    for t in range(S):
+        h = torch.exp(dt[:, t, :, None] * A) * h + (dt[:, t] * u[:, t])[..., None] * Bm[:, t, None, :]
+        ys.append((h * Cm[:, t, None, :]).sum(-1))
+    return F.linear((torch.stack(ys, 1) + u * p["D"]) * F.silu(z), p["out_proj.weight"])
+
+
+@pytest.mark.parametrize("B,S,d", [(1, 7, 128), (2, 72, 256), (1, 333, 768)])
+def test_one_pass_against_64_bits(B, S, d):
+    """A dozen bf16 roundings (1.7e-3 each) lie on the longest way from an input to a gradient; in quadrature 6e-3, and the
+    gradients of dt's side are sums of mixed signs, hence three times that."""
+    from kolmogorov_moe_architecture_b200.models.mamba import Mamba
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops
+    torch.manual_seed(S)
+    with torch.device("cuda"):
+        m = Mamba(d).to(torch.bfloat16)
+    x = torch.randn(B, S, d, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    go = torch.randn(B, S, d, device="cuda").to(torch.bfloat16)
+    names = [n for n, _ in m.named_parameters()]
+    y = m(x)
+    got = (y, *torch.autograd.grad(y, [x, *m.parameters()], go))
+    cuda_ops.check_status()
+    leaves = [t.detach().double().requires_grad_() for t in (x, *m.parameters())]
+    ref = _mixer64(m, leaves[0], dict(zip(names, leaves[1:])))
+    for n, a, b in zip(["y", "x", *names], got, (ref, *torch.autograd.grad(ref, leaves, go.double()))):
+        assert _rel(a, b) < 1.8e-2, n
 
 
 @pytest.mark.parametrize("frozen", ["x_proj", "dt_proj"])

@@ -375,3 +375,63 @@ def test_a_second_derivative_is_refused(which):
     (g,) = torch.autograd.grad(y, x, create_graph=True)
     with pytest.raises(RuntimeError, match="no second derivative"):
         (x.float().square().sum() + g.float().square().sum()).backward()
+
+
+@pytest.mark.parametrize("blocks,spare,d,f,P,split", [
+    ((8, 7, 6), 0, 256, 384, 384, False),     # as dH: one reduction over K-major rows of the weight
+    ((14, 1, 0, 11), 2, 328, 192, 192, False),
+    ((8, 7, 6), 1, 192, 384, 384, True),      # as dX: [dG | dU] against two weights, widths of whole 64-element blocks
+    ((7, 9, 5), 0, 192, 328, 384, True),      # the reduction of each weight ends inside a block, the operand's is padded
+    ((2, 20), 3, 264, 72, 128, True),
+])
+def test_expert_blocks_in_pairs_k_major(blocks, spare, d, f, P, split):
+    """The backward products of the pair schedule: weights [d, f] read along f.  Tolerances as in
+    test_expert_blocks_in_pairs: one rounding to bf16 on fp32 sums of at most 2 * 384 terms."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(6)
+    E, live = len(blocks), sum(blocks)
+    rows = (live + spare) * 128
+    tiles = torch.tensor([e for e, n in enumerate(blocks) for _ in range(n)] + [0] * spare, dtype=torch.int32, device="cuda")
+    nmt = torch.tensor([live], dtype=torch.int32, device="cuda")
+    w1, w2 = (torch.randn(E, d, f, device="cuda").mul(f ** -0.5).bfloat16() for _ in range(2))
+    parts = 2 if split else 1
+    x = torch.zeros(rows, parts * P, device="cuda", dtype=torch.bfloat16)      # zeros between f and P, as the kernels pad
+    for j in range(parts):
+        x[:, j * P:j * P + f] = torch.randn(rows, f, device="cuda").bfloat16()
+    x[live * 128:] = float("nan")
+    out = torch.full((rows, d), 7.0, dtype=torch.bfloat16, device="cuda")
+    kw = dict(B2=w2, k_split=P, b_klen=f) if split else {}
+    c.gemm(x, w1, out, mode=c.GROUPED_M, M=rows, N=d, Kd=parts * P, groups=E, lda=parts * P, ldb=f, ldc=d, b_gs=d * f,
+           tile_group=tiles, num_m_tiles=nmt, **kw)
+    c.check_status()
+    assert bool((out[live * 128:] == 7.0).all())
+    first = 0
+    for e, n in enumerate(blocks):
+        xs, o = x[first * 128:(first + n) * 128].double(), out[first * 128:(first + n) * 128].double()
+        first += n
+        y, mag = 0.0, 0.0
+        for j, w in enumerate((w1, w2)[:parts]):
+            a, b = xs[:, j * P:j * P + f], w[e].double().t()
+            y, mag = y + a @ b, mag + a.abs() @ b.abs()
+        assert bool(((o - y).abs() <= 2.0 ** -8 * y.abs() + 768 * 2.0 ** -24 * mag + 1e-30).all())
+
+
+@pytest.mark.parametrize("T,d,f,E,k", [(2000, 192, 328, 3, 2), (2700, 256, 384, 3, 1)])
+def test_expert_layer_in_pairs(T, d, f, E, k):
+    """Token choice with enough row blocks per expert that every grouped product of both passes runs on CTA pairs."""
+    from kolmogorov_moe_architecture_b200 import ops
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops, eager
+    assert cuda_ops.K.moe_plan(torch.zeros(T * k, dtype=torch.long, device="cuda"), None, E, 0)[1].numel() >= 7 * 128 * E
+    torch.manual_seed(T)
+    ws, x, go = _expert_case(E, d, f), _rand(T, d), _rand(T, d)
+    wts, idx = eager.topk_softmax_route(torch.randn(T, E, device="cuda"), k)
+    wts = wts.to(torch.bfloat16)
+    leaves = [t.clone().requires_grad_() for t in (x, *ws, wts)]
+    out = ops.grouped_swiglu(*leaves[:4], idx, leaves[4])
+    got = (out, *torch.autograd.grad(out, leaves, go))
+    cuda_ops.check_status()
+    rl = [t.double().requires_grad_() for t in (x, *ws, wts)]
+    ref = eager.grouped_swiglu(*rl[:4], idx, rl[4])
+    for g, w in zip(got, (ref, *torch.autograd.grad(ref, rl, go.double()))):
+        if w.norm() > 0:
+            assert _rel(g, w) < EXPERT_TOL
