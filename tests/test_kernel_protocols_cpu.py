@@ -1,12 +1,13 @@
 """Host model of the barrier protocols of the warp-specialised kernels.
 
-The attention kernels (csrc/attention.cu: ``attn_fwd2_kernel``, ``attn_bwd_dq2_kernel``, ``attn_bwd_dkv2_kernel`` and
-the 64-key-wide ``attn_fwd_kernel``, ``attn_bwd_dq_kernel``, ``attn_bwd_dkv_kernel``) and the persistent GEMMs
-(csrc/gemm_umma.cu: ``umma_gemm_kernel``, ``umma_gemm_pair_kernel``) are warp-specialised: a TMA producer, a
-single-thread MMA issuer and softmax / epilogue warps hand shared-memory stages and tensor-memory regions to one
-another through mbarriers that are waited on by phase parity.  This file restates each role's sequence of waits,
-arrivals, loads and MMAs, runs the roles under randomly chosen interleavings (loads and MMAs complete
-asynchronously, MMAs in issue order) and checks for every step count that
+The attention kernels (csrc/attention.cu: ``attn_fwd2_kernel``, ``attn_bwd_dq2_kernel``, ``attn_bwd_dkv2_kernel``, the
+same for both head widths) and the persistent GEMMs (csrc/gemm_umma.cu: ``umma_gemm_kernel``, ``umma_gemm_pair_kernel``)
+are warp-specialised: a TMA producer, a single-thread MMA issuer and softmax / epilogue warps hand shared-memory stages
+and tensor-memory regions to one another through mbarriers that are waited on by phase parity; the GEMM's epilogue hands
+staging buffers to TMA stores through bulk groups, and the dK/dV kernel's clusters meet at cluster barriers.  This file
+restates each role's sequence of waits, arrivals, loads, MMAs and stores, runs the roles under randomly chosen
+interleavings (loads, MMAs and stores complete asynchronously, MMAs of a CTA in issue order) and checks for every step
+count that
 
 * nothing deadlocks (a parity wait that can never be satisfied would show up as one), and
 * every read sees the data it is meant to see: each write tags its buffer with (what, step), each read asserts
@@ -38,13 +39,14 @@ class Bar:
 
 
 class Machine:
-    """Roles are generators that yield ('wait', bar, parity) or None (a scheduling point).  ``pipe`` is the
-    in-order tensor pipe, ``loads`` the TMA requests in flight."""
+    """Roles are generators that yield ('wait', bar, parity), ('until', condition) or None (a scheduling point).
+    ``pipes`` are the in-order tensor pipes (one per CTA, or per pair), ``loads`` the TMA requests in flight, ``stores``
+    the TMA stores of each thread that have not read their buffer yet, oldest first."""
 
-    def __init__(self, seed):
+    def __init__(self, seed, pipes=1):
         self.rng = random.Random(seed)
         self.mem = {}
-        self.pipe, self.loads = [], []
+        self.pipes, self.loads, self.stores = [[] for _ in range(pipes)], [], {}
 
     def write(self, buf, tag):
         self.mem[buf] = tag
@@ -52,15 +54,21 @@ class Machine:
     def read(self, buf, tag):
         assert self.mem.get(buf) == tag, f"{buf}: expected {tag}, found {self.mem.get(buf)}"
 
-    def mma(self, reads, writes):
-        self.pipe.append(("mma", reads, writes))
+    def mma(self, reads, writes, pipe=0):
+        self.pipes[pipe].append(("mma", reads, writes))
 
-    def commit(self, *bars):
+    def commit(self, *bars, pipe=0):
         for b in bars:
-            self.pipe.append(("commit", b))
+            self.pipes[pipe].append(("commit", b))
 
     def load(self, buf, tag, bar):
         self.loads.append((buf, tag, bar))
+
+    def store(self, thread, buf, tag):
+        self.stores.setdefault(thread, []).append((buf, tag))
+
+    def stores_read(self, thread, but):        # cp.async.bulk.wait_group.read `but`
+        return ("until", lambda: len(self.stores.get(thread, ())) <= but)
 
     def run(self, roles):
         roles = [[r, None] for r in roles]
@@ -71,7 +79,7 @@ class Machine:
         skew = self.rng.random() < 0.5
         speed = lambda: self.rng.choice([0.02, 0.2, 1.0, 1.0, 5.0, 50.0]) if skew else 1.0
         w_role = [speed() for _ in roles]
-        w_pipe, w_load = speed(), speed()
+        w_pipe, w_load, w_store = [speed() for _ in self.pipes], speed(), speed()
         steps = 0
         while True:
             steps += 1
@@ -80,12 +88,17 @@ class Machine:
             for i, (gen, st) in enumerate(roles):
                 if st == "done":
                     continue
-                if st is None or (st[0] == "wait" and st[1].passed(st[2])):
+                if st is None or (st[0] == "wait" and st[1].passed(st[2])) or (st[0] == "until" and st[1]()):
                     choices.append(("role", i))
                     weights.append(w_role[i])
-            if self.pipe:
-                choices.append(("pipe", 0))
-                weights.append(w_pipe)
+            for i, pipe in enumerate(self.pipes):
+                if pipe:
+                    choices.append(("pipe", i))
+                    weights.append(w_pipe[i])
+            for t, q in self.stores.items():
+                if q:
+                    choices.append(("store", t))
+                    weights.append(w_store)
             for i in range(len(self.loads)):
                 choices.append(("load", i))
                 weights.append(w_load)
@@ -97,7 +110,7 @@ class Machine:
             if kind == "role":
                 roles[i][1] = next(roles[i][0], "done")
             elif kind == "pipe":
-                item = self.pipe.pop(0)
+                item = self.pipes[i].pop(0)
                 if item[0] == "mma":
                     for buf, tag in item[1]:
                         self.read(buf, tag)
@@ -105,6 +118,8 @@ class Machine:
                         self.write(buf, tag)
                 else:
                     item[1].arrive()
+            elif kind == "store":
+                self.read(*self.stores[i].pop(0))
             else:
                 buf, tag, bar = self.loads.pop(i)
                 self.write(buf, tag)
@@ -172,73 +187,117 @@ def run_dq2(nblk, seed, ds_barriers=2):
     m.run([producer(), issuer()] + [softmax(w) for w in WARPS])
 
 
-def run_dkv2(niter, seed, q_stages=2):
-    """TMEM: S^T | dP^T | dV | dK (single buffers).  Q: ``q_stages`` stages with the row statistics, dO: 2."""
-    m = Machine(seed)
+def run_dkv2(niter, seed, q_stages=3, split=1):
+    """TMEM: S^T | dP^T | dV | dK (single buffers).  Q with its ndelta: ``q_stages`` stages, held until the dK MMAs; dO with
+    its nlse: 2, released by the dV MMAs.  A stage's two loads (tile and statistics) credit one barrier.  ``split`` CTAs of
+    a cluster share the key block: each lays its sums over its own tiles, all meet, each reads its rows of everybody's, and
+    nobody leaves before all have read."""
+    m = Machine(seed, pipes=split)
     NQ = q_stages
-    kv = Bar(1)
-    q_full, q_empty, stat_full = ([Bar(1) for _ in range(NQ)] for _ in range(3))
-    do_full, do_empty = [Bar(1), Bar(1)], [Bar(1), Bar(1)]
-    st_full, dpt_full, p_full, ds_full, acc_full = Bar(1), Bar(1), Bar(8), Bar(8), Bar(1)
+    meet, leave = Bar(10 * split), Bar(10 * split)      # cluster barriers: eight softmax warps, producer, issuer
+    roles = []
 
-    def producer():
-        m.load("KV", ("KV", 0), kv)
-        for it in range(niter):
-            qs, os_ = it % NQ, it & 1
-            yield ("wait", q_empty[qs], ((it // NQ) & 1) ^ 1)
-            m.load(("Q", qs), ("Q", it), q_full[qs])
-            m.write(("stat", qs), ("stat", it))
-            stat_full[qs].arrive()
-            yield ("wait", do_empty[os_], ((it >> 1) & 1) ^ 1)
-            m.load(("dO", os_), ("dO", it), do_full[os_])
+    def finish(c, part):
+        if split == 1:
+            return
+        meet.arrive()
+        yield ("wait", meet, 0)
+        for p in range(split):                         # warps 8 and 9 take their share of the rows as well
+            for w in WARPS:
+                m.read(("part", p, w), ("part", p))
+        yield None
+        leave.arrive()
+        yield ("wait", leave, 0)
+        if part is not None:
+            m.write(("part", c, part), "gone")
 
-    def issuer():
-        yield ("wait", kv, 0)
-        yield ("wait", q_full[0], 0)
-        m.mma([(("Q", 0), ("Q", 0))], [(("ST", w), ("ST", 0)) for w in WARPS])
-        m.commit(st_full)
-        yield ("wait", do_full[0], 0)
-        m.mma([(("dO", 0), ("dO", 0))], [(("DPT", w), ("DPT", 0)) for w in WARPS])
-        m.commit(dpt_full)
-        for it in range(niter):
-            qs, qn, os_, on = it % NQ, (it + 1) % NQ, it & 1, (it & 1) ^ 1
-            yield ("wait", p_full, it & 1)
-            m.mma([(("ST", w), ("PT", it)) for w in WARPS] + [(("dO", os_), ("dO", it))], [("dV", ("dV", it))])
-            m.commit(do_empty[os_])
-            if it + 1 < niter:
-                yield ("wait", q_full[qn], ((it + 1) // NQ) & 1)
-                m.mma([(("Q", qn), ("Q", it + 1))], [(("ST", w), ("ST", it + 1)) for w in WARPS])
-                m.commit(st_full)
-            yield ("wait", ds_full, it & 1)
-            m.mma([(("DPT", w), ("dST", it)) for w in WARPS] + [(("Q", qs), ("Q", it))], [("dK", ("dK", it))])
-            m.commit(q_empty[qs])
-            if it + 1 < niter:
-                yield ("wait", do_full[on], ((it + 1) >> 1) & 1)
-                m.mma([(("dO", on), ("dO", it + 1))], [(("DPT", w), ("DPT", it + 1)) for w in WARPS])
-                m.commit(dpt_full)
-        m.commit(acc_full)
+    def cta(c):
+        kv = Bar(2)
+        q_full, q_empty = [Bar(2) for _ in range(NQ)], [Bar(1) for _ in range(NQ)]
+        do_full, do_empty = [Bar(2), Bar(2)], [Bar(1), Bar(1)]
+        st_full, dpt_full, p_full, ds_full, acc_full = Bar(1), Bar(1), Bar(8), Bar(8), Bar(1)
+        mma = lambda reads, writes: m.mma([((c, b), t) for b, t in reads], [((c, b), t) for b, t in writes], pipe=c)
+        commit = lambda bar: m.commit(bar, pipe=c)
+        read = lambda b, t: m.read((c, b), t)
+        write = lambda b, t: m.write((c, b), t)
 
-    def softmax(h):                                   # warp h owns its rows and column half of S^T and dP^T
-        for it in range(niter):
-            qs = it % NQ
-            yield ("wait", stat_full[qs], (it // NQ) & 1)
-            yield ("wait", st_full, it & 1)
-            m.read(("ST", h), ("ST", it))
-            m.read(("stat", qs), ("stat", it))
-            yield None
-            m.write(("ST", h), ("PT", it))
-            p_full.arrive()
-            yield ("wait", dpt_full, it & 1)
-            m.read(("DPT", h), ("DPT", it))
-            m.read(("stat", qs), ("stat", it))
-            yield None
-            m.write(("DPT", h), ("dST", it))
-            ds_full.arrive()
-        yield ("wait", acc_full, 0)
-        m.read("dV", ("dV", niter - 1))
-        m.read("dK", ("dK", niter - 1))
+        def load_q(it):
+            m.load((c, ("Q", it % NQ)), ("Q", it), q_full[it % NQ])
+            m.load((c, ("ndelta", it % NQ)), ("ndelta", it), q_full[it % NQ])
 
-    m.run([producer(), issuer()] + [softmax(w) for w in WARPS])
+        def load_do(it):
+            m.load((c, ("dO", it & 1)), ("dO", it), do_full[it & 1])
+            m.load((c, ("nlse", it & 1)), ("nlse", it), do_full[it & 1])
+
+        def producer():
+            m.load((c, "K"), "K", kv)
+            load_q(0)
+            m.load((c, "V"), "V", kv)
+            load_do(0)
+            for it in range(1, niter):
+                yield ("wait", q_empty[it % NQ], ((it // NQ) & 1) ^ 1)
+                load_q(it)
+                yield ("wait", do_empty[it & 1], ((it >> 1) & 1) ^ 1)
+                load_do(it)
+            yield from finish(c, None)
+
+        def issuer():
+            yield ("wait", kv, 0)
+            yield ("wait", q_full[0], 0)
+            mma([("K", "K"), (("Q", 0), ("Q", 0))], [(("ST", w), ("ST", 0)) for w in WARPS])
+            commit(st_full)
+            yield ("wait", do_full[0], 0)
+            mma([("V", "V"), (("dO", 0), ("dO", 0))], [(("DPT", w), ("DPT", 0)) for w in WARPS])
+            commit(dpt_full)
+            for it in range(niter):
+                qs, qn, os_, on = it % NQ, (it + 1) % NQ, it & 1, (it & 1) ^ 1
+                yield ("wait", p_full, it & 1)
+                mma([(("ST", w), ("PT", it)) for w in WARPS] + [(("dO", os_), ("dO", it))], [("dV", ("dV", it))])
+                commit(do_empty[os_])
+                if it + 1 < niter:
+                    yield ("wait", q_full[qn], ((it + 1) // NQ) & 1)
+                    mma([("K", "K"), (("Q", qn), ("Q", it + 1))], [(("ST", w), ("ST", it + 1)) for w in WARPS])
+                    commit(st_full)
+                yield ("wait", ds_full, it & 1)
+                mma([(("DPT", w), ("dST", it)) for w in WARPS] + [(("Q", qs), ("Q", it))], [("dK", ("dK", it))])
+                commit(q_empty[qs])
+                if it + 1 < niter:
+                    yield ("wait", do_full[on], ((it + 1) >> 1) & 1)
+                    mma([("V", "V"), (("dO", on), ("dO", it + 1))], [(("DPT", w), ("DPT", it + 1)) for w in WARPS])
+                    commit(dpt_full)
+            commit(acc_full)
+            yield from finish(c, None)
+
+        def softmax(h):                               # warp h owns its rows and column half of S^T and dP^T
+            for it in range(niter):
+                qs, os_ = it % NQ, it & 1
+                yield ("wait", do_full[os_], (it >> 1) & 1)
+                yield ("wait", st_full, it & 1)
+                read(("ST", h), ("ST", it))
+                read(("nlse", os_), ("nlse", it))
+                yield None
+                write(("ST", h), ("PT", it))
+                p_full.arrive()
+                yield ("wait", q_full[qs], (it // NQ) & 1)
+                yield ("wait", dpt_full, it & 1)
+                read(("DPT", h), ("DPT", it))
+                read(("ndelta", qs), ("ndelta", it))
+                yield None
+                write(("DPT", h), ("dST", it))
+                ds_full.arrive()
+            yield ("wait", acc_full, 0)
+            read("dV", ("dV", niter - 1))
+            read("dK", ("dK", niter - 1))
+            if split > 1:                              # the sums go over the tiles: no load may land there any more
+                assert not [b for b, _, _ in m.loads if b[0] == c]
+                m.write(("part", c, h), ("part", c))
+            yield from finish(c, h)
+
+        roles.extend([producer(), issuer()] + [softmax(w) for w in WARPS])
+
+    for c in range(split):
+        cta(c)
+    m.run(roles)
 
 
 def run_fwd2(nb, seed):
@@ -311,179 +370,17 @@ def run_fwd2(nb, seed):
     m.run([producer(), issuer()] + [softmax(w) for w in WARPS])
 
 
-# ---------------------------------------------------------------- the 64-key-wide kernels (head_dim 64 path)
-W4 = range(4)         # these kernels have four softmax warps (thread = accumulator row)
-
-
-def run_fwd64(nblk, seed):
-    """``attn_fwd_kernel``: TMEM S x 2 | O; K, V: 2 stages; P goes through one shared-memory panel."""
-    m = Machine(seed)
-    q_full, p_full, pv_full = Bar(1), Bar(4), Bar(1)
-    k_full, k_empty, v_full, v_empty, s_full = ([Bar(1), Bar(1)] for _ in range(5))
-    s_free = [Bar(4), Bar(4)]
-
-    def producer():
-        m.load("Q", ("Q", 0), q_full)
-        for j in range(nblk):
-            st, par = j & 1, ((j >> 1) & 1) ^ 1
-            yield ("wait", k_empty[st], par)
-            m.load(("K", st), ("K", j), k_full[st])
-            yield ("wait", v_empty[st], par)
-            m.load(("V", st), ("V", j), v_full[st])
-
-    def issue_s(j):
-        st = j & 1
-        yield ("wait", k_full[st], (j >> 1) & 1)
-        yield ("wait", s_free[st], ((j >> 1) & 1) ^ 1)
-        m.mma([("Q", ("Q", 0)), (("K", st), ("K", j))], [(("S", st, w), ("S", j)) for w in W4])
-        m.commit(s_full[st], k_empty[st])
-
-    def issuer():
-        yield ("wait", q_full, 0)
-        yield from issue_s(0)
-        for j in range(nblk):
-            if j + 1 < nblk:
-                yield from issue_s(j + 1)
-            st = j & 1
-            yield ("wait", v_full[st], (j >> 1) & 1)
-            yield ("wait", p_full, j & 1)
-            reads = [(("P", w), ("P", j)) for w in W4] + [(("V", st), ("V", j))]
-            reads += [(("O", w), ("O scaled", j)) for w in W4] if j > 0 else []
-            m.mma(reads, [(("O", w), ("O", j)) for w in W4])
-            m.commit(pv_full, v_empty[st])
-
-    def softmax(w):
-        for j in range(nblk):
-            st = j & 1
-            yield ("wait", s_full[st], (j >> 1) & 1)
-            m.read(("S", st, w), ("S", j))
-            s_free[st].arrive()
-            yield None
-            if j > 0:
-                yield ("wait", pv_full, (j - 1) & 1)
-                m.read(("O", w), ("O", j - 1))
-                m.write(("O", w), ("O scaled", j))
-                yield None
-            m.write(("P", w), ("P", j))             # the panel PV(j - 1) read: free since pv_full
-            p_full.arrive()
-        yield ("wait", pv_full, (nblk - 1) & 1)
-        m.read(("O", w), ("O", nblk - 1))
-
-    m.run([producer(), issuer()] + [softmax(w) for w in W4])
-
-
-def run_dq64(nblk, seed):
-    """``attn_bwd_dq_kernel``: TMEM (S | dP) x 2 | dQ; K, V: 2 stages; dS goes through one shared-memory panel
-    that ``ds_free`` hands back after the step's dQ MMAs."""
-    m = Machine(seed)
-    qdo, ds_full, ds_free, dq_full = Bar(1), Bar(4), Bar(1), Bar(1)
-    k_full, k_empty, v_full, v_empty, sdp_full = ([Bar(1), Bar(1)] for _ in range(5))
-
-    def producer():
-        m.load("QdO", ("QdO", 0), qdo)
-        for j in range(nblk):
-            st, par = j & 1, ((j >> 1) & 1) ^ 1
-            yield ("wait", k_empty[st], par)
-            m.load(("K", st), ("K", j), k_full[st])
-            yield ("wait", v_empty[st], par)
-            m.load(("V", st), ("V", j), v_full[st])
-
-    def issue_sdp(j):
-        st, ph = j & 1, (j >> 1) & 1
-        yield ("wait", k_full[st], ph)
-        yield ("wait", v_full[st], ph)
-        m.mma([("QdO", ("QdO", 0)), (("K", st), ("K", j)), (("V", st), ("V", j))],
-              [(("SdP", st, w), ("SdP", j)) for w in W4])
-        m.commit(sdp_full[st], v_empty[st])
-
-    def issuer():
-        yield ("wait", qdo, 0)
-        yield from issue_sdp(0)
-        for j in range(nblk):
-            st = j & 1
-            if j + 1 < nblk:
-                yield from issue_sdp(j + 1)
-            yield ("wait", ds_full, j & 1)
-            m.mma([(("dS", w), ("dS", j)) for w in W4] + [(("K", st), ("K", j))], [("dQ", ("dQ", j))])
-            m.commit(ds_free, k_empty[st])
-        m.commit(dq_full)
-
-    def softmax(w):
-        for j in range(nblk):
-            yield ("wait", sdp_full[j & 1], (j >> 1) & 1)
-            m.read(("SdP", j & 1, w), ("SdP", j))
-            yield None
-            yield ("wait", ds_free, (j & 1) ^ 1)
-            m.write(("dS", w), ("dS", j))
-            ds_full.arrive()
-        yield ("wait", dq_full, 0)
-        m.read("dQ", ("dQ", nblk - 1))
-
-    m.run([producer(), issuer()] + [softmax(w) for w in W4])
-
-
-def run_dkv64(niter, seed):
-    """``attn_bwd_dkv_kernel``: TMEM (S^T | dP^T) x 2 | dV | dK; Q / dO: 2 stages; P^T and dS^T go through
-    shared-memory panels that ``pds_free`` hands back; the threads stage the row statistics themselves between
-    two CTA-local barriers of the four warps."""
-    m = Machine(seed)
-    kv, pds_full, pds_free, acc_full = Bar(1), Bar(4), Bar(1), Bar(1)
-    q_full, q_empty, st_full = ([Bar(1), Bar(1)] for _ in range(3))
-    sync = [Bar(4) for _ in range(2 * niter)]          # bar.sync 1, 128: one single-use barrier per use
-
-    def producer():
-        m.load("KV", ("KV", 0), kv)
-        for it in range(niter):
-            st = it & 1
-            yield ("wait", q_empty[st], ((it >> 1) & 1) ^ 1)
-            m.load(("QdO", st), ("QdO", it), q_full[st])
-
-    def issue_st(it):
-        st = it & 1
-        yield ("wait", q_full[st], (it >> 1) & 1)
-        m.mma([("KV", ("KV", 0)), (("QdO", st), ("QdO", it))], [(("ST", st, w), ("ST", it)) for w in W4])
-        m.commit(st_full[st])
-
-    def issuer():
-        yield ("wait", kv, 0)
-        yield from issue_st(0)
-        for it in range(niter):
-            st = it & 1
-            if it + 1 < niter:
-                yield from issue_st(it + 1)
-            yield ("wait", pds_full, it & 1)
-            m.mma([(("PdS", w), ("PdS", it)) for w in W4] + [(("QdO", st), ("QdO", it))], [("dKV", ("dKV", it))])
-            m.commit(pds_free, q_empty[st])
-        m.commit(acc_full)
-
-    def softmax(w):
-        for it in range(niter):
-            yield ("wait", st_full[it & 1], (it >> 1) & 1)
-            sync[2 * it].arrive()
-            yield ("wait", sync[2 * it], 0)
-            if w < 2:                                  # rows 0-63 stage the statistics of the step's 64 queries
-                m.write(("stat", w), ("stat", it))
-            sync[2 * it + 1].arrive()
-            yield ("wait", sync[2 * it + 1], 0)
-            m.read(("ST", it & 1, w), ("ST", it))
-            m.read(("stat", 0), ("stat", it))
-            yield None
-            m.read(("stat", 1), ("stat", it))
-            yield ("wait", pds_free, (it & 1) ^ 1)
-            m.write(("PdS", w), ("PdS", it))
-            pds_full.arrive()
-        yield ("wait", acc_full, 0)
-        m.read("dKV", ("dKV", niter - 1))
-
-    m.run([producer(), issuer()] + [softmax(w) for w in W4])
-
-
 # ---------------------------------------------------------------- persistent GEMMs (csrc/gemm_umma.cu)
-def run_gemm(k_blocks, stages, seed, ctas=1):
+W4 = range(4)         # epilogue warps of a CTA
+
+
+def run_gemm(k_blocks, stages, seed, ctas=1, slabs=3, buffers=2):
     """``umma_gemm_kernel`` (ctas=1) and ``umma_gemm_pair_kernel`` (ctas=2) for the tiles one CTA (pair) works
     through: ``k_blocks[i]`` reduction blocks for tile i (0 = a group without rows in a batched product: the
     epilogue writes zeros / the addend and the issuer arrives by itself).  Ring of ``stages`` shared-memory
-    stages, two accumulators, four epilogue warps per CTA.  In the pair the ``full`` and ``tmem_empty`` barriers
+    stages, two accumulators, four epilogue warps per CTA.  A warp takes its accumulator in ``slabs`` column slabs, hands
+    it back with the last one in registers, and sends each slab from one of its ``buffers`` staging buffers by a TMA store
+    that it does not wait for: it waits until all but the latest store have been read.  In the pair the ``full`` and ``tmem_empty`` barriers
     live in the leader, ``empty`` and ``tmem_full`` exist in both CTAs and get the leader's commits."""
     m = Machine(seed)
     C = range(ctas)
@@ -528,14 +425,21 @@ def run_gemm(k_blocks, stages, seed, ctas=1):
                     tmem_full[c][acc].arrive()
 
     def epilogue(c, w):
+        me, n = (c, w), 0
         for i, kb_n in enumerate(k_blocks):
             acc, acc_ph = i & 1, (i >> 1) & 1
             yield ("wait", tmem_full[c][acc], acc_ph)
-            if kb_n > 0:
-                m.read(("acc", c, acc, w), ("acc", i, kb_n - 1))
+            for sl in range(slabs):
+                if kb_n > 0:
+                    m.read(("acc", c, acc, w), ("acc", i, kb_n - 1))
+                if sl == slabs - 1:
+                    tmem_empty[acc].arrive()
+                yield m.stores_read(me, 1)
+                m.write(("stage out", me, n % buffers), ("out", i, sl))
                 yield None
-                m.read(("acc", c, acc, w), ("acc", i, kb_n - 1))      # later slabs of the same tile
-            tmem_empty[acc].arrive()
+                m.store(me, ("stage out", me, n % buffers), ("out", i, sl))
+                n += 1
+        yield m.stores_read(me, 0)
 
     m.run([producer(c) for c in C] + [issuer()] + [epilogue(c, w) for c in C for w in W4])
 
@@ -552,6 +456,13 @@ def test_dkv_kernel_protocol_has_no_deadlock_and_no_stale_read(niter):
         run_dkv2(niter, seed)
 
 
+@pytest.mark.parametrize("split", [2, 4])
+@pytest.mark.parametrize("niter", [1, 2, 3, 4, 7])
+def test_dkv_clusters_meet_and_leave(niter, split):
+    for seed in range(12):
+        run_dkv2(niter, seed, split=split)
+
+
 @pytest.mark.parametrize("nb1", list(range(1, 10)) + [17])
 def test_forward_kernel_protocol_has_no_deadlock_and_no_stale_read(nb1):
     for nb0 in sorted({max(nb1 - 1, 0), nb1}):     # tile 0 ends one key block earlier, or the sequence end cuts both
@@ -559,14 +470,6 @@ def test_forward_kernel_protocol_has_no_deadlock_and_no_stale_read(nb1):
             run_fwd2((nb0, nb1), seed)
     for seed in range(25):                         # the sequence ends inside tile 0: tile 1 has no rows
         run_fwd2((nb1, 0), seed)
-
-
-@pytest.mark.parametrize("n", list(range(1, 8)) + [12, 33])
-def test_the_64_wide_kernels_have_no_deadlock_and_no_stale_read(n):
-    for seed in range(25):
-        run_fwd64(n, seed)
-        run_dq64(n, seed)
-        run_dkv64(n, seed)
 
 
 @pytest.mark.parametrize("ctas", [1, 2])
@@ -590,8 +493,15 @@ def test_one_ds_barrier_for_two_dp_buffers_would_mix_phases():
 
 
 def test_the_model_notices_a_missing_stage():
-    """Sanity of the model itself: with the Q stage released too early (one stage, as if the release were
-    signalled before the dK MMAs), a load overwrites a tile that is still needed and the tag check fires."""
+    """Sanity of the model itself: one Q stage cannot hold the next step's tile for S^T while this step's is still needed
+    for dK, so nothing can proceed."""
     with pytest.raises(AssertionError):
         for seed in range(200):
             run_dkv2(6, seed, q_stages=1)
+
+
+def test_the_model_notices_a_reused_staging_buffer():
+    """With one staging buffer the store in flight would still be reading what the next slab overwrites."""
+    with pytest.raises(AssertionError):
+        for seed in range(50):
+            run_gemm([2, 2, 2], 4, seed, buffers=1)
