@@ -413,16 +413,14 @@ Tensor moe_balanced_assign(const Tensor& probs, int64_t k, int64_t cap) {
   return sel;
 }
 
-Tensor moe_gather_rows(const Tensor& src, const Tensor& row_src, const OptT& assign_scale, const Tensor& meta,
-                       int64_t div) {
+Tensor moe_gather_rows(const Tensor& src, const Tensor& row_src, const Tensor& meta, int64_t div) {
   c10::cuda::CUDAGuard guard(src.device());
   need_bf16(src, "src");
   TORCH_CHECK(src.is_contiguous() && src.dim() == 2);
   const int max_rows = row_src.numel(), d = src.size(1);
   Tensor dst = at::empty({max_rows, d}, src.options());
-  check(kmoe_moe_gather_rows(src.data_ptr(), row_src.data_ptr<int>(), (const float*)ptr_or_null(assign_scale),
-                             meta.data_ptr<int>(), dst.data_ptr(), max_rows, d, (int)div, cur_stream()),
-        "moe_gather_rows");
+  check(kmoe_moe_gather_rows(src.data_ptr(), row_src.data_ptr<int>(), meta.data_ptr<int>(), dst.data_ptr(), max_rows, d,
+                             (int)div, cur_stream()), "moe_gather_rows");
   return dst;
 }
 
@@ -908,7 +906,7 @@ std::vector<Tensor> grouped_swiglu_fwd(const Tensor& x_in, const Tensor& w1, con
   auto plan = moe_plan(idx.reshape({-1}).contiguous(), keep, E, 0);
   const Tensor &pos = plan[0], &row_src = plan[1], &tile_group = plan[4], &meta = plan[5];
   const int64_t R = row_src.numel();
-  Tensor Xp = moe_gather_rows(x, row_src, OptT(), meta, k);
+  Tensor Xp = moe_gather_rows(x, row_src, meta, k);
   Tensor H = at::empty({R, f}, x.options()), G, U;
   if (save) { G = at::empty_like(H); U = at::empty_like(H); }
   auto grouped = [&](Gemm& g, int64_t gs) {

@@ -199,8 +199,8 @@ int kmoe_moe_capacity_mask(const long long* idx, int n, int E, int cap, unsigned
 // sel [T, k] int64 out): see moe_balanced_slot_kernel
 int kmoe_moe_balanced_assign(const float* probs, unsigned char* taken, int* counts, long long* sel, int T, int E,
                              int k, int cap, cudaStream_t st);
-int kmoe_moe_gather_rows(const void* src, const int* row_src, const float* assign_scale, const int* meta, void* dst,
-                         int max_rows, int d, int div, cudaStream_t st);
+int kmoe_moe_gather_rows(const void* src, const int* row_src, const int* meta, void* dst, int max_rows, int d, int div,
+                         cudaStream_t st);
 int kmoe_moe_combine(const void* Y, const int* pos, const float* w, void* out, int T, int k, int d, cudaStream_t st);
 int kmoe_moe_combine_dw(const void* Y, const void* dout, const int* pos, float* dw, int n, int k, int d,
                         cudaStream_t st);

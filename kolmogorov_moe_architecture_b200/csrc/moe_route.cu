@@ -173,12 +173,10 @@ __global__ void moe_balanced_slot_kernel(const float* __restrict__ probs, unsign
   }
 }
 
-// dst[row] = scale(row) * src[row_src[row] / div]  (zero for padding rows), rows < meta[1].
-//   row_scale: optional fp32 per *assignment* multiplier (indexed by row_src), used by the
-//   backward of the combine: dY[row] = w[assignment] * dout[token].
+// dst[row] = src[row_src[row] / div]  (zero for padding rows), rows < meta[1].
 __global__ void moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ row_src,
-                                       const float* __restrict__ assign_scale, const int* __restrict__ meta,
-                                       __nv_bfloat16* __restrict__ dst, int max_rows, int d, int div) {
+                                       const int* __restrict__ meta, __nv_bfloat16* __restrict__ dst, int max_rows,
+                                       int d, int div) {
   const int live_rows = min(meta[1], max_rows);
   const int vec = d / 8;
   const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -191,21 +189,7 @@ __global__ void moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ src, co
       continue;
     }
     const uint4* srow = reinterpret_cast<const uint4*>(src + (size_t)(a / div) * d);
-    if (assign_scale == nullptr) {
-      for (int v = lane; v < vec; v += 32) drow[v] = srow[v];
-    } else {
-      const float s = assign_scale[a];
-      for (int v = lane; v < vec; v += 32) {
-        uint4 r = srow[v];
-        __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&r);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float2 f = __bfloat1622float2(p[i]);
-          p[i] = __floats2bfloat162_rn(f.x * s, f.y * s);
-        }
-        drow[v] = r;
-      }
-    }
+    for (int v = lane; v < vec; v += 32) drow[v] = srow[v];
   }
 }
 
@@ -440,11 +424,11 @@ extern "C" int kmoe_moe_balanced_assign(const float* probs, unsigned char* taken
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-extern "C" int kmoe_moe_gather_rows(const void* src, const int* row_src, const float* assign_scale, const int* meta,
-                                    void* dst, int max_rows, int d, int div, cudaStream_t st) {
+extern "C" int kmoe_moe_gather_rows(const void* src, const int* row_src, const int* meta, void* dst, int max_rows, int d,
+                                    int div, cudaStream_t st) {
   if (d % 8) return -1;
-  moe_gather_rows_kernel<<<148 * 4, 256, 0, st>>>((const __nv_bfloat16*)src, row_src, assign_scale, meta,
-                                                  (__nv_bfloat16*)dst, max_rows, d, div);
+  moe_gather_rows_kernel<<<148 * 4, 256, 0, st>>>((const __nv_bfloat16*)src, row_src, meta, (__nv_bfloat16*)dst, max_rows,
+                                                  d, div);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

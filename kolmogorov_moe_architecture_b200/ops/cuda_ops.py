@@ -702,7 +702,7 @@ class _ExpertChoiceSwiGLU(torch.autograd.Function):
         BC = B * C
         dev = x2.device
         row_src, pos, wdense, meta = K.moe_choice_plan(tok, wts, S, T, status_tensor(dev))   # rows ordered (e, b, c)
-        Xg = K.moe_gather_rows(x2, row_src, None, meta, E)
+        Xg = K.moe_gather_rows(x2, row_src, meta, E)
         H = torch.empty(E * BC, f, dtype=x2.dtype, device=dev)
         G, U = (torch.empty_like(H), torch.empty_like(H)) if grad else (None, None)
         gemm(Xg, w1, H, B2=w2, G=G, U=U, mode=BATCHED, groups=E, epi=EPI_SWIGLU, M=BC, N=f, Kd=d, b_major=MAJ_MN,

@@ -219,7 +219,7 @@ class _GroupedSwiGLUMX(torch.autograd.Function):
             idx.reshape(-1).contiguous(), keep.reshape(-1) if keep is not None else None, E, 0)
         R = row_src.numel()
         nmt, live = meta[0:1], meta[1:2]
-        Xp = K.moe_gather_rows(x.contiguous(), row_src, None, meta, k)
+        Xp = K.moe_gather_rows(x.contiguous(), row_src, meta, k)
         Xq, sX = quant_rows(Xp, live_rows=live)
         W1q, s1 = _weight_quant(w1, "cols")                   # (E, f, d): reduction over d
         W2q, s2 = _weight_quant(w2, "cols")
