@@ -132,9 +132,12 @@ rmsnorm_fwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 }
 
 // A lane carries 8 NCH column sums beside the row itself, so the blocks are small - four warps, three blocks per SM up to
-// 1536 columns, two above (168 registers would spill) - and the warps' column sums meet in shared memory without atomics.  Traffic bound: 8192 x 2048
-// with a residual gradient 41.8 us with 8-warp blocks (one per SM) and shared atomics, 29.4 us this way, 20.5 at the copy
-// rate; 4096 x 1536, which had three generic kernels, forward + backward 38.6 -> 23.8 us.
+// 1536 columns, two above - and the warps' column sums meet in shared memory without atomics.  Three blocks leave a thread
+// 168 registers: at 1536 columns that spills 84 bytes, wider rows need 222 and more.  At 1536 columns two blocks without
+// the spill are as good: forward + backward of 4096 / 8192 / 16384 rows, replayed, 18.3 / 30.2 / 52.4 us with three and
+// 17.3 / 28.6 / 53.8 with two.  Traffic bound: 8192 x 2048 with a residual gradient 41.8 us with 8-warp blocks (one per SM)
+// and shared atomics, 29.4 us this way, 20.5 at the copy rate; 4096 x 1536, which had three generic kernels, forward +
+// backward 38.6 -> 23.8 us with new inputs on each call.
 constexpr int NORM_BWD_WARPS = 4;
 template <int NCH>
 __global__ void __launch_bounds__(32 * NORM_BWD_WARPS, NCH <= 6 ? 3 : 2)
@@ -507,11 +510,11 @@ extern "C" int kmoe_rmsnorm_fwd(const void* x, const void* w, void* y, float* rs
   return kmoe_add_rmsnorm_fwd(x, nullptr, w, nullptr, y, rstd, rows, d, eps, st);
 }
 
-// Rows of fp32 partial column sums a backward pass may write: one per CTA of the register-resident kernel (eight
-// rows per CTA and sweep, at most two CTAs per SM).
+// Rows of fp32 partial column sums a backward pass may write: one per CTA of the register-resident kernel, at most three
+// small CTAs per SM, and no more than one per eight rows (two rows for each of its four warps).
 extern "C" int kmoe_rmsnorm_bwd_num_partials(int rows) {
   int r = (rows + 7) / 8;
-  return r > 444 ? 444 : (r < 1 ? 1 : r);        // three small blocks per SM
+  return r > 444 ? 444 : (r < 1 ? 1 : r);
 }
 
 // `partial` is scratch of kmoe_rmsnorm_bwd_num_partials(rows) * d floats.

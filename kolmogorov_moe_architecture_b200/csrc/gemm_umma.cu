@@ -418,7 +418,7 @@ __device__ __forceinline__ void store_tile_swiglu(const GemmArgs& a, const CUten
 // bytes.  A row count that is a multiple of 64 is described to TMA as (64, K, rows / 64) and the tile is one load;
 // any other count (expert width 2464, vocabulary 50257) as (rows, K), where a load brings one block and the unit
 // zero-fills what lies past the last row.  The second form costs ROWS / 64 issue slots of the producer thread
-// instead of one, which a reduction block of >= 500 ns hides.
+// instead of one, within the 0.4 us that a 256 x 256 x 64 step takes.
 template <int ROWS>
 __device__ __forceinline__ void load_mn_tile(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int k, int row, int g,
                                              int boxed) {
