@@ -221,8 +221,7 @@ def _wgrad_plan(w: torch.Tensor, T: int, device):
 
 def _linear_bwd(dy, x2, w, need_dx: bool, need_dw: bool, dx_acc=None):
     """(dx, dW) of ``y = x2 w^T``; dW is None when it went to the flat gradient buffer."""
-    if not _rows_ok(dy):
-        dy = dy.contiguous()
+    dy = _aligned(dy if _rows_ok(dy) else dy.contiguous())
     sink, dst, kb, kl = _wgrad_plan(w, x2.shape[0], x2.device) if need_dw else (None, None, None, None)
     dx, dw = K.linear_bwd(dy, x2, w, need_dx, dx_acc, need_dw, dst, kb, kl, status_tensor(x2.device))
     _count(int(need_dx) + int(need_dw) + (kb is not None))

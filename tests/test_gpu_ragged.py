@@ -435,3 +435,13 @@ def test_expert_layer_in_pairs(T, d, f, E, k):
     for g, w in zip(got, (ref, *torch.autograd.grad(ref, rl, go.double()))):
         if w.norm() > 0:
             assert _rel(g, w) < EXPERT_TOL
+
+
+@pytest.mark.parametrize("out_f", [24, 64])
+def test_linear_gradient_off_the_16_byte_grid(out_f):
+    from kolmogorov_moe_architecture_b200 import ops
+    torch.manual_seed(out_f)
+    x, w, go = _rand(40, 128), _rand(out_f, 128).requires_grad_(), _rand(40, out_f)
+    y = ops.linear(x, w)
+    (a,), (b,) = (torch.autograd.grad(y, w, g, retain_graph=True) for g in (go, _off(go)))
+    assert torch.equal(a, b)
