@@ -323,8 +323,7 @@ std::tuple<Tensor, Tensor, Tensor> scan_fwd(const Tensor& u, const Tensor& delta
   const int G = A.dim() == 3 ? (int)A.size(0) : 1;
   TORCH_CHECK(A.size(-2) == C && B % G == 0, "A does not match u");
   Tensor out = at::empty_like(u);
-  const int nch = (S + kmoe_scan_chunk() - 1) / kmoe_scan_chunk();
-  Tensor ckpt = save ? at::empty({B, nch, C, N}, A.options()) : at::empty({0}, A.options());
+  Tensor ckpt = at::empty({save ? (int64_t)kmoe_scan_ckpt_floats(B, S, C) : 0}, A.options());
   const int P = kmoe_scan_segments(B, S, C);
   Tensor seg = P > 1 ? at::empty({B, P, N + 1, C}, A.options()) : at::empty({0}, A.options());
   const bool has_z = z.has_value() && z->defined();
@@ -1007,8 +1006,8 @@ std::vector<Tensor> mamba_inner_fwd(const Tensor& xz, const Tensor& conv_w, cons
   Gemm(x_dbl, KM, ld, dt_w, KM, R, delta, C, T, C, R, status).run("dt_proj");
   Tensor y = at::empty({T, C}, xz.options());
   const char* xd = reinterpret_cast<const char*>(x_dbl.data_ptr());
-  const int nch = (int)((S + kmoe_scan_chunk() - 1) / kmoe_scan_chunk()), segs = kmoe_scan_segments((int)B, (int)S, (int)C);
-  Tensor ckpt = save ? at::empty({B, nch, C, N}, f32) : Tensor();
+  const int segs = kmoe_scan_segments((int)B, (int)S, (int)C);
+  Tensor ckpt = save ? at::empty({(int64_t)kmoe_scan_ckpt_floats((int)B, (int)S, (int)C)}, f32) : Tensor();
   Tensor seg = segs > 1 ? at::empty({B * segs * (N + 1) * C}, f32) : at::empty({0}, f32);
   const char* z = reinterpret_cast<const char*>(xz.data_ptr()) + 2 * C;
   check(kmoe_scan_fwd(x.data_ptr(), delta.data_ptr(), z, P, xd + 2 * R, xd + 2 * (R + N), ld, 1, P + 22 * C, P + 21 * C,

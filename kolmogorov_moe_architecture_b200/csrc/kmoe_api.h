@@ -174,11 +174,12 @@ int kmoe_mamba_params_bwd(const float* acc, const float* params, void* out, int 
 int kmoe_mamba_pack_bc(const float* dB, const float* dC, void* out, long long rows, long long ld, cudaStream_t st);
 // Selective scan.  The sequence is processed in kmoe_scan_segments(B, S, C) parallel segments.
 //   Bm, Cm: [B, S, N] with rows ldbc elements apart, bf16 (bc_bf16 != 0) or fp32, rows 16-byte aligned.
-//   ckpt (forward, optional): [B, ceil(S / kmoe_scan_chunk()), C, N] floats, the state before every chunk.
+//   ckpt (forward, optional): kmoe_scan_ckpt_floats(B, S, C) floats, the state before every chunk in the backward pass's
+//        own order.
 //   seg  (required when there is more than one segment): B * segments * C * (N + 1) floats of scratch that the
 //        backward pass reads again;  gseg: [B, segments, C, N] floats of scratch for the backward pass.
 //   C % 8 == 0, N == 16; A and every activation 16-byte aligned.
-int kmoe_scan_chunk(void);
+long long kmoe_scan_ckpt_floats(int B, int S, int C);
 int kmoe_scan_segments(int B, int S, int C);
 int kmoe_scan_fwd(const void* u, const void* delta, const void* z, const float* A, const void* Bm, const void* Cm,
                   long long ldbc, int bc_bf16, const float* D, const float* dt_bias, void* out, float* ckpt, float* seg,
