@@ -2,7 +2,7 @@
 //
 //   warp 0      : TMA producer  (cp.async.bulk.tensor -> 128B-swizzled smem ring, mbarrier tx counts)
 //   warp 1      : MMA issuer    (tcgen05.mma 128 x BN x 16, accumulators in TMEM, double buffered)
-//   warps 2..5  : epilogue      (tcgen05.ld -> registers -> fused epilogue -> global)
+//   warps 4..11 : epilogue      (tcgen05.ld -> registers -> fused epilogue -> global)
 //
 // One CTA per SM walks a static tile list, so the epilogue of tile i overlaps the
 // main loop of tile i+1.  Operands may be K-major or MN-major (the MMA reads either
@@ -31,7 +31,21 @@ namespace kmoe {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int A_STAGE_BYTES = BM * BK * 2;
-constexpr int NUM_THREADS = 192;
+// Three warpgroups: producer and issuer (and two idle warps), two of epilogue.  The register file is split unevenly, 384 x
+// 168 at launch; all take that again before the common end of the kernel.
+constexpr int NUM_THREADS = 384;
+constexpr int EPI_WARPS = 8;
+constexpr int LAUNCH_REGS = 168, EPI_REGS = 216, ROLE_REGS = 72;
+static_assert(256 * EPI_REGS + 128 * ROLE_REGS == NUM_THREADS * LAUNCH_REGS, "register split");
+template <int N>
+__device__ __forceinline__ void set_regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void set_regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+// a warpgroup's warps meet between two changes of their registers (every wait before this is bounded, so all arrive)
+__device__ __forceinline__ void warpgroup_sync() {
+  __syncwarp();
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + (threadIdx.x >> 7)) : "memory");
+}
 
 struct GemmArgs {
   void* C;
@@ -59,6 +73,14 @@ struct GemmArgs {
   const long long* row_ptr;   // optional: address of each output row (may be peer memory); 0 = row not stored
   int* status;
 };
+
+// Reduction ranges of the first groups in shared memory: every role looks up its tiles' ranges one after the other, and
+// from global memory that is 700 clocks each time.
+constexpr int RANGES_MAX = 128;
+__device__ __forceinline__ void fill_ranges(const GemmArgs& a, int2* ranges) {
+  if (a.mode == KMOE_GEMM_BATCHED && a.k_begin != nullptr)
+    for (int g = threadIdx.x; g < min(a.groups, RANGES_MAX); g += NUM_THREADS) ranges[g] = make_int2(a.k_begin[g], a.k_len[g]);
+}
 
 struct Tile {
   int m_tile, n_tile, g_a, g_b, g_c, k0, k_blocks;
@@ -104,7 +126,7 @@ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; 
 
 // Maps a linear work index to a tile of TM x BN outputs. Returns false past the end.
 template <int BN, int TM = BM>
-__device__ __forceinline__ bool get_tile(const GemmArgs& a, int idx, int num_m, int num_n, Tile& t,
+__device__ __forceinline__ bool get_tile(const GemmArgs& a, int idx, int num_m, int num_n, Tile& t, const int2* ranges,
                                          const uint16_t* pair_list = nullptr) {
   const int n_out = (a.epilogue == KMOE_EPI_SWIGLU) ? BN / 2 : BN;
   (void)n_out;
@@ -140,8 +162,8 @@ __device__ __forceinline__ bool get_tile(const GemmArgs& a, int idx, int num_m, 
     int first_m = band * GM;
     int gsz = min(num_m - first_m, GM);
     int r = local - band * GM * num_n;
-    t.m_tile = first_m + r % gsz;
     t.n_tile = r / gsz;
+    t.m_tile = first_m + r - t.n_tile * gsz;
   }
   t.k0 = 0;
   t.k_blocks = ceil_div(a.K, BK);
@@ -164,8 +186,9 @@ __device__ __forceinline__ bool get_tile(const GemmArgs& a, int idx, int num_m, 
     t.g_b = a.b_grouped ? g : 0;
     t.g_c = g;
     if (a.k_begin != nullptr) {
-      t.k0 = a.k_begin[g];
-      t.k_blocks = ceil_div(a.k_len[g], BK);
+      const int2 r = g < RANGES_MAX ? ranges[g] : make_int2(a.k_begin[g], a.k_len[g]);
+      t.k0 = r.x;
+      t.k_blocks = ceil_div(r.y, BK);
     }
   } else {
     t.g_a = t.g_b = t.g_c = 0;
@@ -229,27 +252,26 @@ __device__ __forceinline__ void epilogue_store_chunk_f32(const GemmArgs& a, cons
 }
 
 // ------------------------------------------------------------------ bf16 epilogue
-// An epilogue warp owns 32 accumulator rows (lane = row).  Each 64-column slab is read from tensor memory, finished
-// in registers, rounded into one of the warp's two 4 KB staging buffers (32 rows x 128 bytes in the 128-byte swizzle,
-// so that both the row-per-lane writes and TMA's reads are free of bank conflicts) and sent off by a TMA store, which
-// also clips at M and N.  The warp does not wait for the store: it returns to a buffer two slabs later, and the
-// accumulator goes back to the MMA warp as soon as the last slab is in registers.
+// An epilogue warp owns 32 accumulator rows (lane = row) and every other 64-column slab; two warps share the rows.  A slab
+// is read from tensor memory, finished in registers, rounded into the warp's 4 KB staging buffer (32 rows x 128 bytes in
+// the 128-byte swizzle, so that both the row-per-lane writes and TMA's reads are free of bank conflicts) and sent off by a
+// TMA store, which also clips at M and N.  The warp waits for that store to have read the buffer only when it has the next
+// slab's values, and the accumulator goes back to the MMA warp as soon as the last slab is in registers.
 // A tile whose reduction is shorter than its epilogue is bound by this code (weight gradients of experts with few
-// tokens, orthogonalisation).  The staged form it replaces - shared memory, then one 128-byte line per 8 lanes - took
-// 6.1 us per 256 x 256 tile.
+// tokens, orthogonalisation): a slab is a chain of latencies, 925 clocks, so with one warp per scheduler (four in all, two
+// buffers each) a 256 x 256 tile took 5000 clocks - ten reduction blocks' worth - and takes 3400 to 4000 with two warps per
+// scheduler (weight gradients of the 3B preset's 64 experts: 681 us, 634 with eight warps).
 constexpr int OUT_BUF_BYTES = 32 * 128;
-constexpr int OUT_STAGE_BYTES = 4 * 2 * OUT_BUF_BYTES;     // four epilogue warps, two buffers each
+constexpr int OUT_STAGE_BYTES = EPI_WARPS * OUT_BUF_BYTES;     // one buffer per epilogue warp
 
 struct OutStage {
   uint8_t* base;
-  int buf;
+  int half;        // this warp's slabs: half, half + 2, ...
 };
-__device__ __forceinline__ uint8_t* out_acquire(OutStage& o, int lane) {
-  if (lane == 0) tma_store_wait_read_but_one();
+__device__ __forceinline__ uint8_t* out_acquire(const OutStage& o, int lane) {
+  if (lane == 0) tma_store_wait_read();
   __syncwarp();
-  uint8_t* p = o.base + o.buf * OUT_BUF_BYTES;
-  o.buf ^= 1;
-  return p;
+  return o.base;
 }
 __device__ __forceinline__ void out_put_row(uint8_t* sb, int lane, const uint32_t (&p)[32]) {
 #pragma unroll
@@ -271,10 +293,10 @@ __device__ __forceinline__ void out_send(const CUtensorMap* tm, const uint8_t* s
 // wait() returns once the accumulator is complete (false: gave up), release() hands it back.
 template <int BN, class Wait, class Release>
 __device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtensorMap* tmC, const CUtensorMap* tmT,
-                                                OutStage& out, uint32_t t_row, bool have_acc, int row0, int n0, int g,
+                                                const OutStage& out, uint32_t t_row, bool have_acc, int row0, int n0, int g,
                                                 float scale, float beta, float beta2, bool mirror, int lane,
                                                 Wait wait, Release release) {
-  const int slabs = row0 < a.M ? min(BN / 64, ceil_div(a.N - n0, 64)) : 0;
+  const int slabs = row0 < a.M ? min(BN / 64, ceil_div(a.N - n0, 64)) : 0, first = out.half;
   const __nv_bfloat16* Dp = reinterpret_cast<const __nv_bfloat16*>(a.D);
   const __nv_bfloat16* D2p = reinterpret_cast<const __nv_bfloat16*>(a.D2);
   const bool diag = a.diag_add != 0.f && n0 < row0 + 32 && n0 + BN > row0;
@@ -290,12 +312,12 @@ __device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtenso
                      : make_uint4(0, 0, 0, 0);
     }
   };
-  if (Dp != nullptr && slabs > 0) load_addend(Dp, n0);           // under the wait for the accumulator
+  if (Dp != nullptr && first < slabs) load_addend(Dp, n0 + first * 64);          // under the wait for the accumulator
   if (!wait()) return false;
-  if (slabs == 0) release();
+  if (first >= slabs) release();
   // the loop stays rolled: unrolled, the epilogue outgrows the instruction cache
 #pragma unroll 1
-  for (int sl = 0; sl < slabs; ++sl) {
+  for (int sl = first; sl < slabs; sl += 2) {
     const int col = n0 + sl * 64;
     uint32_t r[64];
     if (have_acc) {
@@ -306,7 +328,7 @@ __device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtenso
 #pragma unroll
       for (int i = 0; i < 64; ++i) r[i] = 0u;
     }
-    if (sl == slabs - 1) release();
+    if (sl + 2 >= slabs) release();
 #pragma unroll
     for (int i = 0; i < 64; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * scale);
     if (diag) {
@@ -340,7 +362,7 @@ __device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtenso
         }
         __syncwarp();
       }
-      if (sl + 1 < slabs) load_addend(Dp, col + 64);
+      if (sl + 2 < slabs) load_addend(Dp, col + 128);
     }
     uint32_t p[32];
 #pragma unroll
@@ -368,14 +390,14 @@ __device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtenso
 // HB gate columns followed by the HB up columns of the same outputs.
 template <int HB, class Release>
 __device__ __forceinline__ void store_tile_swiglu(const GemmArgs& a, const CUtensorMap* tmH, const CUtensorMap* tmG,
-                                                  const CUtensorMap* tmU, OutStage& out, uint32_t t_row, bool have_acc,
+                                                  const CUtensorMap* tmU, const OutStage& out, uint32_t t_row, bool have_acc,
                                                   int row0, int n0, int g, float scale, int lane, Release release) {
   const int slabs = row0 < a.M ? min(HB / 64, ceil_div(a.N - n0, 64)) : 0;
-  if (slabs == 0) release();
+  if (out.half >= slabs) release();
   // Three results per slab, one after the other: reading tensor memory again costs less than holding both slabs in
   // registers (192 of them, which spilled).
 #pragma unroll 1
-  for (int sl = 0; sl < slabs; ++sl) {
+  for (int sl = out.half; sl < slabs; sl += 2) {
     const int col = n0 + sl * 64;
     const int last = a.U_out != nullptr ? 2 : (a.G_out != nullptr ? 1 : 0);
 #pragma unroll 1
@@ -406,7 +428,7 @@ __device__ __forceinline__ void store_tile_swiglu(const GemmArgs& a, const CUten
         for (int i = 0; i < 16; ++i)
           p[h * 16 + i] = pack_bf16(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1]));
       }
-      if (sl == slabs - 1 && what == last) release();
+      if (sl + 2 >= slabs && what == last) release();
       uint8_t* sb = out_acquire(out, lane);
       out_put_row(sb, lane, p);
       out_send(what == 0 ? tmH : (what == 1 ? tmG : tmU), sb, lane, col, row0, g);
@@ -459,6 +481,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __shared__ uint64_t tmem_full[2];
   __shared__ uint64_t tmem_empty[2];
   __shared__ uint32_t tmem_base_slot;
+  __shared__ int2 ranges[RANGES_MAX];
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -470,7 +493,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 4);  // one arrival per epilogue warp
+      mbar_init(&tmem_empty[i], EPI_WARPS);  // one arrival per epilogue warp
     }
     mbar_fence_init();
     prefetch_tmap(&tmA);
@@ -480,6 +503,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tmem_alloc(&tmem_base_slot, TMEM_COLS);
     tmem_relinquish();
   }
+  fill_ranges(args, ranges);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -491,17 +515,20 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (args.mode == KMOE_GEMM_GROUPED_M) num_m = min(num_m, *args.num_m_tiles);
   const int num_n = ceil_div(args.N, n_per_tile);
 
+  if (warp < 4) {
+    set_regs_down<ROLE_REGS>();
+    {
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
       Tile t;
-      for (int idx = blockIdx.x; get_tile<BN>(args, idx, num_m, num_n, t); idx += gridDim.x) {
+      for (int idx = blockIdx.x; get_tile<BN>(args, idx, num_m, num_n, t, ranges); idx += gridDim.x) {
         for (int kb = 0; kb < t.k_blocks; ++kb) {
           if (!mbar_wait(&empty_bar[s], ph ^ 1)) {
             atomicExch(args.status, 1);
-            goto teardown;
+            goto role_done;
           }
           uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + A_STAGE_BYTES;
@@ -540,20 +567,20 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       uint32_t ph = 0;
       int it = 0;
       Tile t;
-      for (int idx = blockIdx.x; get_tile<BN>(args, idx, num_m, num_n, t); idx += gridDim.x) {
+      for (int idx = blockIdx.x; get_tile<BN>(args, idx, num_m, num_n, t, ranges); idx += gridDim.x) {
         const int acc = it & 1;
         const uint32_t acc_ph = (it >> 1) & 1;
         ++it;
         if (!mbar_wait(&tmem_empty[acc], acc_ph ^ 1)) {
           atomicExch(args.status, 2);
-          goto teardown;
+          goto role_done;
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < t.k_blocks; ++kb) {
           if (!mbar_wait(&full_bar[s], ph)) {
             atomicExch(args.status, 3);
-            goto teardown;
+            goto role_done;
           }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
@@ -576,13 +603,20 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           mbar_arrive(&tmem_full[acc]);
       }
     }
+  }
+    }
+  role_done:
+    warpgroup_sync();
+    set_regs_up<LAUNCH_REGS>();
   } else {
+    set_regs_up<EPI_REGS>();
+    {
     // ------------------------------------------------------------ epilogue
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     int it = 0;
     Tile t;
-    OutStage out{smem + stages * STAGE_BYTES + q * 2 * OUT_BUF_BYTES, 0};
-    for (int idx = blockIdx.x; get_tile<BN>(args, idx, num_m, num_n, t); idx += gridDim.x) {
+    const OutStage out{smem + stages * STAGE_BYTES + (warp - 4) * OUT_BUF_BYTES, (warp - 4) >> 2};
+    for (int idx = blockIdx.x; get_tile<BN>(args, idx, num_m, num_n, t, ranges); idx += gridDim.x) {
       const int acc = it & 1;
       const uint32_t acc_ph = (it >> 1) & 1;
       ++it;
@@ -612,10 +646,10 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!swiglu && !args.out_f32 && args.row_ptr == nullptr) {
         if (!store_tile_bf16<BN>(args, &tmC, &tmX, out, t_row, have_acc, row0, t.n_tile * BN, t.g_c, scale, beta, 0.f,
                                  false, lane, wait, release))
-          goto teardown;
+          goto epi_done;
         continue;
       }
-      if (!wait()) goto teardown;
+      if (!wait()) goto epi_done;
       if (swiglu) {
         store_tile_swiglu<BN / 2>(args, &tmC, &tmX, &tmY, out, t_row, have_acc, row0, t.n_tile * (BN / 2), t.g_c, scale,
                                   lane, release);
@@ -628,10 +662,11 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // would emit 32 scattered 16-byte writes per instruction; the 64-column slab is staged in shared
         // memory instead and written back with 8 lanes per row: four full 128-byte lines per instruction.
         const long long row_addr = row_ok ? args.row_ptr[row] : 0;
-        __nv_bfloat16(*stg)[72] = reinterpret_cast<__nv_bfloat16(*)[72]>(out.base);      // 32 rows, within 8 KB
+        __nv_bfloat16(*stg)[72] =
+            reinterpret_cast<__nv_bfloat16(*)[72]>(smem + stages * STAGE_BYTES + q * 2 * OUT_BUF_BYTES);    // 32 rows, 4.5 KB
         const __nv_bfloat16* Dp = reinterpret_cast<const __nv_bfloat16*>(args.D);
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 64) {
+        for (int c = 0; out.half == 0 && c < BN; c += 64) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint32_t r[32];
@@ -669,7 +704,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       } else {
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = out.half * (BN / 2); c < (out.half + 1) * (BN / 2); c += 32) {
           uint32_t r[32];
           if (have_acc) {
             tmem_ld_32x32(t_row + c, r);
@@ -681,10 +716,13 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       release();
     }
+    }
+  epi_done:
+    if (lane == 0) tma_store_wait_all();
+    warpgroup_sync();
+    set_regs_down<LAUNCH_REGS>();
   }
 
-teardown:
-  if (warp >= 2 && lane == 0) tma_store_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -730,7 +768,9 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   __shared__ uint64_t tmem_full[2];
   __shared__ uint64_t tmem_empty[2];
   __shared__ uint32_t tmem_base_slot;
-  __shared__ uint16_t pair_list[PAIR_LIST_MAX];
+  __shared__ __align__(8) uint16_t pair_list[PAIR_LIST_MAX];
+  int2* ranges = reinterpret_cast<int2*>(pair_list);      // one schedule has the list, another the ranges
+  static_assert(sizeof(pair_list) >= RANGES_MAX * sizeof(int2), "ranges fit");
   __shared__ int pair_list_len;
 
   const int warp = threadIdx.x >> 5;
@@ -747,7 +787,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 8);   // four epilogue warps in each CTA of the pair
+      mbar_init(&tmem_empty[i], 2 * EPI_WARPS);   // the epilogue warps of both CTAs
     }
     mbar_fence_init();
     prefetch_tmap(&tmA);
@@ -761,6 +801,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const int n = build_pair_list(args.tile_group, min(ceil_div(args.M, BM), *args.num_m_tiles), pair_list, lane);
     if (lane == 0) pair_list_len = n;
   }
+  fill_ranges(args, ranges);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                 // the peer's barriers exist before anything is signalled across
@@ -772,18 +813,21 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const int num_m = args.mode == KMOE_GEMM_GROUPED_M ? pair_list_len : ceil_div(args.M, PAIR_TM);
   const int num_n = ceil_div(args.N, n_per_tile);
 
+  if (warp < 4) {
+    set_regs_down<ROLE_REGS>();
+    {
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
     if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
       Tile t;
-      for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, pair_list); idx += num_pairs) {
+      for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, ranges, pair_list); idx += num_pairs) {
         const int arow = t.row + (int)rank * BM;
         for (int kb = 0; kb < t.k_blocks; ++kb) {
           if (!mbar_wait(&empty_bar[s], ph ^ 1)) {
             atomicExch(args.status, 11);
-            goto teardown;
+            goto role_done;
           }
           uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + A_STAGE_BYTES;
@@ -815,20 +859,20 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       uint32_t ph = 0;
       int it = 0;
       Tile t;
-      for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, pair_list); idx += num_pairs) {
+      for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, ranges, pair_list); idx += num_pairs) {
         const int acc = it & 1;
         const uint32_t acc_ph = (it >> 1) & 1;
         ++it;
         if (!mbar_wait(&tmem_empty[acc], acc_ph ^ 1)) {
           atomicExch(args.status, 12);
-          goto teardown;
+          goto role_done;
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < t.k_blocks; ++kb) {
           if (!mbar_wait(&full_bar[s], ph)) {
             atomicExch(args.status, 13);
-            goto teardown;
+            goto role_done;
           }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
@@ -852,13 +896,20 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
       }
     }
+  }
+    }
+  role_done:
+    warpgroup_sync();
+    set_regs_up<LAUNCH_REGS>();
   } else {
+    set_regs_up<EPI_REGS>();
+    {
     // ------------------------------------------------------------ epilogue (both CTAs)
     const int q = warp & 3;
     int it = 0;
     Tile t;
-    OutStage out{smem + stages * STAGE_BYTES + q * 2 * OUT_BUF_BYTES, 0};
-    for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, pair_list); idx += num_pairs) {
+    const OutStage out{smem + stages * STAGE_BYTES + (warp - 4) * OUT_BUF_BYTES, (warp - 4) >> 2};
+    for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, ranges, pair_list); idx += num_pairs) {
       const int acc = it & 1;
       const uint32_t acc_ph = (it >> 1) & 1;
       ++it;
@@ -897,10 +948,10 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const bool mirror = args.sym_upper && t.n_tile * BN >= (t.m_tile + 1) * PAIR_TM;
         if (!store_tile_bf16<BN>(args, &tmC, &tmX, out, t_row, have_acc, row0, t.n_tile * BN, t.g_c, scale, beta, beta2,
                                  mirror, lane, wait, release))
-          goto teardown;
+          goto epi_done;
         continue;
       }
-      if (!wait()) goto teardown;
+      if (!wait()) goto epi_done;
       if (swiglu) {
         store_tile_swiglu<HALF_N>(args, &tmC, &tmX, &tmY, out, t_row, have_acc, row0, t.n_tile * HALF_N, t.g_c, scale,
                                   lane, release);
@@ -910,7 +961,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       const long long coff = goff + (long long)row * args.ldc;
       const long long doff = goff + (long long)row * args.ldd;
 #pragma unroll 1
-      for (int c = 0; c < BN; c += 32) {
+      for (int c = out.half * (BN / 2); c < (out.half + 1) * (BN / 2); c += 32) {
         uint32_t r[32];
         if (have_acc) {
           tmem_ld_32x32(t_row + c, r);
@@ -921,10 +972,13 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
       release();
     }
+    }
+  epi_done:
+    if (lane == 0) tma_store_wait_all();
+    warpgroup_sync();
+    set_regs_down<LAUNCH_REGS>();
   }
 
-teardown:
-  if (warp >= 2 && lane == 0) tma_store_wait_all();
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                 // nothing of the peer may still point at this CTA's memory
