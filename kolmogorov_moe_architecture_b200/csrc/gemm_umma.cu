@@ -260,7 +260,8 @@ __device__ __forceinline__ void epilogue_store_chunk_f32(const GemmArgs& a, cons
 // A tile whose reduction is shorter than its epilogue is bound by this code (weight gradients of experts with few
 // tokens, orthogonalisation): a slab is a chain of latencies, 925 clocks, so with one warp per scheduler (four in all, two
 // buffers each) a 256 x 256 tile took 5000 clocks - ten reduction blocks' worth - and takes 3400 to 4000 with two warps per
-// scheduler (weight gradients of the 3B preset's 64 experts: 681 us, 634 with eight warps).
+// scheduler (weight gradients of the 3B preset's 64 experts: 681 us, 634 with eight warps, 552 with the relaxed arrival at
+// the pair's leader).
 constexpr int OUT_BUF_BYTES = 32 * 128;
 constexpr int OUT_STAGE_BYTES = EPI_WARPS * OUT_BUF_BYTES;     // one buffer per epilogue warp
 
@@ -892,7 +893,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           umma_commit_pair(&tmem_full[acc], 3);
         } else {
           mbar_arrive(&tmem_full[acc]);
-          mbar_arrive_cluster(map_to_cta(&tmem_full[acc], 1));
+          mbar_arrive_cluster_relaxed(map_to_cta(&tmem_full[acc], 1));
         }
       }
     }
@@ -940,7 +941,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         __syncwarp();
         if (lane == 0) {
           if (leader) mbar_arrive(&tmem_empty[acc]);
-          else mbar_arrive_cluster(map_to_cta(&tmem_empty[acc], 0));
+          else mbar_arrive_cluster_relaxed(map_to_cta(&tmem_empty[acc], 0));
         }
       };
       if (!swiglu && !args.out_f32) {

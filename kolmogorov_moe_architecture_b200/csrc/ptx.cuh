@@ -217,8 +217,11 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
                : "memory");
   return v;
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// Relaxed: says that tensor memory has been read (the reads have completed, tcgen05.wait::ld), no writes to memory go
+// with it.  With release semantics at cluster scope the arrival waited for the warp's outstanding stores, 1000 to 2000
+// clocks per tile.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // TMA load into this CTA's shared memory whose byte count is credited to a barrier that may live in the
 // pair's leader CTA (`bar_cluster_addr` from map_to_cta).  No multicast: each CTA fetches its own tile.
