@@ -517,17 +517,57 @@ std::tuple<Tensor, Tensor, Tensor> attn_bwd(const Tensor& q, const Tensor& k, co
 }
 
 // ------------------------------------------------------------------------- loss
-Tensor ce_fwd_bwd(Tensor logits, const Tensor& labels, const Tensor& grad_scale, int64_t ignore_index,
-                  bool write_grad) {
+static void ce_rows(Tensor& logits, const Tensor& labels, const Tensor& grad_scale, Tensor& loss_rows, int64_t ignore_index,
+                    bool write_grad) {
   c10::cuda::CUDAGuard guard(logits.device());
   need_bf16(logits, "logits"); need_f32(grad_scale, "grad_scale");
   TORCH_CHECK(logits.dim() == 2 && logits.stride(1) == 1);
   TORCH_CHECK(labels.scalar_type() == at::kLong && labels.is_contiguous() && labels.numel() == logits.size(0));
-  Tensor loss_rows = at::empty({logits.size(0)}, logits.options().dtype(at::kFloat));
   check(kmoe_ce_fwd_bwd(logits.data_ptr(), (const long long*)labels.data_ptr<int64_t>(), loss_rows.data_ptr<float>(),
                         grad_scale.data_ptr<float>(), (int)logits.size(0), (int)logits.size(1), logits.stride(0),
                         ignore_index, write_grad ? 1 : 0, cur_stream()), "ce_fwd_bwd");
+}
+
+Tensor ce_fwd_bwd(Tensor logits, const Tensor& labels, const Tensor& grad_scale, int64_t ignore_index,
+                  bool write_grad) {
+  Tensor loss_rows = at::empty({logits.size(0)}, logits.options().dtype(at::kFloat));
+  ce_rows(logits, labels, grad_scale, loss_rows, ignore_index, write_grad);
   return loss_rows;
+}
+
+void ce_fwd_bwd_out(Tensor logits, const Tensor& labels, const Tensor& grad_scale, Tensor loss_rows, int64_t ignore_index,
+                    bool write_grad) {
+  need_f32(loss_rows, "loss_rows");
+  TORCH_CHECK(loss_rows.is_contiguous() && loss_rows.numel() == logits.size(0));
+  ce_rows(logits, labels, grad_scale, loss_rows, ignore_index, write_grad);
+}
+
+// labels (B, S) -> per head: labels of its rows (heads, B * S), scored ones, gradient scale
+std::tuple<Tensor, Tensor, Tensor> mtp_labels(const Tensor& labels, const Tensor& weights, int64_t ignore_index) {
+  c10::cuda::CUDAGuard guard(labels.device());
+  TORCH_CHECK(labels.is_cuda() && labels.scalar_type() == at::kLong && labels.is_contiguous() && labels.dim() == 2);
+  need_f32(weights, "weights");
+  TORCH_CHECK(weights.is_contiguous() && weights.dim() == 1);
+  Tensor shifted = at::empty({weights.numel(), labels.numel()}, labels.options());
+  Tensor n_valid = at::empty_like(weights), grad_scale = at::empty_like(weights);
+  check(kmoe_mtp_labels((const long long*)labels.data_ptr<int64_t>(), labels.numel(), (int)labels.size(1),
+                        (int)weights.numel(), ignore_index, weights.data_ptr<float>(),
+                        (long long*)shifted.data_ptr<int64_t>(), n_valid.data_ptr<float>(), grad_scale.data_ptr<float>(),
+                        cur_stream()), "mtp_labels");
+  return {shifted, n_valid, grad_scale};
+}
+
+// loss_rows (scored heads, rows) -> (per head, weighted total)
+std::tuple<Tensor, Tensor> mtp_total(const Tensor& loss_rows, const Tensor& weights, const Tensor& n_valid) {
+  c10::cuda::CUDAGuard guard(weights.device());
+  need_f32(loss_rows, "loss_rows"); need_f32(weights, "weights"); need_f32(n_valid, "n_valid");
+  TORCH_CHECK(loss_rows.dim() == 2 && loss_rows.is_contiguous() && weights.is_contiguous() &&
+              n_valid.numel() == weights.numel() && loss_rows.size(0) <= weights.numel());
+  Tensor per = at::empty_like(weights), total = at::empty({}, weights.options());
+  check(kmoe_mtp_total(loss_rows.data_ptr<float>(), loss_rows.size(1), (int)weights.numel(), (int)loss_rows.size(0),
+                       weights.data_ptr<float>(), n_valid.data_ptr<float>(), per.data_ptr<float>(),
+                       total.data_ptr<float>(), cur_stream()), "mtp_total");
+  return {per, total};
 }
 
 // ------------------------------------------------------------- peer-to-peer collectives
@@ -1204,6 +1244,9 @@ TORCH_LIBRARY(kmoe, m) {
   m.def("moe_gather_dw", &moe_gather_dw);
   m.def("moe_choice_plan", &moe_choice_plan);
   m.def("ce_fwd_bwd", &ce_fwd_bwd);
+  m.def("ce_fwd_bwd_out", &ce_fwd_bwd_out);
+  m.def("mtp_labels", &mtp_labels);
+  m.def("mtp_total", &mtp_total);
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
   m.def("p2p_barrier", &p2p_barrier);

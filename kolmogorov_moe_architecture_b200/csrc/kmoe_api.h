@@ -299,6 +299,12 @@ int kmoe_mod_combine_bwd(const void* dout, const void* proc, const float* w, con
 // ---------------------------------------------------------------------------- loss
 int kmoe_ce_fwd_bwd(void* logits, const long long* labels, float* loss_rows, const float* grad_scale, int R, int V,
                     long long ld, long long ignore_index, int write_grad, cudaStream_t st);
+// per head (shift = index + 1): each token's label, how many are scored (at least 1) and weights[h] / that
+int kmoe_mtp_labels(const long long* labels, long long R, int S, int heads, long long ignore_index, const float* weights,
+                    long long* shifted, float* n_valid, float* grad_scale, cudaStream_t st);
+// loss_rows [scored, R] -> per[heads] (0 from `scored` on) and their weighted sum
+int kmoe_mtp_total(const float* loss_rows, long long R, int heads, int scored, const float* weights, const float* n_valid,
+                   float* per, float* total, cudaStream_t st);
 
 #ifdef __cplusplus
 }

@@ -1059,42 +1059,38 @@ class _MTPLoss(torch.autograd.Function):
             kb, kl = _split_k_ranges(V0, parts, hidden.device)
             parts = kb.numel()
             acc32 = torch.empty(parts * min(R, chunk_rows) * d, dtype=torch.float32, device=hidden.device)
-        heads = []                          # (index, weight, labels, gradient scale)
-        dWs: List[Optional[torch.Tensor]] = [None] * len(head_weights)
-        n_valid, loss_sum = [], []
-        for i, W in enumerate(head_weights):
-            shift = i + 1
-            loss_sum.append(torch.zeros((), dtype=torch.float32, device=hidden.device))
-            if shift >= S:
-                n_valid.append(None)
-                continue
-            lab = torch.full((B, S), ignore_index, dtype=torch.long, device=hidden.device)
-            lab[:, : S - shift] = labels[:, shift:]
-            lab = lab.reshape(R)
-            n_valid.append((lab != ignore_index).sum().clamp(min=1).float())
-            Wc = _aligned(W.contiguous())
-            dWs[i] = torch.empty_like(Wc) if need_grad else None
-            heads.append((i, Wc, lab, (float(weights[i]) / n_valid[i]).reshape(1).contiguous()))
+        # Heads the sequence is too short for have nothing to predict: they are the last ones.  Labels of any integer type.
+        scored = min(len(head_weights), max(S - 1, 0))
+        ws = [float(w) for w in weights]
+        if scored > len(ws):
+            raise IndexError(f"{len(ws)} head weights for {scored} heads")
+        wt = _head_weight_tensor(tuple((ws + [0.0] * len(head_weights))[:len(head_weights)]), hidden.device)
+        lab = labels.expand(B, S) if scored else torch.zeros(B, S, device=hidden.device)
+        lab = lab.to(hidden.device, torch.long).contiguous()
+        lab, n_valid, gscale = K.mtp_labels(lab, wt, ignore_index)  # LAUNCHES counts the passes over data, not this and the total
+        loss_rows = torch.empty(scored, R, dtype=torch.float32, device=hidden.device)
+        heads = [_aligned(W.contiguous()) for W in head_weights[:scored]]
+        dWs: List[Optional[torch.Tensor]] = [torch.empty_like(W) if need_grad else None for W in heads]
+        dWs += [None] * (len(head_weights) - scored)
         # row chunks outside, heads inside: what is held beside the results is one chunk's logits and accumulators
         for r0 in range(0, R, chunk_rows):
             r1 = min(R, r0 + chunk_rows)
             n = r1 - r0
             hc = h2[r0:r1]
-            for first, (i, Wc, lab, gscale) in enumerate(heads):
+            for i, Wc in enumerate(heads):
                 V = Wc.shape[0]
                 pitch = -(-V // 64) * 64        # whole 16-byte rows for TMA whatever the vocabulary (50257)
                 buf = torch.empty(n, pitch, dtype=h2.dtype, device=h2.device)
                 # N in whole output vectors: the columns past V are products with rows of W that read as zero
                 gemm(hc, Wc, buf, M=n, N=-(-V // 8) * 8, Kd=d, lda=d, ldb=d, ldc=pitch, b_rows=V)
-                rows = K.ce_fwd_bwd(buf[:, :V], lab[r0:r1].contiguous(), gscale, ignore_index, need_grad)
+                K.ce_fwd_bwd_out(buf[:, :V], lab[i, r0:r1], gscale[i], loss_rows[i, r0:r1], ignore_index, need_grad)
                 _count()
-                loss_sum[i] = loss_sum[i] + rows.sum()
                 if need_grad:
                     dst, kw = dH[r0:r1], {}
                     if parts > 1:
                         dst = acc32[:parts * n * d].view(parts, n, d)
                         kw = dict(mode=BATCHED, groups=parts, k_begin=kb, k_len=kl, c_gs=n * d)
-                    acc = dict(D=dst, beta=1.0) if first > 0 else {}
+                    acc = dict(D=dst, beta=1.0) if i > 0 else {}
                     gemm(buf, Wc, dst, M=n, N=d, Kd=V, b_major=MAJ_MN, lda=pitch, ldb=d, ldc=d, **acc, **kw)
                     acc = dict(D=dWs[i], beta=1.0) if r0 > 0 else {}
                     gemm(buf, hc, dWs[i], M=V, N=d, Kd=n, a_major=MAJ_MN, b_major=MAJ_MN, lda=pitch, ldb=d, ldc=d, **acc)
@@ -1103,9 +1099,9 @@ class _MTPLoss(torch.autograd.Function):
                 _count()
         if need_grad and not heads:
             dH.zero_()
-        per = [s_ if n is None else s_ / n for s_, n in zip(loss_sum, n_valid)]
-        per_t = torch.stack(per)
-        total = (per_t * _head_weight_tensor(tuple(float(w) for w in weights), hidden.device)).sum()
+        per_t, total = K.mtp_total(loss_rows, wt, n_valid)
+        if len(ws) != len(head_weights):
+            total = (per_t * _head_weight_tensor(tuple(ws), hidden.device)).sum()
         ctx.shape = (B, S, d)
         ctx.n_heads = len(head_weights)
         saved = [dH if dH is not None else torch.empty(0, device=hidden.device)]

@@ -1,0 +1,83 @@
+"""Output-head loss: wide rows of cross-entropy, the bookkeeping kernels around the rows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm().clamp(min=1e-30)).item()
+
+
+# one bf16 rounding (8 significant bits) of the result
+ONE_ROUNDING = 2.0 ** -8
+
+
+@pytest.mark.parametrize("R,V", [(1, 16384), (300, 16391), (149, 20000), (5, 57600), (3, 57601)])
+def test_wide_rows(R, V):
+    """More rows than CTAs run at once, a tail, labels in the tail and the last vector, ignored rows, minus infinity and the
+    type's lowest value among the entries."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(V)
+    pitch = -(-V // 64) * 64
+    buf = torch.full((R, pitch), float("nan"), dtype=torch.bfloat16, device="cuda")
+    buf[:, :V] = (torch.randn(R, V, device="cuda") * 3).to(torch.bfloat16)
+    buf[:, 7] = float("-inf")
+    buf[:, V // 2] = torch.finfo(torch.bfloat16).min
+    buf[0, 0] = 60.0
+    lab = torch.randint(8, V // 3, (R,), device="cuda")
+    lab[0] = V - 1
+    if R > 2:
+        lab[1], lab[2] = -100, V // 8 * 8 - 1
+    lg = buf[:, :V].double()
+    ref = torch.nn.functional.cross_entropy(lg, lab, ignore_index=-100, reduction="none")
+    p = (torch.softmax(lg, -1) - torch.nn.functional.one_hot(lab.clamp(min=0), V)) * 0.37
+    p[lab == -100] = 0
+    gs = torch.full((1,), 0.37, device="cuda")
+    only = c.K.ce_fwd_bwd(buf[:, :V], lab, gs, -100, False)
+    assert torch.equal(buf[:, :V].double(), lg)
+    rows = c.K.ce_fwd_bwd(buf[:, :V], lab, gs, -100, True)
+    assert torch.equal(only, rows)
+    assert (rows.double() - ref).abs().max() < 2.0 ** -18 * ref.abs().max().clamp(min=1)     # 32-bit sums
+    assert _rel(buf[:, :V], p) < ONE_ROUNDING
+    assert buf[:, V:].isnan().all()
+
+
+def test_rows_not_finite():
+    """Rows of minus infinity only, with a NaN, with plus infinity: no number, as in torch, and the rows beside them unharmed."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    V = 16400
+    buf = torch.zeros(4, -(-V // 64) * 64, dtype=torch.bfloat16, device="cuda")
+    buf[0], buf[1, 5], buf[2, 6] = float("-inf"), float("nan"), float("inf")
+    rows = c.K.ce_fwd_bwd(buf[:, :V], torch.tensor([3, 4, 5, 6], device="cuda"), torch.ones(1, device="cuda"), -100, True)
+    assert rows[:3].isnan().all() and abs(rows[3].item() - torch.tensor(float(V)).log().item()) < 1e-5
+
+
+@pytest.mark.parametrize("B,S,n", [(3, 1, 2), (2, 3, 4), (1, 70, 2), (2, 129, 3)])
+@pytest.mark.parametrize("dtype", [torch.long, torch.int32])
+def test_heads_and_labels(B, S, n, dtype):
+    """Sequences shorter than the heads reach, every label ignored for one head, labels of another integer type."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(S)
+    V, d = 200, 64
+    h = torch.randn(B, S, d, device="cuda").bfloat16().requires_grad_(True)
+    Ws = [(torch.randn(V, d, device="cuda") * 0.2).bfloat16().requires_grad_(True) for _ in range(n)]
+    lab = torch.randint(0, V, (B, S), device="cuda")
+    lab[:, S // 2:] = -100
+    w = tuple(1.0 / (i + 1) for i in range(n))
+    total, per = c.mtp_cross_entropy(h, Ws, lab.to(dtype), w)
+    hd, Wd = h.detach().double().requires_grad_(True), [W.detach().double().requires_grad_(True) for W in Ws]
+    want = 0.0
+    for i, W in enumerate(Wd):
+        tgt = lab[:, i + 1:].reshape(-1)
+        lg = (hd[:, :max(S - i - 1, 0)] @ W.t()).reshape(-1, V)
+        ce = torch.nn.functional.cross_entropy(lg, tgt, ignore_index=-100, reduction="sum") / max(1, int((tgt != -100).sum()))
+        assert abs(per[i].item() - ce.item()) < 0.01          # logits are rounded to bf16: 2^-8 of values up to 5
+        want = want + w[i] * ce
+    assert abs(total.item() - want.item()) < 0.02
+    assert torch.allclose(total, (per * torch.tensor(w, device="cuda")).sum(), rtol=1e-6)
+    got = torch.autograd.grad(total, [h, *Ws], allow_unused=True)
+    assert [g is None for g in got] == [False] + [i + 1 >= S for i in range(n)]
+    for g, r in zip(got, torch.autograd.grad(want, [hd, *Wd])):
+        if g is not None:
+            assert (g.double() - r).norm() <= 0.02 * r.norm()  # probabilities from rounded logits, two bf16 roundings
