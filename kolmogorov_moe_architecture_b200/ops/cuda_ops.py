@@ -1036,6 +1036,19 @@ def _loss_split(rows: int, d: int, V: int, sms: int = 148) -> int:
     return best
 
 
+def _saved_as_they_are() -> bool:
+    """No saved-tensor hooks are in force: what ``save_for_backward`` takes is what the backward pass gets, and nobody else
+    holds it."""
+    top = getattr(torch._C._autograd, "_top_saved_tensors_default_hooks", None)
+    return top is not None and top(False) is None
+
+
+def _graph_is_released() -> bool:
+    """Inside a backward pass: the graph is not retained, so no further pass will come through this node."""
+    keep = getattr(torch._C._autograd, "_get_current_graph_task_keep_graph", None)
+    return keep is not None and not keep()
+
+
 class _MTPLoss(torch.autograd.Function):
     """Per head: logits chunk = H W^T (tcgen05 GEMM) -> CE kernel writes d logits in place ->
     dH += dlogits W and dW = dlogits^T H.  Gradients are produced during forward (scaled
@@ -1107,6 +1120,7 @@ class _MTPLoss(torch.autograd.Function):
         saved = [dH if dH is not None else torch.empty(0, device=hidden.device)]
         saved += [w if w is not None else torch.empty(0, device=hidden.device) for w in dWs]
         ctx.save_for_backward(*saved)
+        ctx.own = _saved_as_they_are()
         ctx.need_grad = need_grad
         ctx.heads = head_weights
         ctx.mark_non_differentiable(per_t)
@@ -1120,7 +1134,16 @@ class _MTPLoss(torch.autograd.Function):
         B, S, d = ctx.shape
         g32 = g_total.reshape(1).float()
 
+        # The buffers of the forward pass become the gradients, scaled in place, when this is the graph's last pass and they
+        # are nobody else's (four heads of 50257 x 1536: 231 us and 0.6 GB of copies, now 2 us per launch where the
+        # factor is 1); a retained graph gets copies.
+        last = ctx.own and _graph_is_released()
+
         def scaled(t, dst=None):            # one vectorised pass, the factor read from the device
+            if dst is None and last and t.data_ptr() % 16 == 0:
+                K.scale_copy(t, t, g32)
+                _count()
+                return t
             dst = torch.empty_like(t) if dst is None else dst
             if dst.is_contiguous() and dst.data_ptr() % 16 == 0 and t.data_ptr() % 16 == 0:
                 K.scale_copy(t, dst, g32)

@@ -1,4 +1,4 @@
-"""Output-head loss: wide rows of cross-entropy, the bookkeeping kernels around the rows."""
+"""Output-head loss: wide rows of cross-entropy, the bookkeeping kernels around the rows, and who owns the gradients."""
 import pytest
 import torch
 
@@ -81,3 +81,33 @@ def test_heads_and_labels(B, S, n, dtype):
     for g, r in zip(got, torch.autograd.grad(want, [hd, *Wd])):
         if g is not None:
             assert (g.double() - r).norm() <= 0.02 * r.norm()  # probabilities from rounded logits, two bf16 roundings
+
+
+@pytest.mark.parametrize("how", ["retain", "hooks", "scaled"])
+def test_gradients_are_nobody_elses(how):
+    """The forward pass's buffers become the gradients only in the graph's last pass; a retained graph and saved-tensor hooks
+    get copies, whatever the caller does with the first pass's gradients."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(0)
+    h = torch.randn(2, 40, 64, device="cuda").bfloat16().requires_grad_(True)
+    W = (torch.randn(96, 64, device="cuda") * 0.2).bfloat16().requires_grad_(True)
+    lab = torch.randint(0, 96, (2, 40), device="cuda")
+    one = torch.autograd.grad(c.mtp_cross_entropy(h, [W], lab, (1.0,))[0], [h, W])
+    if how == "scaled":
+        got = torch.autograd.grad(c.mtp_cross_entropy(h, [W], lab, (1.0,))[0] * 4.0, [h, W])
+        assert all(torch.equal(g, 4.0 * o) for g, o in zip(got, one))
+    elif how == "retain":
+        total = c.mtp_cross_entropy(h, [W], lab, (1.0,))[0]
+        first = torch.autograd.grad(total, [h, W], retain_graph=True)
+        for g in first:
+            g.zero_()
+        got = torch.autograd.grad(total, [h, W])
+        assert all(torch.equal(g, o) for g, o in zip(got, one)) and not any(g.any() for g in first)
+    else:
+        held = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: held.append(t) or t, lambda t: t):
+            total = c.mtp_cross_entropy(h, [W], lab, (1.0,))[0]
+        before = [t.clone() for t in held]
+        got = torch.autograd.grad(total * 2.0, [h, W])
+        assert all(torch.equal(a, b) for a, b in zip(held, before))
+        assert all(torch.equal(g, 2.0 * o) for g, o in zip(got, one))
