@@ -21,29 +21,57 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf
 // one), before the first of them is looked at.
 // 4 x 2048 x 4096: forward 37.7 -> 36.6 us (20.5 at the copy rate), backward 132.5 -> 88.8 us (30.8) against one
 // channel, 64 steps and one row at a time per thread.
+// The backward kernel is bound by its instructions, fourteen multiply-adds per element: on packed pairs it takes 77.0 us
+// for 88.0 (three CTAs per SM).  The forward kernel, four per element, is not: 40.3 to 42.4 us on pairs (three to six
+// CTAs) for 39.4 with each batch's values widened first, so it keeps single floats.
 constexpr int CONV_T = 32;      // time steps per thread
 constexpr int CONV_WARPS = 8;
 
+// The values P of a thread's V channels at one step: a float or a packed pair, two channels for the arithmetic
+// instructions of one.
 template <int V>
 struct ConvVec;
 template <>
 struct ConvVec<1> {
   using Raw = unsigned short;
+  using P = float;
   __device__ static __forceinline__ Raw load(const __nv_bfloat16* p) { return __ldg(reinterpret_cast<const Raw*>(p)); }
-  __device__ static __forceinline__ void widen(Raw r, float (&v)[1]) { v[0] = __uint_as_float((uint32_t)r << 16); }
-  __device__ static __forceinline__ void store(__nv_bfloat16* p, const float (&v)[1]) { *p = __float2bfloat16(v[0]); }
+  __device__ static __forceinline__ P widen(Raw r) { return __uint_as_float((uint32_t)r << 16); }
+  __device__ static __forceinline__ void store(__nv_bfloat16* p, P v) { *p = __float2bfloat16(v); }
+  __device__ static __forceinline__ P fma(P a, P b, P c) { return fmaf(a, b, c); }
+  __device__ static __forceinline__ P mul(P a, P b) { return a * b; }
+  __device__ static __forceinline__ P add(P a, P b) { return a + b; }
+  __device__ static __forceinline__ P zero() { return 0.f; }
+  __device__ static __forceinline__ P gather(const float* p, int stride) { return p[0]; }
+  template <class F>
+  __device__ static __forceinline__ P map(P v, F f) { return f(v); }
+  __device__ static __forceinline__ void spread(P v, float (&o)[1]) { o[0] = v; }
 };
 template <>
 struct ConvVec<2> {
   using Raw = uint32_t;
+  using P = uint64_t;
   __device__ static __forceinline__ Raw load(const __nv_bfloat16* p) { return __ldg(reinterpret_cast<const Raw*>(p)); }
-  __device__ static __forceinline__ void widen(Raw r, float (&v)[2]) {
-    v[0] = __uint_as_float(r << 16);
-    v[1] = __uint_as_float(r & 0xffff0000u);
+  __device__ static __forceinline__ P widen(Raw r) {
+    return pack_f32x2(__uint_as_float(r << 16), __uint_as_float(r & 0xffff0000u));
   }
-  __device__ static __forceinline__ void store(__nv_bfloat16* p, const float (&v)[2]) {
-    *reinterpret_cast<uint32_t*>(p) = pack_bf16(v[0], v[1]);
+  __device__ static __forceinline__ void store(__nv_bfloat16* p, P v) {
+    float a, b;
+    unpack_f32x2(v, a, b);
+    *reinterpret_cast<uint32_t*>(p) = pack_bf16(a, b);
   }
+  __device__ static __forceinline__ P fma(P a, P b, P c) { return fma_f32x2(a, b, c); }
+  __device__ static __forceinline__ P mul(P a, P b) { return mul_f32x2(a, b); }
+  __device__ static __forceinline__ P add(P a, P b) { return add_f32x2(a, b); }
+  __device__ static __forceinline__ P zero() { return 0ull; }
+  __device__ static __forceinline__ P gather(const float* p, int stride) { return pack_f32x2(p[0], p[stride]); }
+  template <class F>
+  __device__ static __forceinline__ P map(P v, F f) {
+    float a, b;
+    unpack_f32x2(v, a, b);
+    return pack_f32x2(f(a), f(b));
+  }
+  __device__ static __forceinline__ void spread(P v, float (&o)[2]) { unpack_f32x2(v, o[0], o[1]); }
 };
 
 template <int V>
@@ -55,6 +83,7 @@ conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
   if (c >= C || t0 >= S) return;
   const int b = blockIdx.z;
   const int pc = (b / bpg) * C + c;   // parameter row: batch entries [g*bpg, (g+1)*bpg) use parameter set g
+  using CV = ConvVec<V>;
   float wv[V][4], bs[V];
 #pragma unroll
   for (int k = 0; k < V; ++k) {
@@ -69,17 +98,17 @@ conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
   for (int j = 0; j < 3; ++j) {
 #pragma unroll
     for (int k = 0; k < V; ++k) win[j][k] = 0.f;
-    if (t0 - 3 + j >= 0) ConvVec<V>::widen(ConvVec<V>::load(xb + (size_t)(t0 - 3 + j) * ldx), win[j]);
+    if (t0 - 3 + j >= 0) CV::spread(CV::widen(CV::load(xb + (size_t)(t0 - 3 + j) * ldx)), win[j]);
   }
   constexpr int BATCH = 8;
 #pragma unroll 1
   for (int tb = t0; tb < min(t0 + CONV_T, S); tb += BATCH) {
-    typename ConvVec<V>::Raw raw[BATCH];
+    typename CV::Raw raw[BATCH];
 #pragma unroll
-    for (int i = 0; i < BATCH; ++i) raw[i] = ConvVec<V>::load(xb + (size_t)min(tb + i, S - 1) * ldx);
+    for (int i = 0; i < BATCH; ++i) raw[i] = CV::load(xb + (size_t)min(tb + i, S - 1) * ldx);
     float xv[BATCH][V];
 #pragma unroll
-    for (int i = 0; i < BATCH; ++i) ConvVec<V>::widen(raw[i], xv[i]);
+    for (int i = 0; i < BATCH; ++i) CV::spread(CV::widen(raw[i]), xv[i]);
 #pragma unroll
     for (int i = 0; i < BATCH; ++i) {
       float o[V];
@@ -90,7 +119,7 @@ conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
         const float v = bs[k] + wv[k][0] * x0 + wv[k][1] * x1 + wv[k][2] * x2 + wv[k][3] * xv[i][k];
         o[k] = act ? silu_f(v) : v;
       }
-      if (tb + i < S) ConvVec<V>::store(yb + (size_t)(tb + i) * C, o);
+      if (tb + i < S) CV::store(yb + (size_t)(tb + i) * C, CV::gather(o, 1));
     }
 #pragma unroll
     for (int j = 0; j < 3; ++j)
@@ -102,7 +131,7 @@ conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
 // dx (rows lddx apart), and atomically accumulated dw [C,4], dbias [C] (fp32, zeroed by the caller; one addition per
 // channel and CTA).
 template <int V>
-__global__ void __launch_bounds__(32 * CONV_WARPS)
+__global__ void __launch_bounds__(32 * CONV_WARPS, 3)
 conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                   const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
                   float* __restrict__ dbias, int S, int C, long long ldx, long long lddx, int act, int bpg) {
@@ -112,72 +141,70 @@ conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
   const int t0 = (blockIdx.y * CONV_WARPS + warp) * CONV_T;
   const int b = blockIdx.z;
   const int pc = (b / bpg) * C + c;
-  float acc[V][5];                    // dw[0..3], dbias
+  using CV = ConvVec<V>;
+  using P = typename CV::P;
+  P acc[5];                           // dw[0..3], dbias
 #pragma unroll
-  for (int k = 0; k < V; ++k)
-#pragma unroll
-    for (int j = 0; j < 5; ++j) acc[k][j] = 0.f;
+  for (int j = 0; j < 5; ++j) acc[j] = CV::zero();
   if (c < C && t0 < S) {
-    float wv[V][4], bs[V];
+    P wv[4], bs = bias ? CV::gather(bias + pc, 1) : CV::zero();
 #pragma unroll
-    for (int k = 0; k < V; ++k) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) wv[k][j] = w[(size_t)(pc + k) * 4 + j];
-      bs[k] = bias ? bias[pc + k] : 0.f;
-    }
+    for (int j = 0; j < 4; ++j) wv[j] = CV::gather(w + (size_t)pc * 4 + j, 4);
     const __nv_bfloat16* xb = x + (size_t)b * S * ldx + c;
     const __nv_bfloat16* gb = dy + (size_t)b * S * C + c;
     __nv_bfloat16* dxb = dx + (size_t)b * S * lddx + c;
     const int t_own = min(t0 + CONV_T, S);
-    float xw[3][V], pw[3][V];         // x[t-3 .. t-1], dpre[t-3 .. t-1]; the dpre window starts empty, which is exact:
+    P xw[3], pw[3];                   // x[t-3 .. t-1], dpre[t-3 .. t-1]; the dpre window starts empty, which is exact:
 #pragma unroll                        // dx[td >= t0] never reads dpre[< t0]
     for (int j = 0; j < 3; ++j) {
-#pragma unroll
-      for (int k = 0; k < V; ++k) xw[j][k] = pw[j][k] = 0.f;
-      if (t0 - 3 + j >= 0) ConvVec<V>::widen(ConvVec<V>::load(xb + (size_t)(t0 - 3 + j) * ldx), xw[j]);
+      xw[j] = t0 - 3 + j >= 0 ? CV::widen(CV::load(xb + (size_t)(t0 - 3 + j) * ldx)) : CV::zero();
+      pw[j] = CV::zero();
     }
     constexpr int BATCH = 7;          // CONV_T + 3 steps in all: dx[t] needs dpre up to t + 3
     static_assert((CONV_T + 3) % BATCH == 0, "whole batches");
 #pragma unroll 1
     for (int tb = t0; tb < t0 + CONV_T + 3; tb += BATCH) {
-      typename ConvVec<V>::Raw xr[BATCH], gr[BATCH];
+      typename CV::Raw xr[BATCH], gr[BATCH];
 #pragma unroll
       for (int i = 0; i < BATCH; ++i) {
         const int t = min(tb + i, S - 1);
-        xr[i] = ConvVec<V>::load(xb + (size_t)t * ldx);
-        gr[i] = ConvVec<V>::load(gb + (size_t)t * C);
+        xr[i] = CV::load(xb + (size_t)t * ldx);
+        gr[i] = CV::load(gb + (size_t)t * C);
       }
 #pragma unroll
       for (int i = 0; i < BATCH; ++i) {
-        float o[V], xv[V], gv[V];
-        ConvVec<V>::widen(xr[i], xv);
-        ConvVec<V>::widen(gr[i], gv);
-#pragma unroll
-        for (int k = 0; k < V; ++k) {
-          const float x0 = xw[0][k], x1 = xw[1][k], x2 = xw[2][k], x3 = xv[k];
-          float g = tb + i < S ? gv[k] : 0.f;
-          if (act) {
-            const float pre = bs[k] + wv[k][0] * x0 + wv[k][1] * x1 + wv[k][2] * x2 + wv[k][3] * x3;
-            const float sg = sigmoid_f(pre);
-            g *= sg * (1.f + pre * (1.f - sg));
-          }
-          if (tb + i < t_own) {
-            acc[k][0] += g * x0; acc[k][1] += g * x1; acc[k][2] += g * x2; acc[k][3] += g * x3; acc[k][4] += g;
-          }
-          // dx[t - 3] = w0 dpre[t] + w1 dpre[t-1] + w2 dpre[t-2] + w3 dpre[t-3]
-          o[k] = wv[k][0] * g + wv[k][1] * pw[2][k] + wv[k][2] * pw[1][k] + wv[k][3] * pw[0][k];
-          xw[0][k] = x1; xw[1][k] = x2; xw[2][k] = x3;
-          pw[0][k] = pw[1][k]; pw[1][k] = pw[2][k]; pw[2][k] = g;
+        const P x3 = CV::widen(xr[i]);
+        P g = tb + i < S ? CV::widen(gr[i]) : CV::zero();
+        if (act) {
+          const P pre = CV::fma(wv[3], x3, CV::fma(wv[2], xw[2], CV::fma(wv[1], xw[1], CV::fma(wv[0], xw[0], bs))));
+          g = CV::mul(g, CV::map(pre, [](float u) {
+                        const float sg = sigmoid_f(u);
+                        return sg * (1.f + u * (1.f - sg));
+                      }));
         }
+        if (tb + i < t_own) {
+          acc[0] = CV::fma(g, xw[0], acc[0]);
+          acc[1] = CV::fma(g, xw[1], acc[1]);
+          acc[2] = CV::fma(g, xw[2], acc[2]);
+          acc[3] = CV::fma(g, x3, acc[3]);
+          acc[4] = CV::add(g, acc[4]);
+        }
+        // dx[t - 3] = w0 dpre[t] + w1 dpre[t-1] + w2 dpre[t-2] + w3 dpre[t-3]
+        const P o = CV::fma(wv[0], g, CV::fma(wv[1], pw[2], CV::fma(wv[2], pw[1], CV::mul(wv[3], pw[0]))));
+        xw[0] = xw[1]; xw[1] = xw[2]; xw[2] = x3;
+        pw[0] = pw[1]; pw[1] = pw[2]; pw[2] = g;
         const int td = tb + i - 3;
-        if (td >= t0 && td < t_own) ConvVec<V>::store(dxb + (size_t)td * lddx, o);
+        if (td >= t0 && td < t_own) CV::store(dxb + (size_t)td * lddx, o);
       }
     }
   }
 #pragma unroll
-  for (int k = 0; k < V; ++k)
+  for (int j = 0; j < 5; ++j) {
+    float v[V];
+    CV::spread(acc[j], v);
 #pragma unroll
-    for (int j = 0; j < 5; ++j) sums[warp][k * 5 + j][lane] = acc[k][j];
+    for (int k = 0; k < V; ++k) sums[warp][k * 5 + j][lane] = v[k];
+  }
   __syncthreads();
   for (int i = threadIdx.x; i < 5 * V * 32; i += 32 * CONV_WARPS) {
     const int kj = i / 32, l = i % 32, k = kj / 5, j = kj % 5, cc = (blockIdx.x * 32 + l) * V + k;
