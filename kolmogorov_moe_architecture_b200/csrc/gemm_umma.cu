@@ -754,7 +754,8 @@ constexpr int PAIR_TM = 2 * BM;
 // Expert-padded schedule: blocks per expert (counting the padding) from which pairs are taken.  Up / down / dH products
 // in µs, pairs against single CTAs, at d = 2048, f = 2816: 2.6 live blocks per expert 459/234/235 against 434/219/226,
 // 4.6 blocks 351/180/178 against 343/175/185, 6.4 blocks 309/157/156 against 310/165/167, 12.4 blocks 268/132/135 against
-// 272/141/149.
+// 272/141/149.  With eight epilogue warps the sums of the three are within 5 % of each other, either way, from 1.4 to 6.5
+// live blocks per expert (64 experts 633 to 667 against 635 to 643, 32 experts 679 to 703 against 684 to 690).
 constexpr int GROUPED_PAIR_MIN = 7;
 
 template <int BN, int A_MAJOR, int B_MAJOR>

@@ -21,9 +21,10 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf
 // one), before the first of them is looked at.
 // 4 x 2048 x 4096: forward 37.7 -> 36.6 us (20.5 at the copy rate), backward 132.5 -> 88.8 us (30.8) against one
 // channel, 64 steps and one row at a time per thread.
-// The backward kernel is bound by its instructions, fourteen multiply-adds per element: on packed pairs it takes 77.0 us
-// for 88.0 (three CTAs per SM).  The forward kernel, four per element, is not: 40.3 to 42.4 us on pairs (three to six
-// CTAs) for 39.4 with each batch's values widened first, so it keeps single floats.
+// Both are bound by issue slots (68 and 58 % busy) and latency, not by memory (DRAM at 29 and 27 %).  The backward kernel,
+// fourteen multiply-adds per element, takes 77.0 us on packed pairs for 88.0 on single floats (three CTAs per SM).  The
+// forward kernel, four per element, keeps single floats: 40.3 to 42.4 us on pairs (three to six CTAs) for 39.4 with each
+// batch's values widened first.  A batch loaded ahead costs the registers of a CTA: 43 and 81 us.
 constexpr int CONV_T = 32;      // time steps per thread
 constexpr int CONV_WARPS = 8;
 
