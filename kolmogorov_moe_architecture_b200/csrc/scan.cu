@@ -827,6 +827,7 @@ extern "C" int kmoe_scan_fwd(const void* u, const void* delta, const void* z, co
   ScanArgs a{(const __nv_bfloat16*)u, (const __nv_bfloat16*)delta, (const __nv_bfloat16*)z, A, Bm, Cm, D, dt_bias,
              S, C, ldz, ldbc, softplus, groups > 0 ? B / groups : 0, 1, 0};
   if (int rc = kmoe::check(a, bc_bf16, B, N, groups)) return rc;
+  if (B == 0 || S == 0 || C == 0) return 0;    // the kernels need a chunk: their warps finish one after the last
   plan(B, S, C, &a.P, &a.seg_len);
   if (a.P > 1 && seg == nullptr) return -5;
   return bc_bf16 ? launch_fwd<__nv_bfloat16>(a, out, ckpt, seg, B, st) : launch_fwd<float>(a, out, ckpt, seg, B, st);
@@ -843,6 +844,7 @@ extern "C" int kmoe_scan_bwd(const void* u, const void* delta, const void* z, co
              S, C, ldz, ldbc, softplus, groups > 0 ? B / groups : 0, 1, 0};
   if (int rc = kmoe::check(a, bc_bf16, B, N, groups)) return rc;
   if (z != nullptr && lddz % 8) return -4;
+  if (B == 0 || S == 0 || C == 0) return 0;    // as above; the sums stay at the caller's zeros
   plan(B, S, C, &a.P, &a.seg_len);
   if (a.P > 1 && (seg == nullptr || gseg == nullptr)) return -5;
   const int nx = (C + WCH - 1) / WCH;

@@ -59,6 +59,20 @@ def test_segments_chunks_layouts(B, S, C, form, gate):
         assert _rel(g, w) < TOL
 
 
+@pytest.mark.parametrize("B,S,C", [(1, 0, 64), (1, 0, 8), (0, 5, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_nothing_to_scan(B, S, C, dtype):
+    """An empty sequence or batch: an empty result, empty or zero gradients, no kernel."""
+    from kolmogorov_moe_architecture_b200 import ops
+    mk = lambda *s, t=torch.bfloat16: torch.ones(*s, dtype=t, device="cuda").requires_grad_(True)
+    args = [mk(B, S, C), mk(B, S, C), mk(C, 16, t=torch.float32), mk(B, S, 16, t=dtype), mk(B, S, 16, t=dtype),
+            mk(C, t=torch.float32), mk(B, S, C), mk(C, t=torch.float32)]
+    y = ops.selective_scan(*args)
+    assert y.shape == (B, S, C)
+    for g, t in zip(torch.autograd.grad(y, args, torch.ones_like(y)), args):
+        assert g.shape == t.shape and not g.any()
+
+
 def test_no_checkpoints_without_gradients():
     """Under no_grad the state before every chunk (16 fp32 values per channel and 8 steps, four times the output) is not kept."""
     from kolmogorov_moe_architecture_b200 import ops
