@@ -1036,6 +1036,17 @@ def _loss_split(rows: int, d: int, V: int, sms: int = 148) -> int:
     return best
 
 
+def _label_rows(labels: torch.Tensor, B: int, S: int, scored: int, ignore_index: int, device) -> torch.Tensor:
+    """The (B, S) labels that ``scored`` heads read, as int64 on ``device``.  Labels of another shape are what an assignment
+    to each head's slice makes of them: one row serves every sequence, a missing dimension or a wrong length is refused."""
+    if tuple(labels.shape) == (B, S):
+        return labels.to(device, torch.long).contiguous()
+    rows = torch.full((B, S), ignore_index, dtype=torch.long, device=device)
+    for shift in range(scored, 0, -1):
+        rows[:, shift:] = labels[:, shift:]
+    return rows
+
+
 def _saved_as_they_are() -> bool:
     """No saved-tensor hooks are in force: what ``save_for_backward`` takes is what the backward pass gets, and nobody else
     holds it."""
@@ -1072,14 +1083,13 @@ class _MTPLoss(torch.autograd.Function):
             kb, kl = _split_k_ranges(V0, parts, hidden.device)
             parts = kb.numel()
             acc32 = torch.empty(parts * min(R, chunk_rows) * d, dtype=torch.float32, device=hidden.device)
-        # Heads the sequence is too short for have nothing to predict: they are the last ones.  Labels of any integer type.
+        # Heads the sequence is too short for have nothing to predict: they are the last ones.
         scored = min(len(head_weights), max(S - 1, 0))
         ws = [float(w) for w in weights]
         if scored > len(ws):
             raise IndexError(f"{len(ws)} head weights for {scored} heads")
         wt = _head_weight_tensor(tuple((ws + [0.0] * len(head_weights))[:len(head_weights)]), hidden.device)
-        lab = labels.expand(B, S) if scored else torch.zeros(B, S, device=hidden.device)
-        lab = lab.to(hidden.device, torch.long).contiguous()
+        lab = _label_rows(labels, B, S, scored, ignore_index, hidden.device)
         lab, n_valid, gscale = K.mtp_labels(lab, wt, ignore_index)  # LAUNCHES counts the passes over data, not this and the total
         loss_rows = torch.empty(scored, R, dtype=torch.float32, device=hidden.device)
         heads = [_aligned(W.contiguous()) for W in head_weights[:scored]]

@@ -83,6 +83,24 @@ def test_heads_and_labels(B, S, n, dtype):
             assert (g.double() - r).norm() <= 0.02 * r.norm()  # probabilities from rounded logits, two bf16 roundings
 
 
+def test_label_shapes():
+    """One row of labels serves every sequence; labels without a batch dimension, of one column or of another length are
+    refused, and none are looked at where no head has anything to predict."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(0)
+    B, S, V, d = 3, 9, 96, 64
+    h = torch.randn(B, S, d, device="cuda").bfloat16()
+    Ws = [(torch.randn(V, d, device="cuda") * 0.2).bfloat16() for _ in range(2)]
+    row = torch.randint(0, V, (1, S), device="cuda")
+    run = lambda lab, n=2, x=h: c.mtp_cross_entropy(x, Ws[:n], lab, (1.0, 0.5)[:n])
+    assert all(torch.equal(a, b) for a, b in zip(run(row), run(row.repeat(B, 1))))
+    assert all(torch.equal(a, b) for a, b in zip(run(row.cpu().float()), run(row)))
+    for shape in [(S,), (B, 1), (1, 1), (B, S - 1), (B, S + 1), (2, S), (B, S, 1)]:
+        with pytest.raises((IndexError, RuntimeError)):
+            run(torch.zeros(shape, dtype=torch.long, device="cuda"))
+    assert run(torch.zeros(4, dtype=torch.long, device="cuda"), 1, h[:, :1])[0].item() == 0.0
+
+
 @pytest.mark.parametrize("how", ["retain", "hooks", "scaled"])
 def test_gradients_are_nobody_elses(how):
     """The forward pass's buffers become the gradients only in the graph's last pass; a retained graph and saved-tensor hooks
