@@ -307,6 +307,16 @@ inline void check_scan_bc(const Tensor& Bm, const Tensor& Cm) {
               (Bm.scalar_type() == at::kBFloat16 || Bm.scalar_type() == at::kFloat) && row_stride(Bm) == row_stride(Cm),
               "B and C must be bf16 or fp32 [B,S,N] tensors of one layout");
 }
+// What the scan's backward pass reads of the forward pass: the kernel copies whole 16-channel blocks of the checkpoints
+// without a test per channel.
+inline void check_scan_saved(const Tensor& ckpt, const Tensor& seg, int64_t B, int64_t S, int64_t C, int64_t N) {
+  need_f32(ckpt, "ckpt"); need_f32(seg, "seg");
+  TORCH_CHECK(ckpt.is_contiguous() && ckpt.numel() == kmoe_scan_ckpt_floats((int)B, (int)S, (int)C),
+              "checkpoints of the forward pass expected");
+  const int64_t P = kmoe_scan_segments((int)B, (int)S, (int)C);
+  TORCH_CHECK(P == 1 || (seg.is_contiguous() && seg.numel() == B * P * (N + 1) * C),
+              "segment scratch of the forward pass expected");
+}
 inline void need_aligned(const Tensor& t, const char* n) {
   TORCH_CHECK(t.numel() == 0 || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0, n, " must be 16-byte aligned");
 }
@@ -353,7 +363,7 @@ std::vector<Tensor> scan_bwd(const Tensor& u, const Tensor& delta, const OptT& z
   Tensor dD = A.dim() == 3 ? at::zeros({G, C}, f32) : at::zeros({C}, f32);
   Tensor dbias = at::zeros_like(dD);
   const int P = kmoe_scan_segments(B, S, C);
-  TORCH_CHECK(P == 1 || seg.numel() == (int64_t)B * P * (N + 1) * C, "segment scratch of the forward pass expected");
+  check_scan_saved(ckpt, seg, B, S, C, N);
   Tensor gseg = P > 1 ? at::empty({B, P, C, N}, f32) : at::empty({0}, f32);
   check(kmoe_scan_bwd(u.data_ptr(), delta.data_ptr(), has_z ? z->data_ptr() : nullptr, A.data_ptr<float>(),
                       Bm.data_ptr(), Cm.data_ptr(), row_stride(Bm), Bm.scalar_type() == at::kBFloat16,
@@ -1068,6 +1078,7 @@ std::vector<Tensor> mamba_inner_bwd(const Tensor& dy_in, const Tensor& xz, const
   need_bf16(dy, "dy");
   const int64_t B = xz.size(0), S = xz.size(1), C = xz.size(2) / 2, T = B * S, R = dt_w.size(1), N = 16, ld = R + 2 * N;
   TORCH_CHECK(dy.numel() == T * C, "dy does not match");
+  check_scan_saved(ckpt, seg, B, S, C, N);
   auto f32 = xz.options().dtype(at::kFloat);
   // everything that accumulates, zeroed together: the small parameters' gradients, dB, dC
   Tensor acc = at::zeros({23 * C + 2 * T * N}, f32);

@@ -73,6 +73,31 @@ def test_nothing_to_scan(B, S, C, dtype):
         assert g.shape == t.shape and not g.any()
 
 
+def test_backward_takes_its_own_checkpoints_only():
+    """Checkpoints are whole 16-channel blocks; those of a pass without gradients (none) or of the bare channels are refused by
+    the single op and by the mixer."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    K, st = c.K, c.status_tensor(torch.device("cuda", torch.cuda.current_device()))
+    B, S, C, R = 1, 24, 72, 8
+    mk = lambda *s: torch.ones(*s, dtype=torch.bfloat16, device="cuda")
+    u, A, bc = mk(B, S, C), -torch.ones(C, 16, device="cuda"), mk(B, S, 16)
+    _, ckpt, seg = K.scan_fwd(u, u, None, A, bc, bc, None, None, True, True)
+    assert ckpt.numel() == 3 * 80 * 16 and seg.numel() == 0
+    scan = lambda ck: K.scan_bwd(u, u, None, A, bc, bc, None, None, u, ck, seg, True)
+    W = 64                                    # the mixer's width
+    p = [mk(W, 4), mk(W), mk(R + 32, W), mk(W, R), mk(W), mk(W, 16), mk(W)]
+    xz = mk(B, S, 2 * W)
+    y, x, x_dbl, delta, params, ckpt2, seg2 = K.mamba_inner_fwd(xz, *p, True, st)
+    mixer = lambda ck: K.mamba_inner_bwd(y, xz, x, x_dbl, delta, params, ck, seg2, p[2], p[3], True, False, None, None, None,
+                                         False, None, None, None, st)
+    for bwd, own in ((scan, ckpt), (mixer, ckpt2)):
+        bwd(own)
+        for other in (own[:0], own[:-3 * 8 * 16], own.double()):
+            with pytest.raises(RuntimeError, match="ckpt|checkpoints"):
+                bwd(other)
+    c.check_status()
+
+
 def test_no_checkpoints_without_gradients():
     """Under no_grad the state before every chunk (16 fp32 values per channel and 8 steps, four times the output) is not kept."""
     from kolmogorov_moe_architecture_b200 import ops
