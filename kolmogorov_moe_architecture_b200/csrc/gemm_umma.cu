@@ -2,7 +2,7 @@
 //
 //   warp 0      : TMA producer  (cp.async.bulk.tensor -> 128B-swizzled smem ring, mbarrier tx counts)
 //   warp 1      : MMA issuer    (tcgen05.mma 128 x BN x 16, accumulators in TMEM, double buffered)
-//   warps 4..11 : epilogue      (tcgen05.ld -> registers -> fused epilogue -> global)
+//   warps 2..5  : epilogue      (tcgen05.ld -> registers -> fused epilogue -> global); in the CTA-pair kernel 4..11
 //
 // One CTA per SM walks a static tile list, so the epilogue of tile i overlaps the
 // main loop of tile i+1.  Operands may be K-major or MN-major (the MMA reads either
@@ -31,12 +31,15 @@ namespace kmoe {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int A_STAGE_BYTES = BM * BK * 2;
-// Three warpgroups: producer and issuer (and two idle warps), two of epilogue.  The register file is split unevenly, 384 x
-// 168 at launch; all take that again before the common end of the kernel.
-constexpr int NUM_THREADS = 384;
-constexpr int EPI_WARPS = 8;
+// Single-CTA kernel: producer, issuer, four epilogue warps.  It has the small products, and their time is the launch and one
+// tile after another on a mostly idle chip, which a second epilogue warp per scheduler does not shorten: in the
+// pair kernel's form it took 6.3 us for 8 x 512 x 512 (with four warps 5.7), 10.4 for 96 x 1536 x 1536 (9.7).
+constexpr int CTA_THREADS = 192, CTA_EPI_WARPS = 4;
+// CTA-pair kernel: three warpgroups, producer and issuer (and two idle warps), two of epilogue.  The register file is split
+// unevenly, 384 x 168 at launch; all take that again before the common end of the kernel.
+constexpr int PAIR_THREADS = 384, PAIR_EPI_WARPS = 8;
 constexpr int LAUNCH_REGS = 168, EPI_REGS = 216, ROLE_REGS = 72;
-static_assert(256 * EPI_REGS + 128 * ROLE_REGS == NUM_THREADS * LAUNCH_REGS, "register split");
+static_assert(256 * EPI_REGS + 128 * ROLE_REGS == PAIR_THREADS * LAUNCH_REGS, "register split");
 template <int N>
 __device__ __forceinline__ void set_regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
@@ -79,7 +82,7 @@ struct GemmArgs {
 constexpr int RANGES_MAX = 128;
 __device__ __forceinline__ void fill_ranges(const GemmArgs& a, int2* ranges) {
   if (a.mode == KMOE_GEMM_BATCHED && a.k_begin != nullptr)
-    for (int g = threadIdx.x; g < min(a.groups, RANGES_MAX); g += NUM_THREADS) ranges[g] = make_int2(a.k_begin[g], a.k_len[g]);
+    for (int g = threadIdx.x; g < min(a.groups, RANGES_MAX); g += blockDim.x) ranges[g] = make_int2(a.k_begin[g], a.k_len[g]);
 }
 
 struct Tile {
@@ -260,27 +263,41 @@ __device__ __forceinline__ void epilogue_store_chunk_f32(const GemmArgs& a, cons
 }
 
 // ------------------------------------------------------------------ bf16 epilogue
-// An epilogue warp owns 32 accumulator rows (lane = row) and every other 64-column slab; two warps share the rows.  A slab
-// is read from tensor memory, finished in registers, rounded into the warp's 4 KB staging buffer (32 rows x 128 bytes in
-// the 128-byte swizzle, so that both the row-per-lane writes and TMA's reads are free of bank conflicts) and sent off by a
-// TMA store, which also clips at M and N.  The warp waits for that store to have read the buffer only when it has the next
-// slab's values, and the accumulator goes back to the MMA warp as soon as the last slab is in registers.
+// An epilogue warp owns 32 accumulator rows (lane = row); of eight warps two share the rows, each with every other 64-column
+// slab.  A slab is read from tensor memory, finished in registers, rounded into a 4 KB staging buffer (32 rows x 128 bytes
+// in the 128-byte swizzle, so that both the row-per-lane writes and TMA's reads are free of bank conflicts) and sent off by
+// a TMA store, which also clips at M and N.  One of four warps has two buffers, one of eight has one; it waits for a store
+// to have read its buffer only when it has the values that go there next, and the accumulator goes back to the MMA warp
+// as soon as the last slab is in registers.
 // A tile whose reduction is shorter than its epilogue is bound by this code (weight gradients of experts with few
 // tokens, orthogonalisation): a slab is a chain of latencies, 925 clocks, so with one warp per scheduler (four in all, two
 // buffers each) a 256 x 256 tile took 5000 clocks - ten reduction blocks' worth - and takes 3400 to 4000 with two warps per
 // scheduler (weight gradients of the 3B preset's 64 experts: 681 us, 634 with eight warps, 552 with the relaxed arrival at
 // the pair's leader, 514 with `list_div`).
 constexpr int OUT_BUF_BYTES = 32 * 128;
-constexpr int OUT_STAGE_BYTES = EPI_WARPS * OUT_BUF_BYTES;     // one buffer per epilogue warp
+constexpr int OUT_STAGE_BYTES = 8 * OUT_BUF_BYTES;
 
+template <int WARPS>
 struct OutStage {
-  uint8_t* base;
-  int half;        // this warp's slabs: half, half + 2, ...
+  static constexpr int STEP = WARPS / 4, BUFS = 8 / WARPS;
+  uint8_t* base;   // of this warp's BUFS buffers
+  int half;        // this warp's slabs: half, half + STEP, ...
+  int buf;
+  __device__ __forceinline__ OutStage(uint8_t* stage, int epi_warp)
+      : base(stage + (WARPS == 4 ? epi_warp % 4 : epi_warp) * BUFS * OUT_BUF_BYTES),
+        half(WARPS == 4 ? 0 : epi_warp / 4), buf(0) {}
 };
-__device__ __forceinline__ uint8_t* out_acquire(const OutStage& o, int lane) {
-  if (lane == 0) tma_store_wait_read();
+template <int WARPS>
+__device__ __forceinline__ uint8_t* out_acquire(OutStage<WARPS>& o, int lane) {
+  if (lane == 0) {
+    if (OutStage<WARPS>::BUFS == 2) tma_store_wait_read_but_one();
+    else tma_store_wait_read();
+  }
   __syncwarp();
-  return o.base;
+  if (OutStage<WARPS>::BUFS == 1) return o.base;
+  uint8_t* p = o.base + o.buf * OUT_BUF_BYTES;
+  o.buf ^= 1;
+  return p;
 }
 __device__ __forceinline__ void out_put_row(uint8_t* sb, int lane, const uint32_t (&p)[32]) {
 #pragma unroll
@@ -300,9 +317,9 @@ __device__ __forceinline__ void out_send(const CUtensorMap* tm, const uint8_t* s
 // C = scale * acc (+ diag) (+ beta D + beta2 D2), all in fp32 before the one rounding.  `mirror`: the tile lies above
 // the diagonal of a symmetric product and also writes its transpose (tmT: boxes of 32 columns x 64 rows).
 // wait() returns once the accumulator is complete (false: gave up), release() hands it back.
-template <int BN, class Wait, class Release>
+template <int BN, class Stage, class Wait, class Release>
 __device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtensorMap* tmC, const CUtensorMap* tmT,
-                                                const OutStage& out, uint32_t t_row, bool have_acc, int row0, int n0, int g,
+                                                Stage& out, uint32_t t_row, bool have_acc, int row0, int n0, int g,
                                                 float scale, float beta, float beta2, bool mirror, int lane,
                                                 Wait wait, Release release) {
   const int slabs = row0 < a.M ? min(BN / 64, ceil_div(a.N - n0, 64)) : 0, first = out.half;
@@ -326,7 +343,7 @@ __device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtenso
   if (first >= slabs) release();
   // the loop stays rolled: unrolled, the epilogue outgrows the instruction cache
 #pragma unroll 1
-  for (int sl = first; sl < slabs; sl += 2) {
+  for (int sl = first; sl < slabs; sl += Stage::STEP) {
     const int col = n0 + sl * 64;
     uint32_t r[64];
     if (have_acc) {
@@ -337,7 +354,7 @@ __device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtenso
 #pragma unroll
       for (int i = 0; i < 64; ++i) r[i] = 0u;
     }
-    if (sl + 2 >= slabs) release();
+    if (sl + Stage::STEP >= slabs) release();
 #pragma unroll
     for (int i = 0; i < 64; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * scale);
     if (diag) {
@@ -371,7 +388,7 @@ __device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtenso
         }
         __syncwarp();
       }
-      if (sl + 2 < slabs) load_addend(Dp, col + 128);
+      if (sl + Stage::STEP < slabs) load_addend(Dp, col + 64 * Stage::STEP);
     }
     uint32_t p[32];
 #pragma unroll
@@ -397,16 +414,16 @@ __device__ __forceinline__ bool store_tile_bf16(const GemmArgs& a, const CUtenso
 
 // H = silu(gate) * up * scale, with the pre-activations G and U stored as well when asked for.  The accumulator holds
 // HB gate columns followed by the HB up columns of the same outputs.
-template <int HB, class Release>
+template <int HB, class Stage, class Release>
 __device__ __forceinline__ void store_tile_swiglu(const GemmArgs& a, const CUtensorMap* tmH, const CUtensorMap* tmG,
-                                                  const CUtensorMap* tmU, const OutStage& out, uint32_t t_row, bool have_acc,
+                                                  const CUtensorMap* tmU, Stage& out, uint32_t t_row, bool have_acc,
                                                   int row0, int n0, int g, float scale, int lane, Release release) {
   const int slabs = row0 < a.M ? min(HB / 64, ceil_div(a.N - n0, 64)) : 0;
   if (out.half >= slabs) release();
   // Three results per slab, one after the other: reading tensor memory again costs less than holding both slabs in
   // registers (192 of them, which spilled).
 #pragma unroll 1
-  for (int sl = out.half; sl < slabs; sl += 2) {
+  for (int sl = out.half; sl < slabs; sl += Stage::STEP) {
     const int col = n0 + sl * 64;
     const int last = a.U_out != nullptr ? 2 : (a.G_out != nullptr ? 1 : 0);
 #pragma unroll 1
@@ -437,7 +454,7 @@ __device__ __forceinline__ void store_tile_swiglu(const GemmArgs& a, const CUten
         for (int i = 0; i < 16; ++i)
           p[h * 16 + i] = pack_bf16(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1]));
       }
-      if (sl + 2 >= slabs && what == last) release();
+      if (sl + Stage::STEP >= slabs && what == last) release();
       uint8_t* sb = out_acquire(out, lane);
       out_put_row(sb, lane, p);
       out_send(what == 0 ? tmH : (what == 1 ? tmG : tmU), sb, lane, col, row0, g);
@@ -472,7 +489,7 @@ __device__ __forceinline__ void load_mn_tile_pair(uint8_t* dst, const CUtensorMa
 }
 
 template <int BN, int A_MAJOR, int B_MAJOR>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(CTA_THREADS, 1)
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
                  const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY, const GemmArgs args,
@@ -502,7 +519,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], EPI_WARPS);  // one arrival per epilogue warp
+      mbar_init(&tmem_empty[i], CTA_EPI_WARPS);  // one arrival per epilogue warp
     }
     mbar_fence_init();
     prefetch_tmap(&tmA);
@@ -524,9 +541,6 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (args.mode == KMOE_GEMM_GROUPED_M) num_m = min(num_m, *args.num_m_tiles);
   const int num_n = ceil_div(args.N, n_per_tile);
 
-  if (warp < 4) {
-    set_regs_down<ROLE_REGS>();
-    {
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (elect_one()) {
@@ -537,7 +551,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int kb = 0; kb < t.k_blocks; ++kb) {
           if (!mbar_wait(&empty_bar[s], ph ^ 1)) {
             atomicExch(args.status, 1);
-            goto role_done;
+            goto teardown;
           }
           uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + A_STAGE_BYTES;
@@ -582,14 +596,14 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         ++it;
         if (!mbar_wait(&tmem_empty[acc], acc_ph ^ 1)) {
           atomicExch(args.status, 2);
-          goto role_done;
+          goto teardown;
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < t.k_blocks; ++kb) {
           if (!mbar_wait(&full_bar[s], ph)) {
             atomicExch(args.status, 3);
-            goto role_done;
+            goto teardown;
           }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
@@ -612,19 +626,12 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           mbar_arrive(&tmem_full[acc]);
       }
     }
-  }
-    }
-  role_done:
-    warpgroup_sync();
-    set_regs_up<LAUNCH_REGS>();
   } else {
-    set_regs_up<EPI_REGS>();
-    {
     // ------------------------------------------------------------ epilogue
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     int it = 0;
     Tile t;
-    const OutStage out{smem + stages * STAGE_BYTES + (warp - 4) * OUT_BUF_BYTES, (warp - 4) >> 2};
+    OutStage<CTA_EPI_WARPS> out(smem + stages * STAGE_BYTES, q);
     for (int idx = blockIdx.x; get_tile<BN>(args, idx, num_m, num_n, t, ranges); idx += gridDim.x) {
       const int acc = it & 1;
       const uint32_t acc_ph = (it >> 1) & 1;
@@ -655,10 +662,10 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!swiglu && !args.out_f32 && args.row_ptr == nullptr) {
         if (!store_tile_bf16<BN>(args, &tmC, &tmX, out, t_row, have_acc, row0, t.n_tile * BN, t.g_c, scale, beta, 0.f,
                                  false, lane, wait, release))
-          goto epi_done;
+          goto teardown;
         continue;
       }
-      if (!wait()) goto epi_done;
+      if (!wait()) goto teardown;
       if (swiglu) {
         store_tile_swiglu<BN / 2>(args, &tmC, &tmX, &tmY, out, t_row, have_acc, row0, t.n_tile * (BN / 2), t.g_c, scale,
                                   lane, release);
@@ -671,11 +678,10 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // would emit 32 scattered 16-byte writes per instruction; the 64-column slab is staged in shared
         // memory instead and written back with 8 lanes per row: four full 128-byte lines per instruction.
         const long long row_addr = row_ok ? args.row_ptr[row] : 0;
-        __nv_bfloat16(*stg)[72] =
-            reinterpret_cast<__nv_bfloat16(*)[72]>(smem + stages * STAGE_BYTES + q * 2 * OUT_BUF_BYTES);    // 32 rows, 4.5 KB
+        __nv_bfloat16(*stg)[72] = reinterpret_cast<__nv_bfloat16(*)[72]>(out.base);      // 32 rows, within 8 KB
         const __nv_bfloat16* Dp = reinterpret_cast<const __nv_bfloat16*>(args.D);
 #pragma unroll 1
-        for (int c = 0; out.half == 0 && c < BN; c += 64) {
+        for (int c = 0; c < BN; c += 64) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint32_t r[32];
@@ -713,7 +719,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
       } else {
 #pragma unroll 1
-        for (int c = out.half * (BN / 2); c < (out.half + 1) * (BN / 2); c += 32) {
+        for (int c = 0; c < BN; c += 32) {
           uint32_t r[32];
           if (have_acc) {
             tmem_ld_32x32(t_row + c, r);
@@ -725,13 +731,10 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       release();
     }
-    }
-  epi_done:
-    if (lane == 0) tma_store_wait_all();
-    warpgroup_sync();
-    set_regs_down<LAUNCH_REGS>();
   }
 
+teardown:
+  if (warp >= 2 && lane == 0) tma_store_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -759,7 +762,7 @@ constexpr int PAIR_TM = 2 * BM;
 constexpr int GROUPED_PAIR_MIN = 7;
 
 template <int BN, int A_MAJOR, int B_MAJOR>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
                  const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY, const GemmArgs args,
@@ -797,7 +800,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 2 * EPI_WARPS);   // the epilogue warps of both CTAs
+      mbar_init(&tmem_empty[i], 2 * PAIR_EPI_WARPS);   // the epilogue warps of both CTAs
     }
     mbar_fence_init();
     prefetch_tmap(&tmA);
@@ -918,7 +921,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const int q = warp & 3;
     int it = 0;
     Tile t;
-    const OutStage out{smem + stages * STAGE_BYTES + (warp - 4) * OUT_BUF_BYTES, (warp - 4) >> 2};
+    OutStage<PAIR_EPI_WARPS> out(smem + stages * STAGE_BYTES, warp - 4);
     for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, ranges, pair_list); idx += num_pairs) {
       const int acc = it & 1;
       const uint32_t acc_ph = (it >> 1) & 1;
@@ -1103,7 +1106,7 @@ static int launch_variant(const CUtensorMap& tA, const CUtensorMap& tB, const CU
   auto kern = umma_gemm_kernel<BN, AM, BMj>;
   static SmemLimit limit;
   if (!limit.raise(kern, smem)) return -20;
-  kern<<<grid, NUM_THREADS, smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
+  kern<<<grid, CTA_THREADS, smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
@@ -1122,7 +1125,7 @@ static int launch_pair_variant(const CUtensorMap& tA, const CUtensorMap& tB, con
   if (max_clusters == 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * (sms / 2)));
-    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.blockDim = dim3(PAIR_THREADS);
     cfg.dynamicSmemBytes = (size_t)smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1134,7 +1137,7 @@ static int launch_pair_variant(const CUtensorMap& tA, const CUtensorMap& tB, con
   }
   long long pairs = pair_tiles < max_clusters ? pair_tiles : max_clusters;
   if (pairs < 1) pairs = 1;
-  kern<<<(unsigned)(2 * pairs), NUM_THREADS, smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
+  kern<<<(unsigned)(2 * pairs), PAIR_THREADS, smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 

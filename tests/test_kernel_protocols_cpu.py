@@ -371,23 +371,25 @@ def run_fwd2(nb, seed):
 
 
 # ---------------------------------------------------------------- persistent GEMMs (csrc/gemm_umma.cu)
-W8 = range(8)         # epilogue warps of a CTA: two per 32 rows, each with every other column slab
-
-
-def run_gemm(k_blocks, stages, seed, ctas=1, slabs=2, in_flight=0):
+def run_gemm(k_blocks, stages, seed, ctas=1, slabs=None, in_flight=None):
     """``umma_gemm_kernel`` (ctas=1) and ``umma_gemm_pair_kernel`` (ctas=2) for the tiles one CTA (pair) works
     through: ``k_blocks[i]`` reduction blocks for tile i (0 = a group without rows in a batched product: the
     epilogue writes zeros / the addend and the issuer arrives by itself).  Ring of ``stages`` shared-memory
-    stages, two accumulators, eight epilogue warps per CTA.  A warp takes its share of the accumulator in ``slabs`` column
-    slabs, hands it back with the last one in registers, and sends each slab from its staging buffer by a TMA store that it
-    does not wait for: before it writes the next slab, all but ``in_flight`` of its stores have been read.  In the pair the ``full`` and ``tmem_empty`` barriers
-    live in the leader, ``empty`` and ``tmem_full`` exist in both CTAs and get the leader's commits."""
+    stages, two accumulators.  A CTA of the pair has eight epilogue warps, two per 32 rows, each with every other column
+    slab and one staging buffer; the single CTA has four with all slabs and two buffers in turn.  A warp takes its share
+    of the accumulator in ``slabs`` column slabs, hands it back with the last one in registers, and sends each slab from
+    a staging buffer by a TMA store that it does not wait for: before it writes the next slab, all but ``in_flight`` (one
+    less than its buffers) of its stores have been read.  In the pair the ``full`` and ``tmem_empty`` barriers live in
+    the leader, ``empty`` and ``tmem_full`` exist in both CTAs and get the leader's commits."""
     m = Machine(seed)
     C = range(ctas)
+    W, buffers = (range(4), 2) if ctas == 1 else (range(8), 1)
+    slabs = 8 // len(W) * 2 if slabs is None else slabs
+    in_flight = buffers - 1 if in_flight is None else in_flight
     full = [Bar(1 + ctas) for _ in range(stages)]         # the leader's expect_tx + one load group per CTA
     empty = [[Bar(1) for _ in range(stages)] for _ in C]
     tmem_full = [[Bar(1), Bar(1)] for _ in C]
-    tmem_empty = [Bar(8 * ctas), Bar(8 * ctas)]
+    tmem_empty = [Bar(len(W) * ctas), Bar(len(W) * ctas)]
 
     def producer(c):
         s, ph, n = 0, 0, 0
@@ -411,8 +413,8 @@ def run_gemm(k_blocks, stages, seed, ctas=1, slabs=2, in_flight=0):
                 yield ("wait", full[s], ph)
                 reads = [(("stage", c, s), ("AB", n)) for c in C]
                 if kb > 0:
-                    reads += [(("acc", c, acc, w), ("acc", i, kb - 1)) for c in C for w in W8]
-                m.mma(reads, [(("acc", c, acc, w), ("acc", i, kb)) for c in C for w in W8])
+                    reads += [(("acc", c, acc, w), ("acc", i, kb - 1)) for c in C for w in W]
+                m.mma(reads, [(("acc", c, acc, w), ("acc", i, kb)) for c in C for w in W])
                 m.commit(*[empty[c][s] for c in C])
                 n += 1
                 s += 1
@@ -425,7 +427,7 @@ def run_gemm(k_blocks, stages, seed, ctas=1, slabs=2, in_flight=0):
                     tmem_full[c][acc].arrive()
 
     def epilogue(c, w):
-        me = (c, w)
+        me, n = (c, w), 0
         for i, kb_n in enumerate(k_blocks):
             acc, acc_ph = i & 1, (i >> 1) & 1
             yield ("wait", tmem_full[c][acc], acc_ph)
@@ -435,12 +437,13 @@ def run_gemm(k_blocks, stages, seed, ctas=1, slabs=2, in_flight=0):
                 if sl == slabs - 1:
                     tmem_empty[acc].arrive()
                 yield m.stores_read(me, in_flight)
-                m.write(("stage out", me), ("out", i, sl))
+                m.write(("stage out", me, n % buffers), ("out", i, sl))
                 yield None
-                m.store(me, ("stage out", me), ("out", i, sl))
+                m.store(me, ("stage out", me, n % buffers), ("out", i, sl))
+                n += 1
         yield m.stores_read(me, 0)
 
-    m.run([producer(c) for c in C] + [issuer()] + [epilogue(c, w) for c in C for w in W8])
+    m.run([producer(c) for c in C] + [issuer()] + [epilogue(c, w) for c in C for w in W])
 
 
 @pytest.mark.parametrize("nblk", list(range(1, 10)) + [16])
@@ -499,8 +502,9 @@ def test_the_model_notices_a_missing_stage():
             run_dkv2(6, seed, q_stages=1)
 
 
-def test_the_model_notices_a_reused_staging_buffer():
-    """With a store still in flight it would be reading what the next slab overwrites."""
+@pytest.mark.parametrize("ctas", [1, 2])
+def test_the_model_notices_a_reused_staging_buffer(ctas):
+    """With one more store in flight it would be reading what the next slab overwrites."""
     with pytest.raises(AssertionError):
         for seed in range(50):
-            run_gemm([2, 2, 2], 4, seed, in_flight=1)
+            run_gemm([2, 2, 2], 4, seed, ctas=ctas, in_flight=3 - ctas)
