@@ -35,8 +35,11 @@ constexpr int A_STAGE_BYTES = BM * BK * 2;
 // tile after another on a mostly idle chip, which a second epilogue warp per scheduler does not shorten: in the
 // pair kernel's form it took 6.3 us for 8 x 512 x 512 (with four warps 5.7), 10.4 for 96 x 1536 x 1536 (9.7).
 constexpr int CTA_THREADS = 192, CTA_EPI_WARPS = 4;
-// CTA-pair kernel: three warpgroups, producer and issuer (and two idle warps), two of epilogue.  The register file is split
-// unevenly, 384 x 168 at launch; all take that again before the common end of the kernel.
+// CTA-pair kernel: three warpgroups, producer and issuer (and two idle warps), two of epilogue.  The registers, 384 x 168 at
+// launch, are split unevenly, once: an increase waits without a limit for what others give up.  Handed back at the end,
+// they could go round in a pair without a tile: its load and MMA warps took back what the epilogue warps were still
+// waiting for.  (An order between the two by one more barrier would do as well: 0.1 us more for every product of a few
+// tiles, 0.1 to 0.4 us less for B read MN-major at 2048 x 2048 and above.)
 constexpr int PAIR_THREADS = 384, PAIR_EPI_WARPS = 8;
 constexpr int LAUNCH_REGS = 168, EPI_REGS = 216, ROLE_REGS = 72;
 static_assert(256 * EPI_REGS + 128 * ROLE_REGS == PAIR_THREADS * LAUNCH_REGS, "register split");
@@ -44,11 +47,6 @@ template <int N>
 __device__ __forceinline__ void set_regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
 __device__ __forceinline__ void set_regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-// a warpgroup's warps meet between two changes of their registers (every wait before this is bounded, so all arrive)
-__device__ __forceinline__ void warpgroup_sync() {
-  __syncwarp();
-  asm volatile("bar.sync %0, 128;" ::"r"(1 + (threadIdx.x >> 7)) : "memory");
-}
 
 struct GemmArgs {
   void* C;
@@ -826,6 +824,12 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const int num_m = args.mode == KMOE_GEMM_GROUPED_M ? pair_list_len : ceil_div(args.M, PAIR_TM);
   const int num_n = ceil_div(args.N, n_per_tile);
 
+  auto leave = [&]() {                // every wait before it is bounded, so all warps come
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();               // nothing of the peer may still point at this CTA's memory
+  };
+
   if (warp < 4) {
     set_regs_down<ROLE_REGS>();
     {
@@ -912,8 +916,12 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   }
     }
   role_done:
-    warpgroup_sync();
-    set_regs_up<LAUNCH_REGS>();
+    __syncwarp();
+    leave();
+    if (warp == 1) {
+      tc_fence_after();
+      tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    }
   } else {
     set_regs_up<EPI_REGS>();
     {
@@ -988,16 +996,8 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
   epi_done:
     if (lane == 0) tma_store_wait_all();
-    warpgroup_sync();
-    set_regs_down<LAUNCH_REGS>();
-  }
-
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();                 // nothing of the peer may still point at this CTA's memory
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    __syncwarp();
+    leave();
   }
 }
 

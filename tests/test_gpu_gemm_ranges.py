@@ -1,4 +1,5 @@
-"""Batched products over many reduction ranges: more groups than the table in shared memory holds, empty ones among them."""
+"""Schedules read from the device: batched products over many reduction ranges (more groups than the table in shared memory
+holds, empty ones among them), row blocks of groups of which few or none are live."""
 import pytest
 import torch
 
@@ -28,3 +29,26 @@ def test_many_ranges(groups, m, n, dtype):
         # products of bf16 are exact in 32 bits; a sum of l of them is off by at most l * 2^-23 of the sum of their sizes
         bound = eps * (x.t() @ y).abs() + (1 + eps) * l * 2.0 ** -23 * (x.abs().t() @ y.abs())
         assert ((out[g].double() - x.t() @ y).abs() <= bound).all(), (g, l)
+
+
+@pytest.mark.parametrize("groups", [2, 16])                   # on CTA pairs, on single CTAs
+@pytest.mark.parametrize("live", [0, 1, 3])
+def test_most_ctas_have_no_tile(groups, live):
+    """The grid follows from the padded row count, the tiles from the live one.  Many launches: a CTA without a tile ends
+    while its neighbours still work."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(live)
+    M, N, K = 2048, 1024, 128
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(groups, N, K, device="cuda").bfloat16()
+    owner = (torch.arange(M // 128, device="cuda") * groups // (M // 128)).int()
+    n = torch.tensor([live], dtype=torch.int32, device="cuda")
+    out = torch.full((M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    for _ in range(200):
+        c.gemm(a, b, out, mode=c.GROUPED_M, groups=groups, M=M, N=N, Kd=K, lda=K, ldb=K, ldc=N, b_gs=N * K, tile_group=owner,
+               num_m_tiles=n)
+    c.check_status()
+    for t in range(live):
+        x, y = a[t * 128:(t + 1) * 128].double(), b[int(owner[t])].double()
+        bound = 2.0 ** -8 * (x @ y.t()).abs() + 1.01 * K * 2.0 ** -23 * (x.abs() @ y.abs().t())    # exact products, one rounding
+        assert ((out[t * 128:(t + 1) * 128].double() - x @ y.t()).abs() <= bound).all()
+    assert (out[live * 128:] == 7.0).all()

@@ -446,6 +446,54 @@ def run_gemm(k_blocks, stages, seed, ctas=1, slabs=None, in_flight=None):
     m.run([producer(c) for c in C] + [issuer()] + [epilogue(c, w) for c in C for w in W])
 
 
+def run_register_split(tiles, seed, hand_back=False):
+    """``umma_gemm_pair_kernel``: registers per thread move between the warps of a CTA through a pool (setmaxnreg), from 168 for
+    all to 72 for the four load and MMA warps and 216 for the eight epilogue warps.  ``inc`` waits, without a limit, until
+    the pool holds what it takes.  ``hand_back``: everybody takes 168 again at the end, which the kernel must not do."""
+    m = Machine(seed)
+    pool, done = [0], Bar(12)
+    dec = lambda n: pool.__setitem__(0, pool[0] + n)
+
+    def inc(n):
+        yield ("until", lambda: pool[0] >= n, "registers")
+        pool[0] -= n
+
+    def role():
+        dec(168 - 72)
+        for _ in range(tiles):
+            yield None
+        if hand_back:
+            yield from inc(168 - 72)
+        done.arrive()
+        yield ("wait", done, 0)
+
+    def epilogue():
+        yield None
+        yield from inc(216 - 168)
+        for _ in range(tiles):
+            yield None
+        if hand_back:
+            dec(216 - 168)
+        done.arrive()
+        yield ("wait", done, 0)
+
+    m.run([role() for _ in range(4)] + [epilogue() for _ in range(8)])
+
+
+@pytest.mark.parametrize("tiles", [0, 1, 5])
+def test_registers_reach_the_epilogue(tiles):
+    for seed in range(100):
+        run_register_split(tiles, seed)
+
+
+@pytest.mark.parametrize("tiles", [0, 1])
+def test_registers_handed_back_without_order_can_block(tiles):
+    """A CTA with little to do: the load and MMA warps take back what the epilogue warps have not got yet."""
+    with pytest.raises(AssertionError, match="deadlock"):
+        for seed in range(200):
+            run_register_split(tiles, seed, hand_back=True)
+
+
 @pytest.mark.parametrize("nblk", list(range(1, 10)) + [16])
 def test_dq_kernel_protocol_has_no_deadlock_and_no_stale_read(nblk):
     for seed in range(40):
