@@ -28,7 +28,8 @@ def _ref(u, dt, A, Bm, Cm, D, z, bias, softplus):
 
 @pytest.mark.parametrize("B,S,C,form,gate", [
     (1, 1, 8, "slice", True), (2, 7, 72, "float", True), (1, 8, 64, "slice", False), (3, 9, 136, "slice", True),
-    (1, 65, 200, "slice", True), (1, 333, 1536, "slice", True), (2, 517, 64, "float", False), (4, 130, 4096, "slice", True)])
+    (1, 65, 200, "slice", True), (1, 333, 1536, "slice", True), (2, 517, 64, "float", False), (4, 130, 4096, "slice", True),
+    (1, 333, 72, "slice", True), (2, 517, 200, "float", False), (1, 130, 8, "slice", True)])
 def test_segments_chunks_layouts(B, S, C, form, gate):
     from kolmogorov_moe_architecture_b200 import ops
     torch.manual_seed(S + C)
@@ -57,6 +58,15 @@ def test_segments_chunks_layouts(B, S, C, form, gate):
     want = (yr, *torch.autograd.grad(yr, [t for t in ref_args if t is not None], go.double()))
     for g, w in zip(got, want):
         assert _rel(g, w) < TOL
+
+
+@pytest.mark.parametrize("B,S,C", [(1, 333, 72), (2, 517, 200), (1, 130, 8)])
+def test_half_filled_channel_blocks_in_segments(B, S, C):
+    """What the sizes above with C % 16 == 8 are for: their last channel block is half empty and there are several segments."""
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    u, bc = torch.ones(B, S, C, dtype=torch.bfloat16, device="cuda"), torch.ones(B, S, 16, dtype=torch.bfloat16, device="cuda")
+    seg = c.K.scan_fwd(u, u, None, -torch.ones(C, 16, device="cuda"), bc, bc, None, None, True, False)[2]
+    assert C % 16 == 8 and seg.numel() >= 2 * B * 17 * C
 
 
 @pytest.mark.parametrize("B,S,C", [(1, 0, 64), (1, 0, 8), (0, 5, 64)])

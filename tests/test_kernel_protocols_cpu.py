@@ -4,7 +4,9 @@ The attention kernels (csrc/attention.cu: ``attn_fwd2_kernel``, ``attn_bwd_dq2_k
 same for both head widths) and the persistent GEMMs (csrc/gemm_umma.cu: ``umma_gemm_kernel``, ``umma_gemm_pair_kernel``)
 are warp-specialised: a TMA producer, a single-thread MMA issuer and softmax / epilogue warps hand shared-memory stages
 and tensor-memory regions to one another through mbarriers that are waited on by phase parity; the GEMM's epilogue hands
-staging buffers to TMA stores through bulk groups, and the dK/dV kernel's clusters meet at cluster barriers.  This file
+staging buffers to TMA stores through bulk groups, and the dK/dV kernel's clusters meet at cluster barriers.  The selective
+scan's kernels (csrc/scan.cu) are pairs of warps, one that prepares and finishes chunks and one that carries the
+recurrence, which meet at named barriers without a time limit.  This file
 restates each role's sequence of waits, arrivals, loads, MMAs and stores, runs the roles under randomly chosen
 interleavings (loads, MMAs and stores complete asynchronously, MMAs of a CTA in issue order) and checks for every step
 count that
@@ -492,6 +494,200 @@ def test_registers_handed_back_without_order_can_block(tiles):
     with pytest.raises(AssertionError, match="deadlock"):
         for seed in range(200):
             run_register_split(tiles, seed, hand_back=True)
+
+
+# ---------------------------------------------------------------- selective scan (csrc/scan.cu)
+class NamedBar:
+    """bar.sync / bar.arrive of two warps: a phase ends when both have come."""
+
+    def __init__(self):
+        self.here, self.phase = set(), 0
+
+    def arrive(self, warp):
+        assert warp not in self.here, "a warp arrives twice in one phase"
+        self.here.add(warp)
+        if len(self.here) == 2:
+            self.here, self.phase = set(), self.phase + 1
+
+    def sync(self, warp):
+        p = self.phase
+        self.arrive(warp)
+        return ("until", lambda: self.phase > p, "named barrier")
+
+
+class Copies:
+    """cp.async groups of the helper warp: stage(j) brings chunk j and, in the backward pass, its checkpoint."""
+
+    def __init__(self, m, ntiles, ck_buffers=0):
+        self.m, self.ntiles, self.ck_buffers, self.groups = m, ntiles, ck_buffers, []
+
+    def stage(self, j):
+        done = Bar(2 if self.ck_buffers else 1)
+        if j < self.ntiles:
+            self.m.load(("raw", j & 1), ("raw", j), done)
+            if self.ck_buffers:
+                self.m.load(("ck", j % self.ck_buffers), ("ck", j), done)
+        else:
+            done.phase = 1                       # an empty group
+        self.groups.append(done)
+
+    def wait_but_one(self):
+        older = self.groups[:-1]
+        return ("until", lambda: all(g.phase >= 1 for g in older), "copies")
+
+
+def run_scan_fwd(ntiles, seed):
+    """``scan_fwd_kernel``, pass with outputs: both warps meet after every chunk."""
+    m = Machine(seed)
+    step, copies = NamedBar(), Copies(m, ntiles)
+
+    def prepare(j):
+        m.read(("raw", j & 1), ("raw", j))
+        m.write(("prep", j & 1), ("prep", j))
+
+    def helper():
+        copies.stage(0)
+        copies.stage(1)
+        yield copies.wait_but_one()
+        if ntiles > 0:
+            prepare(0)
+        yield step.sync("helper")
+        for j in range(ntiles):
+            if j > 0:
+                m.read(("part", (j - 1) & 1), ("part", j - 1))
+            yield None
+            copies.stage(j + 2)
+            yield copies.wait_but_one()
+            if j + 1 < ntiles:
+                prepare(j + 1)
+            yield step.sync("helper")
+        m.read(("part", (ntiles - 1) & 1), ("part", ntiles - 1))
+
+    def recurrence():
+        yield step.sync("recurrence")
+        for j in range(ntiles):
+            m.read(("prep", j & 1), ("prep", j))
+            yield None
+            m.read(("prep", j & 1), ("prep", j))
+            m.write(("part", j & 1), ("part", j))
+            yield step.sync("recurrence")
+
+    m.run([helper(), recurrence()])
+
+
+def run_scan_carry(ntiles, seed, empty=True):
+    """``scan_bwd_carry_kernel``: the helper is up to two chunks ahead.  ``empty=False`` leaves its wait for a free buffer out."""
+    m = Machine(seed)
+    ready, free, copies = [NamedBar(), NamedBar()], [NamedBar(), NamedBar()], Copies(m, ntiles)
+
+    def prepare(j):
+        m.read(("raw", j & 1), ("raw", j))
+        m.write(("prep", j & 1), ("prep", j))
+
+    def helper():
+        copies.stage(0)
+        copies.stage(1)
+        yield copies.wait_but_one()
+        prepare(0)
+        ready[0].arrive("helper")
+        for j in range(ntiles - 1):
+            copies.stage(j + 2)
+            yield copies.wait_but_one()
+            if j > 0 and empty:
+                yield free[(j + 1) & 1].sync("helper")
+            prepare(j + 1)
+            ready[(j + 1) & 1].arrive("helper")
+
+    def recurrence():
+        for j in range(ntiles):
+            yield ready[j & 1].sync("recurrence")
+            m.read(("prep", j & 1), ("prep", j))
+            yield None
+            m.read(("prep", j & 1), ("prep", j))
+            if j + 2 < ntiles and empty:
+                free[j & 1].arrive("recurrence")
+
+    m.run([helper(), recurrence()])
+
+
+def run_scan_bwd(ntiles, seed, ck_buffers=3, empty=True):
+    """``scan_bwd_kernel``: chunks in halves, the later one first; results of half h lie in buffer h."""
+    m = Machine(seed)
+    ready, full, free = ([NamedBar(), NamedBar()] for _ in range(3))
+    copies = Copies(m, ntiles, ck_buffers)
+
+    def prepare(j):
+        m.read(("raw", j & 1), ("raw", j))
+        m.write(("prep", j & 1), ("prep", j))
+
+    def finish(j, half):
+        m.read(("sums", half), ("sums", j))
+
+    def helper():
+        copies.stage(0)
+        copies.stage(1)
+        yield copies.wait_but_one()
+        if ntiles > 0:
+            prepare(0)
+        ready[0].arrive("helper")
+        for j in range(ntiles):
+            if j > 0:
+                yield full[0].sync("helper")
+                finish(j - 1, 0)
+                yield None
+                finish(j - 1, 0)
+                if empty:
+                    free[0].arrive("helper")
+            copies.stage(j + 2)
+            yield copies.wait_but_one()
+            if j + 1 < ntiles:
+                prepare(j + 1)
+                ready[(j + 1) & 1].arrive("helper")
+            yield full[1].sync("helper")
+            finish(j, 1)
+            yield None
+            finish(j, 1)
+            if j + 1 < ntiles and empty:
+                free[1].arrive("helper")
+        yield full[0].sync("helper")
+        finish(ntiles - 1, 0)
+
+    def recurrence():
+        for j in range(ntiles):
+            yield ready[j & 1].sync("recurrence")
+            for half in (1, 0):
+                m.read(("ck", j % ck_buffers), ("ck", j))
+                m.read(("prep", j & 1), ("prep", j))
+                yield None
+                if j > 0 and empty:
+                    yield free[half].sync("recurrence")
+                m.read(("prep", j & 1), ("prep", j))
+                m.write(("sums", half), ("sums", j))
+                full[half].arrive("recurrence")
+
+    m.run([helper(), recurrence()])
+
+
+@pytest.mark.parametrize("ntiles", list(range(1, 9)) + [33])
+@pytest.mark.parametrize("kernel", [run_scan_fwd, run_scan_carry, run_scan_bwd])
+def test_scan_warps_hand_chunks_over(kernel, ntiles):
+    for seed in range(30):
+        kernel(ntiles, seed)
+
+
+@pytest.mark.parametrize("kernel", [run_scan_fwd, run_scan_bwd])
+def test_the_scan_needs_a_chunk(kernel):
+    """Without one the helper finishes what was never begun (forward) or waits for it (backward): the host does not launch."""
+    with pytest.raises(AssertionError):
+        kernel(0, 0)
+
+
+@pytest.mark.parametrize("run", [lambda s: run_scan_bwd(5, s, ck_buffers=2), lambda s: run_scan_bwd(5, s, empty=False),
+                                 lambda s: run_scan_carry(5, s, empty=False)])
+def test_the_model_notices_a_missing_scan_buffer_or_wait(run):
+    with pytest.raises(AssertionError):
+        for seed in range(200):
+            run(seed)
 
 
 @pytest.mark.parametrize("nblk", list(range(1, 10)) + [16])
