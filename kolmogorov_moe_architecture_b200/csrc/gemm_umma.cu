@@ -2,7 +2,7 @@
 //
 //   warp 0      : TMA producer  (cp.async.bulk.tensor -> 128B-swizzled smem ring, mbarrier tx counts)
 //   warp 1      : MMA issuer    (tcgen05.mma 128 x BN x 16, accumulators in TMEM, double buffered)
-//   warps 2..5  : epilogue      (tcgen05.ld -> registers -> fused epilogue -> global); in the CTA-pair kernel 4..11
+//   warps 2..5  : epilogue      (tcgen05.ld -> registers -> fused epilogue -> global); with eight of them warps 4..11
 //
 // One CTA per SM walks a static tile list, so the epilogue of tile i overlaps the
 // main loop of tile i+1.  Operands may be K-major or MN-major (the MMA reads either
@@ -31,18 +31,15 @@ namespace kmoe {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int A_STAGE_BYTES = BM * BK * 2;
-// Single-CTA kernel: producer, issuer, four epilogue warps.  It has the small products, and their time is the launch and one
-// tile after another on a mostly idle chip, which a second epilogue warp per scheduler does not shorten: in the
-// pair kernel's form it took 6.3 us for 8 x 512 x 512 (with four warps 5.7), 10.4 for 96 x 1536 x 1536 (9.7).
-constexpr int CTA_THREADS = 192, CTA_EPI_WARPS = 4;
-// CTA-pair kernel: three warpgroups, producer and issuer (and two idle warps), two of epilogue.  The registers, 384 x 168 at
-// launch, are split unevenly, once: an increase waits without a limit for what others give up.  Handed back at the end,
-// they could go round in a pair without a tile: its load and MMA warps took back what the epilogue warps were still
-// waiting for.  (An order between the two by one more barrier would do as well: 0.1 us more for every product of a few
-// tiles, 0.1 to 0.4 us less for B read MN-major at 2048 x 2048 and above.)
-constexpr int PAIR_THREADS = 384, PAIR_EPI_WARPS = 8;
+// Four epilogue warps: 192 threads, and every thread has the registers it wants.
+// Eight (CTA pairs with short reductions, see WIDE_K_PLAIN): three warpgroups, producer and issuer (and two idle warps), two of
+// epilogue.  The registers, 384 x 168 at launch, are split unevenly, once: an increase waits without a limit for what
+// others give up.  Handed back at the end, they could go round in a pair without a tile: its load and MMA warps took back
+// what the epilogue warps were still waiting for.
+constexpr int threads_of(int epi_warps) { return epi_warps == 8 ? 384 : 192; }
+constexpr int CTA_EPI_WARPS = 4;
 constexpr int LAUNCH_REGS = 168, EPI_REGS = 216, ROLE_REGS = 72;
-static_assert(256 * EPI_REGS + 128 * ROLE_REGS == PAIR_THREADS * LAUNCH_REGS, "register split");
+static_assert(256 * EPI_REGS + 128 * ROLE_REGS == threads_of(8) * LAUNCH_REGS, "register split");
 template <int N>
 __device__ __forceinline__ void set_regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
@@ -267,11 +264,8 @@ __device__ __forceinline__ void epilogue_store_chunk_f32(const GemmArgs& a, cons
 // a TMA store, which also clips at M and N.  One of four warps has two buffers, one of eight has one; it waits for a store
 // to have read its buffer only when it has the values that go there next, and the accumulator goes back to the MMA warp
 // as soon as the last slab is in registers.
-// A tile whose reduction is shorter than its epilogue is bound by this code (weight gradients of experts with few
-// tokens, orthogonalisation): a slab is a chain of latencies, 925 clocks, so with one warp per scheduler (four in all, two
-// buffers each) a 256 x 256 tile took 5000 clocks - ten reduction blocks' worth - and takes 3400 to 4000 with two warps per
-// scheduler (weight gradients of the 3B preset's 64 experts: 681 us, 634 with eight warps, 552 with the relaxed arrival at
-// the pair's leader, 514 with `list_div`).
+// A tile whose reduction is shorter than its epilogue is bound by this code (weight gradients of experts with few tokens): a
+// slab is a chain of latencies, so two warps per scheduler finish a tile sooner than one (see WIDE_K_PLAIN).
 constexpr int OUT_BUF_BYTES = 32 * 128;
 constexpr int OUT_STAGE_BYTES = 8 * OUT_BUF_BYTES;
 
@@ -487,7 +481,7 @@ __device__ __forceinline__ void load_mn_tile_pair(uint8_t* dst, const CUtensorMa
 }
 
 template <int BN, int A_MAJOR, int B_MAJOR>
-__global__ void __launch_bounds__(CTA_THREADS, 1)
+__global__ void __launch_bounds__(threads_of(CTA_EPI_WARPS), 1)
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
                  const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY, const GemmArgs args,
@@ -755,12 +749,23 @@ constexpr int PAIR_TM = 2 * BM;
 // Expert-padded schedule: blocks per expert (counting the padding) from which pairs are taken.  Up / down / dH products
 // in µs, pairs against single CTAs, at d = 2048, f = 2816: 2.6 live blocks per expert 459/234/235 against 434/219/226,
 // 4.6 blocks 351/180/178 against 343/175/185, 6.4 blocks 309/157/156 against 310/165/167, 12.4 blocks 268/132/135 against
-// 272/141/149.  With eight epilogue warps the sums of the three are within 5 % of each other, either way, from 1.4 to 6.5
-// live blocks per expert (64 experts 633 to 667 against 635 to 643, 32 experts 679 to 703 against 684 to 690).
+// 272/141/149.
 constexpr int GROUPED_PAIR_MIN = 7;
 
-template <int BN, int A_MAJOR, int B_MAJOR>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+// Eight epilogue warps instead of four, by the reduction of a tile (the mean one of ragged products).  They finish a tile
+// sooner, which counts while the epilogue is longer than the reduction it runs beside; where it is not, twice as many
+// warps only take shared memory and issue slots from the products.  The more an epilogue does per tile, the longer the
+// reduction up to which it counts.  In us, eight against four:
+//   plain bf16, more tiles than pairs: 16 products of 2048 x 2816 over K = 128 52 / 60, 256 57 / 64, 384 69 / 72, 448 76 / 75,
+//     768 115 / 111, 1536 200 / 197; 64 of 1792 x 2464 over 128 143 / 172, 384 218 / 220, 448 248 / 231;
+//     8192 x 4096 over 128 22.7 / 24.8, 384 28.3 / 29.0, 640 36.0 / 34.7.  One round of tiles: 0.2 to 0.6 us more.
+//   SwiGLU with both pre-activations: 4096 x 2048 over 512 27.1 / 30.9, 4096 x 4096 over 1536 76.9 / 74.8.
+//   an addend: 8192 x 4096 over 512 57 / 79, 1024 60 / 80, 1536 77 / 82, 2048 97 / 98, 4096 185 / 183, 8192 380 / 366.
+//   fp32 results: never, 2048 x 2048 over 256 15.5 / 12.4, 8192 x 4096 over 1024 80 / 76.
+constexpr int WIDE_K_PLAIN = 384, WIDE_K_SWIGLU = 512, WIDE_K_ADDEND = 2048;
+
+template <int BN, int A_MAJOR, int B_MAJOR, int EPI_WARPS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads_of(EPI_WARPS), 1)
 umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
                  const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmY, const GemmArgs args,
@@ -798,7 +803,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 2 * PAIR_EPI_WARPS);   // the epilogue warps of both CTAs
+      mbar_init(&tmem_empty[i], 2 * EPI_WARPS);   // the epilogue warps of both CTAs
     }
     mbar_fence_init();
     prefetch_tmap(&tmA);
@@ -830,8 +835,10 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     cluster_sync_all();               // nothing of the peer may still point at this CTA's memory
   };
 
-  if (warp < 4) {
-    set_regs_down<ROLE_REGS>();
+  constexpr bool wide = EPI_WARPS == 8;
+  constexpr int FIRST_EPI = wide ? 4 : 2;
+  if (warp < FIRST_EPI) {
+    if (wide) set_regs_down<ROLE_REGS>();
     {
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
@@ -923,13 +930,13 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       tmem_dealloc_pair(tmem_base, TMEM_COLS);
     }
   } else {
-    set_regs_up<EPI_REGS>();
+    if (wide) set_regs_up<EPI_REGS>();
     {
     // ------------------------------------------------------------ epilogue (both CTAs)
     const int q = warp & 3;
     int it = 0;
     Tile t;
-    OutStage<PAIR_EPI_WARPS> out(smem + stages * STAGE_BYTES, warp - 4);
+    OutStage<EPI_WARPS> out(smem + stages * STAGE_BYTES, warp - FIRST_EPI);
     for (int idx = pair; get_tile<BN, PAIR_TM>(args, idx, num_m, num_n, t, ranges, pair_list); idx += num_pairs) {
       const int acc = it & 1;
       const uint32_t acc_ph = (it >> 1) & 1;
@@ -982,7 +989,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       const long long coff = goff + (long long)row * args.ldc;
       const long long doff = goff + (long long)row * args.ldd;
 #pragma unroll 1
-      for (int c = out.half * (BN / 2); c < (out.half + 1) * (BN / 2); c += 32) {
+      for (int c = wide ? out.half * (BN / 2) : 0; c < (wide ? (out.half + 1) * (BN / 2) : BN); c += 32) {
         uint32_t r[32];
         if (have_acc) {
           tmem_ld_32x32(t_row + c, r);
@@ -1106,11 +1113,11 @@ static int launch_variant(const CUtensorMap& tA, const CUtensorMap& tB, const CU
   auto kern = umma_gemm_kernel<BN, AM, BMj>;
   static SmemLimit limit;
   if (!limit.raise(kern, smem)) return -20;
-  kern<<<grid, CTA_THREADS, smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
+  kern<<<grid, threads_of(CTA_EPI_WARPS), smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
-template <int BN, int AM, int BMj>
+template <int BN, int AM, int BMj, int EPI_WARPS>
 static int launch_pair_variant(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2,
                                const CUtensorMap& tC, const CUtensorMap& tX, const CUtensorMap& tY,
                                const GemmArgs& args, long long pair_tiles, int sms, cudaStream_t stream) {
@@ -1118,14 +1125,14 @@ static int launch_pair_variant(const CUtensorMap& tA, const CUtensorMap& tB, con
   int stages = (192 * 1024) / stage_bytes;
   if (stages > 8) stages = 8;
   const int smem = stages * stage_bytes + OUT_STAGE_BYTES + 1024;
-  auto kern = umma_gemm_pair_kernel<BN, AM, BMj>;
+  auto kern = umma_gemm_pair_kernel<BN, AM, BMj, EPI_WARPS>;
   static SmemLimit limit;
   if (!limit.raise(kern, smem)) return -20;
   static int max_clusters = 0;
   if (max_clusters == 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * (sms / 2)));
-    cfg.blockDim = dim3(PAIR_THREADS);
+    cfg.blockDim = dim3(threads_of(EPI_WARPS));
     cfg.dynamicSmemBytes = (size_t)smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1137,7 +1144,7 @@ static int launch_pair_variant(const CUtensorMap& tA, const CUtensorMap& tB, con
   }
   long long pairs = pair_tiles < max_clusters ? pair_tiles : max_clusters;
   if (pairs < 1) pairs = 1;
-  kern<<<(unsigned)(2 * pairs), PAIR_THREADS, smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
+  kern<<<(unsigned)(2 * pairs), threads_of(EPI_WARPS), smem, stream>>>(tA, tB, tB2, tC, tX, tY, args, stages);
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
@@ -1267,8 +1274,14 @@ extern "C" int kmoe_gemm(const KmoeGemmDesc* d, cudaStream_t stream) {
   int grid = (int)(total < sms ? total : sms);
   if (grid < 1) grid = 1;
 
+  const long long mean_k = (long long)d->K / (d->k_begin != nullptr && d->groups > 1 ? d->groups : 1);
+  const bool wide = !d->out_f32 && (d->D != nullptr ? mean_k <= WIDE_K_ADDEND
+                                    : swiglu        ? mean_k <= WIDE_K_SWIGLU
+                                                    : mean_k <= WIDE_K_PLAIN && total > units);
   int lrc = 0;
-#define KMOE_LAUNCH_PAIR(BN_, AM_, BM_) lrc = launch_pair_variant<BN_, AM_, BM_>(tA, tB, tB2, tC, tX, tY, a, total, sms, stream)
+#define KMOE_LAUNCH_PAIR(BN_, AM_, BM_)                                                                        \
+  lrc = wide ? launch_pair_variant<BN_, AM_, BM_, 8>(tA, tB, tB2, tC, tX, tY, a, total, sms, stream)           \
+             : launch_pair_variant<BN_, AM_, BM_, 4>(tA, tB, tB2, tC, tX, tY, a, total, sms, stream)
 #define KMOE_LAUNCH(BN_, AM_, BM_) lrc = launch_variant<BN_, AM_, BM_>(tA, tB, tB2, tC, tX, tY, a, grid, stream)
   if (pair && BN == 256) {
     if (d->a_major == 0 && d->b_major == 0) KMOE_LAUNCH_PAIR(256, 0, 0);

@@ -1,5 +1,6 @@
 """Schedules read from the device: batched products over many reduction ranges (more groups than the table in shared memory
-holds, empty ones among them), row blocks of groups of which few or none are live."""
+holds, empty ones among them), row blocks of groups of which few or none are live; reductions on either side of the lengths
+where the epilogue changes its number of warps."""
 import pytest
 import torch
 
@@ -52,3 +53,31 @@ def test_most_ctas_have_no_tile(groups, live):
         bound = 2.0 ** -8 * (x @ y.t()).abs() + 1.01 * K * 2.0 ** -23 * (x.abs() @ y.abs().t())    # exact products, one rounding
         assert ((out[t * 128:(t + 1) * 128].double() - x @ y.t()).abs() <= bound).all()
     assert (out[live * 128:] == 7.0).all()
+
+
+@pytest.mark.parametrize("form,K", [("plain", 8), ("plain", 384), ("plain", 392), ("addend", 2048), ("addend", 2056),
+                                    ("fp32", 128), ("swiglu", 512), ("swiglu", 520)])
+@pytest.mark.parametrize("M,N", [(2600, 2072), (300, 136)])   # more tiles than pairs, one round
+def test_epilogue_warps(form, K, M, N):
+    from kolmogorov_moe_architecture_b200.ops import cuda_ops as c
+    torch.manual_seed(K)
+    a, b, b2 = (torch.randn(r, K, device="cuda").bfloat16() for r in (M, N, N))
+    x, y = a.double(), b.double()
+    if form == "swiglu":
+        h, g, u = (torch.empty(M, N, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+        b, b2 = b / 8, b2 / 8
+        c.gemm(a, b, h, B2=b2, G=g, U=u, epi=c.EPI_SWIGLU, M=M, N=N, Kd=K, lda=K, ldb=K, ldc=N)
+        c.check_status()
+        gate, up = x @ b.double().t(), x @ b2.double().t()
+        for got, want in ((g, gate), (u, up), (h, torch.nn.functional.silu(gate) * up)):
+            assert (got.double() - want).norm() <= 2.0 ** -8 * want.norm()      # one rounding to 8 bits
+        return
+    d = torch.randn(M, N, device="cuda").bfloat16() if form == "addend" else None
+    out = c.mm_nt(a, b, out_dtype=torch.float32 if form == "fp32" else None, D=d, beta=0.5)
+    c.check_status()
+    more = 0.0 if d is None else 0.5 * d.double()
+    want = x @ y.t() + more
+    # exact products, sums of K + 1 values in 32 bits, one rounding of bf16 results
+    bound = 1.01 * (K + 1) * 2.0 ** -23 * (x.abs() @ y.abs().t() + (more if d is None else more.abs()))
+    bound += 0.0 if form == "fp32" else 2.0 ** -8 * want.abs()
+    assert ((out.double() - want).abs() <= bound).all()

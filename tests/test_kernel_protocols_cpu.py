@@ -373,20 +373,20 @@ def run_fwd2(nb, seed):
 
 
 # ---------------------------------------------------------------- persistent GEMMs (csrc/gemm_umma.cu)
-def run_gemm(k_blocks, stages, seed, ctas=1, slabs=None, in_flight=None):
+def run_gemm(k_blocks, stages, seed, ctas=1, warps=4, slabs=None, in_flight=None):
     """``umma_gemm_kernel`` (ctas=1) and ``umma_gemm_pair_kernel`` (ctas=2) for the tiles one CTA (pair) works
     through: ``k_blocks[i]`` reduction blocks for tile i (0 = a group without rows in a batched product: the
     epilogue writes zeros / the addend and the issuer arrives by itself).  Ring of ``stages`` shared-memory
-    stages, two accumulators.  A CTA of the pair has eight epilogue warps, two per 32 rows, each with every other column
-    slab and one staging buffer; the single CTA has four with all slabs and two buffers in turn.  A warp takes its share
-    of the accumulator in ``slabs`` column slabs, hands it back with the last one in registers, and sends each slab from
-    a staging buffer by a TMA store that it does not wait for: before it writes the next slab, all but ``in_flight`` (one
-    less than its buffers) of its stores have been read.  In the pair the ``full`` and ``tmem_empty`` barriers live in
-    the leader, ``empty`` and ``tmem_full`` exist in both CTAs and get the leader's commits."""
+    stages, two accumulators.  Of eight epilogue ``warps`` of a CTA (pairs only) two share 32 rows, each with every other
+    column slab and one staging buffer; one of four has all slabs of its rows and two buffers in turn.  A warp takes its
+    share of the accumulator in ``slabs`` column slabs, hands it back with the last one in registers, and sends each slab
+    from a staging buffer by a TMA store that it does not wait for: before it writes the next slab, all but ``in_flight``
+    (one less than its buffers) of its stores have been read.  In the pair the ``full`` and ``tmem_empty`` barriers live
+    in the leader, ``empty`` and ``tmem_full`` exist in both CTAs and get the leader's commits."""
     m = Machine(seed)
     C = range(ctas)
-    W, buffers = (range(4), 2) if ctas == 1 else (range(8), 1)
-    slabs = 8 // len(W) * 2 if slabs is None else slabs
+    W, buffers = range(warps), 8 // warps
+    slabs = 16 // warps if slabs is None else slabs
     in_flight = buffers - 1 if in_flight is None else in_flight
     full = [Bar(1 + ctas) for _ in range(stages)]         # the leader's expect_tx + one load group per CTA
     empty = [[Bar(1) for _ in range(stages)] for _ in C]
@@ -449,8 +449,8 @@ def run_gemm(k_blocks, stages, seed, ctas=1, slabs=None, in_flight=None):
 
 
 def run_register_split(tiles, seed, hand_back=False):
-    """``umma_gemm_pair_kernel``: registers per thread move between the warps of a CTA through a pool (setmaxnreg), from 168 for
-    all to 72 for the four load and MMA warps and 216 for the eight epilogue warps.  ``inc`` waits, without a limit, until
+    """``umma_gemm_pair_kernel`` with eight epilogue warps: registers per thread move between the warps of a CTA through a pool
+    (setmaxnreg), from 168 for all to 72 for the four load and MMA warps and 216 for the eight epilogue warps.  ``inc`` waits, without a limit, until
     the pool holds what it takes.  ``hand_back``: everybody takes 168 again at the end, which the kernel must not do."""
     m = Machine(seed)
     pool, done = [0], Bar(12)
@@ -718,15 +718,15 @@ def test_forward_kernel_protocol_has_no_deadlock_and_no_stale_read(nb1):
         run_fwd2((nb1, 0), seed)
 
 
-@pytest.mark.parametrize("ctas", [1, 2])
+@pytest.mark.parametrize("ctas,warps", [(1, 4), (2, 4), (2, 8)])
 @pytest.mark.parametrize("stages", [2, 4, 6])
-def test_gemm_ring_and_accumulator_hand_off(ctas, stages):
+def test_gemm_ring_and_accumulator_hand_off(ctas, warps, stages):
     rng = random.Random(stages * 10 + ctas)
     shapes = [[1], [3], [1, 1, 1, 1, 1], [2, 0, 5, 0, 0, 1], [0], [0, 0, 0], [32, 2, 32], [7] * 9]
     shapes += [[rng.choice([0, 1, 2, 3, 9]) for _ in range(rng.randint(1, 8))] for _ in range(6)]
     for kbs in shapes:
         for seed in range(12):
-            run_gemm(kbs, stages, seed, ctas=ctas)
+            run_gemm(kbs, stages, seed, ctas=ctas, warps=warps)
 
 
 def test_one_ds_barrier_for_two_dp_buffers_would_mix_phases():
@@ -746,9 +746,9 @@ def test_the_model_notices_a_missing_stage():
             run_dkv2(6, seed, q_stages=1)
 
 
-@pytest.mark.parametrize("ctas", [1, 2])
-def test_the_model_notices_a_reused_staging_buffer(ctas):
+@pytest.mark.parametrize("ctas,warps", [(1, 4), (2, 4), (2, 8)])
+def test_the_model_notices_a_reused_staging_buffer(ctas, warps):
     """With one more store in flight it would be reading what the next slab overwrites."""
     with pytest.raises(AssertionError):
         for seed in range(50):
-            run_gemm([2, 2, 2], 4, seed, ctas=ctas, in_flight=3 - ctas)
+            run_gemm([2, 2, 2], 4, seed, ctas=ctas, warps=warps, in_flight=8 // warps)
