@@ -19,12 +19,12 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf
 // CONV_T steps, a CTA eight such stretches.  Both directions stream their operands once; what counts is to have enough
 // loads in flight, so the rows of a batch of steps are requested, unconditionally (rows past the end repeat the last
 // one), before the first of them is looked at.
-// 4 x 2048 x 4096: forward 37.7 -> 36.6 us (20.5 at the copy rate), backward 132.5 -> 88.8 us (30.8) against one
-// channel, 64 steps and one row at a time per thread.
-// Both are bound by issue slots (68 and 58 % busy) and latency, not by memory (DRAM at 29 and 27 %).  The backward kernel,
-// fourteen multiply-adds per element, takes 77.0 us on packed pairs for 88.0 on single floats (three CTAs per SM).  The
-// forward kernel, four per element, keeps single floats: 40.3 to 42.4 us on pairs (three to six CTAs) for 39.4 with each
-// batch's values widened first.  A batch loaded ahead costs the registers of a CTA: 43 and 81 us.
+// 4 x 2048 x 4096: forward 39.4 us (20.5 at the copy rate), backward 77.0 us (30.8).  What bounds both is the latency of a
+// batch of loads and the arithmetic on it, one after the other: neither the issue slots (68 and 58 % busy) nor memory (DRAM
+// at 29 and 27 %) is full.  The backward kernel, fourteen multiply-adds per element, took 88.0 us on single floats
+// instead of packed pairs (three CTAs per SM).  The forward kernel, four per element, keeps single floats: 40.3 to 42.4 us
+// on pairs (three to six CTAs).  A batch loaded ahead costs the registers of a CTA: 43 and 81 us.  Where all CTAs run at once
+// the longer latency of the pairs shows: 1 x 333 x 1536 backward 11.1 us for 10.7, with its two zero fills.
 constexpr int CONV_T = 32;      // time steps per thread
 constexpr int CONV_WARPS = 8;
 

@@ -221,9 +221,12 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
                : "memory");
   return v;
 }
-// Relaxed: says that tensor memory has been read (the reads have completed, tcgen05.wait::ld), no writes to memory go
-// with it.  With release semantics at cluster scope the arrival waited for the warp's outstanding stores, 1000 to 2000
-// clocks per tile.
+// Relaxed: says that tensor memory has been read, and no writes to memory go with it.  What is relied on: tcgen05.wait::ld
+// returns once the warp's reads have completed, i.e. their values are in registers, __syncwarp orders the lanes, and
+// the arrival comes after both in program order, so an MMA issued on the other side behind its wait cannot overtake a
+// read.  (tcgen05.fence::before_thread_sync, which the callers issue too, is defined against a synchronising operation; a
+// relaxed arrival formally is none.)  With release semantics at cluster scope the arrival waited for the warp's
+// outstanding stores, 1000 to 2000 clocks per tile.
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

@@ -15,15 +15,16 @@
 //             from the true state (a short serial combination of the earlier segments) and writes y plus a
 //             state checkpoint every 8 steps.
 //   backward: pass 1 runs dL/dh backwards through each segment from zero; pass 2 starts from the true incoming
-//             value, replays a chunk from its checkpoint - decays and states stay in registers - and walks it in reverse.
+//             value, replays a chunk from its checkpoint and walks it in reverse, in halves of four steps whose decays and
+//             states stay in registers; the later half comes first, so the earlier one is replayed twice.
 // dB and dC are sums over channels: a lane adds its two channels, the warp lays four steps of its lanes' values out in
 // shared memory and each lane of the other warp adds up eight 16-byte pieces and sends them off as one 16-byte global
 // reduction.
 //
-// Bounds: the latency of a step with 1.7 recurrences per scheduler, beside the shared-memory pipe (50 and 71 % busy,
-// forward and backward at 4 x 2048 x 4096) and the issue slots (55 and 50 %); the exponentials alone take 119 us a pass.
-// That size: forward 349 -> 275 us, backward 845 -> 688; 1 x 2048 x 4096 in segments 147 + 284 -> 124 + 247;
-// 1 x 333 x 1536 26 + 46 -> 22 + 44.  Against one channel per lane (the form before this) it is 0.65 of the instructions
+// Bounds: the latency of a step with 1.7 recurrences per scheduler, beside the shared-memory pipe (44 and 62 % busy,
+// forward and backward at 4 x 2048 x 4096) and the issue slots (54 and 50 %).  The exponentials alone take 119 us forward and
+// 178 us backward (twelve steps' worth for eight).  Kernel times there: forward 341 -> 267 us, backward 832 -> 678;
+// 1 x 2048 x 4096 in segments 137 + 270 -> 117 + 233; 1 x 333 x 1536 17 + 34 -> 15 + 30.  Against one channel per lane (the form before this) it is 0.65 of the instructions
 // and half of the shared-memory reads per state.  Also measured: one warp doing everything 437 + 748 (too few warps to
 // hide latency), eight recurrence warps of 200 registers beside eight of 56 in one CTA 970 backward (spills).
 #include <cuda_bf16.h>
