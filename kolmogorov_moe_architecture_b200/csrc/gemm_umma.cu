@@ -759,6 +759,7 @@ constexpr int GROUPED_PAIR_MIN = 7;
 //   plain bf16, more tiles than pairs: 16 products of 2048 x 2816 over K = 128 52 / 60, 256 57 / 64, 384 69 / 72, 448 76 / 75,
 //     768 115 / 111, 1536 200 / 197; 64 of 1792 x 2464 over 128 143 / 172, 384 218 / 220, 448 248 / 231;
 //     8192 x 4096 over 128 22.7 / 24.8, 384 28.3 / 29.0, 640 36.0 / 34.7.  One round of tiles: 0.2 to 0.6 us more.
+//     Uneven groups, whose short ones gain what the long ones lose: as 1 / rank over 16 groups, mean 768, 143 / 142; even 116 / 112.
 //   SwiGLU with both pre-activations: 4096 x 2048 over 512 27.1 / 30.9, 4096 x 4096 over 1536 76.9 / 74.8.
 //   an addend: 8192 x 4096 over 512 57 / 79, 1024 60 / 80, 1536 77 / 82, 2048 97 / 98, 4096 185 / 183, 8192 380 / 366.
 //   fp32 results: never, 2048 x 2048 over 256 15.5 / 12.4, 8192 x 4096 over 1024 80 / 76.
